@@ -1,20 +1,24 @@
-"""Build libbissd.so (the CUDA kernels + C ABI) in-tree with nvcc for sm_100a.
+"""Build libbissd.so (the CUDA kernels + C ABI) and _bissd_torch.so (the operator's native host path) in-tree.
 
     python bi-mamba2_b200/build.py [--force] [--verbose]
 
-The shared library lands in bi-mamba2_b200/ssd/_lib/libbissd.so, next to the Python package that loads it with
-ctypes.  nvcc cross-compiles without a GPU.
+Both land in bi-mamba2_b200/ssd/_lib/.  libbissd.so is compiled by nvcc for sm_100a and has no PyTorch in it (the
+package also loads it with ctypes); _bissd_torch.so is a Python extension compiled by g++ against the installed PyTorch
+and linked to libbissd.so.  Neither needs a GPU to build.
 """
 import argparse
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "ssd", "_lib")
 OUT = os.path.join(OUT_DIR, "libbissd.so")
 SOURCES = ["bissd_api.cu"]
+TORCH_SRC = os.path.join(CSRC, "torch_ops.cpp")
+TORCH_OUT = os.path.join(OUT_DIR, "_bissd_torch.so")
 
 
 def _newest_source_mtime():
@@ -26,8 +30,42 @@ def _newest_source_mtime():
     return newest
 
 
+def _run(cmd, verbose, what):
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+    if res.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed building {what}")
+
+
+def build_torch(force=False, verbose=False):
+    """The extension depends on its own source and the C header only: libbissd.so may be rebuilt beneath it."""
+    header = os.path.join(os.path.dirname(HERE), "include", "bissd.h")
+    newest = max(os.path.getmtime(TORCH_SRC), os.path.getmtime(header))
+    if not force and os.path.exists(TORCH_OUT) and os.path.getmtime(TORCH_OUT) >= newest:
+        return TORCH_OUT
+    import torch
+    from torch.utils import cpp_extension
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    cmd = [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_EXTENSION_NAME=_bissd_torch"]
+    for path in cpp_extension.include_paths() + [os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]:
+        cmd += ["-isystem", path]
+    cmd += [TORCH_SRC, "-o", TORCH_OUT, "-L" + OUT_DIR, "-l:libbissd.so", "-Wl,-rpath,$ORIGIN"]
+    cmd += ["-L" + os.path.join(os.path.dirname(torch.__file__), "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
+            "-ltorch_python"]
+    _run(cmd, verbose, os.path.basename(TORCH_OUT))
+    return TORCH_OUT
+
+
 def build(force=False, verbose=False):
     os.makedirs(OUT_DIR, exist_ok=True)
+    build_library(force, verbose)
+    build_torch(force, verbose)
+    return OUT
+
+
+def build_library(force=False, verbose=False):
     if not force and os.path.exists(OUT) and os.path.getmtime(OUT) >= _newest_source_mtime():
         return OUT
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
@@ -37,11 +75,7 @@ def build(force=False, verbose=False):
     if verbose:
         cmd.insert(1, "-Xptxas")
         cmd.insert(2, "-v")
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if verbose or res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed building libbissd.so")
+    _run(cmd, verbose, os.path.basename(OUT))
     return OUT
 
 

@@ -1,8 +1,10 @@
-"""ctypes binding of libbissd.so - the structs and prototypes of include/bissd.h, nothing else.
+"""ctypes binding of libbissd.so - the structs and prototypes of include/bissd.h - and the loader of the native host path.
 
 There is no fallback: if the shared library is missing or does not load, importing the operator raises.
 """
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 _LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_lib", "libbissd.so")
@@ -132,6 +134,24 @@ def load():
         raise ImportError(f"libbissd ABI {lib.bissd_abi_version()} != binding ABI {ABI_VERSION}; rebuild the library")
     _lib = lib
     return lib
+
+
+_torch_ops = None
+
+
+def torch_ops():
+    """The native host path (csrc/torch_ops.cpp), linked to libbissd.so; raises when it is missing or does not load."""
+    global _torch_ops
+    if _torch_ops is None:
+        load()
+        path = os.path.join(os.path.dirname(_LIB_PATH), "_bissd_torch.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} not found: build it with `python bi-mamba2_b200/build.py`")
+        loader = importlib.machinery.ExtensionFileLoader("_bissd_torch", path)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_bissd_torch", loader))
+        loader.exec_module(module)
+        _torch_ops = module
+    return _torch_ops
 
 
 def launch_count():

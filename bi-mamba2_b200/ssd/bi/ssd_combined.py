@@ -5,9 +5,9 @@ src/ssd/bi/ssd_combined.py): same public function `bimamba_chunk_scan_combined` 
 name `MambaChunkScanCombinedFn` (:555) and the two private entry points the reference's own tests and
 benchmarks call, `_mamba_chunk_scan_combined_fwd` (:297) and `_mamba_chunk_scan_combined_bwd` (:334).
 
-All arithmetic runs in libbissd.so (hand-written CUDA for sm_100a, C ABI in include/bissd.h) through two
-PyTorch custom ops, `bissd::scan_fwd` and `bissd::scan_bwd` (in eager mode their implementations are called
-directly, skipping the dispatcher).  There is no Triton and no CPU or eager fallback:
+All arithmetic runs in libbissd.so (hand-written CUDA for sm_100a, C ABI in include/bissd.h).  In eager mode the
+operator's checks, allocations, library calls and autograd node are native too (csrc/torch_ops.cpp); torch.compile sees
+two PyTorch custom ops, `bissd::scan_fwd` and `bissd::scan_bwd`.  There is no Triton and no CPU or eager fallback:
 without the library, or on CPU tensors, the operator raises.
 """
 import math
@@ -394,5 +394,11 @@ def bimamba_chunk_scan_combined(x, dt, A, B, C, chunk_size, D=None, z=None, dt_b
     Return:
         out: (batch, seqlen, nheads, headdim)
     """
+    if not torch.compiler.is_compiling():
+        res = _cabi.torch_ops().chunk_scan(x, dt, A, B, C, chunk_size, D, z, dt_bias, dt_softplus, dt_limit[0], dt_limit[1],
+                                           return_final_states, initial_states_f, initial_states_b, CHECK_STATUS)
+        if res is not None:
+            return res
+    # torch.compile, tensor subclasses, and arguments that do not check (this path raises the precise error)
     return MambaChunkScanCombinedFn.apply(x, dt, A, B, C, chunk_size, D, z, dt_bias, dt_softplus, dt_limit,
                                           return_final_states, initial_states_f, initial_states_b)
