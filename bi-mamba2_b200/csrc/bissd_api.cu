@@ -13,6 +13,7 @@
 #include "simt_kernels.cuh"
 #include "conv_kernels.cuh"
 #include "norm_kernels.cuh"
+#include "layer_kernels.cuh"
 #include "tc_intra.cuh"
 #include "tc_intra_sums.cuh"
 #include "tc_intra_grp.cuh"
@@ -505,8 +506,13 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
     return BISSD_OK;
 }
 
+// Where dx, dB, dC and ddt go (bissd_backward: contiguous, bissd_backward_into: the caller's strides).
+struct GradViews {
+    MutView dx, dB, dC, ddt;
+};
+
 template <class T>
-static int backward_impl(const bissd_bwd_args &a, const Dims &d, char *ws, cudaStream_t s, bool tcp) {
+static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dims &d, char *ws, cudaStream_t s, bool tcp) {
     const BwdWs w = bwd_layout(d, tcp);
     int *status = reinterpret_cast<int *>(ws);
     auto F = [&](size_t off) { return reinterpret_cast<float *>(ws + off); };
@@ -649,12 +655,12 @@ static int backward_impl(const bissd_bwd_args &a, const Dims &d, char *ws, cudaS
                     };
                     tc::WsArgs wa{};
                     wa.x = x; wa.z = gv; wa.D = a.D; wa.dt_out = a.dt_out; wa.cs_f = a.cs_f; wa.cs_b = a.cs_b;
-                    wa.out = MutView{a.dx, (long long)d.L * d.H * d.P, (long long)d.H * d.P, (long long)d.P};
+                    wa.out = gr.dx;
                     wa.out_x = wa.out;
                     wa.ddt_out = F(w.ddt_out); wa.nf = F(w.nf); wa.nb = F(w.nb); wa.dDpart = F(w.dDpart);
                     wa.wide_x = wide(x.ptr, x.sb, x.sl, x.sh);
                     wa.wide_z = wide(gv.ptr, gv.sb, gv.sl, gv.sh);
-                    wa.wide_o = wide(a.dx, 16, 16, 16) && (d.H * d.P) % 16 == 0;
+                    wa.wide_o = wide(gr.dx.ptr, gr.dx.sb, gr.dx.sl, gr.dx.sh);
                     wa.rows_by_tma = x_rows ? 1 : 0;
                     const size_t smem_t = tc::scan_ws_smem(d.P, d.N, d.Q);
                     const int grid = std::min(sm_count(), bch * nlt_tc);
@@ -705,7 +711,7 @@ static int backward_impl(const bissd_bwd_args &a, const Dims &d, char *ws, cudaS
                     const size_t smem_t = tc::dx_tma_smem(d.P, d.N, d.Q, rounds);
                     BISSD_ALLOW(tc::dx_tma<T>, smem_t);
                     BISSD_LAUNCH("tc_dx_tma", tc::dx_tma<T><<<dim3(bch, nlt_tc), tc::kThreads, smem_t, s>>>(
-                        d, mB, mEf, mEb, mG, x, gv, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cbt), a.dx, F(w.ddt_out), F(w.nf), F(w.nb),
+                        d, mB, mEf, mEb, mG, x, gv, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cbt), gr.dx, F(w.ddt_out), F(w.nf), F(w.nb),
                         F(w.dDpart), rounds, status));
                     dx_done = true;
                 }
@@ -714,11 +720,11 @@ static int backward_impl(const bissd_bwd_args &a, const Dims &d, char *ws, cudaS
             } else if (ntP <= 64) {
                 BISSD_ALLOW((tc::dx_kernel<T, 2>), smem_dx);
                 BISSD_LAUNCH("tc_dx", tc::dx_kernel<T, 2><<<dim3(bch, nlt_tc), tc::kThreads, smem_dx, s>>>(
-                    dg, x, Bm, z, gv, out_x, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cb), E16, a.dx, a.dz, F(w.ddt_out), F(w.dDpart), status));
+                    dg, x, Bm, z, gv, out_x, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cb), E16, gr.dx, a.dz, F(w.ddt_out), F(w.dDpart), status));
             } else {
                 BISSD_ALLOW((tc::dx_kernel<T, 8>), smem_dx);
                 BISSD_LAUNCH("tc_dx", tc::dx_kernel<T, 8><<<dim3(bch, nlt_tc), tc::kThreads, smem_dx, s>>>(
-                    dg, x, Bm, z, gv, out_x, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cb), E16, a.dx, a.dz, F(w.ddt_out), F(w.dDpart), status));
+                    dg, x, Bm, z, gv, out_x, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cb), E16, gr.dx, a.dz, F(w.ddt_out), F(w.dDpart), status));
             }
             bool dbc_done = false;
             if (dx_done) {                                           // the dx kernel has produced nf / nb
@@ -773,7 +779,7 @@ static int backward_impl(const bissd_bwd_args &a, const Dims &d, char *ws, cudaS
     if (!tcp) {
         BISSD_LAUNCH("bmm_cb", simt::bmm_cb<T><<<dim3(d.b * d.nc * d.G, w.nlt, w.nlt), simt::TB, 0, s>>>(d, Cm, Bm, F(w.cb)));
         BISSD_LAUNCH("dx_kernel", simt::dx_kernel<T><<<dim3(bch, w.nlt), simt::TB, q3, s>>>(
-            d, x, Bm, z, dout, out_x, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cb), F(w.E), a.dx, a.dz, F(w.ddt_out), F(w.dDpart)));
+            d, x, Bm, z, dout, out_x, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cb), F(w.E), gr.dx, a.dz, F(w.ddt_out), F(w.dDpart)));
         BISSD_LAUNCH("dbc_states", simt::dbc_states<T><<<dim3(bch, w.nlt, 2), simt::TB, q3, s>>>(
             d, x, Bm, Cm, z, dout, a.dt_out, a.cs_f, a.cs_b, F(w.E), a.states_f, a.states_b, F(w.dB_part), F(w.dC_part),
             F(w.nf), F(w.nb), F(w.pf), F(w.pb)));
@@ -903,23 +909,23 @@ static int backward_impl(const bissd_bwd_args &a, const Dims &d, char *ws, cudaS
             const size_t smem_b = tc::bmm_bwd_tma_smem(d.Q);
             BISSD_ALLOW(tc::bmm_bwd_tma<T>, smem_b);
             BISSD_LAUNCH("tc_bmm_bwd_tma", launch_pdl(tc::bmm_bwd_tma<T>, dim3(d.b * d.nc * d.G * 2, d.Q / 128, d.N / 64), tc::kThreads, smem_b, s, 
-                d, mDm, mDk, mBb, mCb, F(w.dB_part), F(w.dC_part), part_heads, a.dB, a.dC, status));
+                d, mDm, mDk, mBb, mCb, F(w.dB_part), F(w.dC_part), part_heads, gr.dB, gr.dC, status));
         } else if (tcp) {
             bmm_tc = true;
             const size_t smem_n = tc::smem_bytes(ntN, 0);
             BISSD_ALLOW(tc::bmm_bwd<T>, smem_n);
             BISSD_LAUNCH("tc_bmm_bwd", tc::bmm_bwd<T><<<dim3(d.b * d.nc * d.G * 2, nlt_tc, w.nsplit), tc::kThreads, smem_n, s>>>(
-                d, Bm, Cm, F(w.dCB), F(w.dB_part), F(w.dC_part), part_heads, a.dB, a.dC, status));
+                d, Bm, Cm, F(w.dCB), F(w.dB_part), F(w.dC_part), part_heads, gr.dB, gr.dC, status));
         }
     }
     if (!bmm_tc) {
         BISSD_LAUNCH("bmm_bwd", simt::bmm_bwd<T><<<dim3(d.b * d.nc * d.G * 2, w.nlt, ceil_div(d.N, simt::TILE)), simt::TB, 0, s>>>(
-            d, Bm, Cm, F(w.dCB), F(w.dB_part), F(w.dC_part), part_heads, a.dB, a.dC));
+            d, Bm, Cm, F(w.dCB), F(w.dB_part), F(w.dC_part), part_heads, gr.dB, gr.dC));
     }
     BISSD_LAUNCH("cumsum_bwd", launch_pdl(simt::cumsum_bwd, d.b * d.nc * d.H, 256, 0, s, 
         d, a.dt.ptr, a.p.dt_dtype, a.dt.stride_batch, a.dt.stride_seq, a.dt.stride_head, a.A, a.dt_bias, a.dt_out,
         F(w.ddt_out), F(w.nf), F(w.nb), F(w.pf), F(w.pb), use_u4 ? nullptr : F(w.da_f), use_u4 ? nullptr : F(w.da_b),
-        use_u4 ? F(w.u4) : nullptr, u4_tiles, F(w.dTpart), pass_nblk, nsplit, a.ddt,
+        use_u4 ? F(w.u4) : nullptr, u4_tiles, F(w.dTpart), pass_nblk, nsplit, gr.ddt,
         F(w.dApart), F(w.dbiaspart)));
     BISSD_LAUNCH("final_reduce", launch_pdl(simt::final_reduce<1024>, d.H, 1024, 0, s, 
         d, F(w.dApart), F(w.dbiaspart), d.has_D ? F(w.dDpart) : nullptr, dd_slots ? dd_slots : nlt, dd_compact ? 1 : 0, a.dA, d.has_bias ? a.ddt_bias : nullptr,
@@ -1262,6 +1268,35 @@ int bissd_dwconv_silu_backward(const bissd_conv_args *a, void *workspace, size_t
     BISSD_NORM_DISPATCH(conv_backward_impl, a, d, static_cast<char *>(workspace), s);
 }
 
+static int layer_params_check(const bissd_layer_params *a, bool out) {
+    if (!a || !a->A32 || (!out && !a->A) || (out && (!a->dA || !a->dA32))) return BISSD_ERR_NULL;
+    if (a->nheads <= 0 || a->d_elems < 0) return BISSD_ERR_SHAPE;
+    for (int t : {a->a_dtype, a->d_dtype, a->b_dtype})
+        if (t < BISSD_F32 || t > BISSD_F16) return BISSD_ERR_DTYPE;
+    if ((a->D && !a->D32) || (a->dt_bias && !a->dt_bias32)) return BISSD_ERR_NULL;
+    return check_device();
+}
+
+int bissd_layer_params_in(const bissd_layer_params *a, void *stream) {
+    const int rc = layer_params_check(a, false);
+    if (rc != BISSD_OK) return rc;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    BISSD_LAUNCH("layer_params_in", layer::params_in<<<ceil_div(std::max(a->nheads, a->d_elems), 256), 256, 0, s>>>(
+        a->nheads, a->d_elems, a->A, a->a_dtype, a->a_log, a->D, a->d_dtype, a->dt_bias, a->b_dtype, a->A32, a->D32, a->dt_bias32));
+    return BISSD_OK;
+}
+
+int bissd_layer_params_out(const bissd_layer_params *a, void *stream) {
+    const int rc = layer_params_check(a, true);
+    if (rc != BISSD_OK) return rc;
+    if ((a->dD && !a->dD32) || (a->ddt_bias && !a->ddt_bias32)) return BISSD_ERR_NULL;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    BISSD_LAUNCH("layer_params_out", launch_pdl(layer::params_out, ceil_div(std::max(a->nheads, a->d_elems), 256), 256, 0, s,
+        a->nheads, a->d_elems, a->A32, a->dA32, a->dD32, a->ddt_bias32, a->a_log, a->dA, a->a_dtype, a->dD, a->d_dtype,
+        a->ddt_bias, a->b_dtype));
+    return BISSD_OK;
+}
+
 const char *bissd_kernel_path(const bissd_problem *p) {
     if (!p) return "";
     return (!force_simt() && tc_shape_ok(*p)) ? "tcgen05" : "simt";
@@ -1386,6 +1421,11 @@ int bissd_chain_boundaries(const float *left, const float *right, const float *l
 }
 
 int bissd_backward(const bissd_bwd_args *a, void *workspace, size_t workspace_bytes, void *stream) {
+    return bissd_backward_into(a, nullptr, workspace, workspace_bytes, stream);
+}
+
+int bissd_backward_into(const bissd_bwd_args *a, const bissd_grad_strides *gs, void *workspace, size_t workspace_bytes,
+                        void *stream) {
     if (!a) return BISSD_ERR_NULL;
     Dims d;
     int rc = make_dims(a->p, &d);
@@ -1413,10 +1453,19 @@ int bissd_backward(const bissd_bwd_args *a, void *workspace, size_t workspace_by
     if (rc != BISSD_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char *ws = static_cast<char *>(workspace);
+    const long long L = d.L, hp = (long long)d.H * d.P, gn = (long long)d.G * d.N;
+    GradViews gr{MutView{a->dx, L * hp, hp, d.P}, MutView{a->dB, L * gn, gn, d.N}, MutView{a->dC, L * gn, gn, d.N},
+                 MutView{a->ddt, L * d.H, d.H, 1}};
+    if (gs) {
+        auto set = [](MutView &v, const int64_t *st) { v.sb = st[0]; v.sl = st[1]; v.sh = st[2]; };
+        set(gr.dx, gs->dx); set(gr.dB, gs->dB); set(gr.dC, gs->dC); set(gr.ddt, gs->ddt);
+        auto al = [](const MutView &v) { return reinterpret_cast<uintptr_t>(v.ptr) % 16 == 0 && v.sb % 8 == 0 && v.sl % 8 == 0 && v.sh % 8 == 0; };
+        if (tcp && !(al(gr.dx) && al(gr.dB) && al(gr.dC))) return BISSD_ERR_ALIGN;   // 16-byte stores
+    }
     switch (a->p.x_dtype) {
-        case BISSD_F32: return backward_impl<float>(*a, d, ws, s, false);
-        case BISSD_BF16: return backward_impl<__nv_bfloat16>(*a, d, ws, s, tcp);
-        default: return backward_impl<__half>(*a, d, ws, s, tcp);
+        case BISSD_F32: return backward_impl<float>(*a, gr, d, ws, s, false);
+        case BISSD_BF16: return backward_impl<__nv_bfloat16>(*a, gr, d, ws, s, tcp);
+        default: return backward_impl<__half>(*a, gr, d, ws, s, tcp);
     }
 }
 

@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(TB) state_passing_bwd(Dims d, const float *glo
 template <class T>
 __global__ void __launch_bounds__(TB) dx_kernel(Dims d, View x, View Bm, View z, View dout, View out_x, const float *D,
                                                 const float *dt_out, const float *cs_f, const float *cs_b,
-                                                const float *CB, const float *E, void *dx, void *dz, float *ddt_out,
+                                                const float *CB, const float *E, MutView dx, void *dz, float *ddt_out,
                                                 float *dDpart) {
     extern __shared__ float sm[];
     __shared__ GemmSmem gs;
@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(TB) dx_kernel(Dims d, View x, View Bm, View z,
                 }
                 float v = acc[i][j] * sd[l];
                 if (d.has_D) v += (d.D_hdim ? D[h * d.P + p] : D[h]) * gv;
-                st<T>(dx, ((long long)(b * d.L + ls) * d.H + h) * d.P + p, v);
+                stv<T>(dx, b, ls, h, p, v);
                 rowsum[i] += acc[i][j] * xv;
                 colsum[j] += gv * xv;
             }
@@ -779,7 +779,7 @@ __global__ void __launch_bounds__(TB) intra_decay_grad(Dims d, View x, View z, V
 // grid (b*nc*G*2, ceil(Q/64), ceil(N/64)); blockIdx.x & 1: 0 = dB, 1 = dC.
 template <class T>
 __global__ void __launch_bounds__(TB) bmm_bwd(Dims d, View Bm, View Cm, const float *dCB, const float *dB_part,
-                                              const float *dC_part, int part_heads, void *dB, void *dC) {
+                                              const float *dC_part, int part_heads, MutView dB, MutView dC) {
     __shared__ GemmSmem gs;
     const int which = blockIdx.x & 1;
     const int bx = blockIdx.x >> 1;
@@ -805,7 +805,7 @@ __global__ void __launch_bounds__(TB) bmm_bwd(Dims d, View Bm, View Cm, const fl
     }
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const float *part = which ? dC_part : dB_part;
-    void *out = which ? dC : dB;
+    const MutView out = which ? dC : dB;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int l = r0 + ty * 4 + i;
@@ -818,7 +818,7 @@ __global__ void __launch_bounds__(TB) bmm_bwd(Dims d, View Bm, View Cm, const fl
             const int rp = part_heads / d.G;      // partial results per group: one per head, or already summed
             const long long pb = (((long long)b * d.nc * Q + c * Q + l) * part_heads + g * rp) * d.N + n;
             for (int r = 0; r < rp; ++r) v += part[pb + (long long)r * d.N];
-            st<T>(out, (((long long)b * d.L + c * Q + l) * d.G + g) * d.N + n, v);
+            stv<T>(out, b, c * Q + l, g, n, v);
         }
     }
 }
@@ -870,7 +870,7 @@ __global__ void __launch_bounds__(256) cumsum_bwd(Dims d, const void *dt, int dt
                                                       const float *dt_out, const float *ddt_out, const float *nf,
                                                       const float *nb, const float *pf, const float *pb, const float *da_f,
                                                       const float *da_b, const float *u4, int u4_tiles,
-                                                      const float *dTpart, int nblk, int nsplit, void *ddt, float *dApart,
+                                                      const float *dTpart, int nblk, int nsplit, MutView ddt, float *dApart,
                                                       float *dbiaspart) {
     pdl_begin();
     __shared__ float tot[4][8];
@@ -917,7 +917,7 @@ __global__ void __launch_bounds__(256) cumsum_bwd(Dims d, const void *dt, int dt
         const float val = d.softplus ? softplus_ref(pre) : pre;
         if (val < d.dt_min || val > d.dt_max) g = 0.f;
         if (d.softplus && pre <= 20.f) g *= sigmoidf_(pre);
-        st_any(ddt, dt_dtype, ((long long)b * d.L + c * d.Q + l) * d.H + h, g);
+        st_any(ddt.ptr, dt_dtype, b * ddt.sb + (long long)(c * d.Q + l) * ddt.sl + h * ddt.sh, g);
         sumA = ddA * dlo;
         sumB = g;
     }

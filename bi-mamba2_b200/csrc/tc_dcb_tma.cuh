@@ -197,7 +197,7 @@ template <class T>
 __global__ void __launch_bounds__(kThreads, 2)
 bmm_bwd_tma(Dims d, const __grid_constant__ CUtensorMap tmDm, const __grid_constant__ CUtensorMap tmDk,
             const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC, const float *dB_part,
-            const float *dC_part, int part_heads, void *dB, void *dC, int *status) {
+            const float *dC_part, int part_heads, MutView dB, MutView dC, int *status) {
     pdl_begin();
     extern __shared__ uint8_t dyn[];
     __shared__ uint64_t bar_in, bar_done;
@@ -261,7 +261,8 @@ bmm_bwd_tma(Dims d, const __grid_constant__ CUtensorMap tmDm, const __grid_const
         float v[32];
         tmem_ld32(tmem_lane_base(tmem) + c0, v);
         if (row < lim) {
-            T *out = static_cast<T *>(which ? dC : dB) + (((long long)b * d.L + c * Q + row) * d.G + g) * N + n0 + c0;
+            const MutView ov = which ? dC : dB;
+            T *out = static_cast<T *>(ov.ptr) + b * ov.sb + (long long)(c * Q + row) * ov.sl + g * ov.sh + n0 + c0;
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
                 float t[8];

@@ -50,7 +50,7 @@ template <class T>
 __global__ void __launch_bounds__(kThreads, 2)
 dx_tma(Dims d, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmEf,
        const __grid_constant__ CUtensorMap tmEb, const __grid_constant__ CUtensorMap tmG, View x, View g, const float *D,
-       const float *dt_out, const float *cs_f, const float *cs_b, const float *CBt, void *dx, float *ddt_out, float *nf,
+       const float *dt_out, const float *cs_f, const float *cs_b, const float *CBt, MutView dx, float *ddt_out, float *nf,
        float *nb, float *dDpart, int rounds, int *status) {
     extern __shared__ uint8_t dyn[];
     __shared__ ScanShared sh;
@@ -279,7 +279,7 @@ dx_tma(Dims d, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
                         gx[i] = gv[i] * xv[i];
                     }
                     if (l < lim)
-                        *reinterpret_cast<uint4 *>(static_cast<T *>(dx) + ((long long)(b * d.L + c * Q + l) * d.H + h) * P + p0) = pack8<T>(o);
+                        *reinterpret_cast<uint4 *>(static_cast<T *>(dx.ptr) + b * dx.sb + (long long)(c * Q + l) * dx.sl + h * dx.sh + p0) = pack8<T>(o);
                     if (d.has_D) {                              // column sums of g*x over this warp's 32 rows
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {

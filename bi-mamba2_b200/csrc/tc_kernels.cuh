@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(kThreads, BCH <= 2 ? 2 : 1) chunk_scan(Dims d,
 template <class T, int BCH>
 __global__ void __launch_bounds__(kThreads, BCH <= 2 ? 2 : 1) dx_kernel(Dims d, View x, View Bm, View z, View dout, View out_x,
                                                       const float *D, const float *dt_out, const float *cs_f,
-                                                      const float *cs_b, const float *CB, const void *E16, void *dx,
+                                                      const float *cs_b, const float *CB, const void *E16, MutView dx,
                                                       void *dz, float *ddt_out, float *dDpart, int *status) {
     extern __shared__ uint8_t dyn[];
     __shared__ PipeShared sh;
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(kThreads, BCH <= 2 ? 2 : 1) dx_kernel(Dims d, 
                         rowsum += v[j + i] * xv[i];
                         cs8[j + i] = gv[i] * xv[i];
                     }
-                    *reinterpret_cast<uint4 *>(static_cast<T *>(dx) + oo) = pack8<T>(o);
+                    *reinterpret_cast<uint4 *>(static_cast<T *>(dx.ptr) + b * dx.sb + (long long)ls * dx.sl + h * dx.sh + p0) = pack8<T>(o);
                 }
             }
             if (d.has_D) {                                              // column sums of g*x over this warp's 32 rows
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(kThreads) dbc_states(Dims d, View x, View Bm, 
 // grid (b*nc*G*2, ceil(Q/128), nsplit); n_tile = min(round16(N), 128).
 template <class T>
 __global__ void __launch_bounds__(kThreads) bmm_bwd(Dims d, View Bm, View Cm, const float *dCB, const float *dB_part,
-                                                    const float *dC_part, int part_heads, void *dB, void *dC,
+                                                    const float *dC_part, int part_heads, MutView dB, MutView dC,
                                                     int *status) {
     extern __shared__ uint8_t dyn[];
     __shared__ PipeShared sh;
@@ -609,7 +609,8 @@ __global__ void __launch_bounds__(kThreads) bmm_bwd(Dims d, View Bm, View Cm, co
         const int row = r0 + (warp & 3) * 32 + lane;
         const int rp = part_heads / d.G;
         const float *part = (which ? dC_part : dB_part) + (((long long)b * d.nc * Q + c * Q + row) * part_heads + g * rp) * N + n0;
-        T *out = static_cast<T *>(which ? dC : dB) + (((long long)b * d.L + c * Q + row) * d.G + g) * N + n0;
+        const MutView ov = which ? dC : dB;
+        T *out = static_cast<T *>(ov.ptr) + b * ov.sb + (long long)(c * Q + row) * ov.sl + g * ov.sh + n0;
         for (int c0 = (warp >> 2) * 32; c0 < nt; c0 += 64) {
             float v[32];
             tmem_ld32(tmem_lane_base(p.tmem) + c0, v);

@@ -69,7 +69,7 @@ EXPORTS = ("bissd_abi_version", "bissd_strerror", "bissd_last_cuda_error", "biss
            "bissd_backward", "bissd_kernel_path", "bissd_launch_count", "bissd_trace_enable", "bissd_trace_read", "bissd_selftest_gemm", "bissd_read_status",
            "bissd_forward_static_scratch", "bissd_chain_boundaries", "bissd_rmsnorm_gated_workspace_bytes", "bissd_rmsnorm_gated_forward",
            "bissd_rmsnorm_gated_backward", "bissd_dwconv_silu_workspace_bytes", "bissd_dwconv_silu_forward",
-           "bissd_dwconv_silu_backward")
+           "bissd_dwconv_silu_backward", "bissd_backward_into", "bissd_layer_params_in", "bissd_layer_params_out")
 
 STATIC_SCRATCH_BYTES = 16 << 20      # BISSD_STATIC_SCRATCH_BYTES
 ERR_TOO_LARGE = -9

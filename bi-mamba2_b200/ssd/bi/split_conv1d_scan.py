@@ -8,6 +8,10 @@ bidirectional scan does not take) and what its layer leaves commented out behind
 (src/ssd/modules.py:60,129-150).  Here it computes exactly what the layer's step-by-step path computes
 (src/ssd/modules.py:152-187): the same kernels of libbissd in the same order, so both paths give the same numbers.
 
+In eager mode the node is native (csrc/torch_ops.cpp, `layer`, which also serves the layer's step-by-step path, there
+without the recomputation); the Python node below takes what that one does not: torch.compile, autocast, no norm weight
+(the gate inside the scan), and slices of zxbcdt whose rows are not 16-byte aligned.
+
 Saved for the backward pass: zxbcdt, the scan's output (the norm's input), rstd and the parameters.  Recomputed there:
 the convolution's output (x, B, C), the scan's per-chunk quantities (dt after softplus, the cumulative sums and the
 states entering each chunk: the LOCAL phase of the forward library call) and the norm's output (for the output
@@ -18,7 +22,7 @@ import torch
 import torch.nn.functional as F
 
 from ssd import _cabi
-from ssd.bi import conv_silu, layernorm_gated
+from ssd.bi import conv_silu, layernorm_gated, ssd_combined
 from ssd.bi.ssd_combined import _scan_bwd_eager, _scan_fwd_core
 
 
@@ -180,6 +184,16 @@ class BiMambaSplitConv1dScanCombinedFn(torch.autograd.Function):
                 doutproj_weight, doutproj_bias, None, None, None, None)
 
 
+def native_layer(zxbcdt, conv1d_weight, conv1d_bias, dt_bias, A, a_log, D, chunk_size, dt_limit, rmsnorm_weight, rmsnorm_eps,
+                 group_size, norm_before_gate, headdim, ngroups, recompute, outproj_weight=None, outproj_bias=None):
+    """The native node (A is -exp of the given tensor where a_log), or None where its arguments are for the Python path."""
+    if headdim is None:
+        return None
+    return _cabi.torch_ops().layer(zxbcdt, conv1d_weight, conv1d_bias, dt_bias, A, a_log, D, chunk_size, dt_limit[0],
+                                   dt_limit[1], rmsnorm_weight, rmsnorm_eps, group_size, norm_before_gate, headdim, ngroups,
+                                   recompute, outproj_weight, outproj_bias, ssd_combined.CHECK_STATUS)
+
+
 def bimamba_split_conv1d_scan_combined(zxbcdt, conv1d_weight, conv1d_bias, dt_bias, A, D, chunk_size,
                                        dt_limit=(0.0, float("inf")), rmsnorm_weight=None, rmsnorm_eps=1e-6,
                                        outproj_weight=None, outproj_bias=None, headdim=None, ngroups=1,
@@ -200,6 +214,13 @@ def bimamba_split_conv1d_scan_combined(zxbcdt, conv1d_weight, conv1d_bias, dt_bi
     `seq_idx`, `return_final_states` and extra non-SSM channels are not taken (the bidirectional layer has none), and
     arguments outside the kernels' range raise instead of falling back.
     """
+    if rmsnorm_weight is not None and not torch.compiler.is_compiling() and not torch.is_autocast_enabled("cuda"):
+        dim = rmsnorm_weight.shape[0]
+        res = native_layer(zxbcdt, conv1d_weight, conv1d_bias, dt_bias, A, False, D, chunk_size, dt_limit, rmsnorm_weight,
+                           rmsnorm_eps, dim // ngroups if rmsnorm_group_size is None else rmsnorm_group_size,
+                           norm_before_gate, D.shape[1] if D.dim() == 2 else headdim, ngroups, True, outproj_weight, outproj_bias)
+        if res is not None:
+            return res
     return BiMambaSplitConv1dScanCombinedFn.apply(zxbcdt, conv1d_weight, conv1d_bias, dt_bias, A, D, chunk_size, dt_limit,
                                                   rmsnorm_weight, rmsnorm_eps, outproj_weight, outproj_bias, headdim,
                                                   ngroups, norm_before_gate, rmsnorm_group_size)

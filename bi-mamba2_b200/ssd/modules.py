@@ -16,7 +16,7 @@ import torch.nn.functional as F
 
 from ssd.bi.conv_silu import dwconv1d_silu
 from ssd.bi.layernorm_gated import RMSNorm as RMSNormGated
-from ssd.bi.split_conv1d_scan import bimamba_split_conv1d_scan_combined
+from ssd.bi.split_conv1d_scan import bimamba_split_conv1d_scan_combined, native_layer
 from ssd.bi.ssd_combined import bimamba_chunk_scan_combined
 
 
@@ -70,9 +70,25 @@ class BiMamba2(nn.Module):
         self.norm = RMSNormGated(self.d_inner, eps=1e-5, norm_before_gate=True, **factory_kwargs)
         self.out_proj = nn.Linear(self.d_inner, self.d_model, bias=bias, **factory_kwargs)
 
+    def _native_ok(self):
+        """Eager, no autocast, and the norm module as constructed (not replaced or hooked: the node does not call it)."""
+        return not (torch.compiler.is_compiling() or torch.is_autocast_enabled("cuda") or type(self.norm) is not RMSNormGated or
+                    self.norm._forward_hooks or self.norm._forward_pre_hooks or self.norm._backward_hooks or
+                    self.norm._backward_pre_hooks or self.activation not in ("silu", "swish"))
+
     def forward(self, u):
         """u: (batch, seqlen, d_model) -> same shape."""
         zxbcdt = self.in_proj(u)
+        if self._native_ok():
+            # everything between the projections as one native autograd node (with recomputation also the second one)
+            own_out = self.use_mem_eff_path
+            y = native_layer(zxbcdt, self.conv1d.weight, self.conv1d.bias, self.dt_bias, self.A_log, True, self.D,
+                             self.chunk_size, self.dt_limit, self.norm.weight, self.norm.eps,
+                             self.d_inner if self.norm.group_size is None else self.norm.group_size,
+                             self.norm.norm_before_gate, self.headdim, self.ngroups, own_out,
+                             self.out_proj.weight if own_out else None, self.out_proj.bias if own_out else None)
+            if y is not None:
+                return y if own_out else self.out_proj(y)
         A = -torch.exp(self.A_log.float())
         dt_limit_kwargs = {} if self.dt_limit == (0.0, float("inf")) else dict(dt_limit=self.dt_limit)
         if self.use_mem_eff_path:

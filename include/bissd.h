@@ -168,6 +168,16 @@ int bissd_forward_static_scratch(const bissd_fwd_args *args, void *stream);
 /* Backward pass. */
 int bissd_backward(const bissd_bwd_args *args, void *workspace, size_t workspace_bytes, void *stream);
 
+/* The same with dx, dB, dC and ddt written at the given element strides (batch, sequence, head or group; the innermost
+ * dimension stays contiguous) - into slices of a larger tensor, where a layer wants them.  For the tensor-core kernels
+ * dx, dB and dC need 16-byte aligned pointers and strides that are multiples of 8 elements, else BISSD_ERR_ALIGN.
+ * strides == NULL: contiguous, as bissd_backward. */
+typedef struct bissd_grad_strides {
+    int64_t dx[3], dB[3], dC[3], ddt[3];
+} bissd_grad_strides;
+int bissd_backward_into(const bissd_bwd_args *args, const bissd_grad_strides *strides, void *workspace,
+                        size_t workspace_bytes, void *stream);
+
 /* Boundary chaining between the two phases of a sequence-sharded pass (no reference counterpart: the reference is
  * single-GPU; this continues its chunk recurrence, src/ssd/bi/ssd_state_passing.py:60,81, across ranks).  Every rank
  * has gathered all ranks' boundary tensors into LOCAL memory (e.g. with one NCCL all-gather); then
@@ -232,6 +242,23 @@ typedef struct bissd_conv_args {
 int bissd_dwconv_silu_workspace_bytes(const bissd_conv_args *args, size_t *bwd_bytes);
 int bissd_dwconv_silu_forward(const bissd_conv_args *args, void *stream);
 int bissd_dwconv_silu_backward(const bissd_conv_args *args, void *workspace, size_t workspace_bytes, void *stream);
+
+/* ---- the layer's per-head parameters ------------------------------------------------------------------------------
+ * bissd_layer_params_in: A32 = A (a_log == 0) or -exp(A) (a_log != 0: the layer stores A_log, src/ssd/modules.py:125),
+ * D32 = D, dt_bias32 = dt_bias, all fp32 from any bissd_dtype; D and dt_bias may be NULL.
+ * bissd_layer_params_out: the gradients dA32, dD32, ddt_bias32 turned into dA (times A32 where a_log), dD, ddt_bias of
+ * the parameters' dtypes. */
+typedef struct bissd_layer_params {
+    int32_t nheads, d_elems;             /* d_elems: elements of D */
+    int32_t a_log;
+    int32_t a_dtype, d_dtype, b_dtype;   /* bissd_dtype of A, D, dt_bias and of their gradients */
+    const void *A, *D, *dt_bias;
+    float *A32, *D32, *dt_bias32;
+    const float *dA32, *dD32, *ddt_bias32;      /* params_out only, as are the next three */
+    void *dA, *dD, *ddt_bias;
+} bissd_layer_params;
+int bissd_layer_params_in(const bissd_layer_params *args, void *stream);
+int bissd_layer_params_out(const bissd_layer_params *args, void *stream);
 
 /* Name of the kernel family the library selects for `p` ("tcgen05" or "simt"); for reports and tests. */
 const char *bissd_kernel_path(const bissd_problem *p);
