@@ -7,7 +7,9 @@ package also loads it with ctypes); _bissd_torch.so is a Python extension compil
 and linked to libbissd.so.  Neither needs a GPU to build.
 """
 import argparse
+import concurrent.futures
 import os
+import re
 import subprocess
 import sys
 import sysconfig
@@ -16,18 +18,22 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "ssd", "_lib")
 OUT = os.path.join(OUT_DIR, "libbissd.so")
-SOURCES = ["bissd_api.cu"]
+SOURCES = ["bissd_api.cu", "bissd_layer.cu"]
 TORCH_SRC = os.path.join(CSRC, "torch_ops.cpp")
 TORCH_OUT = os.path.join(OUT_DIR, "_bissd_torch.so")
 
 
-def _newest_source_mtime():
-    newest = 0.0
-    for root in (CSRC, os.path.join(os.path.dirname(HERE), "include")):
-        for name in os.listdir(root):
-            if name.endswith((".cu", ".cuh", ".h")):
-                newest = max(newest, os.path.getmtime(os.path.join(root, name)))
-    return newest
+def _newest_source_mtime(source):
+    """Newest of a source file and what it includes from this repository, directly or not."""
+    seen, todo = set(), [os.path.join(CSRC, source)]
+    while todo:
+        path = todo.pop()
+        if path not in seen:
+            seen.add(path)
+            with open(path) as f:
+                names = re.findall(r'^#include "([^"]+)"', f.read(), flags=re.M)
+            todo += [os.path.normpath(os.path.join(os.path.dirname(path), n)) for n in names]
+    return max(os.path.getmtime(p) for p in seen)
 
 
 def _run(cmd, verbose, what):
@@ -66,16 +72,16 @@ def build(force=False, verbose=False):
 
 
 def build_library(force=False, verbose=False):
-    if not force and os.path.exists(OUT) and os.path.getmtime(OUT) >= _newest_source_mtime():
+    if not force and os.path.exists(OUT) and os.path.getmtime(OUT) >= max(map(_newest_source_mtime, SOURCES)):
         return OUT
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    cmd = [nvcc, "-std=c++17", "-O3", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
-           "--expt-relaxed-constexpr", "--extended-lambda", "-Xcompiler", "-fPIC", "-shared",
-           "-o", OUT] + [os.path.join(CSRC, s) for s in SOURCES]
-    if verbose:
-        cmd.insert(1, "-Xptxas")
-        cmd.insert(2, "-v")
-    _run(cmd, verbose, os.path.basename(OUT))
+    flags = ["-std=c++17", "-O3", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a", "--expt-relaxed-constexpr",
+             "--extended-lambda", "-Xcompiler", "-fPIC"] + (["-Xptxas", "-v"] if verbose else [])
+    objs = [os.path.join(OUT_DIR, s.replace(".cu", ".o")) for s in SOURCES]
+    stale = [(s, o) for s, o in zip(SOURCES, objs) if force or not os.path.exists(o) or os.path.getmtime(o) < _newest_source_mtime(s)]
+    with concurrent.futures.ThreadPoolExecutor() as pool:                # one nvcc per translation unit, side by side
+        list(pool.map(lambda so: _run([nvcc, *flags, "-c", "-o", so[1], os.path.join(CSRC, so[0])], verbose, so[0]), stale))
+    _run([nvcc, "-shared", "-o", OUT, *objs], verbose, os.path.basename(OUT))
     return OUT
 
 

@@ -1,19 +1,15 @@
 // C ABI of libbissd (declared in include/bissd.h): argument validation, workspace layout, kernel sequencing.
 #include <algorithm>
-#include <atomic>
-#include <cstdlib>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <utility>
 #include <vector>
 
 #include "common.cuh"
+#include "host.cuh"
 #include "simt_kernels.cuh"
-#include "conv_kernels.cuh"
-#include "norm_kernels.cuh"
-#include "layer_kernels.cuh"
 #include "tc_intra.cuh"
 #include "tc_intra_sums.cuh"
 #include "tc_intra_grp.cuh"
@@ -29,76 +25,12 @@
 
 namespace bissd {
 
-static thread_local char g_cuda_err[256] = "";
-
-static int note_cuda(cudaError_t e, const char *what) {
-    if (e == cudaSuccess) return BISSD_OK;
-    snprintf(g_cuda_err, sizeof(g_cuda_err), "%s: %s", what, cudaGetErrorString(e));
-    return BISSD_ERR_LAUNCH;
-}
-
-// ---- tracing: optional CUDA-event brackets around every kernel launch, and a launch counter -------------
-struct TraceRec {
-    const char *name;
-    cudaEvent_t e0, e1;
-};
-static std::mutex g_trace_mu;
-static std::vector<TraceRec> g_trace;
-static std::atomic<int> g_trace_on{0};
-static std::atomic<unsigned long long> g_launches{0};
-
-struct TraceScope {
-    const char *name;
-    cudaStream_t s;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    TraceScope(const char *n, cudaStream_t st) : name(n), s(st) {
-        if (g_trace_on.load(std::memory_order_relaxed)) {
-            if (cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess) cudaEventRecord(e0, s);
-            else e0 = e1 = nullptr;
-        }
-    }
-    void end() {
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        if (e0 && e1) {
-            cudaEventRecord(e1, s);
-            std::lock_guard<std::mutex> lk(g_trace_mu);
-            g_trace.push_back(TraceRec{name, e0, e1});
-        }
-    }
-};
-
-// Launch `...` (a full kernel<<<>>>() expression) on stream `s`, count it, bracket it with events when tracing.
-// Launch with programmatic stream serialisation: the kernel may be scheduled while its predecessor drains and
-// waits for it in pdl_begin().  Only kernels that open with pdl_begin() go through here.  BISSD_NO_PDL=1 turns
-// the attribute off (plain stream order).
-static bool no_pdl() {
-    static const bool v = std::getenv("BISSD_NO_PDL") != nullptr;
-    return v;
-}
-template <class... Exp, class... Act>
-static cudaError_t launch_pdl(void (*kernel)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act &&...args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = no_pdl() ? 0 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Act>(args)...);
-}
-
-#define BISSD_LAUNCH_ON(stream, name, ...)                        \
-    do {                                                          \
-        TraceScope ts_(name, stream);                             \
-        __VA_ARGS__;                                              \
-        ts_.end();                                                \
-        int rc_ = note_cuda(cudaGetLastError(), name);            \
-        if (rc_ != BISSD_OK) return rc_;                          \
-    } while (0)
-#define BISSD_LAUNCH(name, ...) BISSD_LAUNCH_ON(s, name, __VA_ARGS__)
+// ---- state declared in host.cuh ----------------------------------------------------------------------------
+thread_local char g_cuda_err[256] = "";
+std::mutex g_trace_mu;
+std::vector<TraceRec> g_trace;
+std::atomic<int> g_trace_on{0};
+std::atomic<unsigned long long> g_launches{0};
 
 // A second stream for the two group-walking backward kernels whose results nothing reads before the last product with
 // dCB (prev_terms_grp, dbc_accum_grp): they fork from the caller's stream after the dx kernel and join it again
@@ -179,8 +111,6 @@ static int make_dims(const bissd_problem &p, Dims *d) {
     return BISSD_OK;
 }
 
-static inline size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
-
 // Workspace carving.  The first 256 bytes hold the device status word (nonzero = a bounded device-side wait ran
 // out); everything after it is fp32 scratch.
 constexpr size_t kWsHeader = 256;
@@ -243,31 +173,6 @@ static BwdWs bwd_layout(const Dims &d, bool tc) {
 static View view_of(const bissd_tensor &t) { return View{t.ptr, t.stride_batch, t.stride_seq, t.stride_head}; }
 static MutView mview_of(const bissd_tensor &t) { return MutView{t.ptr, t.stride_batch, t.stride_seq, t.stride_head}; }
 
-// Raise a kernel's dynamic shared-memory limit.  The attribute is per (function, device) and sticks, so it is set the
-// first time a kernel needs `bytes` on a device and remembered (the driver call costs a microsecond or two per launch
-// otherwise - a tenth of the host time of a whole pass).
-static std::mutex g_smem_mu;
-static std::map<std::pair<const void *, int>, size_t> g_smem_granted;   // (kernel, device) -> bytes already allowed
-template <class K> static int allow_smem(K kernel, size_t bytes) {
-    if (bytes <= 48 * 1024) return BISSD_OK;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
-    const std::pair<const void *, int> key(reinterpret_cast<const void *>(kernel), dev);
-    if (dev >= 0) {
-        std::lock_guard<std::mutex> lk(g_smem_mu);
-        auto it = g_smem_granted.find(key);
-        if (it != g_smem_granted.end() && it->second >= bytes) return BISSD_OK;
-    }
-    int rc = note_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes),
-                       "cudaFuncSetAttribute");
-    if (rc == BISSD_OK && dev >= 0) {
-        std::lock_guard<std::mutex> lk(g_smem_mu);
-        size_t &g = g_smem_granted[key];
-        g = std::max(g, bytes);
-    }
-    return rc;
-}
-
 // ---- which kernel family ---------------------------------------------------------------------------------
 static bool tc_shape_ok(const bissd_problem &p) {
     return (p.x_dtype == BISSD_BF16 || p.x_dtype == BISSD_F16) && p.headdim % 8 == 0 && p.dstate % 8 == 0 &&
@@ -287,18 +192,6 @@ static bool no_ws() {    // BISSD_NO_WS=1: keep the one-tile-per-CTA TMA kernels
     static const bool v = [] { const char *e = getenv("BISSD_NO_WS"); return e && e[0] == '1'; }();
     return v;
 }
-static int sm_count() {
-    static int n[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    if (!n[dev]) {
-        int v = 0;
-        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
-        n[dev] = v;
-    }
-    return n[dev];
-}
-
 static bool no_sums() {  // BISSD_NO_SUMS=1: keep the prefix-sweep form of the intra-chunk decay gradient
     static const bool v = [] { const char *e = getenv("BISSD_NO_SUMS"); return e && e[0] == '1'; }();
     return v;
@@ -323,12 +216,6 @@ static bool map_bshd(CUtensorMap *m, int dtype, const void *ptr, long long sb, l
     const unsigned box[4] = {64, 1, rows, 1};
     return tc::make_map4(m, dtype, ptr, dims, str, box);
 }
-
-#define BISSD_ALLOW(kernel, bytes)                  \
-    do {                                             \
-        int rc_ = allow_smem(kernel, bytes);         \
-        if (rc_ != BISSD_OK) return rc_;             \
-    } while (0)
 
 template <class T> struct TcKernels {   // 16-bit types only; the fp32 specialisation below never launches them
     static constexpr bool available = true;
@@ -933,162 +820,9 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
     return BISSD_OK;
 }
 
-static int check_device() {
-    static std::atomic<int> major_of[64];                        // 0 = not asked yet
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return BISSD_ERR_LAUNCH;
-    int major = (dev >= 0 && dev < 64) ? major_of[dev].load(std::memory_order_relaxed) : 0;
-    if (!major) {
-        if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return BISSD_ERR_LAUNCH;
-        if (dev >= 0 && dev < 64) major_of[dev].store(major, std::memory_order_relaxed);
-    }
-    return major == 10 ? BISSD_OK : BISSD_ERR_ARCH;
-}
-
 }  // namespace bissd
 
 using namespace bissd;
-
-// ---- gated RMSNorm ---------------------------------------------------------------------------------------------
-static int norm_check(const bissd_norm_args *a, norm::NormDims *d, bool backward) {
-    if (!a || !a->x || !a->weight || !a->rstd) return BISSD_ERR_NULL;
-    if (!backward && !a->out) return BISSD_ERR_NULL;
-    if (backward && (!a->dout || !a->dx || !a->dweight || (a->z && !a->dz))) return BISSD_ERR_NULL;
-    if (a->rows <= 0 || a->hidden <= 0 || a->hidden % 256 != 0 || a->hidden > 4096) return BISSD_ERR_SHAPE;
-    const int group = a->group_size > 0 ? a->group_size : a->hidden;
-    if (group % 256 != 0 || a->hidden % group != 0) return BISSD_ERR_SHAPE;
-    if (a->x_dtype < BISSD_F32 || a->x_dtype > BISSD_F16) return BISSD_ERR_DTYPE;
-    if (a->w_dtype != BISSD_F32 && a->w_dtype != a->x_dtype) return BISSD_ERR_DTYPE;
-    auto al = [](const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-    if (!al(a->x) || !al(a->z) || !al(a->weight) || !al(a->out) || !al(a->dout) || !al(a->dx) || !al(a->dz))
-        return BISSD_ERR_ALIGN;
-    if (a->stride_x % 8 || a->stride_z % 8 || a->stride_out % 8) return BISSD_ERR_ALIGN;
-    d->rows = a->rows; d->hidden = a->hidden; d->group = group; d->ngroups = a->hidden / group;
-    d->sx = a->stride_x; d->sz = a->stride_z; d->so = a->stride_out;
-    d->has_z = a->z != nullptr; d->norm_before_gate = a->norm_before_gate; d->eps = a->eps;
-    return BISSD_OK;
-}
-static int norm_grid(const norm::NormDims &d) {
-    const long long want = (d.rows + norm::kWarps - 1) / norm::kWarps;
-    return (int)std::min<long long>(want, (long long)sm_count() * 8);
-}
-
-template <class T, class W>
-static int norm_forward_impl(const bissd_norm_args *a, const norm::NormDims &d, cudaStream_t s) {
-    const int grid = norm_grid(d);
-    if (d.hidden <= 2048) {
-        BISSD_LAUNCH("rmsnorm_gated_fwd", norm::rmsnorm_gated_fwd<T, W, 8><<<grid, norm::kThreads, 0, s>>>(
-            d, a->x, a->z, a->weight, a->out, a->rstd));
-    } else {
-        BISSD_LAUNCH("rmsnorm_gated_fwd", norm::rmsnorm_gated_fwd<T, W, 16><<<grid, norm::kThreads, 0, s>>>(
-            d, a->x, a->z, a->weight, a->out, a->rstd));
-    }
-    return BISSD_OK;
-}
-template <class T, class W>
-static int norm_backward_impl(const bissd_norm_args *a, const norm::NormDims &d, float *part, cudaStream_t s) {
-    // two resident CTAs per SM and one partial weight-gradient row per CTA: a larger grid only adds rows to reduce
-    const int grid = std::min(norm_grid(d), 2 * sm_count());
-    const size_t smem = (size_t)norm::kWarps * d.hidden * sizeof(float);
-    if (d.hidden <= 2048) {
-        BISSD_ALLOW((norm::rmsnorm_gated_bwd<T, W, 8>), smem);
-        BISSD_LAUNCH("rmsnorm_gated_bwd", norm::rmsnorm_gated_bwd<T, W, 8><<<grid, norm::kThreads, smem, s>>>(
-            d, a->x, a->z, a->weight, a->dout, a->rstd, a->dx, a->dz, part));
-    } else {
-        BISSD_ALLOW((norm::rmsnorm_gated_bwd<T, W, 16>), smem);
-        BISSD_LAUNCH("rmsnorm_gated_bwd", norm::rmsnorm_gated_bwd<T, W, 16><<<grid, norm::kThreads, smem, s>>>(
-            d, a->x, a->z, a->weight, a->dout, a->rstd, a->dx, a->dz, part));
-    }
-    BISSD_LAUNCH("norm_bwd_reduce", norm::norm_bwd_reduce<W><<<(d.hidden + 255) / 256, norm::kThreads, 0, s>>>(
-        part, grid, d.hidden, a->dweight));
-    return BISSD_OK;
-}
-#define BISSD_NORM_DISPATCH(fn, ...)                                                                \
-    do {                                                                                            \
-        const bool wf = a->w_dtype == BISSD_F32;                                                    \
-        switch (a->x_dtype) {                                                                       \
-            case BISSD_F32: return fn<float, float>(__VA_ARGS__);                                   \
-            case BISSD_BF16: return wf ? fn<__nv_bfloat16, float>(__VA_ARGS__) : fn<__nv_bfloat16, __nv_bfloat16>(__VA_ARGS__); \
-            default: return wf ? fn<__half, float>(__VA_ARGS__) : fn<__half, __half>(__VA_ARGS__); \
-        }                                                                                           \
-    } while (0)
-
-
-// ---- depthwise conv1d + SiLU -----------------------------------------------------------------------------------
-static int conv_check(const bissd_conv_args *a, conv::ConvDims *d, bool backward) {
-    if (!a || !a->x || !a->weight) return BISSD_ERR_NULL;
-    if (!backward && !a->out) return BISSD_ERR_NULL;
-    if (backward && (!a->dout || !a->dx || !a->dweight || (a->bias && !a->dbias))) return BISSD_ERR_NULL;
-    if (a->batch <= 0 || a->seqlen <= 0 || a->channels <= 0 || a->channels % 8 != 0) return BISSD_ERR_SHAPE;
-    if (a->width <= 0 || a->width > conv::kMaxK || a->width % 2 == 0) return BISSD_ERR_SHAPE;
-    if (a->x_dtype < BISSD_F32 || a->x_dtype > BISSD_F16) return BISSD_ERR_DTYPE;
-    if (a->w_dtype != BISSD_F32 && a->w_dtype != a->x_dtype) return BISSD_ERR_DTYPE;
-    auto al = [](const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-    if (!al(a->x) || !al(a->out) || !al(a->dout) || !al(a->dx) || !al(a->bias)) return BISSD_ERR_ALIGN;
-    if (a->x_stride_batch % 8 || a->x_stride_row % 8 || a->out_stride_batch % 8 || a->out_stride_row % 8) return BISSD_ERR_ALIGN;
-    d->batch = a->batch; d->seqlen = a->seqlen; d->channels = a->channels; d->width = a->width;
-    d->xsb = a->x_stride_batch; d->xsl = a->x_stride_row; d->osb = a->out_stride_batch; d->osl = a->out_stride_row;
-    d->has_bias = a->bias != nullptr;
-    return BISSD_OK;
-}
-static inline int conv_row_blocks(int seqlen) { return (seqlen + conv::kRows - 1) / conv::kRows; }
-static inline size_t conv_dpre_bytes(const bissd_conv_args *a) {
-    return align256((size_t)a->batch * a->seqlen * a->channels * (a->x_dtype == BISSD_F32 ? 4 : 2));
-}
-template <class T, class W>
-static int conv_forward_impl(const bissd_conv_args *a, const conv::ConvDims &d, cudaStream_t s) {
-    const dim3 grid((d.channels / 8 + 127) / 128, conv_row_blocks(d.seqlen), d.batch);
-    if constexpr (sizeof(T) == 2) {
-#define BISSD_CONV_FWD(K)                                                                                              \
-    do {                                                                                                               \
-        BISSD_LAUNCH("dwconv_win_fwd", conv::dwconv_win<T, W, 0, K><<<grid, 128, 0, s>>>(d, a->x, a->weight, a->bias,  \
-                                                                                         nullptr, a->out, nullptr));   \
-        return BISSD_OK;                                                                                               \
-    } while (0)
-        if (d.width == 7) BISSD_CONV_FWD(7);                     // rolling-window form for the odd widths
-        if (d.width == 5) BISSD_CONV_FWD(5);
-        if (d.width == 3) BISSD_CONV_FWD(3);
-#undef BISSD_CONV_FWD
-    }
-    BISSD_LAUNCH("dwconv_silu_fwd", conv::dwconv_silu_fwd<T, W><<<grid, 128, 0, s>>>(d, a->x, a->weight, a->bias, a->out));
-    return BISSD_OK;
-}
-template <class T, class W>
-static int conv_backward_impl(const bissd_conv_args *a, const conv::ConvDims &d, char *ws, cudaStream_t s) {
-    const dim3 grid((d.channels / 8 + 127) / 128, conv_row_blocks(d.seqlen), d.batch);
-    void *dpre = ws;
-    float *part = reinterpret_cast<float *>(ws + conv_dpre_bytes(a));
-    // dout is required to be contiguous (checked by the caller), so dpre shares its strides
-    bool win = false;
-    const dim3 grid_dw(grid.x, (d.seqlen + conv::kRowsDw - 1) / conv::kRowsDw, grid.z);   // the window form's dw pass
-    if constexpr (sizeof(T) == 2) {
-#define BISSD_CONV_BWD(K)                                                                                              \
-    do {                                                                                                               \
-        win = true;                                                                                                    \
-        BISSD_LAUNCH("dwconv_win_bwd_pre", conv::dwconv_win<T, W, 1, K><<<grid, 128, 0, s>>>(d, a->x, a->weight,       \
-                                                                                             a->bias, a->dout, dpre, nullptr)); \
-        BISSD_LAUNCH("dwconv_win_bwd_dw", conv::dwconv_win<T, W, 2, K><<<grid_dw, 128, 0, s>>>(d, a->x, nullptr, nullptr, \
-                                                                                            dpre, nullptr, part));    \
-        BISSD_LAUNCH("dwconv_win_bwd_dx", conv::dwconv_win<T, W, 3, K><<<grid, 128, 0, s>>>(d, dpre, a->weight,        \
-                                                                                            nullptr, nullptr, a->dx, nullptr)); \
-    } while (0)
-        if (d.width == 7) BISSD_CONV_BWD(7);                     // rolling-window form for the odd widths
-        else if (d.width == 5) BISSD_CONV_BWD(5);
-        else if (d.width == 3) BISSD_CONV_BWD(3);
-#undef BISSD_CONV_BWD
-    }
-    if (!win) {
-        BISSD_LAUNCH("dwconv_silu_bwd_pre", conv::dwconv_silu_bwd_pre<T, W><<<grid, 128, 0, s>>>(
-            d, a->x, a->weight, a->bias, a->dout, dpre));
-        BISSD_LAUNCH("dwconv_silu_bwd_dw", conv::dwconv_silu_bwd_dw<T><<<grid, 128, 0, s>>>(d, a->x, dpre, part));
-        BISSD_LAUNCH("dwconv_silu_bwd_dx", conv::dwconv_silu_bwd_dx<T, W><<<grid, 128, 0, s>>>(d, dpre, a->weight, a->dx));
-    }
-    const int nparts = d.batch * (win ? (int)grid_dw.y : conv_row_blocks(d.seqlen));
-    const long long n = (long long)d.channels * (conv::kMaxK + 1);
-    BISSD_LAUNCH("conv_bwd_reduce", conv::conv_bwd_reduce<W><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-        part, nparts, d.channels, d.width, a->dweight, a->dbias));
-    return BISSD_OK;
-}
 
 extern "C" {
 
@@ -1197,103 +931,6 @@ int bissd_selftest_gemm(int dtype, int a_mn_major, int b_mn_major, int n, int k,
     else BISSD_SELFTEST_T(__half);
 #undef BISSD_SELFTEST_T
 #undef BISSD_SELFTEST
-    return BISSD_OK;
-}
-
-int bissd_rmsnorm_gated_workspace_bytes(const bissd_norm_args *a, size_t *bwd_bytes) {
-    norm::NormDims d;
-    if (!bwd_bytes) return BISSD_ERR_NULL;
-    if (!a || a->rows <= 0 || a->hidden <= 0) return BISSD_ERR_SHAPE;
-    d.rows = a->rows;
-    *bwd_bytes = (size_t)norm_grid(d) * a->hidden * sizeof(float);
-    return BISSD_OK;
-}
-
-int bissd_rmsnorm_gated_forward(const bissd_norm_args *a, void *stream) {
-    norm::NormDims d;
-    int rc = norm_check(a, &d, false);
-    if (rc != BISSD_OK) return rc;
-    rc = check_device();
-    if (rc != BISSD_OK) return rc;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    BISSD_NORM_DISPATCH(norm_forward_impl, a, d, s);
-}
-
-int bissd_rmsnorm_gated_backward(const bissd_norm_args *a, void *workspace, size_t workspace_bytes, void *stream) {
-    norm::NormDims d;
-    int rc = norm_check(a, &d, true);
-    if (rc != BISSD_OK) return rc;
-    if (!workspace) return BISSD_ERR_NULL;
-    size_t need = 0;
-    bissd_rmsnorm_gated_workspace_bytes(a, &need);
-    if (workspace_bytes < need) return BISSD_ERR_WORKSPACE;
-    rc = check_device();
-    if (rc != BISSD_OK) return rc;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    float *part = static_cast<float *>(workspace);
-    BISSD_NORM_DISPATCH(norm_backward_impl, a, d, part, s);
-}
-
-int bissd_dwconv_silu_workspace_bytes(const bissd_conv_args *a, size_t *bwd_bytes) {
-    if (!a || !bwd_bytes) return BISSD_ERR_NULL;
-    if (a->batch <= 0 || a->seqlen <= 0 || a->channels <= 0) return BISSD_ERR_SHAPE;
-    *bwd_bytes = conv_dpre_bytes(a) +
-                 (size_t)a->batch * conv_row_blocks(a->seqlen) * a->channels * (conv::kMaxK + 1) * sizeof(float);
-    return BISSD_OK;
-}
-
-int bissd_dwconv_silu_forward(const bissd_conv_args *a, void *stream) {
-    conv::ConvDims d;
-    int rc = conv_check(a, &d, false);
-    if (rc != BISSD_OK) return rc;
-    rc = check_device();
-    if (rc != BISSD_OK) return rc;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    BISSD_NORM_DISPATCH(conv_forward_impl, a, d, s);
-}
-
-int bissd_dwconv_silu_backward(const bissd_conv_args *a, void *workspace, size_t workspace_bytes, void *stream) {
-    conv::ConvDims d;
-    int rc = conv_check(a, &d, true);
-    if (rc != BISSD_OK) return rc;
-    if (!workspace) return BISSD_ERR_NULL;
-    size_t need = 0;
-    bissd_dwconv_silu_workspace_bytes(a, &need);
-    if (workspace_bytes < need) return BISSD_ERR_WORKSPACE;
-    if (a->out_stride_row != a->channels || a->out_stride_batch != (int64_t)a->seqlen * a->channels)
-        return BISSD_ERR_ALIGN;                                  // dout (and the dpre scratch) as contiguous rows
-    rc = check_device();
-    if (rc != BISSD_OK) return rc;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    BISSD_NORM_DISPATCH(conv_backward_impl, a, d, static_cast<char *>(workspace), s);
-}
-
-static int layer_params_check(const bissd_layer_params *a, bool out) {
-    if (!a || !a->A32 || (!out && !a->A) || (out && (!a->dA || !a->dA32))) return BISSD_ERR_NULL;
-    if (a->nheads <= 0 || a->d_elems < 0) return BISSD_ERR_SHAPE;
-    for (int t : {a->a_dtype, a->d_dtype, a->b_dtype})
-        if (t < BISSD_F32 || t > BISSD_F16) return BISSD_ERR_DTYPE;
-    if ((a->D && !a->D32) || (a->dt_bias && !a->dt_bias32)) return BISSD_ERR_NULL;
-    return check_device();
-}
-
-int bissd_layer_params_in(const bissd_layer_params *a, void *stream) {
-    const int rc = layer_params_check(a, false);
-    if (rc != BISSD_OK) return rc;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    BISSD_LAUNCH("layer_params_in", layer::params_in<<<ceil_div(std::max(a->nheads, a->d_elems), 256), 256, 0, s>>>(
-        a->nheads, a->d_elems, a->A, a->a_dtype, a->a_log, a->D, a->d_dtype, a->dt_bias, a->b_dtype, a->A32, a->D32, a->dt_bias32));
-    return BISSD_OK;
-}
-
-int bissd_layer_params_out(const bissd_layer_params *a, void *stream) {
-    const int rc = layer_params_check(a, true);
-    if (rc != BISSD_OK) return rc;
-    if ((a->dD && !a->dD32) || (a->ddt_bias && !a->ddt_bias32)) return BISSD_ERR_NULL;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    BISSD_LAUNCH("layer_params_out", launch_pdl(layer::params_out, ceil_div(std::max(a->nheads, a->d_elems), 256), 256, 0, s,
-        a->nheads, a->d_elems, a->A32, a->dA32, a->dD32, a->ddt_bias32, a->a_log, a->dA, a->a_dtype, a->dD, a->d_dtype,
-        a->ddt_bias, a->b_dtype));
     return BISSD_OK;
 }
 

@@ -225,9 +225,8 @@ int bissd_rmsnorm_gated_backward(const bissd_norm_args *args, void *workspace, s
  *     out[b,l,c] = silu(bias[c] + sum_k weight[c,k] x[b, l + k - width/2, c]),   zero outside 0 <= l < seqlen.
  * x, dx: (batch, seqlen, channels) with channel stride 1 and the given batch / row strides (elements, multiples of 8);
  * out, dout: the same shape, contiguous rows of `channels`; weight, dweight: (channels, width) contiguous, bias /
- * dbias: (channels) or NULL; w_dtype fp32 or x's dtype.  channels % 8 == 0, width odd and <= 8, 16-byte aligned
- * pointers.  The backward needs bissd_dwconv_silu_workspace_bytes() of scratch (dpre and the partial weight
- * gradients). */
+ * dbias: (channels) or NULL; w_dtype fp32 or x's dtype.  channels % 8 == 0, width odd and <= 7, 16-byte aligned
+ * pointers.  The backward needs bissd_dwconv_silu_workspace_bytes() of scratch (the partial weight gradients). */
 typedef struct bissd_conv_args {
     int32_t batch, seqlen, channels, width;
     int32_t x_dtype, w_dtype;            /* bissd_dtype */
