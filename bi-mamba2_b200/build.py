@@ -18,7 +18,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "ssd", "_lib")
 OUT = os.path.join(OUT_DIR, "libbissd.so")
-SOURCES = ["bissd_api.cu", "bissd_layer.cu"]
+SOURCES = ["bissd_api.cu", "bissd_layer.cu", "bissd_simt.cu"]
 TORCH_SRC = os.path.join(CSRC, "torch_ops.cpp")
 TORCH_OUT = os.path.join(OUT_DIR, "_bissd_torch.so")
 

@@ -9,6 +9,7 @@
 
 #include "common.cuh"
 #include "host.cuh"
+#include "layouts.cuh"
 #include "simt_kernels.cuh"
 #include "tc_intra.cuh"
 #include "tc_intra_sums.cuh"
@@ -111,68 +112,6 @@ static int make_dims(const bissd_problem &p, Dims *d) {
     return BISSD_OK;
 }
 
-// Workspace carving.  The first 256 bytes hold the device status word (nonzero = a bounded device-side wait ran
-// out); everything after it is fp32 scratch.
-constexpr size_t kWsHeader = 256;
-struct FwdWs {
-    size_t loc, cb, cb16, total;
-};
-struct BwdWs {
-    size_t cb, cbt, cbt16, cb16, cbs, gloc, E, E16, g, dTpart, ddt_out, nf, nb, pf, pb, da_f, da_b, u4, dB_part, dC_part, dCB, dDpart, dApart, dbiaspart, total;
-    int nblk, nlt, nsplit;
-};
-
-static FwdWs fwd_layout(const Dims &d) {
-    FwdWs w;
-    size_t o = kWsHeader;
-    const size_t st = (size_t)d.b * d.nc * d.H * d.P * d.N;
-    w.loc = o; o = align256(o + 2 * st * 4);
-    w.cb = o; o = align256(o + (size_t)d.b * d.nc * d.G * d.Q * d.Q * 4);
-    w.cb16 = o; o = align256(o + (size_t)d.b * d.nc * d.G * d.Q * d.Q * 2);      // C.B^T rounded to bf16 (TMA-fed scan)
-    w.total = o;
-    return w;
-}
-
-// tc: sized for the tensor-core family (16-bit inputs that meet its alignment rules): the passed state gradients are
-// kept in the input dtype only, and the "states" parts of dB / dC arrive summed over the heads of a group.  The
-// CUDA-core family needs the fp32 copy and one partial per head.
-static BwdWs bwd_layout(const Dims &d, bool tc) {
-    BwdWs w;
-    size_t o = kWsHeader;
-    const size_t st = (size_t)d.b * d.nc * d.H * d.P * d.N;
-    const size_t hq = (size_t)d.b * d.H * d.nc * d.Q;
-    w.nblk = ceil_div(d.P * d.N, simt::TB);
-    w.nlt = ceil_div(d.Q, simt::TILE);
-    w.nsplit = ceil_div(d.N, 128);
-    auto take = [&](size_t bytes) { size_t at = o; o = align256(o + bytes); return at; };
-    w.cb = take((size_t)d.b * d.nc * d.G * d.Q * d.Q * 4);
-    w.gloc = take(2 * st * 4);
-    w.E = take(tc ? 0 : 2 * st * 4);                                 // fp32 passed state gradients (CUDA-core family)
-    w.E16 = take(2 * st * 2);                                        // passed state gradients in the input dtype
-    w.g = take((size_t)d.b * d.L * d.H * d.P * 2);                   // gated output gradient dout * silu(z)
-    w.cbt = take((size_t)d.b * d.nc * d.G * d.Q * d.Q * 4);          // CB transposed
-    w.cbs = take((size_t)d.b * d.nc * d.G * d.Q * d.Q * 4);          // CB in strips of 16 columns (tc::intra_sums)
-    w.cbt16 = take((size_t)d.b * d.nc * d.G * d.Q * d.Q * 2);        // CB transposed, rounded to bf16 (TMA-fed dx)
-    w.cb16 = take((size_t)d.b * d.nc * d.G * d.Q * d.Q * 2);         // CB rounded to bf16 (tc::intra_dcb_tile)
-    w.dTpart = take((size_t)2 * d.b * d.H * d.nc * w.nblk * 4);
-    w.ddt_out = take(hq * 4);
-    w.nf = take(hq * 4 * w.nsplit); w.nb = take(hq * 4 * w.nsplit);
-    w.pf = take(hq * 4 * w.nsplit); w.pb = take(hq * 4 * w.nsplit);
-    w.da_f = take(hq * 4); w.da_b = take(hq * 4);
-    w.u4 = take(8 * hq * 4);                                         // u_f / u_b per tile (tc::intra_sums: 2 row tiles; tc::intra_dcb_tile: 4)
-    w.dB_part = take((size_t)d.b * d.nc * d.Q * (tc ? d.G : d.H) * d.N * 4);
-    w.dC_part = take((size_t)d.b * d.nc * d.Q * (tc ? d.G : d.H) * d.N * 4);
-    w.dCB = take((size_t)d.b * d.nc * d.G * d.Q * d.Q * 4);
-    w.dDpart = take((size_t)d.b * d.nc * d.H * std::max(w.nlt, 8) * d.P * 4);   // up to 8 partial rows per (b,c,h)
-    w.dApart = take((size_t)d.b * d.nc * d.H * 4);
-    w.dbiaspart = take((size_t)d.b * d.nc * d.H * 4);
-    w.total = o;
-    return w;
-}
-
-static View view_of(const bissd_tensor &t) { return View{t.ptr, t.stride_batch, t.stride_seq, t.stride_head}; }
-static MutView mview_of(const bissd_tensor &t) { return MutView{t.ptr, t.stride_batch, t.stride_seq, t.stride_head}; }
-
 // ---- which kernel family ---------------------------------------------------------------------------------
 static bool tc_shape_ok(const bissd_problem &p) {
     return (p.x_dtype == BISSD_BF16 || p.x_dtype == BISSD_F16) && p.headdim % 8 == 0 && p.dstate % 8 == 0 &&
@@ -217,13 +156,8 @@ static bool map_bshd(CUtensorMap *m, int dtype, const void *ptr, long long sb, l
     return tc::make_map4(m, dtype, ptr, dims, str, box);
 }
 
-template <class T> struct TcKernels {   // 16-bit types only; the fp32 specialisation below never launches them
-    static constexpr bool available = true;
-};
-template <> struct TcKernels<float> { static constexpr bool available = false; };
-
 template <class T>
-static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaStream_t s, bool tcp) {
+static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaStream_t s) {
     const FwdWs w = fwd_layout(d);
     int *status = reinterpret_cast<int *>(ws);
     float *loc = reinterpret_cast<float *>(ws + w.loc);
@@ -237,170 +171,147 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
         BISSD_LAUNCH("cumsum_fwd", launch_pdl(simt::cumsum_fwd, d.b * d.nc * d.H, 256, 0, s, 
             d, a.dt.ptr, a.p.dt_dtype, a.dt.stride_batch, a.dt.stride_seq, a.dt.stride_head, a.A, a.dt_bias, a.dt_out,
             a.cs_f, a.cs_b));
-        if constexpr (TcKernels<T>::available) {
-            if (tcp) {
-                const size_t smem = tc::smem_bytes(ntP, 2 * d.Q);
-                bool st_done = false;
-                if (!no_tma() && (tc::state_tma_ok(d.P, d.N, d.Q) || (!no_ws() && tc::state_grp_ok(d.P, d.N, d.Q, d.R)))) {
-                    CUtensorMap mRow, mCol;
-                    if (map_bshd(&mRow, a.p.x_dtype, a.B.ptr, a.B.stride_batch, a.B.stride_seq, a.B.stride_head, d.N, d.G, d.L, d.b, d.Q) &&
-                        map_bshd(&mCol, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, d.Q)) {
-                        if (!no_ws() && tc::state_grp_ok(d.P, d.N, d.Q, d.R)) {
-                            const size_t smem_g = tc::state_grp_smem(d.Q);
-                            const int ks = tc::state_grp_ksplit(d.b * d.nc * d.G * ceil_div(d.N, 128), d.R, sm_count());
-                            BISSD_ALLOW((tc::state_gemm_grp<T, 0>), smem_g);
-                            BISSD_LAUNCH("tc_chunk_state_grp", launch_pdl(tc::state_gemm_grp<T, 0>, dim3(d.b * d.nc * d.G * ks, ceil_div(d.N, 128)), tc::kStateGrpThreads, smem_g, s, 
-                                d, mRow, mCol, ks, a.dt_out, a.cs_f, a.cs_b, loc, status));
-                        } else {
-                            const size_t smem_t = tc::state_tma_smem(d.P, d.Q);
-                            BISSD_ALLOW((tc::state_gemm_tma<T, 0>), smem_t);
-                            BISSD_LAUNCH("tc_chunk_state_tma", tc::state_gemm_tma<T, 0><<<dim3(bch, 2, d.N / 128), tc::kThreads, smem_t, s>>>(
-                                d, mRow, mCol, a.dt_out, a.cs_f, a.cs_b, loc, status));
-                        }
-                        st_done = true;
+        {
+            const size_t smem = tc::smem_bytes(ntP, 2 * d.Q);
+            bool st_done = false;
+            if (!no_tma() && (tc::state_tma_ok(d.P, d.N, d.Q) || (!no_ws() && tc::state_grp_ok(d.P, d.N, d.Q, d.R)))) {
+                CUtensorMap mRow, mCol;
+                if (map_bshd(&mRow, a.p.x_dtype, a.B.ptr, a.B.stride_batch, a.B.stride_seq, a.B.stride_head, d.N, d.G, d.L, d.b, d.Q) &&
+                    map_bshd(&mCol, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, d.Q)) {
+                    if (!no_ws() && tc::state_grp_ok(d.P, d.N, d.Q, d.R)) {
+                        const size_t smem_g = tc::state_grp_smem(d.Q);
+                        const int ks = tc::state_grp_ksplit(d.b * d.nc * d.G * ceil_div(d.N, 128), d.R, sm_count());
+                        BISSD_ALLOW((tc::state_gemm_grp<T, 0>), smem_g);
+                        BISSD_LAUNCH("tc_chunk_state_grp", launch_pdl(tc::state_gemm_grp<T, 0>, dim3(d.b * d.nc * d.G * ks, ceil_div(d.N, 128)), tc::kStateGrpThreads, smem_g, s, 
+                            d, mRow, mCol, ks, a.dt_out, a.cs_f, a.cs_b, loc, status));
+                    } else {
+                        const size_t smem_t = tc::state_tma_smem(d.P, d.Q);
+                        BISSD_ALLOW((tc::state_gemm_tma<T, 0>), smem_t);
+                        BISSD_LAUNCH("tc_chunk_state_tma", tc::state_gemm_tma<T, 0><<<dim3(bch, 2, d.N / 128), tc::kThreads, smem_t, s>>>(
+                            d, mRow, mCol, a.dt_out, a.cs_f, a.cs_b, loc, status));
                     }
-                }
-                if (st_done) {
-                } else if (ntP <= 64) {
-                    BISSD_ALLOW((tc::state_gemm<T, 0, 2>), smem);
-                    BISSD_LAUNCH("tc_chunk_state", tc::state_gemm<T, 0, 2><<<dim3(bch, ceil_div(2 * d.N, tc::kTileM)), tc::kThreads, smem, s>>>(
-                        d, Bm, x, z, a.dt_out, a.cs_f, a.cs_b, loc, status));
-                } else {
-                    BISSD_ALLOW((tc::state_gemm<T, 0, 8>), smem);
-                    BISSD_LAUNCH("tc_chunk_state", tc::state_gemm<T, 0, 8><<<dim3(bch, ceil_div(2 * d.N, tc::kTileM)), tc::kThreads, smem, s>>>(
-                        d, Bm, x, z, a.dt_out, a.cs_f, a.cs_b, loc, status));
+                    st_done = true;
                 }
             }
-        }
-        if (!tcp) {
-            BISSD_LAUNCH("chunk_state", simt::chunk_state<T><<<dim3(bch, ceil_div(d.P, simt::TILE), ceil_div(2 * d.N, simt::TILE)), simt::TB, 2 * d.Q * sizeof(float), s>>>(
-                d, x, Bm, a.dt_out, a.cs_f, a.cs_b, loc));
+            if (st_done) {
+            } else if (ntP <= 64) {
+                BISSD_ALLOW((tc::state_gemm<T, 0, 2>), smem);
+                BISSD_LAUNCH("tc_chunk_state", tc::state_gemm<T, 0, 2><<<dim3(bch, ceil_div(2 * d.N, tc::kTileM)), tc::kThreads, smem, s>>>(
+                    d, Bm, x, z, a.dt_out, a.cs_f, a.cs_b, loc, status));
+            } else {
+                BISSD_ALLOW((tc::state_gemm<T, 0, 8>), smem);
+                BISSD_LAUNCH("tc_chunk_state", tc::state_gemm<T, 0, 8><<<dim3(bch, ceil_div(2 * d.N, tc::kTileM)), tc::kThreads, smem, s>>>(
+                    d, Bm, x, z, a.dt_out, a.cs_f, a.cs_b, loc, status));
+            }
         }
     }
     // the recurrence runs in both phases: from zero (or init_*) in LOCAL, again with init_* in FINISH
     const bool need_pass = (a.phases & BISSD_PHASE_LOCAL) || (a.init_f || a.init_b);
     if (need_pass) {
-        if ((d.P * d.N) % 4 == 0) {
-            BISSD_LAUNCH("state_passing_fwd", launch_pdl(simt::state_passing_fwd4<T>, dim3(d.b * d.H, ceil_div(d.P * d.N, 4 * simt::TB), 2), simt::TB, 0, s, 
-                d, loc, a.cs_f, a.cs_b, a.init_f, a.init_b, a.states_f, a.states_b, a.final_f, a.final_b));
-        } else {
-            BISSD_LAUNCH("state_passing_fwd", simt::state_passing_fwd<T><<<dim3(d.b * d.H, ceil_div(d.P * d.N, simt::TB), 2), simt::TB, 0, s>>>(
-                d, loc, a.cs_f, a.cs_b, a.init_f, a.init_b, a.states_f, a.states_b, a.final_f, a.final_b));
-        }
+        BISSD_LAUNCH("state_passing_fwd", launch_pdl(simt::state_passing_fwd4<T>, dim3(d.b * d.H, ceil_div(d.P * d.N, 4 * simt::TB), 2), simt::TB, 0, s,
+            d, loc, a.cs_f, a.cs_b, a.init_f, a.init_b, a.states_f, a.states_b, a.final_f, a.final_b));
     }
     if (a.phases & BISSD_PHASE_FINISH) {
-        if constexpr (TcKernels<T>::available) {
-            if (tcp) {
-                const size_t smem_cb = tc::smem_bytes(ntQ, 0), smem_sc = tc::smem_bytes(ntP, 3 * d.Q);
-                BISSD_ALLOW(tc::bmm_cb<T>, smem_cb);
-                const bool ws_path = !no_tma() && !no_ws() && tc::scan_ws_ok(d.P, d.N, d.Q);
-                __nv_bfloat16 *CB16 = reinterpret_cast<__nv_bfloat16 *>(ws + w.cb16);
-                CUtensorMap mCc, mBc;
-                if (ws_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc)) {
-                    const size_t smem_ct = tc::bmm_cb_tma_smem(d.N);
-                    BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
-                    BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s, 
-                        d, mCc, mBc, CB16, nullptr, nullptr, status));
-                } else
-                BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_cb, s>>>(
-                    d, Cm, Bm, ws_path ? nullptr : CB, nullptr, ws_path ? CB16 : nullptr, nullptr, nullptr, status));
-                bool tma_done = false;
-                if (ws_path) {
-                    CUtensorMap mC, mCB, mSf, mSb, mX, mR;
-                    const unsigned long long dC[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
-                    const unsigned long long sC[3] = {(unsigned long long)a.C.stride_head * 2, (unsigned long long)a.C.stride_seq * 2, (unsigned long long)a.C.stride_batch * 2};
-                    const unsigned bC[4] = {64, 1, 128, 1};
-                    const unsigned long long rows = (unsigned long long)d.b * d.nc * d.H * d.P;
-                    bool maps = tc::make_map4(&mC, a.p.x_dtype, a.C.ptr, dC, sC, bC) &&
-                                map_bshd(&mX, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, 64) &&
-                                tc::make_map2(&mCB, BISSD_BF16, CB16, d.Q, (unsigned long long)d.b * d.nc * d.G * d.Q, 64, 128) &&
-                                tc::make_map2(&mSf, a.p.x_dtype, a.states_f, d.N, rows, 64, d.P) &&
-                                tc::make_map2(&mSb, a.p.x_dtype, a.states_b, d.N, rows, 64, d.P);
-                    // the epilogue's z rows by TMA (a [128 rows x 64] tile per step); without z the map is not used
-                    const bool z_rows = maps && d.has_z &&
-                                        map_bshd(&mR, a.p.x_dtype, a.z.ptr, a.z.stride_batch, a.z.stride_seq, a.z.stride_head, d.P, d.H, d.L, d.b, 128);
-                    if (maps && !z_rows) mR = mX;
-                    if (maps) {
-                        const size_t smem_t = tc::scan_ws_smem(d.P, d.N, d.Q);
-                        const int tiles = bch * (d.Q / tc::kTileM);
-                        const int grid = std::min(sm_count(), tiles);
-                        auto wide = [](const bissd_tensor &t) {   // 32-byte accesses allowed on every row piece
-                            return t.ptr && reinterpret_cast<uintptr_t>(t.ptr) % 32 == 0 && t.stride_batch % 16 == 0 &&
-                                   t.stride_seq % 16 == 0 && t.stride_head % 16 == 0;
-                        };
-                        const int wide_z = d.has_z && wide(a.z);
-                        const int wide_o = wide(a.out) && (!d.has_z || wide(a.out_x));
-                        tc::WsArgs wa{};
-                        wa.x = x; wa.z = z; wa.D = a.D; wa.dt_out = a.dt_out; wa.cs_f = a.cs_f; wa.cs_b = a.cs_b;
-                        wa.out = mview_of(a.out); wa.out_x = mview_of(a.out_x);
-                        wa.wide_z = wide_z; wa.wide_o = wide_o;
-                        wa.rows_by_tma = z_rows ? 1 : 0;
+        {
+            const size_t smem_cb = tc::smem_bytes(ntQ, 0), smem_sc = tc::smem_bytes(ntP, 3 * d.Q);
+            BISSD_ALLOW(tc::bmm_cb<T>, smem_cb);
+            const bool ws_path = !no_tma() && !no_ws() && tc::scan_ws_ok(d.P, d.N, d.Q);
+            __nv_bfloat16 *CB16 = reinterpret_cast<__nv_bfloat16 *>(ws + w.cb16);
+            CUtensorMap mCc, mBc;
+            if (ws_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc)) {
+                const size_t smem_ct = tc::bmm_cb_tma_smem(d.N);
+                BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
+                BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s, 
+                    d, mCc, mBc, CB16, nullptr, nullptr, status));
+            } else
+            BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_cb, s>>>(
+                d, Cm, Bm, ws_path ? nullptr : CB, nullptr, ws_path ? CB16 : nullptr, nullptr, nullptr, status));
+            bool tma_done = false;
+            if (ws_path) {
+                CUtensorMap mC, mCB, mSf, mSb, mX, mR;
+                const unsigned long long dC[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
+                const unsigned long long sC[3] = {(unsigned long long)a.C.stride_head * 2, (unsigned long long)a.C.stride_seq * 2, (unsigned long long)a.C.stride_batch * 2};
+                const unsigned bC[4] = {64, 1, 128, 1};
+                const unsigned long long rows = (unsigned long long)d.b * d.nc * d.H * d.P;
+                bool maps = tc::make_map4(&mC, a.p.x_dtype, a.C.ptr, dC, sC, bC) &&
+                            map_bshd(&mX, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, 64) &&
+                            tc::make_map2(&mCB, BISSD_BF16, CB16, d.Q, (unsigned long long)d.b * d.nc * d.G * d.Q, 64, 128) &&
+                            tc::make_map2(&mSf, a.p.x_dtype, a.states_f, d.N, rows, 64, d.P) &&
+                            tc::make_map2(&mSb, a.p.x_dtype, a.states_b, d.N, rows, 64, d.P);
+                // the epilogue's z rows by TMA (a [128 rows x 64] tile per step); without z the map is not used
+                const bool z_rows = maps && d.has_z &&
+                                    map_bshd(&mR, a.p.x_dtype, a.z.ptr, a.z.stride_batch, a.z.stride_seq, a.z.stride_head, d.P, d.H, d.L, d.b, 128);
+                if (maps && !z_rows) mR = mX;
+                if (maps) {
+                    const size_t smem_t = tc::scan_ws_smem(d.P, d.N, d.Q);
+                    const int tiles = bch * (d.Q / tc::kTileM);
+                    const int grid = std::min(sm_count(), tiles);
+                    auto wide = [](const bissd_tensor &t) {   // 32-byte accesses allowed on every row piece
+                        return t.ptr && reinterpret_cast<uintptr_t>(t.ptr) % 32 == 0 && t.stride_batch % 16 == 0 &&
+                               t.stride_seq % 16 == 0 && t.stride_head % 16 == 0;
+                    };
+                    const int wide_z = d.has_z && wide(a.z);
+                    const int wide_o = wide(a.out) && (!d.has_z || wide(a.out_x));
+                    tc::WsArgs wa{};
+                    wa.x = x; wa.z = z; wa.D = a.D; wa.dt_out = a.dt_out; wa.cs_f = a.cs_f; wa.cs_b = a.cs_b;
+                    wa.out = mview_of(a.out); wa.out_x = mview_of(a.out_x);
+                    wa.wide_z = wide_z; wa.wide_o = wide_o;
+                    wa.rows_by_tma = z_rows ? 1 : 0;
 #define BISSD_SCAN_WS(NSL, NS)                                                                                          \
-    do {                                                                                                                \
-        BISSD_ALLOW((tc::ws_kernel<T, NSL, NS, 0>), smem_t);                                                            \
-        BISSD_LAUNCH("tc_chunk_scan_ws", launch_pdl(tc::ws_kernel<T, NSL, NS, 0>, grid, tc::kWsThreads, smem_t, s,              \
-            d, mC, mCB, mSf, mSb, mX, mR, wa, status));                                                                 \
-    } while (0)
-                        if (d.N == 128 && d.Q == 256) BISSD_SCAN_WS(2, 4);
-                        else if (d.N == 64 && d.Q == 256) BISSD_SCAN_WS(1, 4);
-                        else if (d.N == 128 && d.Q == 128) BISSD_SCAN_WS(2, 2);
-                        else BISSD_SCAN_WS(1, 2);
+do {                                                                                                                \
+    BISSD_ALLOW((tc::ws_kernel<T, NSL, NS, 0>), smem_t);                                                            \
+    BISSD_LAUNCH("tc_chunk_scan_ws", launch_pdl(tc::ws_kernel<T, NSL, NS, 0>, grid, tc::kWsThreads, smem_t, s,              \
+        d, mC, mCB, mSf, mSb, mX, mR, wa, status));                                                                 \
+} while (0)
+                    if (d.N == 128 && d.Q == 256) BISSD_SCAN_WS(2, 4);
+                    else if (d.N == 64 && d.Q == 256) BISSD_SCAN_WS(1, 4);
+                    else if (d.N == 128 && d.Q == 128) BISSD_SCAN_WS(2, 2);
+                    else BISSD_SCAN_WS(1, 2);
 #undef BISSD_SCAN_WS
-                        tma_done = true;
-                    } else {                                     // maps refused: produce the fp32 tile after all
-                        BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_cb, s>>>(
-                            d, Cm, Bm, CB, nullptr, nullptr, nullptr, nullptr, status));
-                    }
-                }
-                if (!tma_done && !no_tma() && tc::scan_tma_ok(d.P, d.N, d.Q)) {
-                    CUtensorMap mC, mSf, mSb, mX;
-                    const unsigned long long dC[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
-                    const unsigned long long sC[3] = {(unsigned long long)a.C.stride_head * 2, (unsigned long long)a.C.stride_seq * 2, (unsigned long long)a.C.stride_batch * 2};
-                    const unsigned bC[4] = {64, 1, 128, 1};
-                    const unsigned long long dX[4] = {(unsigned long long)d.P, (unsigned long long)d.H, (unsigned long long)d.L, (unsigned long long)d.b};
-                    const unsigned long long sX[3] = {(unsigned long long)a.x.stride_head * 2, (unsigned long long)a.x.stride_seq * 2, (unsigned long long)a.x.stride_batch * 2};
-                    const unsigned bX[4] = {64, 1, (unsigned)d.Q, 1};
-                    const unsigned long long rows = (unsigned long long)d.b * d.nc * d.H * d.P;
-                    if (tc::make_map4(&mC, a.p.x_dtype, a.C.ptr, dC, sC, bC) && tc::make_map4(&mX, a.p.x_dtype, a.x.ptr, dX, sX, bX) &&
-                        tc::make_map2(&mSf, a.p.x_dtype, a.states_f, d.N, rows, 64, d.P) &&
-                        tc::make_map2(&mSb, a.p.x_dtype, a.states_b, d.N, rows, 64, d.P)) {
-                        const int rounds = tc::scan_tma_rounds(d.P, d.N, d.Q);
-                        const size_t smem_t = tc::scan_tma_smem(d.P, d.N, d.Q, rounds);
-                        BISSD_ALLOW(tc::chunk_scan_tma<T>, smem_t);
-                        BISSD_LAUNCH("tc_chunk_scan_tma", tc::chunk_scan_tma<T><<<dim3(bch, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_t, s>>>(
-                            d, mC, mSf, mSb, mX, x, z, a.D, a.dt_out, a.cs_f, a.cs_b, CB, mview_of(a.out), mview_of(a.out_x), rounds, status));
-                        tma_done = true;
-                    }
-                }
-                if (tma_done) {
-                } else if (ntP <= 64) {
-                    BISSD_ALLOW((tc::chunk_scan<T, 2>), smem_sc);
-                    BISSD_LAUNCH("tc_chunk_scan", tc::chunk_scan<T, 2><<<dim3(bch, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_sc, s>>>(
-                        d, x, Cm, z, a.D, a.dt_out, a.cs_f, a.cs_b, CB, a.states_f, a.states_b, mview_of(a.out), mview_of(a.out_x), status));
-                } else {
-                    BISSD_ALLOW((tc::chunk_scan<T, 8>), smem_sc);
-                    BISSD_LAUNCH("tc_chunk_scan", tc::chunk_scan<T, 8><<<dim3(bch, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_sc, s>>>(
-                        d, x, Cm, z, a.D, a.dt_out, a.cs_f, a.cs_b, CB, a.states_f, a.states_b, mview_of(a.out), mview_of(a.out_x), status));
+                    tma_done = true;
+                } else {                                     // maps refused: produce the fp32 tile after all
+                    BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_cb, s>>>(
+                        d, Cm, Bm, CB, nullptr, nullptr, nullptr, nullptr, status));
                 }
             }
-        }
-        if (!tcp) {
-            BISSD_LAUNCH("bmm_cb", simt::bmm_cb<T><<<dim3(d.b * d.nc * d.G, ceil_div(d.Q, simt::TILE), ceil_div(d.Q, simt::TILE)), simt::TB, 0, s>>>(d, Cm, Bm, CB));
-            BISSD_LAUNCH("chunk_scan", simt::chunk_scan<T><<<dim3(bch, ceil_div(d.Q, simt::TILE), ceil_div(d.P, simt::TILE)), simt::TB, 3 * d.Q * sizeof(float), s>>>(
-                d, x, Cm, z, a.D, a.dt_out, a.cs_f, a.cs_b, CB, a.states_f, a.states_b, mview_of(a.out), mview_of(a.out_x)));
+            if (!tma_done && !no_tma() && tc::scan_tma_ok(d.P, d.N, d.Q)) {
+                CUtensorMap mC, mSf, mSb, mX;
+                const unsigned long long dC[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
+                const unsigned long long sC[3] = {(unsigned long long)a.C.stride_head * 2, (unsigned long long)a.C.stride_seq * 2, (unsigned long long)a.C.stride_batch * 2};
+                const unsigned bC[4] = {64, 1, 128, 1};
+                const unsigned long long dX[4] = {(unsigned long long)d.P, (unsigned long long)d.H, (unsigned long long)d.L, (unsigned long long)d.b};
+                const unsigned long long sX[3] = {(unsigned long long)a.x.stride_head * 2, (unsigned long long)a.x.stride_seq * 2, (unsigned long long)a.x.stride_batch * 2};
+                const unsigned bX[4] = {64, 1, (unsigned)d.Q, 1};
+                const unsigned long long rows = (unsigned long long)d.b * d.nc * d.H * d.P;
+                if (tc::make_map4(&mC, a.p.x_dtype, a.C.ptr, dC, sC, bC) && tc::make_map4(&mX, a.p.x_dtype, a.x.ptr, dX, sX, bX) &&
+                    tc::make_map2(&mSf, a.p.x_dtype, a.states_f, d.N, rows, 64, d.P) &&
+                    tc::make_map2(&mSb, a.p.x_dtype, a.states_b, d.N, rows, 64, d.P)) {
+                    const int rounds = tc::scan_tma_rounds(d.P, d.N, d.Q);
+                    const size_t smem_t = tc::scan_tma_smem(d.P, d.N, d.Q, rounds);
+                    BISSD_ALLOW(tc::chunk_scan_tma<T>, smem_t);
+                    BISSD_LAUNCH("tc_chunk_scan_tma", tc::chunk_scan_tma<T><<<dim3(bch, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_t, s>>>(
+                        d, mC, mSf, mSb, mX, x, z, a.D, a.dt_out, a.cs_f, a.cs_b, CB, mview_of(a.out), mview_of(a.out_x), rounds, status));
+                    tma_done = true;
+                }
+            }
+            if (tma_done) {
+            } else if (ntP <= 64) {
+                BISSD_ALLOW((tc::chunk_scan<T, 2>), smem_sc);
+                BISSD_LAUNCH("tc_chunk_scan", tc::chunk_scan<T, 2><<<dim3(bch, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_sc, s>>>(
+                    d, x, Cm, z, a.D, a.dt_out, a.cs_f, a.cs_b, CB, a.states_f, a.states_b, mview_of(a.out), mview_of(a.out_x), status));
+            } else {
+                BISSD_ALLOW((tc::chunk_scan<T, 8>), smem_sc);
+                BISSD_LAUNCH("tc_chunk_scan", tc::chunk_scan<T, 8><<<dim3(bch, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_sc, s>>>(
+                    d, x, Cm, z, a.D, a.dt_out, a.cs_f, a.cs_b, CB, a.states_f, a.states_b, mview_of(a.out), mview_of(a.out_x), status));
+            }
         }
     }
     return BISSD_OK;
 }
 
-// Where dx, dB, dC and ddt go (bissd_backward: contiguous, bissd_backward_into: the caller's strides).
-struct GradViews {
-    MutView dx, dB, dC, ddt;
-};
-
 template <class T>
-static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dims &d, char *ws, cudaStream_t s, bool tcp) {
-    const BwdWs w = bwd_layout(d, tcp);
+static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dims &d, char *ws, cudaStream_t s) {
+    const BwdWs w = bwd_layout(d, true);
     int *status = reinterpret_cast<int *>(ws);
     auto F = [&](size_t off) { return reinterpret_cast<float *>(ws + off); };
     const View x = view_of(a.x), Bm = view_of(a.B), Cm = view_of(a.C), z = view_of(a.z), dout = view_of(a.dout),
@@ -414,69 +325,57 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
     Dims dg = d;
     View gv = dout;
     void *E16 = ws + w.E16;
-    if (tcp && d.has_z) {
+    if (d.has_z) {
         dg.has_z = 0;
         gv = View{ws + w.g, (long long)d.L * d.H * d.P, (long long)d.H * d.P, (long long)d.P};
     }
     if (a.phases & BISSD_PHASE_LOCAL) {
         int rc = note_cuda(cudaMemsetAsync(ws, 0, kWsHeader, s), "cudaMemsetAsync");
         if (rc != BISSD_OK) return rc;
-        if constexpr (TcKernels<T>::available) {
-            if (tcp && d.has_z) {
-                const long long chunks = (long long)d.b * d.L * d.H * (d.P / 8);
-                BISSD_LAUNCH("gate_bwd", launch_pdl(tc::gate_bwd<T>, (unsigned)((chunks + 255) / 256), 256, 0, s, 
-                    d, dout, z, out_x, ws + w.g, a.dz));
-            }
-            if (tcp) {
-                const size_t smem = tc::smem_bytes(ntP, 2 * d.Q);
-                bool st_done = false;
-                if (!no_tma() && (tc::state_tma_ok(d.P, d.N, d.Q) || (!no_ws() && tc::state_grp_ok(d.P, d.N, d.Q, d.R)))) {
-                    CUtensorMap mRow, mCol;
-                    if (map_bshd(&mRow, a.p.x_dtype, a.C.ptr, a.C.stride_batch, a.C.stride_seq, a.C.stride_head, d.N, d.G, d.L, d.b, d.Q) &&
-                        map_bshd(&mCol, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, d.Q)) {
-                        if (!no_ws() && tc::state_grp_ok(d.P, d.N, d.Q, d.R)) {
-                            const size_t smem_g = tc::state_grp_smem(d.Q);
-                            const int ks = tc::state_grp_ksplit(d.b * d.nc * d.G * ceil_div(d.N, 128), d.R, sm_count());
-                            BISSD_ALLOW((tc::state_gemm_grp<T, 1>), smem_g);
-                            BISSD_LAUNCH("tc_dstates_grp", launch_pdl(tc::state_gemm_grp<T, 1>, dim3(d.b * d.nc * d.G * ks, ceil_div(d.N, 128)), tc::kStateGrpThreads, smem_g, s, 
-                                d, mRow, mCol, ks, a.dt_out, a.cs_f, a.cs_b, F(w.gloc), status));
-                        } else {
-                            const size_t smem_t = tc::state_tma_smem(d.P, d.Q);
-                            BISSD_ALLOW((tc::state_gemm_tma<T, 1>), smem_t);
-                            BISSD_LAUNCH("tc_dstates_tma", tc::state_gemm_tma<T, 1><<<dim3(bch, 2, d.N / 128), tc::kThreads, smem_t, s>>>(
-                                d, mRow, mCol, a.dt_out, a.cs_f, a.cs_b, F(w.gloc), status));
-                        }
-                        st_done = true;
-                    }
-                }
-                if (st_done) {
-                } else if (ntP <= 64) {
-                    BISSD_ALLOW((tc::state_gemm<T, 1, 2>), smem);
-                    BISSD_LAUNCH("tc_dstates", tc::state_gemm<T, 1, 2><<<dim3(bch, ceil_div(2 * d.N, tc::kTileM)), tc::kThreads, smem, s>>>(
-                        dg, Cm, gv, z, a.dt_out, a.cs_f, a.cs_b, F(w.gloc), status));
-                } else {
-                    BISSD_ALLOW((tc::state_gemm<T, 1, 8>), smem);
-                    BISSD_LAUNCH("tc_dstates", tc::state_gemm<T, 1, 8><<<dim3(bch, ceil_div(2 * d.N, tc::kTileM)), tc::kThreads, smem, s>>>(
-                        dg, Cm, gv, z, a.dt_out, a.cs_f, a.cs_b, F(w.gloc), status));
-                }
-            }
+        if (d.has_z) {
+            const long long chunks = (long long)d.b * d.L * d.H * (d.P / 8);
+            BISSD_LAUNCH("gate_bwd", launch_pdl(tc::gate_bwd<T>, (unsigned)((chunks + 255) / 256), 256, 0, s, 
+                d, dout, z, out_x, ws + w.g, a.dz));
         }
-        if (!tcp) {
-            BISSD_LAUNCH("dstates", simt::dstates<T><<<dim3(bch, ceil_div(d.P, simt::TILE), ceil_div(2 * d.N, simt::TILE)), simt::TB, 2 * d.Q * sizeof(float), s>>>(
-                d, dout, z, Cm, a.cs_f, a.cs_b, F(w.gloc)));
+        {
+            const size_t smem = tc::smem_bytes(ntP, 2 * d.Q);
+            bool st_done = false;
+            if (!no_tma() && (tc::state_tma_ok(d.P, d.N, d.Q) || (!no_ws() && tc::state_grp_ok(d.P, d.N, d.Q, d.R)))) {
+                CUtensorMap mRow, mCol;
+                if (map_bshd(&mRow, a.p.x_dtype, a.C.ptr, a.C.stride_batch, a.C.stride_seq, a.C.stride_head, d.N, d.G, d.L, d.b, d.Q) &&
+                    map_bshd(&mCol, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, d.Q)) {
+                    if (!no_ws() && tc::state_grp_ok(d.P, d.N, d.Q, d.R)) {
+                        const size_t smem_g = tc::state_grp_smem(d.Q);
+                        const int ks = tc::state_grp_ksplit(d.b * d.nc * d.G * ceil_div(d.N, 128), d.R, sm_count());
+                        BISSD_ALLOW((tc::state_gemm_grp<T, 1>), smem_g);
+                        BISSD_LAUNCH("tc_dstates_grp", launch_pdl(tc::state_gemm_grp<T, 1>, dim3(d.b * d.nc * d.G * ks, ceil_div(d.N, 128)), tc::kStateGrpThreads, smem_g, s, 
+                            d, mRow, mCol, ks, a.dt_out, a.cs_f, a.cs_b, F(w.gloc), status));
+                    } else {
+                        const size_t smem_t = tc::state_tma_smem(d.P, d.Q);
+                        BISSD_ALLOW((tc::state_gemm_tma<T, 1>), smem_t);
+                        BISSD_LAUNCH("tc_dstates_tma", tc::state_gemm_tma<T, 1><<<dim3(bch, 2, d.N / 128), tc::kThreads, smem_t, s>>>(
+                            d, mRow, mCol, a.dt_out, a.cs_f, a.cs_b, F(w.gloc), status));
+                    }
+                    st_done = true;
+                }
+            }
+            if (st_done) {
+            } else if (ntP <= 64) {
+                BISSD_ALLOW((tc::state_gemm<T, 1, 2>), smem);
+                BISSD_LAUNCH("tc_dstates", tc::state_gemm<T, 1, 2><<<dim3(bch, ceil_div(2 * d.N, tc::kTileM)), tc::kThreads, smem, s>>>(
+                    dg, Cm, gv, z, a.dt_out, a.cs_f, a.cs_b, F(w.gloc), status));
+            } else {
+                BISSD_ALLOW((tc::state_gemm<T, 1, 8>), smem);
+                BISSD_LAUNCH("tc_dstates", tc::state_gemm<T, 1, 8><<<dim3(bch, ceil_div(2 * d.N, tc::kTileM)), tc::kThreads, smem, s>>>(
+                    dg, Cm, gv, z, a.dt_out, a.cs_f, a.cs_b, F(w.gloc), status));
+            }
         }
     }
     const bool need_pass = (a.phases & BISSD_PHASE_LOCAL) || (a.dfinal_f || a.dfinal_b);
-    int pass_nblk = ((d.P * d.N) % 4 == 0) ? ceil_div(d.P * d.N, 4 * simt::TB) : w.nblk;   // dT partial slots per chunk
+    const int pass_nblk = ceil_div(d.P * d.N, 4 * simt::TB);     // dT partial slots per chunk
     if (need_pass) {
-        if ((d.P * d.N) % 4 == 0) {
-            pass_nblk = ceil_div(d.P * d.N, 4 * simt::TB);
-            BISSD_LAUNCH("state_passing_bwd", launch_pdl(simt::state_passing_bwd4<T>, dim3(d.b * d.H, pass_nblk, 2), simt::TB, 0, s, 
-                d, F(w.gloc), a.states_f, a.states_b, a.cs_f, a.cs_b, a.dfinal_f, a.dfinal_b, tcp ? nullptr : F(w.E), tcp ? E16 : nullptr, F(w.dTpart), a.dinit_f, a.dinit_b));
-        } else {
-            BISSD_LAUNCH("state_passing_bwd", simt::state_passing_bwd<T><<<dim3(d.b * d.H, w.nblk, 2), simt::TB, 0, s>>>(
-                d, F(w.gloc), a.states_f, a.states_b, a.cs_f, a.cs_b, a.dfinal_f, a.dfinal_b, tcp ? nullptr : F(w.E), tcp ? E16 : nullptr, F(w.dTpart), a.dinit_f, a.dinit_b));
-        }
+        BISSD_LAUNCH("state_passing_bwd", launch_pdl(simt::state_passing_bwd4<T>, dim3(d.b * d.H, pass_nblk, 2), simt::TB, 0, s,
+            d, F(w.gloc), a.states_f, a.states_b, a.cs_f, a.cs_b, a.dfinal_f, a.dfinal_b, nullptr, E16, F(w.dTpart), a.dinit_f, a.dinit_b));
     }
     if (!(a.phases & BISSD_PHASE_FINISH)) return BISSD_OK;
     int nlt = w.nlt, nsplit = 1, part_heads = d.H;
@@ -488,300 +387,278 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
     int u4_tiles = 2;                                            // (u_f, u_b) vector pairs per chunk in u4
     int dd_slots = 0;                                            // dD partial rows per (b,c,h) when not nlt
     bool dd_compact = false;                                     // per-head D from the persistent dx kernel: dd_slots scalars, no channel axis
-    if constexpr (TcKernels<T>::available) {
-        if (tcp) {
-            nlt = nlt_tc;
-            nsplit = w.nsplit;
-            part_heads = d.G;
-            const size_t smem_cb = tc::smem_bytes(ntQ, 0), smem_dx = tc::smem_bytes(ntP, 3 * d.Q), smem_n = tc::smem_bytes(ntN, 0);
-            BISSD_ALLOW(tc::bmm_cb<T>, smem_cb);
-            const bool ws_path = !no_tma() && !no_ws() && tc::scan_ws_ok(d.P, d.N, d.Q);
-            const bool sums_path = !no_tma() && !no_sums() && tc::scan_tma_ok(d.P, d.N, d.Q);
-            __nv_bfloat16 *CBt16 = reinterpret_cast<__nv_bfloat16 *>(ws + w.cbt16);
-            __nv_bfloat16 *CB16b = reinterpret_cast<__nv_bfloat16 *>(ws + w.cb16);
-            CUtensorMap mCc, mBc;
-            if (ws_path && sums_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc)) {
-                // the fused dCB / decay-gradient kernel reads the bf16 tile by TMA; the separate intra_sums kernel
-                // reads the fp32 strips
-                fused_cb = !no_fused() && tc::intra_tile_ok(d.P, d.Q);
-                const size_t smem_ct = tc::bmm_cb_tma_smem(d.N);
-                BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
-                BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s, 
-                    d, mCc, mBc, fused_cb ? CB16b : nullptr, CBt16, fused_cb ? nullptr : F(w.cbs), status));
-            } else
+    {
+        nlt = nlt_tc;
+        nsplit = w.nsplit;
+        part_heads = d.G;
+        const size_t smem_cb = tc::smem_bytes(ntQ, 0), smem_dx = tc::smem_bytes(ntP, 3 * d.Q), smem_n = tc::smem_bytes(ntN, 0);
+        BISSD_ALLOW(tc::bmm_cb<T>, smem_cb);
+        const bool ws_path = !no_tma() && !no_ws() && tc::scan_ws_ok(d.P, d.N, d.Q);
+        const bool sums_path = !no_tma() && !no_sums() && tc::scan_tma_ok(d.P, d.N, d.Q);
+        __nv_bfloat16 *CBt16 = reinterpret_cast<__nv_bfloat16 *>(ws + w.cbt16);
+        __nv_bfloat16 *CB16b = reinterpret_cast<__nv_bfloat16 *>(ws + w.cb16);
+        CUtensorMap mCc, mBc;
+        if (ws_path && sums_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc)) {
+            // the fused dCB / decay-gradient kernel reads the bf16 tile by TMA; the separate intra_sums kernel
+            // reads the fp32 strips
+            fused_cb = !no_fused() && tc::intra_tile_ok(d.P, d.Q);
+            const size_t smem_ct = tc::bmm_cb_tma_smem(d.N);
+            BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
+            BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s, 
+                d, mCc, mBc, fused_cb ? CB16b : nullptr, CBt16, fused_cb ? nullptr : F(w.cbs), status));
+        } else
+        BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
+            d, Cm, Bm, (sums_path && ws_path) ? nullptr : F(w.cb), ws_path ? nullptr : F(w.cbt), nullptr,
+            ws_path ? CBt16 : nullptr, sums_path ? F(w.cbs) : nullptr, status));   // only the copies that will be read
+        have_fp32_cb = !ws_path;                             // ws path: only the copies its kernels read were written
+        auto ensure_fp32_cb = [&]() -> int {                 // for the kernels that read them, should a planned path fall through
+            if (have_fp32_cb) return BISSD_OK;
             BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
-                d, Cm, Bm, (sums_path && ws_path) ? nullptr : F(w.cb), ws_path ? nullptr : F(w.cbt), nullptr,
-                ws_path ? CBt16 : nullptr, sums_path ? F(w.cbs) : nullptr, status));   // only the copies that will be read
-            have_fp32_cb = !ws_path;                             // ws path: only the copies its kernels read were written
-            auto ensure_fp32_cb = [&]() -> int {                 // for the kernels that read them, should a planned path fall through
-                if (have_fp32_cb) return BISSD_OK;
-                BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
-                    d, Cm, Bm, F(w.cb), F(w.cbt), nullptr, nullptr, nullptr, status));
-                have_fp32_cb = true;
-                return BISSD_OK;
-            };
-            bool dx_done = false;
-            if (ws_path) {
-                CUtensorMap mB, mCBt, mEf, mEb, mG, mR;
-                const unsigned long long dB4[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
-                const unsigned long long sB4[3] = {(unsigned long long)a.B.stride_head * 2, (unsigned long long)a.B.stride_seq * 2, (unsigned long long)a.B.stride_batch * 2};
-                const unsigned bB4[4] = {64, 1, 128, 1};
-                const unsigned long long rows = (unsigned long long)d.b * d.nc * d.H * d.P;
-                const char *e16 = static_cast<const char *>(E16);
-                const bool maps = tc::make_map4(&mB, a.p.x_dtype, a.B.ptr, dB4, sB4, bB4) &&
-                                  map_bshd(&mG, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, 64) &&
-                                  tc::make_map2(&mCBt, BISSD_BF16, CBt16, d.Q, (unsigned long long)d.b * d.nc * d.G * d.Q, 64, 128) &&
-                                  tc::make_map2(&mEf, a.p.x_dtype, e16, d.N, rows, 64, d.P) &&
-                                  tc::make_map2(&mEb, a.p.x_dtype, e16 + rows * d.N * 2, d.N, rows, 64, d.P);
-                // the epilogue's x rows by TMA (a [128 rows x 64] tile per step)
-                const bool x_rows = maps && map_bshd(&mR, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, 128);
-                if (maps && !x_rows) mR = mG;
-                if (maps) {
-                    auto wide = [](const void *ptr, long long sb, long long sl, long long sh) {
-                        return ptr && reinterpret_cast<uintptr_t>(ptr) % 32 == 0 && sb % 16 == 0 && sl % 16 == 0 && sh % 16 == 0;
-                    };
-                    tc::WsArgs wa{};
-                    wa.x = x; wa.z = gv; wa.D = a.D; wa.dt_out = a.dt_out; wa.cs_f = a.cs_f; wa.cs_b = a.cs_b;
-                    wa.out = gr.dx;
-                    wa.out_x = wa.out;
-                    wa.ddt_out = F(w.ddt_out); wa.nf = F(w.nf); wa.nb = F(w.nb); wa.dDpart = F(w.dDpart);
-                    wa.wide_x = wide(x.ptr, x.sb, x.sl, x.sh);
-                    wa.wide_z = wide(gv.ptr, gv.sb, gv.sl, gv.sh);
-                    wa.wide_o = wide(gr.dx.ptr, gr.dx.sb, gr.dx.sl, gr.dx.sh);
-                    wa.rows_by_tma = x_rows ? 1 : 0;
-                    const size_t smem_t = tc::scan_ws_smem(d.P, d.N, d.Q);
-                    const int grid = std::min(sm_count(), bch * nlt_tc);
+                d, Cm, Bm, F(w.cb), F(w.cbt), nullptr, nullptr, nullptr, status));
+            have_fp32_cb = true;
+            return BISSD_OK;
+        };
+        bool dx_done = false;
+        if (ws_path) {
+            CUtensorMap mB, mCBt, mEf, mEb, mG, mR;
+            const unsigned long long dB4[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
+            const unsigned long long sB4[3] = {(unsigned long long)a.B.stride_head * 2, (unsigned long long)a.B.stride_seq * 2, (unsigned long long)a.B.stride_batch * 2};
+            const unsigned bB4[4] = {64, 1, 128, 1};
+            const unsigned long long rows = (unsigned long long)d.b * d.nc * d.H * d.P;
+            const char *e16 = static_cast<const char *>(E16);
+            const bool maps = tc::make_map4(&mB, a.p.x_dtype, a.B.ptr, dB4, sB4, bB4) &&
+                              map_bshd(&mG, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, 64) &&
+                              tc::make_map2(&mCBt, BISSD_BF16, CBt16, d.Q, (unsigned long long)d.b * d.nc * d.G * d.Q, 64, 128) &&
+                              tc::make_map2(&mEf, a.p.x_dtype, e16, d.N, rows, 64, d.P) &&
+                              tc::make_map2(&mEb, a.p.x_dtype, e16 + rows * d.N * 2, d.N, rows, 64, d.P);
+            // the epilogue's x rows by TMA (a [128 rows x 64] tile per step)
+            const bool x_rows = maps && map_bshd(&mR, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, 128);
+            if (maps && !x_rows) mR = mG;
+            if (maps) {
+                auto wide = [](const void *ptr, long long sb, long long sl, long long sh) {
+                    return ptr && reinterpret_cast<uintptr_t>(ptr) % 32 == 0 && sb % 16 == 0 && sl % 16 == 0 && sh % 16 == 0;
+                };
+                tc::WsArgs wa{};
+                wa.x = x; wa.z = gv; wa.D = a.D; wa.dt_out = a.dt_out; wa.cs_f = a.cs_f; wa.cs_b = a.cs_b;
+                wa.out = gr.dx;
+                wa.out_x = wa.out;
+                wa.ddt_out = F(w.ddt_out); wa.nf = F(w.nf); wa.nb = F(w.nb); wa.dDpart = F(w.dDpart);
+                wa.wide_x = wide(x.ptr, x.sb, x.sl, x.sh);
+                wa.wide_z = wide(gv.ptr, gv.sb, gv.sl, gv.sh);
+                wa.wide_o = wide(gr.dx.ptr, gr.dx.sb, gr.dx.sl, gr.dx.sh);
+                wa.rows_by_tma = x_rows ? 1 : 0;
+                const size_t smem_t = tc::scan_ws_smem(d.P, d.N, d.Q);
+                const int grid = std::min(sm_count(), bch * nlt_tc);
 #define BISSD_DX_WS(NSL, NS)                                                                                            \
-    do {                                                                                                                \
-        BISSD_ALLOW((tc::ws_kernel<T, NSL, NS, 1>), smem_t);                                                            \
-        BISSD_LAUNCH("tc_dx_ws", launch_pdl(tc::ws_kernel<T, NSL, NS, 1>, grid, tc::kWsThreads, smem_t, s,                      \
-            d, mB, mCBt, mEf, mEb, mG, mR, wa, status));                                                                \
-    } while (0)
-                    if (d.N == 128 && d.Q == 256) BISSD_DX_WS(2, 4);
-                    else if (d.N == 64 && d.Q == 256) BISSD_DX_WS(1, 4);
-                    else if (d.N == 128 && d.Q == 128) BISSD_DX_WS(2, 2);
-                    else BISSD_DX_WS(1, 2);
+do {                                                                                                                \
+    BISSD_ALLOW((tc::ws_kernel<T, NSL, NS, 1>), smem_t);                                                            \
+    BISSD_LAUNCH("tc_dx_ws", launch_pdl(tc::ws_kernel<T, NSL, NS, 1>, grid, tc::kWsThreads, smem_t, s,                      \
+        d, mB, mCBt, mEf, mEb, mG, mR, wa, status));                                                                \
+} while (0)
+                if (d.N == 128 && d.Q == 256) BISSD_DX_WS(2, 4);
+                else if (d.N == 64 && d.Q == 256) BISSD_DX_WS(1, 4);
+                else if (d.N == 128 && d.Q == 128) BISSD_DX_WS(2, 2);
+                else BISSD_DX_WS(1, 2);
 #undef BISSD_DX_WS
-                    dx_done = true;
-                    if (fused_cb && (lease.sd = side_acquire(s)) != nullptr) {      // the two group-walking kernels branch off here
-                        if (cudaEventRecord(lease.sd->fork, s) == cudaSuccess && cudaStreamWaitEvent(lease.sd->st, lease.sd->fork, 0) == cudaSuccess) {
-                            s_side = lease.sd->st;
-                        } else {
-                            cudaGetLastError();
-                        }
-                    }
-                    dd_slots = nlt_tc * 4;
-                    if (d.has_D && !d.D_hdim) {
-                        dd_slots = nlt_tc * 8;                       // one scalar per epilogue warp and tile
-                        dd_compact = true;
-                    }
-                }
-            }
-            if (!dx_done) {
-                const int rc = ensure_fp32_cb();
-                if (rc != BISSD_OK) return rc;
-            }
-            if (!dx_done && !no_tma() && tc::scan_tma_ok(d.P, d.N, d.Q)) {
-                CUtensorMap mB, mEf, mEb, mG;
-                const unsigned long long dB4[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
-                const unsigned long long sB4[3] = {(unsigned long long)a.B.stride_head * 2, (unsigned long long)a.B.stride_seq * 2, (unsigned long long)a.B.stride_batch * 2};
-                const unsigned bB4[4] = {64, 1, 128, 1};
-                const unsigned long long dG4[4] = {(unsigned long long)d.P, (unsigned long long)d.H, (unsigned long long)d.L, (unsigned long long)d.b};
-                const unsigned long long sG4[3] = {(unsigned long long)gv.sh * 2, (unsigned long long)gv.sl * 2, (unsigned long long)gv.sb * 2};
-                const unsigned bG4[4] = {64, 1, (unsigned)d.Q, 1};
-                const unsigned long long rows = (unsigned long long)d.b * d.nc * d.H * d.P;
-                const char *e16 = static_cast<const char *>(E16);
-                if (tc::make_map4(&mB, a.p.x_dtype, a.B.ptr, dB4, sB4, bB4) && tc::make_map4(&mG, a.p.x_dtype, gv.ptr, dG4, sG4, bG4) &&
-                    tc::make_map2(&mEf, a.p.x_dtype, e16, d.N, rows, 64, d.P) &&
-                    tc::make_map2(&mEb, a.p.x_dtype, e16 + rows * d.N * 2, d.N, rows, 64, d.P)) {
-                    const int rounds = tc::scan_tma_rounds(d.P, d.N, d.Q);
-                    const size_t smem_t = tc::dx_tma_smem(d.P, d.N, d.Q, rounds);
-                    BISSD_ALLOW(tc::dx_tma<T>, smem_t);
-                    BISSD_LAUNCH("tc_dx_tma", tc::dx_tma<T><<<dim3(bch, nlt_tc), tc::kThreads, smem_t, s>>>(
-                        d, mB, mEf, mEb, mG, x, gv, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cbt), gr.dx, F(w.ddt_out), F(w.nf), F(w.nb),
-                        F(w.dDpart), rounds, status));
-                    dx_done = true;
-                }
-            }
-            if (dx_done) {
-            } else if (ntP <= 64) {
-                BISSD_ALLOW((tc::dx_kernel<T, 2>), smem_dx);
-                BISSD_LAUNCH("tc_dx", tc::dx_kernel<T, 2><<<dim3(bch, nlt_tc), tc::kThreads, smem_dx, s>>>(
-                    dg, x, Bm, z, gv, out_x, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cb), E16, gr.dx, a.dz, F(w.ddt_out), F(w.dDpart), status));
-            } else {
-                BISSD_ALLOW((tc::dx_kernel<T, 8>), smem_dx);
-                BISSD_LAUNCH("tc_dx", tc::dx_kernel<T, 8><<<dim3(bch, nlt_tc), tc::kThreads, smem_dx, s>>>(
-                    dg, x, Bm, z, gv, out_x, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cb), E16, gr.dx, a.dz, F(w.ddt_out), F(w.dDpart), status));
-            }
-            bool dbc_done = false;
-            if (dx_done) {                                           // the dx kernel has produced nf / nb
-                CUtensorMap mC, mEf, mEb, mSf, mSb;
-                const unsigned long long dC4[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
-                const unsigned long long sC4[3] = {(unsigned long long)a.C.stride_head * 2, (unsigned long long)a.C.stride_seq * 2, (unsigned long long)a.C.stride_batch * 2};
-                const unsigned bC4[4] = {64, 1, 128, 1};
-                const unsigned long long rows = (unsigned long long)d.b * d.nc * d.H * d.P;
-                const char *e16 = static_cast<const char *>(E16);
-                if (tc::make_map4(&mC, a.p.x_dtype, a.C.ptr, dC4, sC4, bC4) &&
-                    tc::make_map2(&mEf, a.p.x_dtype, e16, d.N, rows, 64, d.P) &&
-                    tc::make_map2(&mEb, a.p.x_dtype, e16 + rows * d.N * 2, d.N, rows, 64, d.P) &&
-                    tc::make_map2(&mSf, a.p.x_dtype, a.states_f, d.N, rows, 64, d.P) &&
-                    tc::make_map2(&mSb, a.p.x_dtype, a.states_b, d.N, rows, 64, d.P)) {
-                    const size_t smem_p = tc::prev_tma_smem(d.P, d.N), smem_a = tc::dbc_tma_smem(d.P, std::min(d.N, 128));
-                    CUtensorMap mX128, mG128;
-                    if (!map_bshd(&mX128, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, 128) ||
-                        !map_bshd(&mG128, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, 128))
-                        return BISSD_ERR_ALIGN;
-                    if (!no_ws() && tc::prev_grp_ok(d.P, d.N, d.Q, d.R)) {
-                        const size_t smem_g = tc::prev_grp_smem(d.N, d.Q);
-                        const int ks = tc::state_grp_ksplit(d.b * d.nc * d.G, d.R, sm_count());
-                        BISSD_ALLOW(tc::prev_terms_grp<T>, smem_g);
-                        BISSD_LAUNCH_ON(s_side, "tc_prev_terms_grp", launch_pdl(tc::prev_terms_grp<T>, dim3(d.b * d.nc * d.G * ks), tc::kPrevGrpThreads, smem_g, s_side, 
-                            d, mC, mSf, mSb, mG128, ks, a.cs_f, a.cs_b, F(w.pf), F(w.pb), status));
+                dx_done = true;
+                if (fused_cb && (lease.sd = side_acquire(s)) != nullptr) {      // the two group-walking kernels branch off here
+                    if (cudaEventRecord(lease.sd->fork, s) == cudaSuccess && cudaStreamWaitEvent(lease.sd->st, lease.sd->fork, 0) == cudaSuccess) {
+                        s_side = lease.sd->st;
                     } else {
-                        BISSD_ALLOW(tc::prev_terms_tma<T>, smem_p);
-                        BISSD_LAUNCH("tc_prev_terms_tma", tc::prev_terms_tma<T><<<dim3(bch, nlt_tc), tc::kThreads, smem_p, s>>>(
-                            d, mC, mSf, mSb, gv, a.cs_f, a.cs_b, F(w.pf), F(w.pb), status));
+                        cudaGetLastError();
                     }
-                    BISSD_ALLOW(tc::dbc_accum_tma<T>, smem_a);
-                    if (!no_ws() && tc::dbc_grp_ok(d.P, d.N, d.Q)) {
-                        const size_t smem_g = tc::dbc_grp_smem(d.Q, std::min(d.N, 128));
-                        BISSD_ALLOW(tc::dbc_accum_grp<T>, smem_g);
-                        BISSD_LAUNCH_ON(s_side, "tc_dbc_accum_grp", launch_pdl(tc::dbc_accum_grp<T>, dim3(d.b * d.nc * d.G * w.nsplit, 1, 2), tc::kDbcGrpThreads, smem_g, s_side, 
-                            d, mEf, mEb, mSf, mSb, mX128, mG128, a.dt_out, a.cs_f, a.cs_b, F(w.dB_part), F(w.dC_part), status));
-                    } else
-                    BISSD_LAUNCH("tc_dbc_accum_tma", tc::dbc_accum_tma<T><<<dim3(d.b * d.nc * d.G * w.nsplit, nlt_tc, 2), tc::kThreads, smem_a, s>>>(
-                        d, mEf, mEb, mSf, mSb, mX128, mG128, a.dt_out, a.cs_f, a.cs_b, F(w.dB_part), F(w.dC_part), status));
-                    dbc_done = true;
-                    nsplit = 1;                                      // nf/nb/pf/pb now hold complete row sums
                 }
-            }
-            if (!dbc_done) {
-                BISSD_ALLOW(tc::dbc_states<T>, smem_n);
-                BISSD_LAUNCH("tc_dbc_states", tc::dbc_states<T><<<dim3(d.b * d.nc * d.G * w.nsplit, nlt_tc, 2), tc::kThreads, smem_n, s>>>(
-                    dg, x, Bm, Cm, z, gv, a.dt_out, a.cs_f, a.cs_b, E16, a.states_f, a.states_b, F(w.dB_part), F(w.dC_part),
-                    F(w.nf), F(w.nb), F(w.pf), F(w.pb), status));
+                dd_slots = nlt_tc * 4;
+                if (d.has_D && !d.D_hdim) {
+                    dd_slots = nlt_tc * 8;                       // one scalar per epilogue warp and tile
+                    dd_compact = true;
+                }
             }
         }
+        if (!dx_done) {
+            const int rc = ensure_fp32_cb();
+            if (rc != BISSD_OK) return rc;
+        }
+        if (!dx_done && !no_tma() && tc::scan_tma_ok(d.P, d.N, d.Q)) {
+            CUtensorMap mB, mEf, mEb, mG;
+            const unsigned long long dB4[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
+            const unsigned long long sB4[3] = {(unsigned long long)a.B.stride_head * 2, (unsigned long long)a.B.stride_seq * 2, (unsigned long long)a.B.stride_batch * 2};
+            const unsigned bB4[4] = {64, 1, 128, 1};
+            const unsigned long long dG4[4] = {(unsigned long long)d.P, (unsigned long long)d.H, (unsigned long long)d.L, (unsigned long long)d.b};
+            const unsigned long long sG4[3] = {(unsigned long long)gv.sh * 2, (unsigned long long)gv.sl * 2, (unsigned long long)gv.sb * 2};
+            const unsigned bG4[4] = {64, 1, (unsigned)d.Q, 1};
+            const unsigned long long rows = (unsigned long long)d.b * d.nc * d.H * d.P;
+            const char *e16 = static_cast<const char *>(E16);
+            if (tc::make_map4(&mB, a.p.x_dtype, a.B.ptr, dB4, sB4, bB4) && tc::make_map4(&mG, a.p.x_dtype, gv.ptr, dG4, sG4, bG4) &&
+                tc::make_map2(&mEf, a.p.x_dtype, e16, d.N, rows, 64, d.P) &&
+                tc::make_map2(&mEb, a.p.x_dtype, e16 + rows * d.N * 2, d.N, rows, 64, d.P)) {
+                const int rounds = tc::scan_tma_rounds(d.P, d.N, d.Q);
+                const size_t smem_t = tc::dx_tma_smem(d.P, d.N, d.Q, rounds);
+                BISSD_ALLOW(tc::dx_tma<T>, smem_t);
+                BISSD_LAUNCH("tc_dx_tma", tc::dx_tma<T><<<dim3(bch, nlt_tc), tc::kThreads, smem_t, s>>>(
+                    d, mB, mEf, mEb, mG, x, gv, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cbt), gr.dx, F(w.ddt_out), F(w.nf), F(w.nb),
+                    F(w.dDpart), rounds, status));
+                dx_done = true;
+            }
+        }
+        if (dx_done) {
+        } else if (ntP <= 64) {
+            BISSD_ALLOW((tc::dx_kernel<T, 2>), smem_dx);
+            BISSD_LAUNCH("tc_dx", tc::dx_kernel<T, 2><<<dim3(bch, nlt_tc), tc::kThreads, smem_dx, s>>>(
+                dg, x, Bm, z, gv, out_x, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cb), E16, gr.dx, a.dz, F(w.ddt_out), F(w.dDpart), status));
+        } else {
+            BISSD_ALLOW((tc::dx_kernel<T, 8>), smem_dx);
+            BISSD_LAUNCH("tc_dx", tc::dx_kernel<T, 8><<<dim3(bch, nlt_tc), tc::kThreads, smem_dx, s>>>(
+                dg, x, Bm, z, gv, out_x, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cb), E16, gr.dx, a.dz, F(w.ddt_out), F(w.dDpart), status));
+        }
+        bool dbc_done = false;
+        if (dx_done) {                                           // the dx kernel has produced nf / nb
+            CUtensorMap mC, mEf, mEb, mSf, mSb;
+            const unsigned long long dC4[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
+            const unsigned long long sC4[3] = {(unsigned long long)a.C.stride_head * 2, (unsigned long long)a.C.stride_seq * 2, (unsigned long long)a.C.stride_batch * 2};
+            const unsigned bC4[4] = {64, 1, 128, 1};
+            const unsigned long long rows = (unsigned long long)d.b * d.nc * d.H * d.P;
+            const char *e16 = static_cast<const char *>(E16);
+            if (tc::make_map4(&mC, a.p.x_dtype, a.C.ptr, dC4, sC4, bC4) &&
+                tc::make_map2(&mEf, a.p.x_dtype, e16, d.N, rows, 64, d.P) &&
+                tc::make_map2(&mEb, a.p.x_dtype, e16 + rows * d.N * 2, d.N, rows, 64, d.P) &&
+                tc::make_map2(&mSf, a.p.x_dtype, a.states_f, d.N, rows, 64, d.P) &&
+                tc::make_map2(&mSb, a.p.x_dtype, a.states_b, d.N, rows, 64, d.P)) {
+                const size_t smem_p = tc::prev_tma_smem(d.P, d.N), smem_a = tc::dbc_tma_smem(d.P, std::min(d.N, 128));
+                CUtensorMap mX128, mG128;
+                if (!map_bshd(&mX128, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, 128) ||
+                    !map_bshd(&mG128, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, 128))
+                    return BISSD_ERR_ALIGN;
+                if (!no_ws() && tc::prev_grp_ok(d.P, d.N, d.Q, d.R)) {
+                    const size_t smem_g = tc::prev_grp_smem(d.N, d.Q);
+                    const int ks = tc::state_grp_ksplit(d.b * d.nc * d.G, d.R, sm_count());
+                    BISSD_ALLOW(tc::prev_terms_grp<T>, smem_g);
+                    BISSD_LAUNCH_ON(s_side, "tc_prev_terms_grp", launch_pdl(tc::prev_terms_grp<T>, dim3(d.b * d.nc * d.G * ks), tc::kPrevGrpThreads, smem_g, s_side, 
+                        d, mC, mSf, mSb, mG128, ks, a.cs_f, a.cs_b, F(w.pf), F(w.pb), status));
+                } else {
+                    BISSD_ALLOW(tc::prev_terms_tma<T>, smem_p);
+                    BISSD_LAUNCH("tc_prev_terms_tma", tc::prev_terms_tma<T><<<dim3(bch, nlt_tc), tc::kThreads, smem_p, s>>>(
+                        d, mC, mSf, mSb, gv, a.cs_f, a.cs_b, F(w.pf), F(w.pb), status));
+                }
+                BISSD_ALLOW(tc::dbc_accum_tma<T>, smem_a);
+                if (!no_ws() && tc::dbc_grp_ok(d.P, d.N, d.Q)) {
+                    const size_t smem_g = tc::dbc_grp_smem(d.Q, std::min(d.N, 128));
+                    BISSD_ALLOW(tc::dbc_accum_grp<T>, smem_g);
+                    BISSD_LAUNCH_ON(s_side, "tc_dbc_accum_grp", launch_pdl(tc::dbc_accum_grp<T>, dim3(d.b * d.nc * d.G * w.nsplit, 1, 2), tc::kDbcGrpThreads, smem_g, s_side, 
+                        d, mEf, mEb, mSf, mSb, mX128, mG128, a.dt_out, a.cs_f, a.cs_b, F(w.dB_part), F(w.dC_part), status));
+                } else
+                BISSD_LAUNCH("tc_dbc_accum_tma", tc::dbc_accum_tma<T><<<dim3(d.b * d.nc * d.G * w.nsplit, nlt_tc, 2), tc::kThreads, smem_a, s>>>(
+                    d, mEf, mEb, mSf, mSb, mX128, mG128, a.dt_out, a.cs_f, a.cs_b, F(w.dB_part), F(w.dC_part), status));
+                dbc_done = true;
+                nsplit = 1;                                      // nf/nb/pf/pb now hold complete row sums
+            }
+        }
+        if (!dbc_done) {
+            BISSD_ALLOW(tc::dbc_states<T>, smem_n);
+            BISSD_LAUNCH("tc_dbc_states", tc::dbc_states<T><<<dim3(d.b * d.nc * d.G * w.nsplit, nlt_tc, 2), tc::kThreads, smem_n, s>>>(
+                dg, x, Bm, Cm, z, gv, a.dt_out, a.cs_f, a.cs_b, E16, a.states_f, a.states_b, F(w.dB_part), F(w.dC_part),
+                F(w.nf), F(w.nb), F(w.pf), F(w.pb), status));
+        }
     }
-    if (!tcp) {
-        BISSD_LAUNCH("bmm_cb", simt::bmm_cb<T><<<dim3(d.b * d.nc * d.G, w.nlt, w.nlt), simt::TB, 0, s>>>(d, Cm, Bm, F(w.cb)));
-        BISSD_LAUNCH("dx_kernel", simt::dx_kernel<T><<<dim3(bch, w.nlt), simt::TB, q3, s>>>(
-            d, x, Bm, z, dout, out_x, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cb), F(w.E), gr.dx, a.dz, F(w.ddt_out), F(w.dDpart)));
-        BISSD_LAUNCH("dbc_states", simt::dbc_states<T><<<dim3(bch, w.nlt, 2), simt::TB, q3, s>>>(
-            d, x, Bm, Cm, z, dout, a.dt_out, a.cs_f, a.cs_b, F(w.E), a.states_f, a.states_b, F(w.dB_part), F(w.dC_part),
-            F(w.nf), F(w.nb), F(w.pf), F(w.pb)));
-    }
-    bool intra_tc = false;
     bool bmm_tma = false;                                        // dCB is then a 16-bit array read by TMA
     CUtensorMap mBb, mCb, mDm, mDk;
-    if constexpr (TcKernels<T>::available) {
-        if (tcp) {
-            intra_tc = true;
-            const int ntQ128 = std::min(ntQ, 128);
-            const size_t smem_dcb = tc::smem_bytes(ntQ128, 3 * d.Q), smem_in = tc::smem_bytes(ntQ, 4 * d.Q + tc::kTileM * 8);
-            bool dcb_done = false;
-            bool fused_done = false;
-            if (fused_cb) {
-                // one kernel for dCB and the intra-chunk decay gradients: a CTA per (batch, chunk, group, row tile)
-                CUtensorMap mG, mX128, mCB;
+    {
+        const int ntQ128 = std::min(ntQ, 128);
+        const size_t smem_dcb = tc::smem_bytes(ntQ128, 3 * d.Q), smem_in = tc::smem_bytes(ntQ, 4 * d.Q + tc::kTileM * 8);
+        bool dcb_done = false;
+        bool fused_done = false;
+        if (fused_cb) {
+            // one kernel for dCB and the intra-chunk decay gradients: a CTA per (batch, chunk, group, row tile)
+            CUtensorMap mG, mX128, mCB;
+            const unsigned long long dBC4[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
+            const unsigned long long sB4[3] = {(unsigned long long)a.B.stride_head * 2, (unsigned long long)a.B.stride_seq * 2, (unsigned long long)a.B.stride_batch * 2};
+            const unsigned long long sC4b[3] = {(unsigned long long)a.C.stride_head * 2, (unsigned long long)a.C.stride_seq * 2, (unsigned long long)a.C.stride_batch * 2};
+            const unsigned bx4[4] = {64, 1, 128, 1};
+            const unsigned long long dcb_rows = (unsigned long long)d.b * d.nc * d.G * d.Q;
+            if (map_bshd(&mG, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, 128) &&
+                map_bshd(&mX128, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, 128) &&
+                tc::make_map2(&mCB, BISSD_BF16, ws + w.cb16, d.Q, dcb_rows, 64, 128) &&
+                tc::bmm_bwd_tma_ok(d.N, d.Q) &&
+                tc::make_map4(&mBb, a.p.x_dtype, a.B.ptr, dBC4, sB4, bx4) && tc::make_map4(&mCb, a.p.x_dtype, a.C.ptr, dBC4, sC4b, bx4) &&
+                tc::make_map2(&mDm, a.p.x_dtype, F(w.dCB), d.Q, dcb_rows, 64, d.Q) &&
+                tc::make_map2(&mDk, a.p.x_dtype, F(w.dCB), d.Q, dcb_rows, 64, 128)) {
+                const size_t smem_f = tc::intra_tile_smem(d.Q);
+                BISSD_ALLOW(tc::intra_dcb_tile<T>, smem_f);
+                BISSD_LAUNCH("tc_intra_dcb_tile", launch_pdl(tc::intra_dcb_tile<T>, dim3(d.b * d.nc * d.G, nlt_tc, nlt_tc), tc::kIntraTileThreads, smem_f, s,
+                    dg, mG, mX128, mCB, a.dt_out, a.cs_f, a.cs_b, F(w.u4), (long long)d.b * d.H * d.nc * d.Q,
+                    static_cast<void *>(F(w.dCB)), status));
+                u4_tiles = nlt_tc * nlt_tc;
+                fused_done = dcb_done = true;
+                bmm_tma = true;
+                use_u4 = true;
+            } else {
+                return BISSD_ERR_ALIGN;                      // the bf16 tile was written for this kernel only
+            }
+        }
+        if (!dcb_done && !no_tma() && tc::scan_tma_ok(d.P, d.N, d.Q)) {
+            CUtensorMap mG, mX;
+            const unsigned long long dX4[4] = {(unsigned long long)d.P, (unsigned long long)d.H, (unsigned long long)d.L, (unsigned long long)d.b};
+            const unsigned long long sX4[3] = {(unsigned long long)a.x.stride_head * 2, (unsigned long long)a.x.stride_seq * 2, (unsigned long long)a.x.stride_batch * 2};
+            const unsigned long long sG4[3] = {(unsigned long long)gv.sh * 2, (unsigned long long)gv.sl * 2, (unsigned long long)gv.sb * 2};
+            const unsigned bx4[4] = {64, 1, 128, 1};
+            if (tc::make_map4(&mX, a.p.x_dtype, a.x.ptr, dX4, sX4, bx4) && tc::make_map4(&mG, a.p.x_dtype, gv.ptr, dX4, sG4, bx4)) {
+                // the product with B / C reads dCB by TMA from a 16-bit copy when it can
                 const unsigned long long dBC4[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
                 const unsigned long long sB4[3] = {(unsigned long long)a.B.stride_head * 2, (unsigned long long)a.B.stride_seq * 2, (unsigned long long)a.B.stride_batch * 2};
                 const unsigned long long sC4b[3] = {(unsigned long long)a.C.stride_head * 2, (unsigned long long)a.C.stride_seq * 2, (unsigned long long)a.C.stride_batch * 2};
-                const unsigned bx4[4] = {64, 1, 128, 1};
                 const unsigned long long dcb_rows = (unsigned long long)d.b * d.nc * d.G * d.Q;
-                if (map_bshd(&mG, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, 128) &&
-                    map_bshd(&mX128, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, 128) &&
-                    tc::make_map2(&mCB, BISSD_BF16, ws + w.cb16, d.Q, dcb_rows, 64, 128) &&
-                    tc::bmm_bwd_tma_ok(d.N, d.Q) &&
-                    tc::make_map4(&mBb, a.p.x_dtype, a.B.ptr, dBC4, sB4, bx4) && tc::make_map4(&mCb, a.p.x_dtype, a.C.ptr, dBC4, sC4b, bx4) &&
-                    tc::make_map2(&mDm, a.p.x_dtype, F(w.dCB), d.Q, dcb_rows, 64, d.Q) &&
-                    tc::make_map2(&mDk, a.p.x_dtype, F(w.dCB), d.Q, dcb_rows, 64, 128)) {
-                    const size_t smem_f = tc::intra_tile_smem(d.Q);
-                    BISSD_ALLOW(tc::intra_dcb_tile<T>, smem_f);
-                    BISSD_LAUNCH("tc_intra_dcb_tile", launch_pdl(tc::intra_dcb_tile<T>, dim3(d.b * d.nc * d.G, nlt_tc, nlt_tc), tc::kIntraTileThreads, smem_f, s,
-                        dg, mG, mX128, mCB, a.dt_out, a.cs_f, a.cs_b, F(w.u4), (long long)d.b * d.H * d.nc * d.Q,
-                        static_cast<void *>(F(w.dCB)), status));
-                    u4_tiles = nlt_tc * nlt_tc;
-                    fused_done = dcb_done = true;
-                    bmm_tma = true;
-                    use_u4 = true;
-                } else {
-                    return BISSD_ERR_ALIGN;                      // the bf16 tile was written for this kernel only
-                }
-            }
-            if (!dcb_done && !no_tma() && tc::scan_tma_ok(d.P, d.N, d.Q)) {
-                CUtensorMap mG, mX;
-                const unsigned long long dX4[4] = {(unsigned long long)d.P, (unsigned long long)d.H, (unsigned long long)d.L, (unsigned long long)d.b};
-                const unsigned long long sX4[3] = {(unsigned long long)a.x.stride_head * 2, (unsigned long long)a.x.stride_seq * 2, (unsigned long long)a.x.stride_batch * 2};
-                const unsigned long long sG4[3] = {(unsigned long long)gv.sh * 2, (unsigned long long)gv.sl * 2, (unsigned long long)gv.sb * 2};
-                const unsigned bx4[4] = {64, 1, 128, 1};
-                if (tc::make_map4(&mX, a.p.x_dtype, a.x.ptr, dX4, sX4, bx4) && tc::make_map4(&mG, a.p.x_dtype, gv.ptr, dX4, sG4, bx4)) {
-                    // the product with B / C reads dCB by TMA from a 16-bit copy when it can
-                    const unsigned long long dBC4[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
-                    const unsigned long long sB4[3] = {(unsigned long long)a.B.stride_head * 2, (unsigned long long)a.B.stride_seq * 2, (unsigned long long)a.B.stride_batch * 2};
-                    const unsigned long long sC4b[3] = {(unsigned long long)a.C.stride_head * 2, (unsigned long long)a.C.stride_seq * 2, (unsigned long long)a.C.stride_batch * 2};
-                    const unsigned long long dcb_rows = (unsigned long long)d.b * d.nc * d.G * d.Q;
-                    bmm_tma = !no_ws() && tc::bmm_bwd_tma_ok(d.N, d.Q) &&
-                              tc::make_map4(&mBb, a.p.x_dtype, a.B.ptr, dBC4, sB4, bx4) && tc::make_map4(&mCb, a.p.x_dtype, a.C.ptr, dBC4, sC4b, bx4) &&
-                              tc::make_map2(&mDm, a.p.x_dtype, F(w.dCB), d.Q, dcb_rows, 64, d.Q) &&
-                              tc::make_map2(&mDk, a.p.x_dtype, F(w.dCB), d.Q, dcb_rows, 64, 128);
-                    const size_t smem_t = tc::dcb_tma_smem(d.P, d.Q);
-                    BISSD_ALLOW(tc::dcb_tma<T>, smem_t);
-                    BISSD_LAUNCH("tc_dcb_tma", launch_pdl(tc::dcb_tma<T>, dim3(d.b * d.nc * d.G, nlt_tc, nlt_tc), tc::kThreads, smem_t, s, 
-                        d, mG, mX, a.dt_out, a.cs_f, a.cs_b, bmm_tma ? nullptr : F(w.dCB), bmm_tma ? static_cast<void *>(F(w.dCB)) : nullptr, status));
-                    dcb_done = true;
-                }
-            }
-            if (!dcb_done) {
-                BISSD_ALLOW(tc::dcb_kernel<T>, smem_dcb);
-                BISSD_LAUNCH("tc_dcb", tc::dcb_kernel<T><<<dim3(d.b * d.nc * d.G, nlt_tc, nlt_tc), tc::kThreads, smem_dcb, s>>>(
-                    dg, x, z, gv, a.dt_out, a.cs_f, a.cs_b, F(w.dCB), status));
-            }
-            bool intra_done = fused_done;
-            const bool sums_path = !no_tma() && !no_sums() && tc::scan_tma_ok(d.P, d.N, d.Q);
-            if (sums_path && !intra_done) {
-                CUtensorMap mG, mX;
-                if (map_bshd(&mG, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, 128) &&
-                    map_bshd(&mX, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, d.Q)) {
-                    const size_t smem_s = tc::intra_sums_smem(d.Q);
-                    BISSD_ALLOW(tc::intra_sums<T>, smem_s);
-                    BISSD_LAUNCH("tc_intra_sums", launch_pdl(tc::intra_sums<T>, dim3(bch, nlt_tc), tc::kThreads, smem_s, s, 
-                        dg, mG, mX, a.dt_out, a.cs_f, a.cs_b, F(w.cbs), F(w.u4), (long long)d.b * d.H * d.nc * d.Q, status));
-                    intra_done = true;
-                    use_u4 = true;
-                }
-            }
-            if (!intra_done && !have_fp32_cb) {                  // the prefix-sweep kernels read the fp32 matrix
-                const size_t smem_cb = tc::smem_bytes(ntQ, 0);
-                BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
-                    d, Cm, Bm, F(w.cb), F(w.cbt), nullptr, nullptr, nullptr, status));
-                have_fp32_cb = true;
-            }
-            if (!intra_done && !no_tma() && tc::scan_tma_ok(d.P, d.N, d.Q)) {
-                CUtensorMap mG, mX;
-                if (map_bshd(&mG, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, 128) &&
-                    map_bshd(&mX, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, d.Q)) {
-                    BISSD_ALLOW((tc::intra_decay_grad<T, true>), smem_in);
-                    BISSD_LAUNCH("tc_intra_decay_grad", tc::intra_decay_grad<T, true><<<dim3(bch, nlt_tc), tc::kThreads, smem_in, s>>>(
-                        dg, mG, mX, x, z, gv, a.dt_out, a.cs_f, a.cs_b, F(w.cb), F(w.da_f), F(w.da_b), status));
-                    intra_done = true;
-                }
-            }
-            if (!intra_done) {
-                CUtensorMap none{};
-                BISSD_ALLOW((tc::intra_decay_grad<T, false>), smem_in);
-                BISSD_LAUNCH("tc_intra_decay_grad", tc::intra_decay_grad<T, false><<<dim3(bch, nlt_tc), tc::kThreads, smem_in, s>>>(
-                    dg, none, none, x, z, gv, a.dt_out, a.cs_f, a.cs_b, F(w.cb), F(w.da_f), F(w.da_b), status));
+                bmm_tma = !no_ws() && tc::bmm_bwd_tma_ok(d.N, d.Q) &&
+                          tc::make_map4(&mBb, a.p.x_dtype, a.B.ptr, dBC4, sB4, bx4) && tc::make_map4(&mCb, a.p.x_dtype, a.C.ptr, dBC4, sC4b, bx4) &&
+                          tc::make_map2(&mDm, a.p.x_dtype, F(w.dCB), d.Q, dcb_rows, 64, d.Q) &&
+                          tc::make_map2(&mDk, a.p.x_dtype, F(w.dCB), d.Q, dcb_rows, 64, 128);
+                const size_t smem_t = tc::dcb_tma_smem(d.P, d.Q);
+                BISSD_ALLOW(tc::dcb_tma<T>, smem_t);
+                BISSD_LAUNCH("tc_dcb_tma", launch_pdl(tc::dcb_tma<T>, dim3(d.b * d.nc * d.G, nlt_tc, nlt_tc), tc::kThreads, smem_t, s, 
+                    d, mG, mX, a.dt_out, a.cs_f, a.cs_b, bmm_tma ? nullptr : F(w.dCB), bmm_tma ? static_cast<void *>(F(w.dCB)) : nullptr, status));
+                dcb_done = true;
             }
         }
-    }
-    if (!intra_tc) {
-        BISSD_LAUNCH("dcb_kernel", simt::dcb_kernel<T><<<dim3(d.b * d.nc * d.G, w.nlt, w.nlt), simt::TB, 0, s>>>(
-            d, x, z, dout, a.dt_out, a.cs_f, a.cs_b, F(w.dCB)));
-        const size_t smem = (3 * d.Q + 2 * simt::TILE * (d.Q + 1)) * sizeof(float);
-        BISSD_ALLOW(simt::intra_decay_grad<T>, smem);
-        BISSD_LAUNCH("intra_decay_grad", simt::intra_decay_grad<T><<<bch, simt::TB, smem, s>>>(
-            d, x, z, dout, a.dt_out, a.cs_f, a.cs_b, F(w.cb), F(w.da_f), F(w.da_b)));
+        if (!dcb_done) {
+            BISSD_ALLOW(tc::dcb_kernel<T>, smem_dcb);
+            BISSD_LAUNCH("tc_dcb", tc::dcb_kernel<T><<<dim3(d.b * d.nc * d.G, nlt_tc, nlt_tc), tc::kThreads, smem_dcb, s>>>(
+                dg, x, z, gv, a.dt_out, a.cs_f, a.cs_b, F(w.dCB), status));
+        }
+        bool intra_done = fused_done;
+        const bool sums_path = !no_tma() && !no_sums() && tc::scan_tma_ok(d.P, d.N, d.Q);
+        if (sums_path && !intra_done) {
+            CUtensorMap mG, mX;
+            if (map_bshd(&mG, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, 128) &&
+                map_bshd(&mX, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, d.Q)) {
+                const size_t smem_s = tc::intra_sums_smem(d.Q);
+                BISSD_ALLOW(tc::intra_sums<T>, smem_s);
+                BISSD_LAUNCH("tc_intra_sums", launch_pdl(tc::intra_sums<T>, dim3(bch, nlt_tc), tc::kThreads, smem_s, s, 
+                    dg, mG, mX, a.dt_out, a.cs_f, a.cs_b, F(w.cbs), F(w.u4), (long long)d.b * d.H * d.nc * d.Q, status));
+                intra_done = true;
+                use_u4 = true;
+            }
+        }
+        if (!intra_done && !have_fp32_cb) {                  // the prefix-sweep kernels read the fp32 matrix
+            const size_t smem_cb = tc::smem_bytes(ntQ, 0);
+            BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
+                d, Cm, Bm, F(w.cb), F(w.cbt), nullptr, nullptr, nullptr, status));
+            have_fp32_cb = true;
+        }
+        if (!intra_done && !no_tma() && tc::scan_tma_ok(d.P, d.N, d.Q)) {
+            CUtensorMap mG, mX;
+            if (map_bshd(&mG, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, 128) &&
+                map_bshd(&mX, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, d.Q)) {
+                BISSD_ALLOW((tc::intra_decay_grad<T, true>), smem_in);
+                BISSD_LAUNCH("tc_intra_decay_grad", tc::intra_decay_grad<T, true><<<dim3(bch, nlt_tc), tc::kThreads, smem_in, s>>>(
+                    dg, mG, mX, x, z, gv, a.dt_out, a.cs_f, a.cs_b, F(w.cb), F(w.da_f), F(w.da_b), status));
+                intra_done = true;
+            }
+        }
+        if (!intra_done) {
+            CUtensorMap none{};
+            BISSD_ALLOW((tc::intra_decay_grad<T, false>), smem_in);
+            BISSD_LAUNCH("tc_intra_decay_grad", tc::intra_decay_grad<T, false><<<dim3(bch, nlt_tc), tc::kThreads, smem_in, s>>>(
+                dg, none, none, x, z, gv, a.dt_out, a.cs_f, a.cs_b, F(w.cb), F(w.da_f), F(w.da_b), status));
+        }
     }
     if (s_side != s) {                                           // the group-walking kernels rejoin before their results are read
         int rcj = note_cuda(cudaEventRecord(lease.sd->join, s_side), "cudaEventRecord");
@@ -789,31 +666,25 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
         if (rcj != BISSD_OK) return rcj;
         s_side = s;
     }
-    bool bmm_tc = false;
-    if constexpr (TcKernels<T>::available) {
-        if (tcp && bmm_tma) {
-            bmm_tc = true;
-            const size_t smem_b = tc::bmm_bwd_tma_smem(d.Q);
-            BISSD_ALLOW(tc::bmm_bwd_tma<T>, smem_b);
-            BISSD_LAUNCH("tc_bmm_bwd_tma", launch_pdl(tc::bmm_bwd_tma<T>, dim3(d.b * d.nc * d.G * 2, d.Q / 128, d.N / 64), tc::kThreads, smem_b, s, 
-                d, mDm, mDk, mBb, mCb, F(w.dB_part), F(w.dC_part), part_heads, gr.dB, gr.dC, status));
-        } else if (tcp) {
-            bmm_tc = true;
-            const size_t smem_n = tc::smem_bytes(ntN, 0);
-            BISSD_ALLOW(tc::bmm_bwd<T>, smem_n);
-            BISSD_LAUNCH("tc_bmm_bwd", tc::bmm_bwd<T><<<dim3(d.b * d.nc * d.G * 2, nlt_tc, w.nsplit), tc::kThreads, smem_n, s>>>(
-                d, Bm, Cm, F(w.dCB), F(w.dB_part), F(w.dC_part), part_heads, gr.dB, gr.dC, status));
-        }
+    if (bmm_tma) {
+        const size_t smem_b = tc::bmm_bwd_tma_smem(d.Q);
+        BISSD_ALLOW(tc::bmm_bwd_tma<T>, smem_b);
+        BISSD_LAUNCH("tc_bmm_bwd_tma", launch_pdl(tc::bmm_bwd_tma<T>, dim3(d.b * d.nc * d.G * 2, d.Q / 128, d.N / 64), tc::kThreads, smem_b, s, 
+            d, mDm, mDk, mBb, mCb, F(w.dB_part), F(w.dC_part), part_heads, gr.dB, gr.dC, status));
+    } else {
+        const size_t smem_n = tc::smem_bytes(ntN, 0);
+        BISSD_ALLOW(tc::bmm_bwd<T>, smem_n);
+        BISSD_LAUNCH("tc_bmm_bwd", tc::bmm_bwd<T><<<dim3(d.b * d.nc * d.G * 2, nlt_tc, w.nsplit), tc::kThreads, smem_n, s>>>(
+            d, Bm, Cm, F(w.dCB), F(w.dB_part), F(w.dC_part), part_heads, gr.dB, gr.dC, status));
     }
-    if (!bmm_tc) {
-        BISSD_LAUNCH("bmm_bwd", simt::bmm_bwd<T><<<dim3(d.b * d.nc * d.G * 2, w.nlt, ceil_div(d.N, simt::TILE)), simt::TB, 0, s>>>(
-            d, Bm, Cm, F(w.dCB), F(w.dB_part), F(w.dC_part), part_heads, gr.dB, gr.dC));
-    }
-    BISSD_LAUNCH("cumsum_bwd", launch_pdl(simt::cumsum_bwd, d.b * d.nc * d.H, 256, 0, s, 
-        d, a.dt.ptr, a.p.dt_dtype, a.dt.stride_batch, a.dt.stride_seq, a.dt.stride_head, a.A, a.dt_bias, a.dt_out,
-        F(w.ddt_out), F(w.nf), F(w.nb), F(w.pf), F(w.pb), use_u4 ? nullptr : F(w.da_f), use_u4 ? nullptr : F(w.da_b),
-        use_u4 ? F(w.u4) : nullptr, u4_tiles, F(w.dTpart), pass_nblk, nsplit, gr.ddt,
-        F(w.dApart), F(w.dbiaspart)));
+    simt::CumsumBwd cs{};
+    cs.dt = a.dt.ptr; cs.dt_dtype = a.p.dt_dtype; cs.dsb = a.dt.stride_batch; cs.dsl = a.dt.stride_seq; cs.dsh = a.dt.stride_head;
+    cs.A = a.A; cs.dt_bias = a.dt_bias; cs.dt_out = a.dt_out; cs.ddt_out = F(w.ddt_out);
+    cs.nf = F(w.nf); cs.nb = F(w.nb); cs.pf = F(w.pf); cs.pb = F(w.pb);
+    if (use_u4) { cs.u4 = F(w.u4); cs.u4_tiles = u4_tiles; }
+    else { cs.da_f = F(w.da_f); cs.da_b = F(w.da_b); }
+    cs.dTpart = F(w.dTpart); cs.nblk = pass_nblk; cs.nsplit = nsplit; cs.ddt = gr.ddt; cs.dApart = F(w.dApart); cs.dbiaspart = F(w.dbiaspart);
+    BISSD_LAUNCH("cumsum_bwd", launch_pdl(simt::cumsum_bwd, d.b * d.nc * d.H, 256, 0, s, d, cs));
     BISSD_LAUNCH("final_reduce", launch_pdl(simt::final_reduce<1024>, d.H, 1024, 0, s, 
         d, F(w.dApart), F(w.dbiaspart), d.has_D ? F(w.dDpart) : nullptr, dd_slots ? dd_slots : nlt, dd_compact ? 1 : 0, a.dA, d.has_bias ? a.ddt_bias : nullptr,
         d.has_D ? a.dD : nullptr));
@@ -976,11 +847,8 @@ int bissd_forward(const bissd_fwd_args *a, void *workspace, size_t workspace_byt
     char *ws = static_cast<char *>(workspace);
     const bool tcp = !force_simt() && tc_shape_ok(a->p) && aligned16(a->x) && aligned16(a->B) && aligned16(a->C) &&
                      aligned16(a->z) && aligned16(a->out) && aligned16(a->out_x);
-    switch (a->p.x_dtype) {
-        case BISSD_F32: return forward_impl<float>(*a, d, ws, s, false);
-        case BISSD_BF16: return forward_impl<__nv_bfloat16>(*a, d, ws, s, tcp);
-        default: return forward_impl<__half>(*a, d, ws, s, tcp);
-    }
+    if (!tcp) return simt_forward(*a, d, ws, s);
+    return a->p.x_dtype == BISSD_BF16 ? forward_impl<__nv_bfloat16>(*a, d, ws, s) : forward_impl<__half>(*a, d, ws, s);
 }
 
 // ---- forward pass on library-owned scratch -------------------------------------------------------------------
@@ -1099,11 +967,8 @@ int bissd_backward_into(const bissd_bwd_args *a, const bissd_grad_strides *gs, v
         auto al = [](const MutView &v) { return reinterpret_cast<uintptr_t>(v.ptr) % 16 == 0 && v.sb % 8 == 0 && v.sl % 8 == 0 && v.sh % 8 == 0; };
         if (tcp && !(al(gr.dx) && al(gr.dB) && al(gr.dC))) return BISSD_ERR_ALIGN;   // 16-byte stores
     }
-    switch (a->p.x_dtype) {
-        case BISSD_F32: return backward_impl<float>(*a, gr, d, ws, s, false);
-        case BISSD_BF16: return backward_impl<__nv_bfloat16>(*a, gr, d, ws, s, tcp);
-        default: return backward_impl<__half>(*a, gr, d, ws, s, tcp);
-    }
+    if (!tcp) return simt_backward(*a, gr, d, ws, s);
+    return a->p.x_dtype == BISSD_BF16 ? backward_impl<__nv_bfloat16>(*a, gr, d, ws, s) : backward_impl<__half>(*a, gr, d, ws, s);
 }
 
 }  // extern "C"

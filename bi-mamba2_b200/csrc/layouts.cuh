@@ -1,0 +1,90 @@
+// Workspace layouts shared by the launch code of the kernel families.  The first 256 bytes hold the device status word
+// (nonzero = a bounded device-side wait ran out); everything after it is scratch.
+#pragma once
+#include "host.cuh"
+#include "simt_tile.cuh"
+
+namespace bissd {
+
+constexpr size_t kWsHeader = 256;
+struct FwdWs {
+    size_t loc, cb, cb16, total;
+};
+struct BwdWs {
+    size_t cb, cbt, cbt16, cb16, cbs, gloc, E, E16, g, dTpart, ddt_out, nf, nb, pf, pb, da_f, da_b, u4, dB_part, dC_part, dCB, dDpart, dApart, dbiaspart, total;
+    int nblk, nlt, nsplit, hsplit;
+};
+
+inline FwdWs fwd_layout(const Dims &d) {
+    FwdWs w;
+    size_t o = kWsHeader;
+    const size_t st = (size_t)d.b * d.nc * d.H * d.P * d.N;
+    w.loc = o; o = align256(o + 2 * st * 4);
+    w.cb = o; o = align256(o + (size_t)d.b * d.nc * d.G * d.Q * d.Q * 4);
+    w.cb16 = o; o = align256(o + (size_t)d.b * d.nc * d.G * d.Q * d.Q * 2);      // C.B^T rounded to bf16 (TMA-fed scan)
+    w.total = o;
+    return w;
+}
+
+// Blocks the heads of a group are dealt to in the CUDA-core dCB product, each with a partial dCB of its own: one, unless
+// the problem has too few (batch, chunk, group, tile)s for two blocks an SM; a divisor of the heads per group.
+inline int simt_hsplit(const Dims &d) {
+    const int nt = ceil_div(d.Q, simt::TILE);
+    const long long blocks = (long long)d.b * d.nc * d.G * nt * nt;
+    int hs = 1;
+    for (int k = 2; k <= d.R && blocks * hs < 2LL * sm_count(); ++k)
+        if (d.R % k == 0) hs = k;
+    return hs;
+}
+
+// tc: sized for the tensor-core family (16-bit inputs that meet its alignment rules): the passed state gradients are
+// kept in the input dtype only, and the "states" parts of dB / dC arrive summed over the heads of a group.  The
+// CUDA-core family needs the fp32 copy and one partial per head.
+inline BwdWs bwd_layout(const Dims &d, bool tc) {
+    BwdWs w;
+    size_t o = kWsHeader;
+    const size_t st = (size_t)d.b * d.nc * d.H * d.P * d.N;
+    const size_t hq = (size_t)d.b * d.H * d.nc * d.Q, qq = (size_t)d.b * d.nc * d.G * d.Q * d.Q;
+    w.nblk = ceil_div(d.P * d.N, simt::TB);
+    w.nlt = ceil_div(d.Q, simt::TILE);
+    w.nsplit = tc ? ceil_div(d.N, 128) : 1;
+    w.hsplit = tc ? 1 : simt_hsplit(d);
+    auto take = [&](size_t bytes) { size_t at = o; o = align256(o + bytes); return at; };
+    w.cb = take(qq * 4);
+    w.gloc = take(2 * st * 4);
+    w.E = take(tc ? 0 : 2 * st * 4);                                 // fp32 passed state gradients (CUDA-core family)
+    w.E16 = take(tc ? 2 * st * 2 : 0);                               // passed state gradients in the input dtype
+    w.g = take(tc ? (size_t)d.b * d.L * d.H * d.P * 2 : 0);          // gated output gradient dout * silu(z)
+    w.cbt = take(tc ? qq * 4 : 0);                                   // CB transposed
+    w.cbs = take(tc ? qq * 4 : 0);                                   // CB in strips of 16 columns (tc::intra_sums)
+    w.cbt16 = take(tc ? qq * 2 : 0);                                 // CB transposed, rounded to bf16 (TMA-fed dx)
+    w.cb16 = take(tc ? qq * 2 : 0);                                  // CB rounded to bf16 (tc::intra_dcb_tile)
+    w.dTpart = take((size_t)2 * d.b * d.H * d.nc * w.nblk * 4);
+    w.ddt_out = take(hq * 4);
+    w.nf = take(hq * 4 * w.nsplit); w.nb = take(hq * 4 * w.nsplit);
+    w.pf = take(hq * 4 * w.nsplit); w.pb = take(hq * 4 * w.nsplit);
+    w.da_f = take(tc ? hq * 4 : 0); w.da_b = take(tc ? hq * 4 : 0);
+    w.u4 = take((tc ? 8 : 4 * w.nlt) * hq * 4);                      // u_f / u_b per tile (tc::intra_sums: 2 row tiles; tc::intra_dcb_tile: 4; simt: 2 nlt)
+    w.dB_part = take((size_t)d.b * d.nc * d.Q * (tc ? d.G : d.H) * d.N * 4);
+    w.dC_part = take((size_t)d.b * d.nc * d.Q * (tc ? d.G : d.H) * d.N * 4);
+    w.dCB = take(qq * 4 * w.hsplit);
+    w.dDpart = take((size_t)d.b * d.nc * d.H * std::max(w.nlt, 8) * d.P * 4);   // up to 8 partial rows per (b,c,h)
+    w.dApart = take((size_t)d.b * d.nc * d.H * 4);
+    w.dbiaspart = take((size_t)d.b * d.nc * d.H * 4);
+    w.total = o;
+    return w;
+}
+
+inline View view_of(const bissd_tensor &t) { return View{t.ptr, t.stride_batch, t.stride_seq, t.stride_head}; }
+inline MutView mview_of(const bissd_tensor &t) { return MutView{t.ptr, t.stride_batch, t.stride_seq, t.stride_head}; }
+
+// Where dx, dB, dC and ddt go (bissd_backward: contiguous, bissd_backward_into: the caller's strides).
+struct GradViews {
+    MutView dx, dB, dC, ddt;
+};
+
+// The CUDA-core family (bissd_simt.cu): fp32 inputs, and 16-bit ones outside the tensor-core family's shapes or alignment.
+int simt_forward(const bissd_fwd_args &a, const Dims &d, char *ws, cudaStream_t s);
+int simt_backward(const bissd_bwd_args &a, const GradViews &gr, const Dims &d, char *ws, cudaStream_t s);
+
+}  // namespace bissd
