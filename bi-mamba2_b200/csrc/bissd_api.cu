@@ -208,7 +208,7 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
     // the recurrence runs in both phases: from zero (or init_*) in LOCAL, again with init_* in FINISH
     const bool need_pass = (a.phases & BISSD_PHASE_LOCAL) || (a.init_f || a.init_b);
     if (need_pass) {
-        BISSD_LAUNCH("state_passing_fwd", launch_pdl(simt::state_passing_fwd4<T>, dim3(d.b * d.H, ceil_div(d.P * d.N, 4 * simt::TB), 2), simt::TB, 0, s,
+        BISSD_LAUNCH("state_passing_fwd", launch_pdl(pass_ahead(d) ? simt::state_passing_fwd4<T, 8> : simt::state_passing_fwd4<T, 1>, pass_grid(d), pass_threads(d), 0, s,
             d, loc, a.cs_f, a.cs_b, a.init_f, a.init_b, a.states_f, a.states_b, a.final_f, a.final_b));
     }
     if (a.phases & BISSD_PHASE_FINISH) {
@@ -372,9 +372,8 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
         }
     }
     const bool need_pass = (a.phases & BISSD_PHASE_LOCAL) || (a.dfinal_f || a.dfinal_b);
-    const int pass_nblk = ceil_div(d.P * d.N, 4 * simt::TB);     // dT partial slots per chunk
     if (need_pass) {
-        BISSD_LAUNCH("state_passing_bwd", launch_pdl(simt::state_passing_bwd4<T>, dim3(d.b * d.H, pass_nblk, 2), simt::TB, 0, s,
+        BISSD_LAUNCH("state_passing_bwd", launch_pdl(pass_ahead(d) ? simt::state_passing_bwd4<T, 8> : simt::state_passing_bwd4<T, 1>, pass_grid(d), pass_threads(d), 0, s,
             d, F(w.gloc), a.states_f, a.states_b, a.cs_f, a.cs_b, a.dfinal_f, a.dfinal_b, nullptr, E16, F(w.dTpart), a.dinit_f, a.dinit_b));
     }
     if (!(a.phases & BISSD_PHASE_FINISH)) return BISSD_OK;
@@ -683,7 +682,7 @@ do {                                                                            
     cs.nf = F(w.nf); cs.nb = F(w.nb); cs.pf = F(w.pf); cs.pb = F(w.pb);
     if (use_u4) { cs.u4 = F(w.u4); cs.u4_tiles = u4_tiles; }
     else { cs.da_f = F(w.da_f); cs.da_b = F(w.da_b); }
-    cs.dTpart = F(w.dTpart); cs.nblk = pass_nblk; cs.nsplit = nsplit; cs.ddt = gr.ddt; cs.dApart = F(w.dApart); cs.dbiaspart = F(w.dbiaspart);
+    cs.dTpart = F(w.dTpart); cs.nblk = w.nslots; cs.nsplit = nsplit; cs.ddt = gr.ddt; cs.dApart = F(w.dApart); cs.dbiaspart = F(w.dbiaspart);
     BISSD_LAUNCH("cumsum_bwd", launch_pdl(simt::cumsum_bwd, d.b * d.nc * d.H, 256, 0, s, d, cs));
     BISSD_LAUNCH("final_reduce", launch_pdl(simt::final_reduce<1024>, d.H, 1024, 0, s, 
         d, F(w.dApart), F(w.dbiaspart), d.has_D ? F(w.dDpart) : nullptr, dd_slots ? dd_slots : nlt, dd_compact ? 1 : 0, a.dA, d.has_bias ? a.ddt_bias : nullptr,

@@ -57,8 +57,8 @@ template <class T> static int forward_t(const bissd_fwd_args &a, const Dims &d, 
     if (rc != BISSD_OK) return rc;
     // the recurrence runs in both phases: from zero (or init_*) in LOCAL, again with init_* in FINISH
     if (local || a.init_f || a.init_b) {
-        if ((d.P * d.N) % 4 == 0) {
-            BISSD_LAUNCH("state_passing_fwd", launch_pdl(simt::state_passing_fwd4<T>, dim3(d.b * d.H, ceil_div(d.P * d.N, 4 * simt::TB), 2), simt::TB, 0, s,
+        if (pass_by4(d)) {
+            BISSD_LAUNCH("state_passing_fwd", launch_pdl(pass_ahead(d) ? simt::state_passing_fwd4<T, 8> : simt::state_passing_fwd4<T, 1>, pass_grid(d), pass_threads(d), 0, s,
                 d, loc, a.cs_f, a.cs_b, a.init_f, a.init_b, a.states_f, a.states_b, a.final_f, a.final_b));
         } else {
             BISSD_LAUNCH("state_passing_fwd", simt::state_passing_fwd<T><<<dim3(d.b * d.H, ceil_div(d.P * d.N, simt::TB), 2), simt::TB, 0, s>>>(
@@ -94,14 +94,12 @@ template <class T> static int backward_t(const bissd_bwd_args &a, const GradView
     sa.cs_f = const_cast<float *>(a.cs_f); sa.cs_b = const_cast<float *>(a.cs_b); sa.out = F(w.gloc);
     int rc = launch_states<T, true>(d, sa, Cm, Bm, F(w.cb), vec, local, finish, local ? reinterpret_cast<int *>(ws) : nullptr, s);
     if (rc != BISSD_OK) return rc;
-    const bool by4 = (d.P * d.N) % 4 == 0;
-    const int pass_nblk = by4 ? ceil_div(d.P * d.N, 4 * simt::TB) : w.nblk;   // dT partial slots per chunk
     if (local || a.dfinal_f || a.dfinal_b) {
-        if (by4) {
-            BISSD_LAUNCH("state_passing_bwd", launch_pdl(simt::state_passing_bwd4<T>, dim3(d.b * d.H, pass_nblk, 2), simt::TB, 0, s,
+        if (pass_by4(d)) {
+            BISSD_LAUNCH("state_passing_bwd", launch_pdl(pass_ahead(d) ? simt::state_passing_bwd4<T, 8> : simt::state_passing_bwd4<T, 1>, pass_grid(d), pass_threads(d), 0, s,
                 d, F(w.gloc), a.states_f, a.states_b, a.cs_f, a.cs_b, a.dfinal_f, a.dfinal_b, F(w.E), nullptr, F(w.dTpart), a.dinit_f, a.dinit_b));
         } else {
-            BISSD_LAUNCH("state_passing_bwd", simt::state_passing_bwd<T><<<dim3(d.b * d.H, pass_nblk, 2), simt::TB, 0, s>>>(
+            BISSD_LAUNCH("state_passing_bwd", simt::state_passing_bwd<T><<<dim3(d.b * d.H, ceil_div(d.P * d.N, simt::TB), 2), simt::TB, 0, s>>>(
                 d, F(w.gloc), a.states_f, a.states_b, a.cs_f, a.cs_b, a.dfinal_f, a.dfinal_b, F(w.E), nullptr, F(w.dTpart), a.dinit_f, a.dinit_b));
         }
     }
@@ -129,7 +127,7 @@ template <class T> static int backward_t(const bissd_bwd_args &a, const GradView
     cs.dt = a.dt.ptr; cs.dt_dtype = a.p.dt_dtype; cs.dsb = a.dt.stride_batch; cs.dsl = a.dt.stride_seq; cs.dsh = a.dt.stride_head;
     cs.A = a.A; cs.dt_bias = a.dt_bias; cs.dt_out = a.dt_out; cs.ddt_out = F(w.ddt_out);
     cs.nf = F(w.nf); cs.nb = F(w.nb); cs.pf = F(w.pf); cs.pb = F(w.pb); cs.u4 = F(w.u4); cs.u4_tiles = 2 * nt;
-    cs.dTpart = F(w.dTpart); cs.nblk = pass_nblk; cs.nsplit = 1; cs.ddt = gr.ddt; cs.dApart = F(w.dApart); cs.dbiaspart = F(w.dbiaspart);
+    cs.dTpart = F(w.dTpart); cs.nblk = w.nslots; cs.nsplit = 1; cs.ddt = gr.ddt; cs.dApart = F(w.dApart); cs.dbiaspart = F(w.dbiaspart);
     const int bmm = bcg * 2 * nt * ceil_div(d.N, twn);
     rc = by_width<T>(twn, [&](auto width) -> int {
         BISSD_LAUNCH("bmm_bwd_cumsum_bwd", launch_pdl(simt::backward3<T, decltype(width)::value>, bmm + bch, simt::TB, sizeof(simt::Panels), s,

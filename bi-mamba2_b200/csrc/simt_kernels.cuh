@@ -200,7 +200,7 @@ struct CumsumBwd {
     int dt_dtype;
     long long dsb, dsl, dsh;
     const float *A, *dt_bias, *dt_out, *ddt_out, *nf, *nb, *pf, *pb, *da_f, *da_b, *u4;
-    int u4_tiles;
+    int u4_tiles;                                                // 0 without u4
     const float *dTpart;
     int nblk, nsplit;
     MutView ddt;
@@ -217,29 +217,63 @@ __device__ __forceinline__ void cumsum_bwd_role(const Dims &d, const CumsumBwd &
     const long long split_stride = (long long)d.b * d.H * d.nc * d.Q;   // a.nf/a.nb/a.pf/a.pb hold a.nsplit partial copies
     // the four scanned sequences: a.nf (+u_f) and a.pb ascending, a.nb (+u_b) and a.pf descending
     float v1 = 0.f, v2 = 0.f, w1 = 0.f, w2 = 0.f, ex = 0.f, dto = 0.f, dlo = 0.f, pre = 0.f;
+    // Every load is requested before the first is used: with the sums next to their loads this kernel was one memory
+    // latency per term.
+    float ts[4] = {0.f, 0.f, 0.f, 0.f}, te[4] = {0.f, 0.f, 0.f, 0.f};
+    const float *slots_b = a.dTpart + ((long long)d.b * d.H * d.nc + tix) * a.nblk, *slots_f = a.dTpart + tix * a.nblk;
+    const bool last = warp == (d.Q - 1) >> 5;                    // the warp of position Q - 1
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (warp == 0 && lane + 32 * i < a.nblk) ts[i] = slots_b[lane + 32 * i];
+        if (last && lane + 32 * i < a.nblk) te[i] = slots_f[lane + 32 * i];
+    }
     if (l < d.Q) {
-        for (int k = 0; k < a.nsplit; ++k) {
-            v1 += a.nf[k * split_stride + base + l];
-            v2 += a.pb[k * split_stride + base + l];
-            w1 += a.nb[k * split_stride + base + l];
-            w2 += a.pf[k * split_stride + base + l];
+        const float n0 = a.nf[base + l], p0 = a.pb[base + l], q0 = a.nb[base + l], r0 = a.pf[base + l];
+        float uf[4] = {0.f, 0.f, 0.f, 0.f}, ub[4] = {0.f, 0.f, 0.f, 0.f};
+        if (a.u4) {                                              // (u_f, u_b) pairs, one per tile of the chunk
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (t < a.u4_tiles) {
+                    uf[t] = a.u4[(2 * t) * split_stride + base + l];
+                    ub[t] = a.u4[(2 * t + 1) * split_stride + base + l];
+                }
+        } else {
+            ex = a.da_f[base + l] + a.da_b[base + l];
         }
-        if (a.u4) {                                                         // (u_f, u_b) pairs, one per tile of the chunk
-            for (int t = 0; t < a.u4_tiles; ++t) {
-                v1 += a.u4[(2 * t) * split_stride + base + l];
-                w1 += a.u4[(2 * t + 1) * split_stride + base + l];
-            }
-        }
-        if (a.da_f) ex = a.da_f[base + l] + a.da_b[base + l];
-        if (l == 0)                                                       // dT_b enters at index 0, dT_f at index Q-1
-            for (int k = 0; k < a.nblk; ++k) v2 += a.dTpart[((long long)d.b * d.H * d.nc + tix) * a.nblk + k];
-        if (l == d.Q - 1)
-            for (int k = 0; k < a.nblk; ++k) w2 += a.dTpart[tix * a.nblk + k];
         if (l < lim) {
             dto = a.ddt_out[base + l];
             dlo = a.dt_out[base + l];
             pre = ld_any(a.dt, a.dt_dtype, b * a.dsb + (long long)(c * d.Q + l) * a.dsl + h * a.dsh) + (d.has_bias ? a.dt_bias[h] : 0.f);
         }
+        v1 = n0; v2 = p0; w1 = q0; w2 = r0;
+        for (int k = 1; k < a.nsplit; ++k) {
+            v1 += a.nf[k * split_stride + base + l];
+            v2 += a.pb[k * split_stride + base + l];
+            w1 += a.nb[k * split_stride + base + l];
+            w2 += a.pf[k * split_stride + base + l];
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            v1 += uf[t];
+            w1 += ub[t];
+        }
+        for (int t = 4; t < a.u4_tiles; ++t) {
+            v1 += a.u4[(2 * t) * split_stride + base + l];
+            w1 += a.u4[(2 * t + 1) * split_stride + base + l];
+        }
+    }
+    // dT_b enters at index 0, dT_f at index Q-1; the warp of that position adds up the slots
+    if (warp == 0) {
+        float t = (ts[0] + ts[1]) + (ts[2] + ts[3]);
+        for (int k = lane + 128; k < a.nblk; k += 32) t += slots_b[k];
+        t = warp_sum(t);
+        if (lane == 0) v2 += t;
+    }
+    if (last) {
+        float t = (te[0] + te[1]) + (te[2] + te[3]);
+        for (int k = lane + 128; k < a.nblk; k += 32) t += slots_f[k];
+        t = warp_sum(t);
+        if (l == d.Q - 1) w2 += t;
     }
     float s1 = v1, s2 = v2, r1 = w1, r2 = w2;
     block_scan4(s1, s2, r1, r2, tot);
@@ -383,8 +417,8 @@ template <class T> __device__ __forceinline__ float4 ld4(const void *p, long lon
     return make_float4(to_f<T>(v[0]), to_f<T>(v[1]), to_f<T>(v[2]), to_f<T>(v[3]));
 }
 
-// grid (b*H, ceil(P*N/1024), 2)
-template <class T>
+// grid (b*H, ceil(P*N/4/blockDim), 2)
+template <class T, int U>
 __global__ void __launch_bounds__(TB) state_passing_fwd4(Dims d, const float *loc, const float *cs_f, const float *cs_b,
                                                          const float *init_f, const float *init_b, void *states_f,
                                                          void *states_b, float *final_f, float *final_b) {
@@ -392,7 +426,7 @@ __global__ void __launch_bounds__(TB) state_passing_fwd4(Dims d, const float *lo
     const int h = blockIdx.x % d.H, b = blockIdx.x / d.H;
     const int dir = blockIdx.z;
     const int PN = d.P * d.N;
-    const int e = (blockIdx.y * TB + threadIdx.x) * 4;
+    const int e = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     if (e >= PN) return;
     const long long per_dir = (long long)d.b * d.nc * d.H * PN;
     const float *lp = loc + dir * per_dir;
@@ -403,69 +437,93 @@ __global__ void __launch_bounds__(TB) state_passing_fwd4(Dims d, const float *lo
     const long long cstride = (long long)d.H * PN;
     const long long off0 = ((long long)b * d.nc * d.H + h) * PN + e;
     const long long cb0 = (long long)(b * d.H + h) * d.nc * d.Q;
-#pragma unroll 4
-    for (int i = 0; i < d.nc; ++i) {
-        const int c = dir ? d.nc - 1 - i : i;
-        const long long off = off0 + c * cstride;
-        const float4 v = __ldg(reinterpret_cast<const float4 *>(lp + off));
-        const float dec = expf(dir ? cs_b[cb0 + (long long)c * d.Q] : cs_f[cb0 + (long long)c * d.Q + d.Q - 1]);
-        st4<T>(states, off, run.x, run.y, run.z, run.w);
-        run.x = dec * run.x + v.x;
-        run.y = dec * run.y + v.y;
-        run.z = dec * run.z + v.z;
-        run.w = dec * run.w + v.w;
+    for (int i0 = 0; i0 < d.nc; i0 += U) {
+        float4 v[U];
+        float dec[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = dir ? d.nc - 1 - i0 - u : i0 + u;
+            const bool have = i0 + u < d.nc;
+            v[u] = have ? __ldg(reinterpret_cast<const float4 *>(lp + off0 + c * cstride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            dec[u] = have ? (dir ? cs_b[cb0 + (long long)c * d.Q] : cs_f[cb0 + (long long)c * d.Q + d.Q - 1]) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i0 + u >= d.nc) break;
+            const int c = dir ? d.nc - 1 - i0 - u : i0 + u;
+            const float ed = expf(dec[u]);
+            st4<T>(states, off0 + c * cstride, run.x, run.y, run.z, run.w);
+            run.x = ed * run.x + v[u].x;
+            run.y = ed * run.y + v[u].y;
+            run.z = ed * run.z + v[u].z;
+            run.w = ed * run.w + v[u].w;
+        }
     }
     if (fin) *reinterpret_cast<float4 *>(fin + (long long)(b * d.H + h) * PN + e) = run;
 }
 
-// grid (b*H, nblk4 = ceil(P*N/1024), 2); dTpart has nblk4 slots per (dir, b, h, c)
-template <class T>
+// grid (b*H, ceil(P*N/4/blockDim), 2), blockDim a multiple of 32; dTpart has one slot per warp of a (dir, b, h): gridDim.y *
+// blockDim / 32 - one per warp instead of one per block keeps barriers out of the loop (b8 H24 nc8 P64 N128 bf16: 43 -> 39
+// us).  U: chunks whose loads are in flight together, see pass_ahead().
+template <class T, int U>
 __global__ void __launch_bounds__(TB) state_passing_bwd4(Dims d, const float *gloc, const void *states_f,
                                                          const void *states_b, const float *cs_f, const float *cs_b,
                                                          const float *dfinal_f, const float *dfinal_b, float *E,
                                                          void *E16, float *dTpart, float *dinit_f, float *dinit_b) {
     pdl_begin();
-    __shared__ float red[TB / 32];
     const int h = blockIdx.x % d.H, b = blockIdx.x / d.H;
     const int dir = blockIdx.z;
     const int PN = d.P * d.N;
-    const int nblk = gridDim.y;
-    const int e = (blockIdx.y * TB + threadIdx.x) * 4;
+    const int nslots = gridDim.y * (blockDim.x >> 5), slot = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int e = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     const bool on = e < PN;
     const long long per_dir = (long long)d.b * d.nc * d.H * PN;
     const float *gp = gloc + dir * per_dir;
     const void *states = dir ? states_b : states_f;
     const float *dfin = dir ? dfinal_b : dfinal_f;
     float *dinit = dir ? dinit_b : dinit_f;
-    float4 run = (on && dfin) ? *reinterpret_cast<const float4 *>(dfin + (long long)(b * d.H + h) * PN + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 run = (on && dfin) ? *reinterpret_cast<const float4 *>(dfin + (long long)(b * d.H + h) * PN + e) : zero;
     const long long cstride = (long long)d.H * PN;
     const long long off0 = ((long long)b * d.nc * d.H + h) * PN + e;
-    const long long cb0 = (long long)(b * d.H + h) * d.nc * d.Q;
-    for (int i = 0; i < d.nc; ++i) {
-        const int c = dir ? i : d.nc - 1 - i;
-        const long long off = off0 + c * cstride;
-        const float dec = expf(dir ? cs_b[cb0 + (long long)c * d.Q] : cs_f[cb0 + (long long)c * d.Q + d.Q - 1]);
-        float part = 0.f;
-        if (on) {
-            const float4 gv = __ldg(reinterpret_cast<const float4 *>(gp + off));
-            const float4 sv = ld4<T>(states, off);
-            if (E) *reinterpret_cast<float4 *>(E + dir * per_dir + off) = run;
-            if (E16) st4<T>(E16, dir * per_dir + off, run.x, run.y, run.z, run.w);
-            part = dec * (sv.x * run.x + sv.y * run.y + sv.z * run.z + sv.w * run.w);
-            run.x = dec * run.x + gv.x;
-            run.y = dec * run.y + gv.y;
-            run.z = dec * run.z + gv.z;
-            run.w = dec * run.w + gv.w;
+    const float *total = (dir ? cs_b : cs_f + d.Q - 1) + (long long)(b * d.H + h) * d.nc * d.Q;      // T of chunk 0
+    float *slots = dTpart + ((long long)dir * d.b * d.H * d.nc + (long long)(b * d.H + h) * d.nc) * nslots + slot;
+    for (int i0 = 0; i0 < d.nc; i0 += U) {
+        float4 gv[U], sv[U];
+        float dec[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = dir ? i0 + u : d.nc - 1 - i0 - u;
+            const bool have = on && i0 + u < d.nc;
+            gv[u] = have ? __ldg(reinterpret_cast<const float4 *>(gp + off0 + c * cstride)) : zero;
+            sv[u] = have ? ld4<T>(states, off0 + c * cstride) : zero;
+            dec[u] = i0 + u < d.nc ? total[(long long)c * d.Q] : 0.f;
         }
-        part = warp_sum(part);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float s = 0.f;
-            for (int w = 0; w < TB / 32; ++w) s += red[w];
-            dTpart[((long long)dir * d.b * d.H * d.nc + (long long)(b * d.H + h) * d.nc + c) * nblk + blockIdx.y] = s;
+        float part[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = dir ? i0 + u : d.nc - 1 - i0 - u;
+            const long long off = off0 + c * cstride;
+            const float ed = expf(dec[u]);
+            part[u] = ed * (sv[u].x * run.x + sv[u].y * run.y + sv[u].z * run.z + sv[u].w * run.w);
+            if (i0 + u < d.nc) {
+                if (on) {
+                    if (E) *reinterpret_cast<float4 *>(E + dir * per_dir + off) = run;
+                    if (E16) st4<T>(E16, dir * per_dir + off, run.x, run.y, run.z, run.w);
+                }
+                run.x = ed * run.x + gv[u].x;
+                run.y = ed * run.y + gv[u].y;
+                run.z = ed * run.z + gv[u].z;
+                run.w = ed * run.w + gv[u].w;
+            }
         }
-        __syncthreads();
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < U; ++u) part[u] += __shfl_xor_sync(0xffffffffu, part[u], o);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if ((threadIdx.x & 31) == 0 && i0 + u < d.nc) slots[(long long)(dir ? i0 + u : d.nc - 1 - i0 - u) * nslots] = part[u];
     }
     if (on && dinit) *reinterpret_cast<float4 *>(dinit + (long long)(b * d.H + h) * PN + e) = run;
 }

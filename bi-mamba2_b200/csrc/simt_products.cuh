@@ -14,8 +14,9 @@
 //
 // Decay factors, masks, gates and the two directions are applied while a panel is put into shared memory; where a product
 // runs over both directions its depth is simply [forward | reverse].
-// Bound by shared-memory reads and by block latency.  fp32, b1 L256 H4 P32 N16 Q64, forward + backward: 156 -> see
-// DISPATCH below; b2 L8192 H4 G4 P16 N16 Q128: one product per launch with 64-wide tiles and a panel of 16 before.
+// Bound by shared-memory reads and instruction issue, small problems by block and launch latency.  Device time of a
+// forward + backward pass, fp32, against one product per launch with 64-wide tiles and 16-deep panels filled element by
+// element: b1 L256 H4 P32 N16 Q64 156 -> 48 us (17 -> 8 launches), b2 L8192 H4 G4 P16 N16 Q128 1012 -> 311 us.
 #pragma once
 #include "simt_kernels.cuh"
 
@@ -25,7 +26,7 @@ namespace simt {
 struct Panels {                                                  // dynamic shared memory of every kernel here
     float a[TILE * LD];
     float b[TILE * LD];
-    float v[4][256];                                             // per-position vectors of the chunk
+    float v[5][256];                                             // per-position vectors of the chunk (16-byte aligned)
     float red[8][2][TILE];
 };
 
@@ -72,20 +73,40 @@ __device__ __forceinline__ void fetch_gated(Frag &fr, int sh, const Dims &d, con
         });
     }
 }
-// Decay between two positions of a chunk, both directions (both on the diagonal).
-__device__ __forceinline__ float decay2(const float *sf, const float *sb, int to, int from) {
-    float w = 0.f;
-    if (from <= to) w += expf(sf[to] - sf[from]);
-    if (from >= to) w += expf(sb[to] - sb[from]);
-    return w;
-}
-__device__ __forceinline__ void load_vectors(Panels &sm, const Dims &d, const Where &w, const float *dt_out, const float *cs_f, const float *cs_b) {
-    for (int l = threadIdx.x; l < d.Q; l += TB) {
-        sm.v[0][l] = cs_f[w.base + l];
-        sm.v[1][l] = cs_b[w.base + l];
-        sm.v[2][l] = dt_out[w.base + l];
-    }
+// The chunk's per-position vectors: cumulative sums, Delta, and the decay inside each quad of positions - to its last
+// position (reverse: its first), so that four adjacent weights cost one exponential and four products.
+struct Vectors {
+    const float *sf, *sb, *sd, *qf, *qb;
+};
+__device__ __forceinline__ Vectors load_vectors(Panels &sm, const Dims &d, const Where &w, const float *dt_out, const float *cs_f, const float *cs_b) {
+    const int l = threadIdx.x;                                   // beyond the chunk: finite values that meet zeros only
+    const float f = cs_f[w.base + min(l, d.Q - 1)], r = l < d.Q ? cs_b[w.base + l] : 0.f;
+    sm.v[0][l] = f;
+    sm.v[1][l] = r;
+    sm.v[2][l] = l < d.Q ? dt_out[w.base + l] : 0.f;
+    // a quad's ends are in this thread's warp
+    const float fe = __shfl_sync(0xffffffffu, f, (l & 31) | 3), re = __shfl_sync(0xffffffffu, r, l & 28);
+    sm.v[3][l] = expf(fe - f);
+    sm.v[4][l] = expf(re - r);
     __syncthreads();
+    return Vectors{sm.v[0], sm.v[1], sm.v[2], sm.v[3], sm.v[4]};
+}
+// Decay from positions from ... from + 3 (a quad) to position `to` of a chunk, both directions (both on the diagonal).
+// All exponents are <= 0.
+__device__ __forceinline__ float4 decay4(const Vectors &v, int to, int from) {
+    const bool below = from + 3 < to, above = from > to;
+    if (below || above) {
+        const float e = below ? expf(v.sf[to] - v.sf[from + 3]) : expf(v.sb[to] - v.sb[from]);
+        const float4 q = *reinterpret_cast<const float4 *>((below ? v.qf : v.qb) + from);
+        return make_float4(e * q.x, e * q.y, e * q.z, e * q.w);
+    }
+    float w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int s = from + i;
+        w[i] = (s <= to ? expf(v.sf[to] - v.sf[s]) : 0.f) + (s >= to ? expf(v.sb[to] - v.sb[s]) : 0.f);
+    }
+    return make_float4(w[0], w[1], w[2], w[3]);
 }
 
 // Local chunk states, or their gradients, for both directions: out[dir][b,c,h,p,n] = sum_l X[l,p] Y[l,n] w_dir[l], as a
@@ -131,8 +152,8 @@ __device__ __forceinline__ void states_role(Panels &sm, const Dims &d, const Sta
     }
     __syncthreads();
     const int shA = shift_for(2 * d.N - m0), shB = shift_for(min(d.P - p0, TW));
-    Acc<TW> acc;
-    acc.zero();
+    Mul mul;
+    mul.zero();
     Frag fa, fb;
     panels(w.lim, [&](int k0) {
         pieces(shA, [&](int u, int r, int c) {
@@ -149,7 +170,8 @@ __device__ __forceinline__ void states_role(Panels &sm, const Dims &d, const Sta
     }, [&](int) {
         put_rows(fa, shA, sm.a);
         put_rows(fb, shB, sm.b);
-    }, [&](int, int depth) { compute_tn<TW>(acc, sm.a, sm.b, depth); });
+    }, [&](int, int depth) { compute_tn<TW>(mul, sm.a, sm.b, depth); });
+    const Acc<TW> acc = finish<TW>(mul, sm.a);
     const long long per_dir = (long long)d.b * d.nc * d.H * d.P * d.N;
     float *out = a.out + ((long long)(w.b * d.nc + w.c) * d.H + w.h) * d.P * d.N;
 #pragma unroll
@@ -170,16 +192,17 @@ template <class T> __device__ __forceinline__ void cb_role(Panels &sm, const Dim
     const int nt = ceil_div(d.Q, TILE), tile = block % (nt * nt), bcg = block / (nt * nt);
     const int g = bcg % d.G, c = (bcg / d.G) % d.nc, b = bcg / (d.G * d.nc), lim = min(d.Q, d.L - c * d.Q);
     const int l0 = tile / nt * TILE, s0 = tile % nt * TILE, sh = shift_for(min(d.N, TILE));
-    Acc<64> acc;
-    acc.zero();
+    Mul mul;
+    mul.zero();
     Frag fa, fb;
-    panels(d.N, [&](int k0) {
+    panels<false>(d.N, [&](int k0) {
         fetch<T>(fa, sh, row_ptr<T>(Cm, b, c * d.Q + l0, g) + k0, Cm.sl, lim - l0, d.N - k0, vec & VEC_BC);
         fetch<T>(fb, sh, row_ptr<T>(Bm, b, c * d.Q + s0, g) + k0, Bm.sl, lim - s0, d.N - k0, vec & VEC_BC);
     }, [&](int) {
         put_rows(fa, sh, sm.a);
         put_transposed(fb, sh, sm.b);
-    }, [&](int, int depth) { compute_nn<64>(acc, sm.a, sm.b, depth); });
+    }, [&](int, int depth) { compute_nn<64, true>(mul, sm.a, sm.b, depth); });
+    const Acc<64> acc = finish<64>(mul, sm.a);
     const int s = s0 + Acc<64>::col0();
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -200,7 +223,7 @@ struct ScanArgs {
     const void *states_f, *states_b;
     MutView out, out_x;
 };
-template <class T, int TW> __global__ void __launch_bounds__(TB, 2) chunk_scan(Dims d, ScanArgs a, int vec) {
+template <class T, int TW> __global__ void __launch_bounds__(TB, TW == 64 ? 2 : 3) chunk_scan(Dims d, ScanArgs a, int vec) {
     extern __shared__ char smem[];
     Panels &sm = *reinterpret_cast<Panels *>(smem);
     pdl_begin();
@@ -208,16 +231,16 @@ template <class T, int TW> __global__ void __launch_bounds__(TB, 2) chunk_scan(D
     const Where w(d, blockIdx.x / (lt * pt));
     const int l0 = tile % lt * TILE, p0 = tile / lt * TW;
     if (l0 >= w.lim) return;
-    load_vectors(sm, d, w, a.dt_out, a.cs_f, a.cs_b);
-    const float *sf = sm.v[0], *sb = sm.v[1], *sd = sm.v[2];
+    const Vectors v = load_vectors(sm, d, w, a.dt_out, a.cs_f, a.cs_b);
+    const float *sf = v.sf, *sb = v.sb, *sd = v.sd;
     const float *cb = a.CB + (((long long)w.b * d.nc + w.c) * d.G + w.g) * d.Q * d.Q;
     const long long st = (((long long)w.b * d.nc + w.c) * d.H + w.h) * d.P * N;
     const T *Sf = static_cast<const T *>(a.states_f) + st, *Sb = static_cast<const T *>(a.states_b) + st;
-    Acc<TW> acc;
-    acc.zero();
+    Mul mul;
+    mul.zero();
     Frag fa, fb;
     const int rows = w.lim - l0, shN = shift_for(2 * N);
-    panels(2 * N, [&](int k0) {
+    panels<false>(2 * N, [&](int k0) {
         pieces(shN, [&](int u, int r, int c) {
             const int k = k0 + c;
             fa.v[u] = fb.v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -234,16 +257,21 @@ template <class T, int TW> __global__ void __launch_bounds__(TB, 2) chunk_scan(D
     }, [&](int) {
         put_rows(fa, shN, sm.a);
         put_transposed(fb, shN, sm.b);
-    }, [&](int, int depth) { compute_nn<TW>(acc, sm.a, sm.b, depth); });
+    }, [&](int, int depth) { compute_nn<TW, true>(mul, sm.a, sm.b, depth); });
     const int shQ = shift_for(w.lim), shP = shift_for(min(d.P - p0, TW));
     panels(w.lim, [&](int k0) {
         fetch<float>(fa, shQ, cb + (long long)l0 * d.Q + k0, d.Q, rows, w.lim - k0, vec & VEC_Q);
         fetch<T>(fb, shP, row_ptr<T>(a.x, w.b, w.l0 + k0, w.h) + p0, a.x.sl, w.lim - k0, d.P - p0, vec & VEC_X);
     }, [&](int k0) {
-        scale(fa, shQ, [&](int r, int c) { return r < rows && k0 + c < w.lim ? sd[k0 + c] * decay2(sf, sb, l0 + r, k0 + c) : 0.f; });
+        pieces(shQ, [&](int u, int r, int c) {
+            if (r >= rows || k0 + c >= w.lim) return;            // zeros already
+            const float4 e = decay4(v, l0 + r, k0 + c), t = *reinterpret_cast<const float4 *>(sd + k0 + c);
+            fa.v[u] = make_float4(fa.v[u].x * (e.x * t.x), fa.v[u].y * (e.y * t.y), fa.v[u].z * (e.z * t.z), fa.v[u].w * (e.w * t.w));
+        });
         put_rows(fa, shQ, sm.a);
         put_rows(fb, shP, sm.b);
-    }, [&](int, int depth) { compute_nn<TW>(acc, sm.a, sm.b, depth); });
+    }, [&](int, int depth) { compute_nn<TW, false>(mul, sm.a, sm.b, depth); });
+    const Acc<TW> acc = finish<TW>(mul, sm.a);
     const int p = p0 + Acc<TW>::col0(), n = d.P - p;
     if (n <= 0) return;
 #pragma unroll
@@ -292,8 +320,8 @@ struct BwdArgs {
 template <class T, int TW> __device__ __forceinline__ void dx_role(Panels &sm, const Dims &d, const BwdArgs &a, int vec, int block) {
     const int lt = ceil_div(d.Q, TILE), N = d.N, l0 = block % lt * TILE;
     const Where w(d, block / lt);
-    load_vectors(sm, d, w, a.dt_out, a.cs_f, a.cs_b);
-    const float *sf = sm.v[0], *sb = sm.v[1], *sd = sm.v[2];
+    const Vectors v = load_vectors(sm, d, w, a.dt_out, a.cs_f, a.cs_b);
+    const float *sf = v.sf, *sb = v.sb, *sd = v.sd;
     const float Tf = sf[d.Q - 1], Tb = sb[0];
     const float *cb = a.CB + (((long long)w.b * d.nc + w.c) * d.G + w.g) * d.Q * d.Q;
     const long long st = (((long long)w.b * d.nc + w.c) * d.H + w.h) * d.P * N;
@@ -303,10 +331,10 @@ template <class T, int TW> __device__ __forceinline__ void dx_role(Panels &sm, c
 #pragma unroll
     for (int i = 0; i < Acc<TW>::RI; ++i) rowsum[i] = 0.f;
     for (int p0 = 0; p0 < d.P; p0 += TW) {
-        Acc<TW> acc;
-        acc.zero();
+        Mul mul;
+        mul.zero();
         Frag fa, fb;
-        panels(2 * N, [&](int k0) {
+        panels<false>(2 * N, [&](int k0) {
             pieces(shN, [&](int u, int r, int c) {
                 const int k = k0 + c;
                 fa.v[u] = fb.v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -323,16 +351,21 @@ template <class T, int TW> __device__ __forceinline__ void dx_role(Panels &sm, c
         }, [&](int) {
             put_rows(fa, shN, sm.a);
             put_transposed(fb, shN, sm.b);
-        }, [&](int, int depth) { compute_nn<TW>(acc, sm.a, sm.b, depth); });
+        }, [&](int, int depth) { compute_nn<TW, true>(mul, sm.a, sm.b, depth); });
         const int shP = shift_for(min(d.P - p0, TW));
         panels(w.lim, [&](int k0) {
             fetch<float>(fa, shL, cb + (long long)k0 * d.Q + l0, d.Q, w.lim - k0, rows, vec & VEC_Q);
             fetch_gated<T>(fb, shP, d, a.dout, a.z, w.b, w.l0 + k0, w.h, p0, w.lim - k0, d.P - p0, vec & VEC_X);
         }, [&](int k0) {
-            scale(fa, shL, [&](int r, int c) { return k0 + r < w.lim && c < rows ? decay2(sf, sb, k0 + r, l0 + c) : 0.f; });
+            pieces(shL, [&](int u, int r, int c) {
+                if (k0 + r >= w.lim || c >= rows) return;        // zeros already
+                const float4 e = decay4(v, k0 + r, l0 + c);
+                fa.v[u] = make_float4(fa.v[u].x * e.x, fa.v[u].y * e.y, fa.v[u].z * e.z, fa.v[u].w * e.w);
+            });
             put_rows(fa, shL, sm.a);
             put_rows(fb, shP, sm.b);
-        }, [&](int, int depth) { compute_tn<TW>(acc, sm.a, sm.b, depth); });
+        }, [&](int, int depth) { compute_tn<TW>(mul, sm.a, sm.b, depth); });
+        const Acc<TW> acc = finish<TW>(mul, sm.a);
         const int p = p0 + Acc<TW>::col0(), n = d.P - p;
         float colsum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -413,17 +446,19 @@ __device__ __forceinline__ void dbc_half(Panels &sm, const Dims &d, const BwdArg
         const int shN = shift_for(min(N - n0, TW));
 #pragma unroll
         for (int dir = 0; dir < 2; ++dir) {
-            acc[dir].zero();
+            Mul mul;
+            mul.zero();
             const S *from = (dir ? Sb : Sf) + n0;
             Frag fa, fb;
-            panels(d.P, [&](int k0) {
+            panels<false>(d.P, [&](int k0) {
                 if (which) fetch_gated<T>(fa, shP, d, a.dout, a.z, w.b, w.l0 + l0, w.h, k0, rows, d.P - k0, vec & VEC_X);
                 else fetch<T>(fa, shP, row_ptr<T>(a.x, w.b, w.l0 + l0, w.h) + k0, a.x.sl, rows, d.P - k0, vec & VEC_X);
                 fetch<S>(fb, shN, from + (long long)k0 * N, N, d.P - k0, N - n0, vec & VEC_N);
             }, [&](int) {
                 put_rows(fa, shP, sm.a);
                 put_rows(fb, shN, sm.b);
-            }, [&](int, int depth) { compute_nn<TW>(acc[dir], sm.a, sm.b, depth); });
+            }, [&](int, int depth) { compute_nn<TW, false>(mul, sm.a, sm.b, depth); });
+            acc[dir] = finish<TW>(mul, sm.a);
         }
         const int nn = n0 + Acc<TW>::col0();
 #pragma unroll
@@ -480,54 +515,73 @@ template <class T> __device__ __forceinline__ void dcb_role(Panels &sm, const Di
     const int lt = tile / nt, st = tile % nt, l0 = lt * TILE, s0 = st * TILE, heads = d.R / a.hsplit, shP = shift_for(d.P);
     const int lr = l0 + Acc<64>::row0(), sc = s0 + Acc<64>::col0(), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long stride = (long long)d.b * d.H * d.nc * d.Q;
-    float cbv[4][4], tot[4][4];
+    float tot[4][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float4 v = lr + i < lim ? load4<float>(a.CB + ((long long)bcg * d.Q + lr + i) * d.Q + sc, d.Q - sc, vec & VEC_Q) : make_float4(0.f, 0.f, 0.f, 0.f);
-        cbv[i][0] = v.x; cbv[i][1] = v.y; cbv[i][2] = v.z; cbv[i][3] = v.w;
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) tot[i][j] = 0.f;
-    }
     for (int r = 0; r < heads; ++r) {
         Where w(d, (b * d.nc + c) * d.H + g * d.R + part * heads + r);
         __syncthreads();                                         // the vectors' and sums' last readers are done
-        load_vectors(sm, d, w, a.dt_out, a.cs_f, a.cs_b);
-        const float *sf = sm.v[0], *sb = sm.v[1], *sd = sm.v[2];
-        Acc<64> acc;
-        acc.zero();
+        const Vectors vec4 = load_vectors(sm, d, w, a.dt_out, a.cs_f, a.cs_b);
+        const float *sf = vec4.sf, *sb = vec4.sb, *sd = vec4.sd;
+        Mul mul;
+        mul.zero();
         Frag fa, fb;
-        panels(d.P, [&](int k0) {
+        panels<false>(d.P, [&](int k0) {
             fetch_gated<T>(fa, shP, d, a.dout, a.z, b, w.l0 + l0, w.h, k0, lim - l0, d.P - k0, vec & VEC_X);
             fetch<T>(fb, shP, row_ptr<T>(a.x, b, w.l0 + s0, w.h) + k0, a.x.sl, lim - s0, d.P - k0, vec & VEC_X);
         }, [&](int) {
             put_rows(fa, shP, sm.a);
             put_transposed(fb, shP, sm.b);
-        }, [&](int, int depth) { compute_nn<64>(acc, sm.a, sm.b, depth); });
-        float rowf[4], rowb[4], colf[4], colb[4];
+        }, [&](int, int depth) { compute_nn<64, true>(mul, sm.a, sm.b, depth); });
+        const Acc<64> acc = finish<64>(mul, sm.a);
+        float rowf[4], rowb[4], colf[4], colb[4], et[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) rowf[i] = rowb[i] = colf[i] = colb[i] = 0.f;
+        for (int j = 0; j < 4; ++j) {
+            rowf[j] = rowb[j] = colf[j] = colb[j] = 0.f;
+            et[j] = sc + j < lim ? sd[sc + j] : 0.f;
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int l = lr + i;
+            if (l >= lim) continue;
+            const float4 cq = load4<float>(a.CB + ((long long)bcg * d.Q + l) * d.Q + sc, d.Q - sc, vec & VEC_Q);
+            const float cbv[4] = {cq.x, cq.y, cq.z, cq.w};
+            if (sc + 3 < l || sc > l) {                          // the four columns lie on one side of the diagonal
+                const float4 e = decay4(vec4, l, sc);
+                const float es[4] = {e.x, e.y, e.z, e.w};
+                float row = 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float v = acc.v[i][j] * (et[j] * es[j]), u = v * cbv[j];
+                    tot[i][j] += v;
+                    row += u;
+                    if (sc > l) colb[j] += u;
+                    else colf[j] += u;
+                }
+                if (sc > l) rowb[i] += row;
+                else rowf[i] += row;
+                continue;
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int s = sc + j;
-                if (l >= lim || s >= lim) continue;
-                const float t = acc.v[i][j] * sd[s];
+                const float t = acc.v[i][j] * et[j];
                 if (s <= l) {
                     const float v = t * expf(sf[l] - sf[s]);
                     tot[i][j] += v;
                     if (s < l) {
-                        rowf[i] += v * cbv[i][j];
-                        colf[j] += v * cbv[i][j];
+                        rowf[i] += v * cbv[j];
+                        colf[j] += v * cbv[j];
                     }
                 }
                 if (s >= l) {
                     const float v = t * expf(sb[l] - sb[s]);
                     tot[i][j] += v;
                     if (s > l) {
-                        rowb[i] += v * cbv[i][j];
-                        colb[j] += v * cbv[i][j];
+                        rowb[i] += v * cbv[j];
+                        colb[j] += v * cbv[j];
                     }
                 }
             }
@@ -573,8 +627,8 @@ template <class T, int TW> __device__ __forceinline__ void bmm_bwd_role(Panels &
     const float *dcb = a.dCB + (long long)bcg * a.hsplit * d.Q * d.Q;
     const View &Y = which ? a.Bm : a.Cm;
     const int shR = shift_for(which ? lim : lim - r0), shN = shift_for(min(d.N - n0, TW));
-    Acc<TW> acc;
-    acc.zero();
+    Mul mul;
+    mul.zero();
     Frag fa, fb;
     panels(lim, [&](int k0) {                                    // dC: rows r0 of dCB, depth along them; dB: the other way
         const int fr = which ? r0 : k0, fc = which ? k0 : r0;
@@ -591,9 +645,10 @@ template <class T, int TW> __device__ __forceinline__ void bmm_bwd_role(Panels &
         put_rows(fa, shR, sm.a);
         put_rows(fb, shN, sm.b);
     }, [&](int, int depth) {
-        if (which) compute_nn<TW>(acc, sm.a, sm.b, depth);
-        else compute_tn<TW>(acc, sm.a, sm.b, depth);
+        if (which) compute_nn<TW, false>(mul, sm.a, sm.b, depth);
+        else compute_tn<TW>(mul, sm.a, sm.b, depth);
     });
+    const Acc<TW> acc = finish<TW>(mul, sm.a);
     const float *part = which ? a.dC_part : a.dB_part;
     const MutView &out = which ? a.dC : a.dB;
     const int nn = n0 + Acc<TW>::col0();
@@ -616,7 +671,7 @@ template <class T, int TW> __device__ __forceinline__ void bmm_bwd_role(Panels &
 // Blocks of the first role come first; `first` and `second` are the roles' block counts.  The first kernel of a pass
 // clears the workspace header (the status word, which these kernels never raise).
 template <class T, bool GRAD, int TW>
-__global__ void __launch_bounds__(TB, 2) states_and_cb(Dims d, StateArgs a, View Cm, View Bm, float *CB, int vec, int first, int *header) {
+__global__ void __launch_bounds__(TB, 3) states_and_cb(Dims d, StateArgs a, View Cm, View Bm, float *CB, int vec, int first, int *header) {
     extern __shared__ char smem[];
     Panels &sm = *reinterpret_cast<Panels *>(smem);
     pdl_begin();
@@ -633,7 +688,7 @@ template <class T, int TWP, int TWN> __global__ void __launch_bounds__(TB, 2) ba
     else if (block < first + second) dx_role<T, TWP>(sm, d, a, vec, block - first);
     else dbc_role<T, TWN>(sm, d, a, vec, block - first - second);
 }
-template <class T, int TWN> __global__ void __launch_bounds__(TB, 2) backward3(Dims d, BwdArgs a, CumsumBwd cs, int vec, int first) {
+template <class T, int TWN> __global__ void __launch_bounds__(TB, TWN == 64 ? 2 : 3) backward3(Dims d, BwdArgs a, CumsumBwd cs, int vec, int first) {
     extern __shared__ char smem[];
     Panels &sm = *reinterpret_cast<Panels *>(smem);
     pdl_begin();

@@ -2,8 +2,8 @@
 // 64 x 64 in shared memory filled from global memory four elements at a time.
 //
 // A block has 256 threads.  TW (16, 32 or 64) is the width of what the tile's columns run over - headdim, dstate or
-// chunk positions - so that narrow heads do not pay for 64 columns: thread (ty, tx) holds TW / 16 adjacent rows and four
-// adjacent columns.  Panels are at most 64 deep; the next panel's global loads are in flight while one is multiplied.
+// chunk positions - so that narrow heads do not pay for 64 columns.  Panels are at most 64 deep; where several follow one
+// another the next one's global loads are in flight while one is multiplied.
 #pragma once
 #include "common.cuh"
 
@@ -16,67 +16,100 @@ constexpr int LD = TILE + 4; // floats per panel row: 16-byte rows, and the four
 
 __host__ __device__ inline int width_for(int n) { return n <= 16 ? 16 : (n <= 32 ? 32 : 64); }
 
+// A finished tile: thread (ty, tx) holds TW / 16 adjacent rows and four adjacent columns.
 template <int TW> struct Acc {
     static constexpr int RI = TW / 16, NTX = TW / 4;
     float v[RI][4];
-    __device__ __forceinline__ void zero() {
-#pragma unroll
-        for (int i = 0; i < RI; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[i][j] = 0.f;
-    }
     static __device__ __forceinline__ int row0() { return threadIdx.x / NTX * RI; }
     static __device__ __forceinline__ int col0() { return threadIdx.x % NTX * 4; }
 };
 
-// acc += A B over kb panel steps.  A row-major: As[m][k];  B: Bs[k][n].
-template <int TW> __device__ __forceinline__ void compute_nn(Acc<TW> &acc, const float *As, const float *Bs, int kb) {
-    constexpr int RI = Acc<TW>::RI;
-    const float *a0 = As + Acc<TW>::row0() * LD, *b0 = Bs + Acc<TW>::col0();
-#pragma unroll 2
-    for (int k = 0; k < kb; k += 4) {
-        float4 a[RI];
+// A tile being multiplied: 4 x 4 values per thread whatever TW, so that a shared-memory read feeds four rows or columns
+// (a 16-byte read costs a warp four cycles of the shared-memory pipe even where lanes read the same bytes; with TW / 16
+// rows per thread that pipe was the limit).  The 64 / TW thread groups this leaves take every (64 / TW)-th step of the
+// depth; finish() adds them up.
+struct Mul {
+    float v[4][4];
+    __device__ __forceinline__ void zero() {
 #pragma unroll
-        for (int i = 0; i < RI; ++i) a[i] = *reinterpret_cast<const float4 *>(a0 + i * LD + k);
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float4 b = *reinterpret_cast<const float4 *>(b0 + (k + q) * LD);
+            for (int j = 0; j < 4; ++j) v[i][j] = 0.f;
+    }
+    __device__ __forceinline__ void step(const float (&a)[4], float4 b) {
 #pragma unroll
-            for (int i = 0; i < RI; ++i) {
-                const float s = q == 0 ? a[i].x : (q == 1 ? a[i].y : (q == 2 ? a[i].z : a[i].w));
-                acc.v[i][0] = fmaf(s, b.x, acc.v[i][0]);
-                acc.v[i][1] = fmaf(s, b.y, acc.v[i][1]);
-                acc.v[i][2] = fmaf(s, b.z, acc.v[i][2]);
-                acc.v[i][3] = fmaf(s, b.w, acc.v[i][3]);
-            }
+        for (int i = 0; i < 4; ++i) {
+            v[i][0] = fmaf(a[i], b.x, v[i][0]);
+            v[i][1] = fmaf(a[i], b.y, v[i][1]);
+            v[i][2] = fmaf(a[i], b.z, v[i][2]);
+            v[i][3] = fmaf(a[i], b.w, v[i][3]);
         }
+    }
+};
+template <int TW> struct MulAt {
+    static constexpr int NG = 64 / TW, NT = TB / NG, NTX = TW / 4;
+    int grp, row, col;
+    __device__ __forceinline__ MulAt() {
+        const int t = threadIdx.x % NT;
+        grp = threadIdx.x / NT; row = t / NTX * 4; col = t % NTX * 4;
+    }
+};
+
+// m += A B over kb panel steps.  A row-major: As[m][k];  B: Bs[k][n], its columns swizzled by put_transposed where SWZ.
+template <int TW, bool SWZ> __device__ __forceinline__ void compute_nn(Mul &m, const float *As, const float *Bs, int kb) {
+    const MulAt<TW> at;
+    const float *a0 = As + at.row * LD;
+#pragma unroll 2
+    for (int k = at.grp * 4; k < kb; k += 4 * MulAt<TW>::NG) {
+        float4 a[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4 *>(a0 + i * LD + k);
+        const float *b0 = Bs + k * LD + (SWZ ? at.col ^ (k & 28) : at.col);
+        const float ax[4] = {a[0].x, a[1].x, a[2].x, a[3].x}, ay[4] = {a[0].y, a[1].y, a[2].y, a[3].y};
+        const float az[4] = {a[0].z, a[1].z, a[2].z, a[3].z}, aw[4] = {a[0].w, a[1].w, a[2].w, a[3].w};
+        m.step(ax, *reinterpret_cast<const float4 *>(b0));
+        m.step(ay, *reinterpret_cast<const float4 *>(b0 + LD));
+        m.step(az, *reinterpret_cast<const float4 *>(b0 + 2 * LD));
+        m.step(aw, *reinterpret_cast<const float4 *>(b0 + 3 * LD));
     }
 }
 // The same with A stored step-major: As[k][m].
-template <int TW> __device__ __forceinline__ void compute_tn(Acc<TW> &acc, const float *As, const float *Bs, int kb) {
-    constexpr int RI = Acc<TW>::RI;
-    const float *a0 = As + Acc<TW>::row0(), *b0 = Bs + Acc<TW>::col0();
+template <int TW> __device__ __forceinline__ void compute_tn(Mul &m, const float *As, const float *Bs, int kb) {
+    const MulAt<TW> at;
 #pragma unroll 4
-    for (int k = 0; k < kb; ++k) {
-        float a[RI];
-        if constexpr (RI == 4) {
-            const float4 t = *reinterpret_cast<const float4 *>(a0 + k * LD);
-            a[0] = t.x; a[1] = t.y; a[2] = t.z; a[3] = t.w;
-        } else if constexpr (RI == 2) {
-            const float2 t = *reinterpret_cast<const float2 *>(a0 + k * LD);
-            a[0] = t.x; a[1] = t.y;
-        } else {
-            a[0] = a0[k * LD];
-        }
-        const float4 b = *reinterpret_cast<const float4 *>(b0 + k * LD);
+    for (int k = at.grp; k < kb; k += MulAt<TW>::NG) {
+        const float4 a = *reinterpret_cast<const float4 *>(As + k * LD + at.row);
+        const float av[4] = {a.x, a.y, a.z, a.w};
+        m.step(av, *reinterpret_cast<const float4 *>(Bs + k * LD + at.col));
+    }
+}
+// The groups' partial tiles added in order; buf: 4096 floats that no one reads any more after the barrier.
+template <int TW> __device__ __forceinline__ Acc<TW> finish(const Mul &m, float *buf) {
+    Acc<TW> acc;
+    if constexpr (TW == 64) {
 #pragma unroll
-        for (int i = 0; i < RI; ++i) {
-            acc.v[i][0] = fmaf(a[i], b.x, acc.v[i][0]);
-            acc.v[i][1] = fmaf(a[i], b.y, acc.v[i][1]);
-            acc.v[i][2] = fmaf(a[i], b.z, acc.v[i][2]);
-            acc.v[i][3] = fmaf(a[i], b.w, acc.v[i][3]);
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc.v[i][j] = m.v[i][j];
+    } else {
+        const MulAt<TW> at;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<float4 *>(buf + (at.grp * TILE + at.row + i) * TW + at.col) = make_float4(m.v[i][0], m.v[i][1], m.v[i][2], m.v[i][3]);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < Acc<TW>::RI; ++i) {
+            float4 t = *reinterpret_cast<const float4 *>(buf + (Acc<TW>::row0() + i) * TW + Acc<TW>::col0());
+#pragma unroll
+            for (int g = 1; g < MulAt<TW>::NG; ++g) {
+                const float4 o = *reinterpret_cast<const float4 *>(buf + (g * TILE + Acc<TW>::row0() + i) * TW + Acc<TW>::col0());
+                t.x += o.x; t.y += o.y; t.z += o.z; t.w += o.w;
+            }
+            acc.v[i][0] = t.x; acc.v[i][1] = t.y; acc.v[i][2] = t.z; acc.v[i][3] = t.w;
         }
     }
+    return acc;
 }
 
 // Four adjacent elements as fp32; `n` of them exist (n >= 4: all).  vec: the address is aligned to the four.
@@ -133,32 +166,29 @@ template <class T> __device__ __forceinline__ void fetch(Frag &fr, int sh, const
 __device__ __forceinline__ void put_rows(const Frag &fr, int sh, float *dst) {
     pieces(sh, [&](int u, int r, int c) { *reinterpret_cast<float4 *>(dst + r * LD + c) = fr.v[u]; });
 }
+// Transposed: source row r becomes column r ^ (step & 28) of the steps c ... c + 3 - without the exclusive or the lanes of a
+// warp, four steps apart, would meet in two banks.
 __device__ __forceinline__ void put_transposed(const Frag &fr, int sh, float *dst) {
     pieces(sh, [&](int u, int r, int c) {
-        dst[c * LD + r] = fr.v[u].x;
-        dst[(c + 1) * LD + r] = fr.v[u].y;
-        dst[(c + 2) * LD + r] = fr.v[u].z;
-        dst[(c + 3) * LD + r] = fr.v[u].w;
-    });
-}
-template <class F> __device__ __forceinline__ void scale(Frag &fr, int sh, F f) {   // f(row, column) multiplies
-    pieces(sh, [&](int u, int r, int c) {
-        fr.v[u].x *= f(r, c);
-        fr.v[u].y *= f(r, c + 1);
-        fr.v[u].z *= f(r, c + 2);
-        fr.v[u].w *= f(r, c + 3);
+        float *to = dst + c * LD + (r ^ (c & 28));
+        to[0] = fr.v[u].x;
+        to[LD] = fr.v[u].y;
+        to[2 * LD] = fr.v[u].z;
+        to[3 * LD] = fr.v[u].w;
     });
 }
 
 // The panel loop: load(k0) fetches this thread's pieces of the panels at k0, put(k0) stores them to As / Bs,
-// mul(k0, depth) multiplies.
-template <class L, class P, class M> __device__ __forceinline__ void panels(int K, L load, P put, M mul) {
-    load(0);
+// mul(k0, depth) multiplies.  PREFETCH: the next panel is fetched during the multiplication - for depths that usually take
+// several panels; where one is the rule, the registers are better spent otherwise.
+template <bool PREFETCH = true, class L, class P, class M> __device__ __forceinline__ void panels(int K, L load, P put, M mul) {
+    if (PREFETCH) load(0);
     for (int k0 = 0; k0 < K; k0 += TILE) {
+        if (!PREFETCH) load(k0);
         __syncthreads();                                         // the panels' last readers are done
         put(k0);
         __syncthreads();
-        if (k0 + TILE < K) load(k0 + TILE);
+        if (PREFETCH && k0 + TILE < K) load(k0 + TILE);
         mul(k0, min(TILE, K - k0));
     }
 }
