@@ -543,8 +543,9 @@ do {                                                                            
                 if (!no_ws() && tc::dbc_grp_ok(d.P, d.N, d.Q)) {
                     const size_t smem_g = tc::dbc_grp_smem(d.Q, std::min(d.N, 128));
                     BISSD_ALLOW(tc::dbc_accum_grp<T>, smem_g);
-                    BISSD_LAUNCH_ON(s_side, "tc_dbc_accum_grp", launch_pdl(tc::dbc_accum_grp<T>, dim3(d.b * d.nc * d.G * w.nsplit, 1, 2), tc::kDbcGrpThreads, smem_g, s_side, 
-                        d, mEf, mEb, mSf, mSb, mX128, mG128, a.dt_out, a.cs_f, a.cs_b, F(w.dB_part), F(w.dC_part), status));
+                    BISSD_LAUNCH_ON(s_side, "tc_dbc_accum_grp", launch_pdl(tc::dbc_accum_grp<T>, dim3(d.b * d.nc * d.G * w.nsplit * w.dbc_ks, 1, 2), tc::kDbcGrpThreads, smem_g, s_side,
+                        d, mEf, mEb, mSf, mSb, mX128, mG128, a.dt_out, a.cs_f, a.cs_b, F(w.dB_part), F(w.dC_part), w.dbc_ks, status));
+                    part_heads = d.G * dbc_slots(d, w.dbc_ks);
                 } else
                 BISSD_LAUNCH("tc_dbc_accum_tma", tc::dbc_accum_tma<T><<<dim3(d.b * d.nc * d.G * w.nsplit, nlt_tc, 2), tc::kThreads, smem_a, s>>>(
                     d, mEf, mEb, mSf, mSb, mX128, mG128, a.dt_out, a.cs_f, a.cs_b, F(w.dB_part), F(w.dC_part), status));
@@ -582,10 +583,12 @@ do {                                                                            
                 tc::make_map2(&mDm, a.p.x_dtype, F(w.dCB), d.Q, dcb_rows, 64, d.Q) &&
                 tc::make_map2(&mDk, a.p.x_dtype, F(w.dCB), d.Q, dcb_rows, 64, 128)) {
                 const size_t smem_f = tc::intra_tile_smem(d.Q);
-                BISSD_ALLOW(tc::intra_dcb_tile<T>, smem_f);
-                BISSD_LAUNCH("tc_intra_dcb_tile", launch_pdl(tc::intra_dcb_tile<T>, dim3(d.b * d.nc * d.G, nlt_tc, nlt_tc), tc::kIntraTileThreads, smem_f, s,
+                const auto intra = head_parts(d) > 1 ? tc::intra_dcb_tile<T, true> : tc::intra_dcb_tile<T, false>;
+                BISSD_ALLOW(intra, smem_f);
+                const int ks = tc::intra_ksplit(d, sm_count());
+                BISSD_LAUNCH("tc_intra_dcb_tile", launch_cluster(intra, dim3(d.b * d.nc * d.G * ks, nlt_tc, nlt_tc), tc::kIntraTileThreads, smem_f, s, ks,
                     dg, mG, mX128, mCB, a.dt_out, a.cs_f, a.cs_b, F(w.u4), (long long)d.b * d.H * d.nc * d.Q,
-                    static_cast<void *>(F(w.dCB)), status));
+                    static_cast<void *>(F(w.dCB)), ks, status));
                 u4_tiles = nlt_tc * nlt_tc;
                 fused_done = dcb_done = true;
                 bmm_tma = true;

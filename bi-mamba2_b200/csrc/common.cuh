@@ -28,6 +28,18 @@ struct MutView {
 
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// Parts the heads of a group are summed in by the kernels that walk them (dCB, dB, dC): heads R i / S ... R (i + 1) / S of part
+// i, the parts' sums then added in a fixed order.  Blocks may share the parts or one block take them all - the numbers
+// are the same, and the rule looks at one row of the batch only, so a row's results do not depend on how many rows there
+// are.  One part where a row alone brings 32 tiles (b >= 5 such rows fill the chip; summing in parts costs one block 5 %)
+// or the heads are few.
+__host__ __device__ inline int head_parts(const Dims &d) {
+    const int nt = ceil_div(d.Q, 128);
+    return d.nc * d.G * nt * nt >= 32 ? 1 : (d.R >= 16 ? 4 : (d.R >= 8 ? 2 : 1));
+}
+// Partial dB / dC of a group that dbc_accum_grp writes when ks blocks share its parts: one per pair of parts, or per part.
+__host__ __device__ inline int dbc_slots(const Dims &d, int ks) { const int S = head_parts(d); return ks == S ? S : S / 2; }
+
 template <class T> __device__ __forceinline__ float to_f(T v);
 template <> __device__ __forceinline__ float to_f<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }

@@ -12,7 +12,7 @@ struct FwdWs {
 };
 struct BwdWs {
     size_t cb, cbt, cbt16, cb16, cbs, gloc, E, E16, g, dTpart, ddt_out, nf, nb, pf, pb, da_f, da_b, u4, dB_part, dC_part, dCB, dDpart, dApart, dbiaspart, total;
-    int nslots, nlt, nsplit, hsplit;
+    int nslots, nlt, nsplit, hsplit, dbc_ks;
 };
 
 // The recurrence over chunks: four elements of the (headdim, dstate) state per thread where their number allows.
@@ -55,6 +55,23 @@ inline int simt_hsplit(const Dims &d) {
     return hs;
 }
 
+// Blocks the heads of a group are dealt to in dbc_accum_grp (one block an SM, about 2 us a head), each writing a partial
+// dB / dC that the last product adds up again: more than one only where the blocks leave SMs idle.
+inline int dbc_ksplit(const Dims &d) {
+    const long long tiles = 2LL * d.b * d.nc * d.G * ceil_div(d.N, 128);
+    int best = 1;
+    float least = 0.f;
+    for (int ks = 1; ks <= head_parts(d); ks *= 2) {
+        const long long waves = (tiles * ks + sm_count() - 1) / sm_count();
+        const float t = waves * (2.f * ceil_div(d.R, ks) + 5.f) + ks;
+        if (ks == 1 || t < least) {
+            best = ks;
+            least = t;
+        }
+    }
+    return best;
+}
+
 // tc: sized for the tensor-core family (16-bit inputs that meet its alignment rules): the passed state gradients are
 // kept in the input dtype only, and the "states" parts of dB / dC arrive summed over the heads of a group.  The
 // CUDA-core family needs the fp32 copy and one partial per head.
@@ -67,6 +84,8 @@ inline BwdWs bwd_layout(const Dims &d, bool tc) {
     w.nlt = ceil_div(d.Q, simt::TILE);
     w.nsplit = tc ? ceil_div(d.N, 128) : 1;
     w.hsplit = tc ? 1 : simt_hsplit(d);
+    w.dbc_ks = tc ? dbc_ksplit(d) : 1;
+    const int slots = dbc_slots(d, w.dbc_ks);
     auto take = [&](size_t bytes) { size_t at = o; o = align256(o + bytes); return at; };
     w.cb = take(qq * 4);
     w.gloc = take(2 * st * 4);
@@ -83,8 +102,8 @@ inline BwdWs bwd_layout(const Dims &d, bool tc) {
     w.pf = take(hq * 4 * w.nsplit); w.pb = take(hq * 4 * w.nsplit);
     w.da_f = take(tc ? hq * 4 : 0); w.da_b = take(tc ? hq * 4 : 0);
     w.u4 = take((tc ? 8 : 4 * w.nlt) * hq * 4);                      // u_f / u_b per tile (tc::intra_sums: 2 row tiles; tc::intra_dcb_tile: 4; simt: 2 nlt)
-    w.dB_part = take((size_t)d.b * d.nc * d.Q * (tc ? d.G : d.H) * d.N * 4);
-    w.dC_part = take((size_t)d.b * d.nc * d.Q * (tc ? d.G : d.H) * d.N * 4);
+    w.dB_part = take((size_t)d.b * d.nc * d.Q * (tc ? d.G * slots : d.H) * d.N * 4);
+    w.dC_part = take((size_t)d.b * d.nc * d.Q * (tc ? d.G * slots : d.H) * d.N * 4);
     w.dCB = take(qq * 4 * w.hsplit);
     w.dDpart = take((size_t)d.b * d.nc * d.H * std::max(w.nlt, 8) * d.P * 4);   // up to 8 partial rows per (b,c,h)
     w.dApart = take((size_t)d.b * d.nc * d.H * 4);

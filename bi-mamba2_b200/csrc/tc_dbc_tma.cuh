@@ -168,9 +168,11 @@ dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
 // are fetched once instead of once per row block, and the x / g tile once.  Roles as in state_gemm_grp: warps 0-7
 // turn the left tile as it landed into its two row-scaled copies (one buffer: the copies of head i + 1 are written
 // once the MMAs of head i are done), lane 0 of warp 8 issues every TMA load and every MMA; two stages of (left
-// tile + 2 right tiles).  All heads accumulate in tensor memory, which is read once at the end.  Bounded waits,
-// ids 51-56 in the status word.
-// grid (b*nc*G*nsplit, 1, 2); blockIdx.z: 0 = dB, 1 = dC.
+// tile + 2 right tiles).  The heads accumulate in tensor memory, two parts of them (head_parts) side by side; a pair of
+// parts is read out together.  With few blocks the parts are dealt to ks of them (dbc_ksplit).  Bounded waits, ids 51-56
+// in the status word.
+// grid (b*nc*G*ks*nsplit, 1, 2); blockIdx.z: 0 = dB, 1 = dC.  part layout [b, nc*Q, G, slots, N] fp32: a slot per pair of
+// parts, or per part where every block has one.
 struct DbcGrpShared {
     uint64_t full[2], scaled, done[2], wbar;
     uint32_t tmem_base;
@@ -187,24 +189,28 @@ __global__ void __launch_bounds__(kDbcGrpThreads, 1)
 dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_constant__ CUtensorMap tmEb,
               const __grid_constant__ CUtensorMap tmSf, const __grid_constant__ CUtensorMap tmSb,
               const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG, const float *dt_out,
-              const float *cs_f, const float *cs_b, float *dB_part, float *dC_part, int *status) {
+              const float *cs_f, const float *cs_b, float *dB_part, float *dC_part, int ks, int *status) {
     pdl_begin();
     extern __shared__ uint8_t dyn[];
     __shared__ DbcGrpShared sh;
     constexpr int P = 64;
-    const int N = d.N, Q = d.Q, R = d.R;
+    const int N = d.N, Q = d.Q;
     const int nsplit = (N + 127) / 128, nt = min(N, 128), nnb = nt / 64, nrb = Q / 128;
     const int left_bytes = Q * 128, right_bytes = 2 * nnb * P * 128, stage_bytes = left_bytes + right_bytes;
     uint8_t *base_sm = smem_align1024(dyn);                     // per stage: left [Q rows x 128 B], right [dir][nnb][P x 128 B]
     uint8_t *smScaled = base_sm + 2 * stage_bytes;              // [dir][Q rows x 128 B]
     float *sc = reinterpret_cast<float *>(smScaled + 2 * left_bytes);   // [2 bufs][2 dirs][Q]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int split = blockIdx.x % nsplit, bx = blockIdx.x / nsplit;
+    const int split = blockIdx.x % nsplit, part_id = blockIdx.x / nsplit % ks, bx = blockIdx.x / nsplit / ks;
     const int grp = bx % d.G, c = (bx / d.G) % d.nc, b = bx / (d.G * d.nc);
     const int which = blockIdx.z;
     const int lim = min(Q, d.L - c * Q);
-    const int n0 = split * 128, h0 = grp * R;
-    const uint32_t ncols = tmem_cols(nrb * nt);
+    // this block's parts of the heads (head_parts): S / ks of them from `first` on, heads h0 ... h0 + R - 1
+    const int n0 = split * 128, S = head_parts(d), nparts = S / ks, first = nparts * part_id, r0 = d.R * first / S;
+    const int h0 = grp * d.R + r0, R = d.R * (first + nparts) / S - r0;
+    const int slots = dbc_slots(d, ks);
+    auto part_end = [&](int p) { return d.R * (first + p + 1) / S - r0; };   // first head after local part p
+    const uint32_t acc_cols = nrb * nt, ncols = tmem_cols(nparts > 1 ? 2 * acc_cols : acc_cols);   // two parts have an accumulator each
     volatile int *fail = &sh.fail;
     auto load_head = [&](int i) {                               // the left tile and both state tiles of head i
         uint8_t *sl = base_sm + (i & 1) * stage_bytes, *sr = sl + left_bytes;
@@ -268,7 +274,12 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
         if (lane == 0) {
             bool ok = true;
             const uint32_t idesc = instr_desc(AbFmt<T>::v, false, true, nt);
+            int p = 0, start = 0;                               // local part of head i and its first head
             for (int i = 0; i < R && ok; ++i) {
+                if (i == part_end(p)) {
+                    ++p;
+                    start = i;
+                }
                 if (i >= 1 && i + 1 < R) {                      // stage (i + 1) & 1 is free once the MMAs of head i - 1 are done
                     ok = ws_wait(&sh.done[(i - 1) & 1], ((i - 1) >> 1) & 1, fail, 51);
                     if (ok) load_head(i + 1);
@@ -281,14 +292,40 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
                     for (int dir = 0; dir < 2; ++dir)
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk)
-                            umma(tmem + rb * nt, smem_desc(sl + (dir * nrb + rb) * 16384 + kk * 32, 16, 1024),
+                            umma(tmem + (p & 1) * acc_cols + rb * nt, smem_desc(sl + (dir * nrb + rb) * 16384 + kk * 32, 16, 1024),
                                  smem_desc(sr + dir * nnb * P * 128 + kk * 16 * 128, (uint32_t)P * 128, 1024), idesc,
-                                 (i > 0 || dir > 0 || kk > 0) ? 1u : 0u);
+                                 (i > start || dir > 0 || kk > 0) ? 1u : 0u);
                 umma_commit(&sh.done[i & 1]);
             }
         }
     } else {
+        // the sum of local parts 2 pair and 2 pair + 1 (`two`) as this block's next partial result
+        auto write_out = [&](int pair, bool two) {
+            tc_fence_after();
+            const int slot = slots == S ? part_id : first / 2 + pair;
+            for (int rb = 0; rb < nrb; ++rb) {
+                const int l = rb * 128 + (warp & 3) * 32 + lane;
+                float *part = (which ? dC_part : dB_part) + (((long long)b * d.nc * Q + c * Q + l) * d.G * slots + grp * slots + slot) * N + n0;
+                for (int c0 = (warp >> 2) * 32; c0 < nt; c0 += 64) {
+                    float v[32];
+                    tmem_ld32(tmem_lane_base(tmem) + rb * nt + c0, v);
+                    if (two) {
+                        float t[32];
+                        tmem_ld32(tmem_lane_base(tmem) + acc_cols + rb * nt + c0, t);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] += t[j];
+                    }
+                    if (l < lim) {
+#pragma unroll
+                        for (int j = 0; j < 32; j += 4)
+                            *reinterpret_cast<float4 *>(part + c0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                    }
+                }
+            }
+            tc_fence_before();
+        };
         bool ok = true;
+        int pair = 0;
 #pragma unroll 1
         for (int i = 0; i < R && ok; ++i) {
             uint8_t *sl = base_sm + (i & 1) * stage_bytes;
@@ -296,6 +333,7 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
             // the scaled copies of head i - 1 have been read by its MMAs
             if (ok && i >= 1) ok = ws_wait_warp(&sh.done[(i - 1) & 1], ((i - 1) >> 1) & 1, fail, 56);
             if (!ok) break;
+            if (nparts > 2 && i == part_end(2 * pair + 1)) write_out(pair++, true);   // both accumulators are complete: out, before the next part starts
             const float *wf = sc + ((i & 1) * 2) * Q, *wb = wf + Q;
             for (int q = tid; q < Q * 8; q += kThreads) {
                 const uint4 raw = reinterpret_cast<const uint4 *>(sl)[q];
@@ -315,22 +353,7 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
             ok = ws_wait_warp(&sh.wbar, i & 1, fail, 54);
         }
         if (ok) ok = ws_wait_warp(&sh.done[(R - 1) & 1], ((R - 1) >> 1) & 1, fail, 55);
-        if (ok) {
-            tc_fence_after();
-            for (int rb = 0; rb < nrb; ++rb) {
-                const int l = rb * 128 + (warp & 3) * 32 + lane;
-                float *part = (which ? dC_part : dB_part) + (((long long)b * d.nc * Q + c * Q + l) * d.G + grp) * N + n0;
-                for (int c0 = (warp >> 2) * 32; c0 < nt; c0 += 64) {
-                    float v[32];
-                    tmem_ld32(tmem_lane_base(tmem) + rb * nt + c0, v);
-                    if (l < lim) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4)
-                            *reinterpret_cast<float4 *>(part + c0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                    }
-                }
-            }
-        }
+        if (ok) write_out((nparts - 1) / 2, nparts > 1);
     }
     tc_fence_before();
     __syncthreads();

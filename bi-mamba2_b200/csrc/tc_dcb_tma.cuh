@@ -246,13 +246,26 @@ bmm_bwd_tma(Dims d, const __grid_constant__ CUtensorMap tmDm, const __grid_const
     float o[32];                                                // the partial sums are on their way while the MMAs run
 #pragma unroll
     for (int j = 0; j < 32; ++j) o[j] = 0.f;
-    if (row < lim)
-        for (int q = 0; q < rp; ++q)
+    if (row < lim) {                                            // pairs of partial results first, as dbc_accum_grp adds them itself
+        auto pair = [&](const float *p, int n, float (&v)[32]) {
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
-                const float4 t = *reinterpret_cast<const float4 *>(part + (long long)q * N + j);
-                o[j] += t.x, o[j + 1] += t.y, o[j + 2] += t.z, o[j + 3] += t.w;
+                float4 t = *reinterpret_cast<const float4 *>(p + j);
+                if (n > 1) {
+                    const float4 u = *reinterpret_cast<const float4 *>(p + N + j);
+                    t.x += u.x, t.y += u.y, t.z += u.z, t.w += u.w;
+                }
+                v[j] = t.x, v[j + 1] = t.y, v[j + 2] = t.z, v[j + 3] = t.w;
             }
+        };
+        pair(part, min(rp, 2), o);
+        for (int q = 2; q < rp; q += 2) {
+            float t[32];
+            pair(part + (long long)q * N, min(rp - q, 2), t);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) o[j] += t[j];
+        }
+    }
     if (ok) ok = mbar_wait(&bar_done, 0);
     ok = __syncthreads_and(ok);
     tc_fence_after();

@@ -15,7 +15,8 @@
 // memory - over g and x, which are dead once G2 exists; a second chain with a lower-triangular ones matrix,
 // D[m,s] = sum_{l<=m} V[l,s], yields the column totals (row 127) and, in tiles on the diagonal, their split at the
 // diagonal (D[m,m]).  Row sums are taken over the values as rounded for that chain, so that row and column sums
-// telescope exactly.  While one CTA weights a head the other one's loads and products are in flight.  A tile writes two
+// telescope exactly.  With few tiles the heads of a group are dealt to a cluster of up to four CTAs, which add their dCB
+// tiles through distributed shared memory at the end (one CTA adds the same parts in tensor memory).  While one CTA weights a head the other one's loads and products are in flight.  A tile writes two
 // Q-long vectors (forward / reverse part): + column sums at its columns, - row sums at its rows, zero elsewhere;
 // cumsum_bwd adds the vectors of a chunk's tiles.  Tiles off the diagonal hold one direction only and no mixed strip.
 //
@@ -35,6 +36,7 @@ namespace tc {
 struct IntraGrpShared {
     uint64_t bar_cb, bar_in, bar_m1, bar_m2;
     uint32_t tmem_base;
+    int h0, heads, part_end, parts_done;         // of this block; kept here, not in registers (see below)
 };
 
 constexpr int kIntraTileThreads = 256;
@@ -42,18 +44,48 @@ constexpr float kMixedSpan = 60.f;                              // log2 of the l
 inline size_t intra_tile_smem(int Q) { return 1024 + 32768 + 32768 + 32768 + 6 * (size_t)Q * 4; }
 inline bool intra_tile_ok(int P, int Q) { return P == 64 && (Q == 128 || Q == 256); }
 
-template <class T>
+// One block walking all heads of a group is the kernel's length where tiles are few (98 us for 24 heads whatever the rest of
+// the chip does).  There the heads are summed in parts (head_parts): one block takes all of them, or each block of a cluster
+// one.  A block alone on its SM takes about 4 us a head, two sharing one 2.75 us a head each in turn; a split adds its start
+// and the exchange of the partial tiles.
+inline int intra_ksplit(const Dims &d, int sms) {
+    const int S = head_parts(d);
+    const long long tiles = (long long)d.b * d.nc * d.G * (d.Q / 128) * (d.Q / 128);
+    auto cost = [&](int ks) {
+        const int n = (int)((tiles * ks + sms - 1) / sms), h = (d.R + ks - 1) / ks;
+        return (n == 1 ? 4.f * h : 2.75f * n * h) + (ks == 1 ? 4.f : 7.f) * ((n + 1) / 2);
+    };
+    return cost(S) < cost(1) ? S : 1;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster(uint32_t smem_addr, int rank) {   // 16 bytes at the same address of another block
+    uint32_t at;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
+}
+
+// The head after the i-th part of a block that takes all parts, or a head that never comes where that part is the last (or
+// the block has one part only).
+__device__ __forceinline__ int part_end_of(int R, int S, int ks, int i) { return ks == 1 && i + 1 < S ? R * (i + 1) / S : 1 << 30; }
+
+// PARTS: the heads are summed in parts (head_parts > 1).  grid (b nc G ks, Q / 128, Q / 128), clusters of ks blocks along x.
+template <class T, bool PARTS>
 __global__ void __launch_bounds__(kIntraTileThreads, 2)
 intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_constant__ CUtensorMap tmX,
                const __grid_constant__ CUtensorMap tmCB, const float *dt_out, const float *cs_f, const float *cs_b,
-               float *u4, long long hq, void *dCB16, int *status) {
+               float *u4, long long hq, void *dCB16, int ks, int *status) {
     pdl_begin();
     extern __shared__ uint8_t dyn[];
     __shared__ IntraGrpShared sh;
     __shared__ float rsum[2][2][kTileM];                          // [column half][direction][row]
     __shared__ float dg[kTileM];                                  // D[m, m] of a diagonal tile
     __shared__ __align__(16) float tot[kTileM];                   // D[127, s]
-    const int Q = d.Q, R = d.R;
+    const int Q = d.Q, part = PARTS ? blockIdx.x % ks : 0, bx = PARTS ? blockIdx.x / ks : blockIdx.x;
     uint8_t *base_sm = smem_align1024(dyn);
     uint8_t *smCB = base_sm;                                      // two slabs [128 x 64] bf16, K-major
     uint8_t *smG = smCB + 32768;                                  // [128 x 64], K-major
@@ -62,7 +94,7 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
     uint8_t *smTri = smG + 32768;                                 // two slabs [128 x 64] bf16, K-major
     float *tab = reinterpret_cast<float *>(smTri + 32768);        // [6][Q]: f2, b2, tf, tb, colF, colB
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = blockIdx.x % d.G, c = (blockIdx.x / d.G) % d.nc, b = blockIdx.x / (d.G * d.nc);
+    const int g = bx % d.G, c = (bx / d.G) % d.nc, b = bx / (d.G * d.nc);
     // Launch order (x, then y, then z) puts the tiles on the diagonal first: they carry the dearer strips, and the
     // second CTA an SM receives is then mostly one off the diagonal.
     const int ty = blockIdx.y ^ blockIdx.z, tz = blockIdx.y;
@@ -74,8 +106,21 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
     const int wl_min = l0 + quad * 32, wl_max = wl_min + 31;      // rows handled by this warp
     const int tile = ty * gridDim.z + tz;
     if (warp == 0) tmem_alloc(&sh.tmem_base, 256);
+    // The registers are full (64 of them hold the tile): what the head loop needs once per head is read from shared memory.
+    // Eight spilled bytes in it cost 8 % of the kernel's time, and the code for the parts alone 3 %, hence the template.
+    if (PARTS) {
+        if (tid == 0) {
+            sh.heads = d.R * (part + 1) / ks - d.R * part / ks;
+            sh.h0 = g * d.R + d.R * part / ks;
+            sh.parts_done = 0;
+            sh.part_end = part_end_of(d.R, head_parts(d), ks, 0);
+        }
+        __syncthreads();
+    }
+    auto first_head = [&] { return PARTS ? sh.h0 : g * d.R; };
+    auto heads = [&] { return PARTS ? sh.heads : d.R; };
     auto load_head = [&](int hr) {                                // one thread: g and x of head hr
-        const int h = g * R + hr;
+        const int h = first_head() + hr;
         mbar_expect_tx(&sh.bar_in, 32768u);
         tma_load4(smG, &tmG, 0, h, c * Q + l0, b, &sh.bar_in);
         tma_load4(smX, &tmX, 0, h, c * Q + s0, b, &sh.bar_in);
@@ -93,7 +138,7 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
     }
     float pcf = 0.f, pcb = 0.f, pdt = 1.f, pcfr = 0.f, pcbr = 0.f;
     auto fetch_tab = [&](int hr) {
-        const int h = g * R + hr;
+        const int h = first_head() + hr;
         const long long base = ((long long)(b * d.H + h) * d.nc + c) * Q;
         if (tid < Q) {
             pcf = cs_f[base + tid];
@@ -127,13 +172,14 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
     }
     fetch_tab(0);
     write_tab();
-    if (R > 1) fetch_tab(1);
+    if (heads() > 1) fetch_tab(1);
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
-    const uint32_t tG2 = tmem, tD2 = tmem + 128;
+    // D2 takes the columns of G2, which is dead by then; the others hold the sum of the finished parts of the heads
+    const uint32_t tG2 = tmem, tD2 = tmem;
     auto issue_g2 = [&](int hr) -> bool {                         // thread 0: G2 of head hr
         if (!mbar_wait(&sh.bar_in, hr & 1)) return false;
         tc_fence_after();
@@ -159,7 +205,7 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
                                    (((jc & 7) ^ (kl & 7)) << 4)) = v;
     };
 #pragma unroll 1
-    for (int hr = 0; hr < R; ++hr) {
+    for (int hr = 0; hr < heads(); ++hr) {
         ok = mbar_wait_cta(&sh.bar_m1, hr & 1, ok);               // G2 of head hr is in tensor memory
         tc_fence_after();
         if (hr == 0 && ok && ty == tz && chalf == ((r >> 4) & 1)) {
@@ -272,17 +318,17 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
             umma_issue_stage<false, true>(tD2, 128, 1, smTri + 16384, smV + 16384, 1u);
             umma_commit(&sh.bar_m2);
         }
-        if (hr + 1 < R) {                                         // single set of tables: the next head's go in here,
+        if (hr + 1 < heads()) {                                  // single set of tables: the next head's go in here,
             write_tab();                                          // while the triangular product runs
-            if (hr + 2 < R) fetch_tab(hr + 2);
+            if (hr + 2 < heads()) fetch_tab(hr + 2);
         }
         ok = mbar_wait_cta(&sh.bar_m2, hr & 1, ok);               // column sums done: V (= g, x) may be overwritten
         tc_fence_after();
-        if (tid == 0 && ok && hr + 1 < R) load_head(hr + 1);
+        if (tid == 0 && ok && hr + 1 < heads()) load_head(hr + 1);
         if (ok) {
             if (ty == tz && chalf == (quad >> 1)) {   // the diagonal element of this thread's row
                 float v[32];
-                tmem_ld32(tl + 128 + quad * 32, v);
+                tmem_ld32(tl + quad * 32, v);
                 float x = 0.f;
 #pragma unroll
                 for (int j = 0; j < 32; ++j) x = (lane == j) ? v[j] : x;
@@ -292,7 +338,7 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
 #pragma unroll
                 for (int c0 = 0; c0 < 64; c0 += 32) {
                     float v[32];
-                    tmem_ld32(tl + 128 + cbeg + c0, v);
+                    tmem_ld32(tl + cbeg + c0, v);
                     if (lane == 31) {
 #pragma unroll
                         for (int j = 0; j < 32; j += 4)
@@ -304,9 +350,9 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
         tc_fence_before();
         ok = __syncthreads_and(ok);
         if (!ok) break;
-        if (tid == 0 && hr + 1 < R) ok = issue_g2(hr + 1);        // its loads have had the read-out above to land
+        if (tid == 0 && hr + 1 < heads()) ok = issue_g2(hr + 1);        // its loads have had the read-out above to land
         if (tid < Q) {
-            const int h = g * R + hr;
+            const int h = first_head() + hr;
             const long long base = ((long long)(b * d.H + h) * d.nc + c) * Q;
             const int j = tid, mc = j - s0, mr = j - l0;          // position as a column / as a row of this tile
             const bool incol = mc >= 0 && mc < kTileM, inrow = mr >= 0 && mr < kTileM;
@@ -330,9 +376,70 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
             u4[(tile * 2 + 0) * hq + base + j] = uf;
             u4[(tile * 2 + 1) * hq + base + j] = ub;
         }
+        if (PARTS && __builtin_expect(hr + 1 == sh.part_end, 0)) {         // a part is complete, not the last: add it to the sum
+            const bool more = sh.parts_done > 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const uint32_t at = tl + 128 + chalf * 64 + q * 8;
+                if (more) {
+                    uint32_t u[8];
+                    tmem_ld8_nowait(at, u);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) acc[q * 8 + j] = __uint_as_float(u[j]) + acc[q * 8 + j];
+                }
+                tmem_st8(at, *reinterpret_cast<float(*)[8]>(&acc[q * 8]));
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[q * 8 + j] = 0.f;
+            }
+            tmem_st_wait();
+            __syncthreads();                                      // everyone has read the counters
+            if (tid == 0) {
+                ++sh.parts_done;
+                sh.part_end = part_end_of(d.R, head_parts(d), 1, sh.parts_done);
+            }
+        }
     }
     if (!ok && tid == 0) atomicExch(status, kErrMmaTimeout);
-    if (ok && l < Q) {                                            // the rounded dCB tile; zero outside the sequence
+    if (PARTS && ok && sh.parts_done > 0) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            uint32_t u[8];
+            tmem_ld8_nowait(tl + 128 + chalf * 64 + q * 8, u);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[q * 8 + j] = __uint_as_float(u[j]) + acc[q * 8 + j];
+        }
+    }
+    if (PARTS && ks > 1) {
+        // The cluster's blocks hold partial sums of the same tile.  Each puts its own into its shared memory in fp32 (over
+        // C.B^T and V, both dead; 16-byte pieces swizzled by row), then adds up 128 / ks rows over the cluster.
+        float4 *mine = reinterpret_cast<float4 *>(base_sm);
+#pragma unroll
+        for (int j0 = 0; j0 < 64; j0 += 4) {
+            const int col = ((j0 >> 4) * 2 + chalf) * 16 + (j0 & 15);
+            mine[r * 32 + ((col >> 2) ^ (r & 31))] = make_float4(acc[j0], acc[j0 + 1], acc[j0 + 2], acc[j0 + 3]);
+        }
+        cluster_sync();
+        const int rows = kTileM / ks;
+        const uint32_t at = smem_u32(base_sm);
+        for (int i = tid; i < rows * 32; i += kIntraTileThreads) {
+            const int rr = part * rows + (i >> 5), c4 = i & 31;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int k = 0; k < ks; ++k) {
+                const float4 t = ld_cluster(at + (rr * 32 + (c4 ^ (rr & 31))) * 16, k);
+                v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+            }
+            const int row = l0 + rr, col = s0 + c4 * 4;
+            if (row < Q) {
+                const bool on = row < lim;                        // zero outside the sequence
+                T *out = static_cast<T *>(dCB16) + ((long long)(b * d.nc + c) * d.G + g) * Q * Q + (long long)row * Q + col;
+                *reinterpret_cast<uint2 *>(out) = make_uint2(pack2<T>(on && col < lim ? v.x : 0.f, on && col + 1 < lim ? v.y : 0.f),
+                                                             pack2<T>(on && col + 2 < lim ? v.z : 0.f, on && col + 3 < lim ? v.w : 0.f));
+            }
+        }
+        cluster_sync();                                           // no block leaves while its tile is being read
+    } else if (ok && l < Q) {                                     // the rounded dCB tile; zero outside the sequence
         T *out = static_cast<T *>(dCB16) + ((long long)(b * d.nc + c) * d.G + g) * Q * Q + (long long)l * Q + s0;
 #pragma unroll
         for (int j0 = 0; j0 < 64; j0 += 8) {
