@@ -33,16 +33,16 @@ std::vector<TraceRec> g_trace;
 std::atomic<int> g_trace_on{0};
 std::atomic<unsigned long long> g_launches{0};
 
-// A second stream for the two group-walking backward kernels whose results nothing reads before the last product with
-// dCB (prev_terms_grp, dbc_accum_grp): they fork from the caller's stream after the dx kernel and join it again
-// before that product, so that they share the GPU with the fused dCB / decay-gradient kernel, which depends on
-// neither - each of the three leaves a seventh of the SMs idle when it runs alone.  Stream order as the caller sees it is unchanged, also
-// under stream capture (the side stream joins the capture through the event).  A call leases one (stream, two events)
-// set of its device for its duration; sets are created on first need - in practice by the first call on a device, so
-// not inside a later capture.  BISSD_NO_SIDE=1 keeps everything on the caller's stream.
+// A second stream for the group-walking backward kernels: prev_terms_grp, which nothing before cumsum_bwd reads, forks from
+// the caller's stream after the dx kernel and shares the GPU with the fused dCB / decay-gradient kernel; dbc_accum_grp goes
+// with it where it writes partial results, or follows that kernel where it finishes dB and dC itself, then beside
+// cumsum_bwd and final_reduce.  Each of these leaves a seventh of the SMs idle when it runs alone.  Stream order as the
+// caller sees it is unchanged, also under stream capture (the side stream joins the capture through the events).  A call
+// leases one (stream, events) set of its device for its duration; sets are created on first need - in practice by the
+// first call on a device, so not inside a later capture.  BISSD_NO_SIDE=1 keeps everything on the caller's stream.
 struct Side {
     cudaStream_t st = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaEvent_t fork = nullptr, fork2 = nullptr, join = nullptr;
     int dev = -1;
     bool busy = false;
 };
@@ -66,15 +66,16 @@ static Side *side_acquire(cudaStream_t s) {
         return nullptr;
     }
     cudaStream_t st = nullptr;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
     if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&e0, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&e1, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&e1, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&e2, cudaEventDisableTiming) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;                                           // no side stream: the launch stays in line
     }
     Side *sd = new Side;
-    sd->st = st; sd->fork = e0; sd->join = e1; sd->dev = dev; sd->busy = true;
+    sd->st = st; sd->fork = e0; sd->join = e1; sd->fork2 = e2; sd->dev = dev; sd->busy = true;
     g_side.push_back(sd);
     return sd;
 }
@@ -95,6 +96,11 @@ template <class Args> static bool make_cb_maps(const Args &a, const Dims &d, CUt
     const unsigned long long sB[3] = {(unsigned long long)a.B.stride_head * 2, (unsigned long long)a.B.stride_seq * 2, (unsigned long long)a.B.stride_batch * 2};
     const unsigned box[4] = {64, 1, 128, 1};
     return tc::make_map4(mC, a.p.x_dtype, a.C.ptr, dims, sC, box) && tc::make_map4(mB, a.p.x_dtype, a.B.ptr, dims, sB, box);
+}
+
+// A 16-bit [Q x Q] tile per (batch, chunk, group) in boxes of 64 columns x 128 rows
+static bool make_tile_map(const Dims &d, const void *ptr, CUtensorMap *m) {
+    return tc::make_map2(m, BISSD_BF16, ptr, d.Q, (unsigned long long)d.b * d.nc * d.G * d.Q, 64, 128);
 }
 
 static int make_dims(const bissd_problem &p, Dims *d) {
@@ -217,12 +223,12 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
             BISSD_ALLOW(tc::bmm_cb<T>, smem_cb);
             const bool ws_path = !no_tma() && !no_ws() && tc::scan_ws_ok(d.P, d.N, d.Q);
             __nv_bfloat16 *CB16 = reinterpret_cast<__nv_bfloat16 *>(ws + w.cb16);
-            CUtensorMap mCc, mBc;
-            if (ws_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc)) {
-                const size_t smem_ct = tc::bmm_cb_tma_smem(d.N);
+            CUtensorMap mCc, mBc, mCBo;
+            if (ws_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc) && make_tile_map(d, CB16, &mCBo)) {
+                const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, false);
                 BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
-                BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s, 
-                    d, mCc, mBc, CB16, nullptr, nullptr, status));
+                BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
+                    d, mCc, mBc, mCBo, mCBo, true, false, nullptr, status));
             } else
             BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_cb, s>>>(
                 d, Cm, Bm, ws_path ? nullptr : CB, nullptr, ws_path ? CB16 : nullptr, nullptr, nullptr, status));
@@ -317,7 +323,6 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
     const View x = view_of(a.x), Bm = view_of(a.B), Cm = view_of(a.C), z = view_of(a.z), dout = view_of(a.dout),
                out_x = view_of(a.out_x);
     const int bch = d.b * d.nc * d.H;
-    const size_t q3 = 3 * d.Q * sizeof(float);
     const int ntP = tc::round_up(d.P, 16), ntQ = tc::round_up(d.Q, 16), ntN = std::min(tc::round_up(d.N, 16), 128);
     const int nlt_tc = ceil_div(d.Q, tc::kTileM);
     // Tensor-core family: the gate is applied once (gate_bwd writes g = dout * silu(z) and dz); every later kernel
@@ -378,6 +383,15 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
     }
     if (!(a.phases & BISSD_PHASE_FINISH)) return BISSD_OK;
     int nlt = w.nlt, nsplit = 1, part_heads = d.H;
+    CUtensorMap mEf, mEb, mSf, mSb, mX128, mG128;                // operands of dbc_accum_grp
+    bool dbc_last = false;                                       // it finishes dB and dC after the dCB kernel
+    auto launch_dbc = [&](auto kernel, const tc::LastMaps &last, cudaStream_t st) -> int {
+        const size_t smem_g = tc::dbc_grp_smem(d.Q, std::min(d.N, 128));
+        BISSD_ALLOW(kernel, smem_g);
+        BISSD_LAUNCH_ON(st, "tc_dbc_accum_grp", launch_pdl(kernel, dim3(d.b * d.nc * d.G * w.nsplit * w.dbc_ks, 1, 2), tc::kDbcGrpThreads, smem_g, st,
+            d, mEf, mEb, mSf, mSb, mX128, mG128, a.dt_out, a.cs_f, a.cs_b, F(w.dB_part), F(w.dC_part), w.dbc_ks, last, status));
+        return BISSD_OK;
+    };
     bool have_fp32_cb = true;                                    // fp32 CB (and its transpose) are in the workspace
     bool use_u4 = false;                                         // decay gradients arrive as u_f / u_b (tc::intra_sums)
     bool fused_cb = false;                                       // the bf16 C.B^T tile for tc::intra_dcb_tile has been written
@@ -396,15 +410,16 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
         const bool sums_path = !no_tma() && !no_sums() && tc::scan_tma_ok(d.P, d.N, d.Q);
         __nv_bfloat16 *CBt16 = reinterpret_cast<__nv_bfloat16 *>(ws + w.cbt16);
         __nv_bfloat16 *CB16b = reinterpret_cast<__nv_bfloat16 *>(ws + w.cb16);
-        CUtensorMap mCc, mBc;
-        if (ws_path && sums_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc)) {
+        CUtensorMap mCc, mBc, mCBo, mCBto;
+        if (ws_path && sums_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc) && make_tile_map(d, CB16b, &mCBo) &&
+            make_tile_map(d, CBt16, &mCBto)) {
             // the fused dCB / decay-gradient kernel reads the bf16 tile by TMA; the separate intra_sums kernel
             // reads the fp32 strips
             fused_cb = !no_fused() && tc::intra_tile_ok(d.P, d.Q);
-            const size_t smem_ct = tc::bmm_cb_tma_smem(d.N);
+            const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, true);
             BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
-            BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s, 
-                d, mCc, mBc, fused_cb ? CB16b : nullptr, CBt16, fused_cb ? nullptr : F(w.cbs), status));
+            BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
+                d, mCc, mBc, mCBo, mCBto, fused_cb, true, fused_cb ? nullptr : F(w.cbs), status));
         } else
         BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
             d, Cm, Bm, (sums_path && ws_path) ? nullptr : F(w.cb), ws_path ? nullptr : F(w.cbt), nullptr,
@@ -512,7 +527,7 @@ do {                                                                            
         }
         bool dbc_done = false;
         if (dx_done) {                                           // the dx kernel has produced nf / nb
-            CUtensorMap mC, mEf, mEb, mSf, mSb;
+            CUtensorMap mC;
             const unsigned long long dC4[4] = {(unsigned long long)d.N, (unsigned long long)d.G, (unsigned long long)d.L, (unsigned long long)d.b};
             const unsigned long long sC4[3] = {(unsigned long long)a.C.stride_head * 2, (unsigned long long)a.C.stride_seq * 2, (unsigned long long)a.C.stride_batch * 2};
             const unsigned bC4[4] = {64, 1, 128, 1};
@@ -524,7 +539,6 @@ do {                                                                            
                 tc::make_map2(&mSf, a.p.x_dtype, a.states_f, d.N, rows, 64, d.P) &&
                 tc::make_map2(&mSb, a.p.x_dtype, a.states_b, d.N, rows, 64, d.P)) {
                 const size_t smem_p = tc::prev_tma_smem(d.P, d.N), smem_a = tc::dbc_tma_smem(d.P, std::min(d.N, 128));
-                CUtensorMap mX128, mG128;
                 if (!map_bshd(&mX128, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, 128) ||
                     !map_bshd(&mG128, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, 128))
                     return BISSD_ERR_ALIGN;
@@ -541,11 +555,12 @@ do {                                                                            
                 }
                 BISSD_ALLOW(tc::dbc_accum_tma<T>, smem_a);
                 if (!no_ws() && tc::dbc_grp_ok(d.P, d.N, d.Q)) {
-                    const size_t smem_g = tc::dbc_grp_smem(d.Q, std::min(d.N, 128));
-                    BISSD_ALLOW(tc::dbc_accum_grp<T>, smem_g);
-                    BISSD_LAUNCH_ON(s_side, "tc_dbc_accum_grp", launch_pdl(tc::dbc_accum_grp<T>, dim3(d.b * d.nc * d.G * w.nsplit * w.dbc_ks, 1, 2), tc::kDbcGrpThreads, smem_g, s_side,
-                        d, mEf, mEb, mSf, mSb, mX128, mG128, a.dt_out, a.cs_f, a.cs_b, F(w.dB_part), F(w.dC_part), w.dbc_ks, status));
-                    part_heads = d.G * dbc_slots(d, w.dbc_ks);
+                    dbc_last = fused_cb && head_parts(d) == 1 && tc::bmm_bwd_tma_ok(d.N, d.Q);   // launched after the dCB kernel, below
+                    if (!dbc_last) {
+                        const int rc = launch_dbc(tc::dbc_accum_grp<T, false>, tc::LastMaps{}, s_side);
+                        if (rc != BISSD_OK) return rc;
+                        part_heads = d.G * dbc_slots(d, w.dbc_ks);
+                    }
                 } else
                 BISSD_LAUNCH("tc_dbc_accum_tma", tc::dbc_accum_tma<T><<<dim3(d.b * d.nc * d.G * w.nsplit, nlt_tc, 2), tc::kThreads, smem_a, s>>>(
                     d, mEf, mEb, mSf, mSb, mX128, mG128, a.dt_out, a.cs_f, a.cs_b, F(w.dB_part), F(w.dC_part), status));
@@ -662,16 +677,29 @@ do {                                                                            
                 dg, none, none, x, z, gv, a.dt_out, a.cs_f, a.cs_b, F(w.cb), F(w.da_f), F(w.da_b), status));
         }
     }
-    if (s_side != s) {                                           // the group-walking kernels rejoin before their results are read
+    auto join = [&]() -> int {                                   // the side stream's kernels rejoin before their results are read
+        if (s_side == s) return BISSD_OK;
         int rcj = note_cuda(cudaEventRecord(lease.sd->join, s_side), "cudaEventRecord");
         if (rcj == BISSD_OK) rcj = note_cuda(cudaStreamWaitEvent(s, lease.sd->join, 0), "cudaStreamWaitEvent");
+        return rcj;
+    };
+    {
+        const int rcj = join();
         if (rcj != BISSD_OK) return rcj;
-        s_side = s;
     }
-    if (bmm_tma) {
+    if (dbc_last) {
+        if (!bmm_tma) return BISSD_ERR_ALIGN;                    // its operands are the ones the dCB kernel's branch has mapped
+        if (s_side != s) {
+            int rcj = note_cuda(cudaEventRecord(lease.sd->fork2, s), "cudaEventRecord");
+            if (rcj == BISSD_OK) rcj = note_cuda(cudaStreamWaitEvent(s_side, lease.sd->fork2, 0), "cudaStreamWaitEvent");
+            if (rcj != BISSD_OK) return rcj;
+        }
+        const int rcl = launch_dbc(tc::dbc_accum_grp<T, true>, tc::LastMaps{mDm, mDk, mBb, mCb, gr.dB, gr.dC}, s_side);
+        if (rcl != BISSD_OK) return rcl;
+    } else if (bmm_tma) {
         const size_t smem_b = tc::bmm_bwd_tma_smem(d.Q);
         BISSD_ALLOW(tc::bmm_bwd_tma<T>, smem_b);
-        BISSD_LAUNCH("tc_bmm_bwd_tma", launch_pdl(tc::bmm_bwd_tma<T>, dim3(d.b * d.nc * d.G * 2, d.Q / 128, d.N / 64), tc::kThreads, smem_b, s, 
+        BISSD_LAUNCH("tc_bmm_bwd_tma", launch_pdl(tc::bmm_bwd_tma<T>, dim3(d.b * d.nc * d.G * 2, d.Q / 128, d.N / 64), tc::kThreads, smem_b, s,
             d, mDm, mDk, mBb, mCb, F(w.dB_part), F(w.dC_part), part_heads, gr.dB, gr.dC, status));
     } else {
         const size_t smem_n = tc::smem_bytes(ntN, 0);
@@ -690,7 +718,7 @@ do {                                                                            
     BISSD_LAUNCH("final_reduce", launch_pdl(simt::final_reduce<1024>, d.H, 1024, 0, s, 
         d, F(w.dApart), F(w.dbiaspart), d.has_D ? F(w.dDpart) : nullptr, dd_slots ? dd_slots : nlt, dd_compact ? 1 : 0, a.dA, d.has_bias ? a.ddt_bias : nullptr,
         d.has_D ? a.dD : nullptr));
-    return BISSD_OK;
+    return dbc_last ? join() : BISSD_OK;
 }
 
 }  // namespace bissd

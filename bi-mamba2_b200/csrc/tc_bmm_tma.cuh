@@ -1,8 +1,10 @@
 // CB[b,c,g,l,s] = C[l].B[s] with both operands by TMA (see tc::bmm_cb for the thread-staged form and the layouts).
 // One shot per CTA: a 128 x 128 tile of (l, s); the C rows and the B rows arrive as K-major tiles of dstate/64 slabs,
-// one MMA chain gives the tile, a second one with the operands swapped gives the same tile of the transpose, so that
-// every store is a row-contiguous vector.  Outputs, each optional: CB16 (bf16), CBt16 (bf16, transposed), CBs (fp32
-// in strips of 16 columns, [Q/16][Q rows][16]).  Rows past the end of the sequence read as zeros.
+// one MMA chain gives the tile, a second one with the operands swapped gives the same tile of the transpose.  Outputs,
+// each optional: the bf16 tile (tmO), its transpose (tmOt), CBs (fp32 in strips of 16 columns, [Q/16][Q rows][16]).
+// The 16-bit tiles leave by TMA from shared memory, over C and B, which are dead by then: as per-lane row pieces, 32
+// different lines per store instruction, they were most of this kernel's time (b2 L8192 G8: 51 us a launch; bound by
+// the 67 or 134 MB it writes).  Rows past the end of the sequence read as zeros.
 // grid (b*nc*G, Q/128, Q/128).
 #pragma once
 #include "tc_scan_tma.cuh"
@@ -11,12 +13,16 @@ namespace bissd {
 namespace tc {
 
 inline bool bmm_cb_tma_ok(int N, int Q) { return N % 64 == 0 && N <= 256 && (Q == 128 || Q == 256); }
-inline size_t bmm_cb_tma_smem(int N) { return 1024 + 2 * (size_t)(N / 64) * 16384; }
+inline size_t bmm_cb_tma_smem(int N, bool transposed) {         // C and B, then the tile and its transpose
+    const size_t in = 2 * (size_t)(N / 64) * 16384, out = transposed ? 65536 : 32768;
+    return 1024 + (in > out ? in : out);
+}
 
 template <class T>
 __global__ void __launch_bounds__(kThreads)
-bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmB, __nv_bfloat16 *CB16,
-           __nv_bfloat16 *CBt16, float *CBs, int *status) {
+bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmB,
+           const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmOt, bool plain, bool transposed, float *CBs,
+           int *status) {
     pdl_begin();
     extern __shared__ uint8_t dyn[];
     __shared__ uint64_t bar_in, bar_done;
@@ -26,7 +32,7 @@ bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constan
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = blockIdx.x % d.G, c = (blockIdx.x / d.G) % d.nc, b = blockIdx.x / (d.G * d.nc);
     const int l0 = blockIdx.y * kTileM, s0 = blockIdx.z * 128;
-    const uint32_t ncols = CBt16 ? 256 : 128;
+    const uint32_t ncols = transposed ? 256 : 128;
     if (warp == 0) tmem_alloc(&tmem_slot, ncols);
     if (tid == 32) {                                            // barriers and loads by the same thread, before the sync
         mbar_init(&bar_in, 1);
@@ -48,7 +54,7 @@ bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constan
         if (ok) {
             tc_fence_after();
             const uint32_t idesc = instr_desc(AbFmt<T>::v, false, false, 128);
-            for (int t = 0; t < (CBt16 ? 2 : 1); ++t)
+            for (int t = 0; t < (transposed ? 2 : 1); ++t)
                 for (int j = 0; j < nsl; ++j)
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk) {
@@ -64,11 +70,19 @@ bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constan
     tc_fence_after();
     if (!ok && tid == 0) atomicExch(status, kErrMmaTimeout);
     if (ok) {
-        const int r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 64;     // this thread: row r, columns c0 .. c0 + 63 of either tile
+        const int r = (warp & 3) * 32 + lane, half = warp >> 2, c0 = half * 64;   // this thread: row r, columns c0 .. c0 + 63 of either tile
         const long long tile = ((long long)(b * d.nc + c) * d.G + g) * Q * Q;
         const uint32_t tl = tmem_lane_base(tmem) + c0;
-        if (CB16 || CBs) {
-            const int l = l0 + r;
+        // 32 values of row r as four swizzled 16-byte pieces of slab `half` (rows of 128 bytes)
+        auto stage = [&](uint8_t *slab, int hc, const float (&v)[32]) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 8) {
+                const float o[8] = {v[j], v[j + 1], v[j + 2], v[j + 3], v[j + 4], v[j + 5], v[j + 6], v[j + 7]};
+                *reinterpret_cast<uint4 *>(slab + r * 128 + ((((hc + j) >> 3) ^ (r & 7)) << 4)) = pack8<__nv_bfloat16>(o);
+            }
+        };
+        uint8_t *so = smC, *st = smC + 32768;                   // [2 slabs of 128 x 64]
+        if (plain || CBs) {
 #pragma unroll
             for (int hc = 0; hc < 64; hc += 32) {
                 float v[32];
@@ -77,30 +91,29 @@ bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constan
                 if (CBs) {
 #pragma unroll
                     for (int j = 0; j < 32; j += 4)
-                        *reinterpret_cast<float4 *>(CBs + tile + (long long)((sc + j) >> 4) * Q * 16 + l * 16 + ((sc + j) & 15)) =
+                        *reinterpret_cast<float4 *>(CBs + tile + (long long)((sc + j) >> 4) * Q * 16 + (l0 + r) * 16 + ((sc + j) & 15)) =
                             make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
                 }
-                if (CB16) {
-#pragma unroll
-                    for (int j = 0; j < 32; j += 8) {
-                        const float o[8] = {v[j], v[j + 1], v[j + 2], v[j + 3], v[j + 4], v[j + 5], v[j + 6], v[j + 7]};
-                        *reinterpret_cast<uint4 *>(CB16 + tile + (long long)l * Q + sc + j) = pack8<__nv_bfloat16>(o);
-                    }
-                }
+                if (plain) stage(so + half * 16384, hc, v);
             }
         }
-        if (CBt16) {
-            const int srow = s0 + r;
+        if (transposed) {
 #pragma unroll
             for (int hc = 0; hc < 64; hc += 32) {
                 float v[32];
                 tmem_ld32(tl + 128 + hc, v);
-#pragma unroll
-                for (int j = 0; j < 32; j += 8) {
-                    const float o[8] = {v[j], v[j + 1], v[j + 2], v[j + 3], v[j + 4], v[j + 5], v[j + 6], v[j + 7]};
-                    *reinterpret_cast<uint4 *>(CBt16 + tile + (long long)srow * Q + l0 + c0 + hc + j) = pack8<__nv_bfloat16>(o);
-                }
+                stage(st + half * 16384, hc, v);
             }
+        }
+        fence_async_smem();
+        __syncthreads();
+        if (tid == 0) {
+            const int row = ((b * d.nc + c) * d.G + g) * Q;
+            for (int k = 0; k < 2; ++k) {
+                if (plain) tma_store2(&tmO, so + k * 16384, s0 + k * 64, row + l0);
+                if (transposed) tma_store2(&tmOt, st + k * 16384, l0 + k * 64, row + s0);
+            }
+            tma_store_wait();
         }
     }
     tc_fence_before();

@@ -169,12 +169,18 @@ dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
 // turn the left tile as it landed into its two row-scaled copies (one buffer: the copies of head i + 1 are written
 // once the MMAs of head i are done), lane 0 of warp 8 issues every TMA load and every MMA; two stages of (left
 // tile + 2 right tiles).  The heads accumulate in tensor memory, two parts of them (head_parts) side by side; a pair of
-// parts is read out together.  With few blocks the parts are dealt to ks of them (dbc_ksplit).  Bounded waits, ids 51-56
+// parts is read out together.  With few blocks the parts are dealt to ks of them (dbc_ksplit).  Bounded waits, ids 51-58
 // in the status word.
 // grid (b*nc*G*ks*nsplit, 1, 2); blockIdx.z: 0 = dB, 1 = dC.  part layout [b, nc*Q, G, slots, N] fp32: a slot per pair of
 // parts, or per part where every block has one.
+//
+// LAST: the kernel also adds the product with dCB (dB += dCB^T C, dC += dCB B, see bmm_bwd_tma) to the same accumulators
+// and writes dB and dC themselves: after the last head both operands land in the ring's and the scaled copies' memory -
+// [Q x Q] of dCB and [Q x 128] of C or B fit exactly - and 2 Q / 16 more MMAs follow.  Saves the round trip of the fp32
+// partial results (268 MB at b2 L8192 G8 N128) and a launch; taken where the heads are one part (head_parts), so that
+// the order of additions does not depend on the batch.
 struct DbcGrpShared {
-    uint64_t full[2], scaled, done[2], wbar;
+    uint64_t full[2], scaled, done[2], wbar, last_in, last_done;
     uint32_t tmem_base;
     int fail;
 };
@@ -183,13 +189,17 @@ inline size_t dbc_grp_smem(int Q, int nt) {
     return 1024 + 2 * ((size_t)Q * 128 + 2 * (size_t)(nt / 64) * 64 * 128) + 2 * (size_t)Q * 128 + 2 * 2 * (size_t)Q * 4;
 }
 constexpr int kDbcGrpThreads = kThreads + 32;
+struct LastMaps {                                               // operands and results of the product with dCB
+    CUtensorMap Dm, Dk, B, C;
+    MutView dB, dC;
+};
 
-template <class T>
+template <class T, bool LAST>
 __global__ void __launch_bounds__(kDbcGrpThreads, 1)
 dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_constant__ CUtensorMap tmEb,
               const __grid_constant__ CUtensorMap tmSf, const __grid_constant__ CUtensorMap tmSb,
               const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG, const float *dt_out,
-              const float *cs_f, const float *cs_b, float *dB_part, float *dC_part, int ks, int *status) {
+              const float *cs_f, const float *cs_b, float *dB_part, float *dC_part, int ks, const __grid_constant__ LastMaps last, int *status) {
     pdl_begin();
     extern __shared__ uint8_t dyn[];
     __shared__ DbcGrpShared sh;
@@ -231,6 +241,8 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
             mbar_init(&sh.full[i], 1);
             mbar_init(&sh.done[i], 1);
         }
+        mbar_init(&sh.last_in, 1);
+        mbar_init(&sh.last_done, 1);
         sh.fail = 0;
         fence_mbar_init();
         load_head(0);
@@ -297,6 +309,34 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
                                  (i > start || dir > 0 || kk > 0) ? 1u : 0u);
                 umma_commit(&sh.done[i & 1]);
             }
+            if (LAST) {                                         // every buffer is free once the last head's MMAs are done
+                ok = ok && ws_wait(&sh.done[(R - 1) & 1], ((R - 1) >> 1) & 1, fail, 55);
+                if (ok) {
+                    const int row0 = ((b * d.nc + c) * d.G + grp) * Q, nsl = Q / 64;
+                    uint8_t *smD = base_sm, *smY = base_sm + Q * Q * 2;
+                    mbar_expect_tx(&sh.last_in, (uint32_t)(Q * Q * 2 + Q * nt * 2));
+                    if (which == 0)                             // [l x 64 s] blocks: dCB^T as it lies, MN-major
+                        for (int j = 0; j < nsl; ++j) tma_load2(smD + j * Q * 128, &last.Dm, j * 64, row0, &sh.last_in);
+                    else
+                        for (int rb = 0; rb < nrb; ++rb)
+                            for (int j = 0; j < nsl; ++j) tma_load2(smD + (rb * nsl + j) * 16384, &last.Dk, j * 64, row0 + rb * 128, &sh.last_in);
+                    for (int nb = 0; nb < nnb; ++nb)
+                        for (int rb = 0; rb < nrb; ++rb)
+                            tma_load4(smY + nb * Q * 128 + rb * 16384, which ? &last.B : &last.C, n0 + nb * 64, grp, c * Q + rb * 128, b, &sh.last_in);
+                    ok = ws_wait(&sh.last_in, 0, fail, 57);
+                    if (ok) {
+                        tc_fence_after();
+                        const uint32_t id2 = instr_desc(AbFmt<T>::v, which == 0, true, nt);
+                        for (int rb = 0; rb < nrb; ++rb)
+                            for (int kk = 0; kk < Q / 16; ++kk) {
+                                const uint64_t da = which == 0 ? smem_desc(smem_u32(smD) + rb * Q * 256 + kk * 2048, (uint32_t)Q * 128, 1024)
+                                                               : smem_desc(smem_u32(smD) + (rb * nsl + (kk >> 2)) * 16384 + (kk & 3) * 32, 16, 1024);
+                                umma(tmem + rb * nt, da, smem_desc(smem_u32(smY) + kk * 2048, (uint32_t)Q * 128, 1024), id2, 1u);
+                            }
+                        umma_commit(&sh.last_done);
+                    }
+                }
+            }
         }
     } else {
         // the sum of local parts 2 pair and 2 pair + 1 (`two`) as this block's next partial result
@@ -352,8 +392,28 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
             // every scaling warp is done with head i and the factors of head i + 1 are written
             ok = ws_wait_warp(&sh.wbar, i & 1, fail, 54);
         }
-        if (ok) ok = ws_wait_warp(&sh.done[(R - 1) & 1], ((R - 1) >> 1) & 1, fail, 55);
-        if (ok) write_out((nparts - 1) / 2, nparts > 1);
+        if (LAST) {
+            if (ok) ok = ws_wait_warp(&sh.last_done, 0, fail, 58);
+            if (ok) {
+                tc_fence_after();
+                const MutView ov = which ? last.dC : last.dB;
+                for (int rb = 0; rb < nrb; ++rb) {
+                    const int l = rb * 128 + (warp & 3) * 32 + lane;
+                    T *out = static_cast<T *>(ov.ptr) + b * ov.sb + (long long)(c * Q + l) * ov.sl + grp * ov.sh + n0;
+                    for (int c0 = (warp >> 2) * 32; c0 < nt; c0 += 64) {
+                        float v[32];
+                        tmem_ld32(tmem_lane_base(tmem) + rb * nt + c0, v);
+                        if (l < lim) {
+#pragma unroll
+                            for (int j = 0; j < 32; j += 8) *reinterpret_cast<uint4 *>(out + c0 + j) = pack8<T>(*reinterpret_cast<float(*)[8]>(&v[j]));
+                        }
+                    }
+                }
+            }
+        } else {
+            if (ok) ok = ws_wait_warp(&sh.done[(R - 1) & 1], ((R - 1) >> 1) & 1, fail, 55);
+            if (ok) write_out((nparts - 1) / 2, nparts > 1);
+        }
     }
     tc_fence_before();
     __syncthreads();

@@ -76,6 +76,17 @@ __device__ __forceinline__ void tma_load2(void *dst, const CUtensorMap *m, int x
         ::"r"(smem_u32(dst)), "l"(m), "r"(smem_u32(bar)), "r"(x), "r"(y)
         : "memory");
 }
+// Store a box from shared memory; the shared memory may be reused, and the block may end, after tma_store_wait by the same
+// thread.  The threads that wrote the box call fence_async_smem and meet in a barrier first.
+__device__ __forceinline__ void tma_store2(const CUtensorMap *m, const void *src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
+                 ::"l"(m), "r"(smem_u32(src)), "r"(x), "r"(y)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_store_wait() {
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
 __device__ __forceinline__ float ex2_approx(float v) {
     float r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
