@@ -1,5 +1,6 @@
 // C ABI of libbissd (declared in include/bissd.h): argument validation, workspace layout, kernel sequencing.
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -23,6 +24,7 @@
 #include "tc_scan_ws.cuh"
 #include "tc_selftest.cuh"
 #include "tc_state_tma.cuh"
+#include "tc_walk_tma.cuh"
 
 namespace bissd {
 
@@ -162,6 +164,46 @@ static bool map_bshd(CUtensorMap *m, int dtype, const void *ptr, long long sb, l
     return tc::make_map4(m, dtype, ptr, dims, str, box);
 }
 
+// The walk of tc_walk_tma.cuh, where it applies: its tensor maps and whether it is the faster way.
+struct Walk {
+    bool use = false;
+    CUtensorMap mRow, mCol, mSf, mSb;
+};
+// The walk takes a fixed time per chunk whatever else runs, one CTA an SM; the two kernels it replaces take the time of their
+// memory traffic.  Measured (us, forward and backward averaged): a chunk of the walk 1.0 / 1.4 at chunk 128 / 256 and headdim
+// 64, 2.1 / 2.9 at headdim 128; the two kernels 8 + 2.5 per million state elements, both directions.  So the walk wins unless
+// a long sequence of few heads leaves most SMs without one (b1 L8192 H8 chunk 256: 46 us against 16).
+static bool walk_pays(const Dims &d) {
+    const double ctas = 2.0 * d.b * d.H * tc::walk_tiles(d), waves = std::ceil(ctas / sm_count());
+    const double walk = 4.0 + waves * d.nc * (d.P / 64) * (0.6 + 0.8 * d.Q / 256);
+    const double apart = 8.0 + 2.5e-6 * 2.0 * d.b * d.nc * d.H * d.P * d.N;
+    return walk < apart;
+}
+static Walk plan_walk(const Dims &d, int dtype, int phases, const bissd_tensor &row, const View &col, const float *dt_out,
+                      const float *cs_f, const float *cs_b, const void *states_f, const void *states_b) {
+    Walk w;
+    if (no_tma() || no_ws() || (phases & 3) != 3 || !tc::walk_ok(d.P, d.N, d.Q) || !walk_pays(d)) return w;
+    if ((reinterpret_cast<uintptr_t>(dt_out) | reinterpret_cast<uintptr_t>(cs_f) | reinterpret_cast<uintptr_t>(cs_b)) % 16) return w;
+    const unsigned rows = tc::walk_rows(d.P / 64);
+    const unsigned long long srows = (unsigned long long)d.b * d.nc * d.H * d.P;
+    w.use = map_bshd(&w.mRow, dtype, row.ptr, row.stride_batch, row.stride_seq, row.stride_head, d.N, d.G, d.L, d.b, rows) &&
+            map_bshd(&w.mCol, dtype, col.ptr, col.sb, col.sl, col.sh, d.P, d.H, d.L, d.b, rows) &&
+            tc::make_map2(&w.mSf, dtype, states_f, d.N, srows, 64, d.P) && tc::make_map2(&w.mSb, dtype, states_b, d.N, srows, 64, d.P);
+    return w;
+}
+template <class T, int MODE>
+static int launch_walk(const Dims &d, const Walk &w, const tc::WalkArgs &args, int *status, cudaStream_t s) {
+    auto launch = [&](auto kernel) -> int {
+        const size_t smem = tc::walk_smem(d.P, MODE);
+        BISSD_ALLOW(kernel, smem);
+        BISSD_LAUNCH(MODE ? "tc_dstate_walk" : "tc_state_walk", launch_pdl(kernel, dim3(2 * d.b * d.H * tc::walk_tiles(d)), tc::kWalkThreads, smem, s,
+            d, w.mRow, w.mCol, w.mSf, w.mSb, args, status));
+        return BISSD_OK;
+    };
+    if (d.N == 64) return d.P == 64 ? launch(tc::state_walk<T, MODE, 1, true>) : launch(tc::state_walk<T, MODE, 2, true>);
+    return d.P == 64 ? launch(tc::state_walk<T, MODE, 1, false>) : launch(tc::state_walk<T, MODE, 2, false>);
+}
+
 template <class T>
 static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaStream_t s) {
     const FwdWs w = fwd_layout(d);
@@ -171,13 +213,14 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
     const View x = view_of(a.x), Bm = view_of(a.B), Cm = view_of(a.C), z = view_of(a.z);
     const int bch = d.b * d.nc * d.H;
     const int ntP = tc::round_up(d.P, 16), ntQ = tc::round_up(d.Q, 16);
+    const Walk walk = plan_walk(d, a.p.x_dtype, a.phases, a.B, x, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
     if (a.phases & BISSD_PHASE_LOCAL) {
         int rc = note_cuda(cudaMemsetAsync(ws, 0, kWsHeader, s), "cudaMemsetAsync");
         if (rc != BISSD_OK) return rc;
         BISSD_LAUNCH("cumsum_fwd", launch_pdl(simt::cumsum_fwd, d.b * d.nc * d.H, 256, 0, s, 
             d, a.dt.ptr, a.p.dt_dtype, a.dt.stride_batch, a.dt.stride_seq, a.dt.stride_head, a.A, a.dt_bias, a.dt_out,
             a.cs_f, a.cs_b));
-        {
+        if (!walk.use) {
             const size_t smem = tc::smem_bytes(ntP, 2 * d.Q);
             bool st_done = false;
             if (!no_tma() && (tc::state_tma_ok(d.P, d.N, d.Q) || (!no_ws() && tc::state_grp_ok(d.P, d.N, d.Q, d.R)))) {
@@ -213,7 +256,11 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
     }
     // the recurrence runs in both phases: from zero (or init_*) in LOCAL, again with init_* in FINISH
     const bool need_pass = (a.phases & BISSD_PHASE_LOCAL) || (a.init_f || a.init_b);
-    if (need_pass) {
+    if (walk.use) {
+        const tc::WalkArgs wa{a.dt_out, a.cs_f, a.cs_b, a.init_f, a.init_b, a.final_f, a.final_b, a.states_f, a.states_b, nullptr};
+        const int rc = launch_walk<T, 0>(d, walk, wa, status, s);
+        if (rc != BISSD_OK) return rc;
+    } else if (need_pass) {
         BISSD_LAUNCH("state_passing_fwd", launch_pdl(pass_ahead(d) ? simt::state_passing_fwd4<T, 8> : simt::state_passing_fwd4<T, 1>, pass_grid(d), pass_threads(d), 0, s,
             d, loc, a.cs_f, a.cs_b, a.init_f, a.init_b, a.states_f, a.states_b, a.final_f, a.final_b));
     }
@@ -334,6 +381,7 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
         dg.has_z = 0;
         gv = View{ws + w.g, (long long)d.L * d.H * d.P, (long long)d.H * d.P, (long long)d.P};
     }
+    const Walk walk = plan_walk(d, a.p.x_dtype, a.phases, a.C, gv, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
     if (a.phases & BISSD_PHASE_LOCAL) {
         int rc = note_cuda(cudaMemsetAsync(ws, 0, kWsHeader, s), "cudaMemsetAsync");
         if (rc != BISSD_OK) return rc;
@@ -342,7 +390,7 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
             BISSD_LAUNCH("gate_bwd", launch_pdl(tc::gate_bwd<T>, (unsigned)((chunks + 255) / 256), 256, 0, s, 
                 d, dout, z, out_x, ws + w.g, a.dz));
         }
-        {
+        if (!walk.use) {
             const size_t smem = tc::smem_bytes(ntP, 2 * d.Q);
             bool st_done = false;
             if (!no_tma() && (tc::state_tma_ok(d.P, d.N, d.Q) || (!no_ws() && tc::state_grp_ok(d.P, d.N, d.Q, d.R)))) {
@@ -377,7 +425,12 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
         }
     }
     const bool need_pass = (a.phases & BISSD_PHASE_LOCAL) || (a.dfinal_f || a.dfinal_b);
-    if (need_pass) {
+    if (walk.use) {
+        const tc::WalkArgs wa{a.dt_out, a.cs_f, a.cs_b, a.dfinal_f, a.dfinal_b, a.dinit_f, a.dinit_b, E16,
+                              static_cast<char *>(E16) + (size_t)d.b * d.nc * d.H * d.P * d.N * 2, F(w.dTpart)};
+        const int rc = launch_walk<T, 1>(d, walk, wa, status, s);
+        if (rc != BISSD_OK) return rc;
+    } else if (need_pass) {
         BISSD_LAUNCH("state_passing_bwd", launch_pdl(pass_ahead(d) ? simt::state_passing_bwd4<T, 8> : simt::state_passing_bwd4<T, 1>, pass_grid(d), pass_threads(d), 0, s,
             d, F(w.gloc), a.states_f, a.states_b, a.cs_f, a.cs_b, a.dfinal_f, a.dfinal_b, nullptr, E16, F(w.dTpart), a.dinit_f, a.dinit_b));
     }
@@ -713,7 +766,7 @@ do {                                                                            
     cs.nf = F(w.nf); cs.nb = F(w.nb); cs.pf = F(w.pf); cs.pb = F(w.pb);
     if (use_u4) { cs.u4 = F(w.u4); cs.u4_tiles = u4_tiles; }
     else { cs.da_f = F(w.da_f); cs.da_b = F(w.da_b); }
-    cs.dTpart = F(w.dTpart); cs.nblk = w.nslots; cs.nsplit = nsplit; cs.ddt = gr.ddt; cs.dApart = F(w.dApart); cs.dbiaspart = F(w.dbiaspart);
+    cs.dTpart = F(w.dTpart); cs.nblk = walk.use ? tc::walk_slots(d) : pass_slots(d); cs.nsplit = nsplit; cs.ddt = gr.ddt; cs.dApart = F(w.dApart); cs.dbiaspart = F(w.dbiaspart);
     BISSD_LAUNCH("cumsum_bwd", launch_pdl(simt::cumsum_bwd, d.b * d.nc * d.H, 256, 0, s, d, cs));
     BISSD_LAUNCH("final_reduce", launch_pdl(simt::final_reduce<1024>, d.H, 1024, 0, s, 
         d, F(w.dApart), F(w.dbiaspart), d.has_D ? F(w.dDpart) : nullptr, dd_slots ? dd_slots : nlt, dd_compact ? 1 : 0, a.dA, d.has_bias ? a.ddt_bias : nullptr,

@@ -81,6 +81,7 @@ inline BwdWs bwd_layout(const Dims &d, bool tc) {
     const size_t st = (size_t)d.b * d.nc * d.H * d.P * d.N;
     const size_t hq = (size_t)d.b * d.H * d.nc * d.Q, qq = (size_t)d.b * d.nc * d.G * d.Q * d.Q;
     w.nslots = pass_slots(d);
+    if (tc) w.nslots = std::max(w.nslots, 8 * ceil_div(d.N, 128));   // tc::state_walk: one per warp
     w.nlt = ceil_div(d.Q, simt::TILE);
     w.nsplit = tc ? ceil_div(d.N, 128) : 1;
     w.hsplit = tc ? 1 : simt_hsplit(d);

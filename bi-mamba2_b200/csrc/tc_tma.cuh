@@ -76,6 +76,11 @@ __device__ __forceinline__ void tma_load2(void *dst, const CUtensorMap *m, int x
         ::"r"(smem_u32(dst)), "l"(m), "r"(smem_u32(bar)), "r"(x), "r"(y)
         : "memory");
 }
+// `bytes` (a multiple of 16) from a 16-byte aligned address to a 16-byte aligned place in shared memory
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
 // Store a box from shared memory; the shared memory may be reused, and the block may end, after tma_store_wait by the same
 // thread.  The threads that wrote the box call fence_async_smem and meet in a barrier first.
 __device__ __forceinline__ void tma_store2(const CUtensorMap *m, const void *src, int x, int y) {
