@@ -19,6 +19,7 @@
 #include "tc_dbc_tma.cuh"
 #include "tc_dcb_tma.cuh"
 #include "tc_bmm_tma.cuh"
+#include "tc_cumsum.cuh"
 #include "tc_dx_tma.cuh"
 #include "tc_scan_tma.cuh"
 #include "tc_scan_ws.cuh"
@@ -130,6 +131,9 @@ static bool aligned16(const bissd_tensor &t) {
     return (reinterpret_cast<uintptr_t>(t.ptr) % 16 == 0) && t.stride_batch % 8 == 0 && t.stride_seq % 8 == 0 &&
            t.stride_head % 8 == 0;
 }
+static bool all_aligned16(const float *a, const float *b, const float *c) {
+    return (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) % 16 == 0;
+}
 static bool force_simt() {
     static const bool v = [] { const char *e = getenv("BISSD_FORCE_SIMT"); return e && e[0] == '1'; }();
     return v;
@@ -183,7 +187,7 @@ static Walk plan_walk(const Dims &d, int dtype, int phases, const bissd_tensor &
                       const float *cs_f, const float *cs_b, const void *states_f, const void *states_b) {
     Walk w;
     if (no_tma() || no_ws() || (phases & 3) != 3 || !tc::walk_ok(d.P, d.N, d.Q) || !walk_pays(d)) return w;
-    if ((reinterpret_cast<uintptr_t>(dt_out) | reinterpret_cast<uintptr_t>(cs_f) | reinterpret_cast<uintptr_t>(cs_b)) % 16) return w;
+    if (!all_aligned16(dt_out, cs_f, cs_b)) return w;
     const unsigned rows = tc::walk_rows(d.P / 64);
     const unsigned long long srows = (unsigned long long)d.b * d.nc * d.H * d.P;
     w.use = map_bshd(&w.mRow, dtype, row.ptr, row.stride_batch, row.stride_seq, row.stride_head, d.N, d.G, d.L, d.b, rows) &&
@@ -217,9 +221,9 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
     if (a.phases & BISSD_PHASE_LOCAL) {
         int rc = note_cuda(cudaMemsetAsync(ws, 0, kWsHeader, s), "cudaMemsetAsync");
         if (rc != BISSD_OK) return rc;
-        BISSD_LAUNCH("cumsum_fwd", launch_pdl(simt::cumsum_fwd, d.b * d.nc * d.H, 256, 0, s, 
+        BISSD_LAUNCH("cumsum_fwd", launch_pdl(d.Q <= 128 ? tc::cumsum_fwd<4> : tc::cumsum_fwd<8>, tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s,
             d, a.dt.ptr, a.p.dt_dtype, a.dt.stride_batch, a.dt.stride_seq, a.dt.stride_head, a.A, a.dt_bias, a.dt_out,
-            a.cs_f, a.cs_b));
+            a.cs_f, a.cs_b, all_aligned16(a.dt_out, a.cs_f, a.cs_b)));
         if (!walk.use) {
             const size_t smem = tc::smem_bytes(ntP, 2 * d.Q);
             bool st_done = false;
@@ -334,16 +338,15 @@ do {                                                                            
                 const unsigned bC[4] = {64, 1, 128, 1};
                 const unsigned long long dX[4] = {(unsigned long long)d.P, (unsigned long long)d.H, (unsigned long long)d.L, (unsigned long long)d.b};
                 const unsigned long long sX[3] = {(unsigned long long)a.x.stride_head * 2, (unsigned long long)a.x.stride_seq * 2, (unsigned long long)a.x.stride_batch * 2};
-                const unsigned bX[4] = {64, 1, (unsigned)d.Q, 1};
+                const unsigned bX[4] = {64, 1, 64, 1};
                 const unsigned long long rows = (unsigned long long)d.b * d.nc * d.H * d.P;
                 if (tc::make_map4(&mC, a.p.x_dtype, a.C.ptr, dC, sC, bC) && tc::make_map4(&mX, a.p.x_dtype, a.x.ptr, dX, sX, bX) &&
                     tc::make_map2(&mSf, a.p.x_dtype, a.states_f, d.N, rows, 64, d.P) &&
                     tc::make_map2(&mSb, a.p.x_dtype, a.states_b, d.N, rows, 64, d.P)) {
-                    const int rounds = tc::scan_tma_rounds(d.P, d.N, d.Q);
-                    const size_t smem_t = tc::scan_tma_smem(d.P, d.N, d.Q, rounds);
+                    const size_t smem_t = tc::scan_tma_smem(d.P, d.Q);
                     BISSD_ALLOW(tc::chunk_scan_tma<T>, smem_t);
-                    BISSD_LAUNCH("tc_chunk_scan_tma", tc::chunk_scan_tma<T><<<dim3(bch, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_t, s>>>(
-                        d, mC, mSf, mSb, mX, x, z, a.D, a.dt_out, a.cs_f, a.cs_b, CB, mview_of(a.out), mview_of(a.out_x), rounds, status));
+                    BISSD_LAUNCH("tc_chunk_scan_tma", launch_pdl(tc::chunk_scan_tma<T>, dim3(bch, d.Q / tc::kTileM), tc::kThreads, smem_t, s,
+                        d, mC, mSf, mSb, mX, x, z, a.D, a.dt_out, a.cs_f, a.cs_b, CB, mview_of(a.out), mview_of(a.out_x), status));
                     tma_done = true;
                 }
             }
@@ -553,18 +556,17 @@ do {                                                                            
             const unsigned bB4[4] = {64, 1, 128, 1};
             const unsigned long long dG4[4] = {(unsigned long long)d.P, (unsigned long long)d.H, (unsigned long long)d.L, (unsigned long long)d.b};
             const unsigned long long sG4[3] = {(unsigned long long)gv.sh * 2, (unsigned long long)gv.sl * 2, (unsigned long long)gv.sb * 2};
-            const unsigned bG4[4] = {64, 1, (unsigned)d.Q, 1};
+            const unsigned bG4[4] = {64, 1, 64, 1};
             const unsigned long long rows = (unsigned long long)d.b * d.nc * d.H * d.P;
             const char *e16 = static_cast<const char *>(E16);
             if (tc::make_map4(&mB, a.p.x_dtype, a.B.ptr, dB4, sB4, bB4) && tc::make_map4(&mG, a.p.x_dtype, gv.ptr, dG4, sG4, bG4) &&
                 tc::make_map2(&mEf, a.p.x_dtype, e16, d.N, rows, 64, d.P) &&
                 tc::make_map2(&mEb, a.p.x_dtype, e16 + rows * d.N * 2, d.N, rows, 64, d.P)) {
-                const int rounds = tc::scan_tma_rounds(d.P, d.N, d.Q);
-                const size_t smem_t = tc::dx_tma_smem(d.P, d.N, d.Q, rounds);
+                const size_t smem_t = tc::dx_tma_smem(d.P, d.Q);
                 BISSD_ALLOW(tc::dx_tma<T>, smem_t);
-                BISSD_LAUNCH("tc_dx_tma", tc::dx_tma<T><<<dim3(bch, nlt_tc), tc::kThreads, smem_t, s>>>(
+                BISSD_LAUNCH("tc_dx_tma", launch_pdl(tc::dx_tma<T>, dim3(bch, nlt_tc), tc::kThreads, smem_t, s,
                     d, mB, mEf, mEb, mG, x, gv, a.D, a.dt_out, a.cs_f, a.cs_b, F(w.cbt), gr.dx, F(w.ddt_out), F(w.nf), F(w.nb),
-                    F(w.dDpart), rounds, status));
+                    F(w.dDpart), status));
                 dx_done = true;
             }
         }
@@ -767,7 +769,8 @@ do {                                                                            
     if (use_u4) { cs.u4 = F(w.u4); cs.u4_tiles = u4_tiles; }
     else { cs.da_f = F(w.da_f); cs.da_b = F(w.da_b); }
     cs.dTpart = F(w.dTpart); cs.nblk = walk.use ? tc::walk_slots(d) : pass_slots(d); cs.nsplit = nsplit; cs.ddt = gr.ddt; cs.dApart = F(w.dApart); cs.dbiaspart = F(w.dbiaspart);
-    BISSD_LAUNCH("cumsum_bwd", launch_pdl(simt::cumsum_bwd, d.b * d.nc * d.H, 256, 0, s, d, cs));
+    BISSD_LAUNCH("cumsum_bwd", launch_pdl(d.Q <= 128 ? tc::cumsum_bwd<4> : tc::cumsum_bwd<8>, tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s,
+        d, cs, all_aligned16(a.dt_out, a.dt_out, a.dt_out)));
     BISSD_LAUNCH("final_reduce", launch_pdl(simt::final_reduce<1024>, d.H, 1024, 0, s, 
         d, F(w.dApart), F(w.dbiaspart), d.has_D ? F(w.dDpart) : nullptr, dd_slots ? dd_slots : nlt, dd_compact ? 1 : 0, a.dA, d.has_bias ? a.ddt_bias : nullptr,
         d.has_D ? a.dD : nullptr));

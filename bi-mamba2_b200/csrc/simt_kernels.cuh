@@ -170,21 +170,6 @@ __device__ __forceinline__ void chunk_cumsum(const Dims &d, const void *dt, int 
     float dummy1 = 0.f, dummy2 = 0.f;
     block_scan4(f, dummy1, r, dummy2, tot);
 }
-static __global__ void __launch_bounds__(256) cumsum_fwd(Dims d, const void *dt, int dt_dtype, long long dsb, long long dsl,
-                                                      long long dsh, const float *A, const float *dt_bias, float *dt_out,
-                                                      float *cs_f, float *cs_b) {
-    pdl_begin();
-    __shared__ float tot[4][8];
-    const int h = blockIdx.x % d.H, c = (blockIdx.x / d.H) % d.nc, b = blockIdx.x / (d.H * d.nc);
-    const long long base = ((long long)(b * d.H + h) * d.nc + c) * d.Q;
-    float v, f, r;
-    chunk_cumsum(d, dt, dt_dtype, dsb, dsl, dsh, A, dt_bias, b, c, h, min(d.Q, d.L - c * d.Q), tot, v, f, r);
-    if (threadIdx.x < d.Q) {
-        dt_out[base + threadIdx.x] = v;
-        cs_f[base + threadIdx.x] = f;
-        cs_b[base + threadIdx.x] = r;
-    }
-}
 
 // ---------------------------------------------------------------------------------------------------------
 // Assemble d(a) from its six terms, go back through the discretisation.  One CTA per (batch, chunk, head), see above.
@@ -305,12 +290,6 @@ __device__ __forceinline__ void cumsum_bwd_role(const Dims &d, const CumsumBwd &
         a.dApart[(long long)(b * d.nc + c) * d.H + h] = ta;
         a.dbiaspart[(long long)(b * d.nc + c) * d.H + h] = tb;
     }
-}
-static __global__ void __launch_bounds__(256) cumsum_bwd(Dims d, CumsumBwd a) {
-    pdl_begin();
-    __shared__ float tot[4][8];
-    __shared__ float red[2][8];
-    cumsum_bwd_role(d, a, blockIdx.x, tot, red);
 }
 
 // ---------------------------------------------------------------------------------------------------------

@@ -1,14 +1,17 @@
 // Forward chunk scan, TMA-fed variant (see simt::chunk_scan for the formula).
 //
-// Per CTA: one (batch, chunk, head) and 128 rows l.  C, the two entering states and x arrive by TMA and stay resident
-// in shared memory; the two state products C.S_f^T and C.S_b^T go straight from those tiles into their own TMEM
-// accumulators (the row factors e^{cs_f[l]}, e^{cs_b[l]} are applied in the epilogue), and only the masked-decay
-// matrix M[l,s] = CB[l,s] Delta[s] (L_f + L_b)[l,s] is built by the threads, 64 columns at a time, in two stage buffers
-// that reuse the C / state tiles once those products have completed.  M is evaluated in the log2 domain with
-// per-column tables tf[s] = cs_f[s] log2e - log2 Delta[s] (tb likewise): M = CB * 2^(f2[l] - tf[s]) below the
-// diagonal, CB * 2^(b2[l] - tb[s]) above it, twice that on it.
+// Per CTA: one (batch, chunk, head) and 128 rows l; two CTAs an SM - one tile is a chain of loads, products and sums, and the
+// other CTA's work fills the waits (headdim 128, dstate 256, b8 L1024 H16 chunk 128: one CTA an SM, everything resident,
+// took 129 us).  For that the products C.S_f^T and C.S_b^T take 64 dstate columns at a time: a slot holds a slab of C and
+// of both entering states, the next slab lands in the second slot meanwhile.  Both products have a TMEM accumulator; when
+// they are complete their sum, weighted by e^{cs_f[l]} and e^{cs_b[l]}, replaces the first of them, and the masked-decay
+// product is accumulated on top: 2 P columns of tensor memory instead of 3 P, which would round up to all of it.
+// The masked-decay matrix M[l,s] = CB[l,s] Delta[s] (L_f + L_b)[l,s] is built by the threads, 64 columns at a time, in two stage
+// buffers in the slot of the last slab; the x rows of the same 64 columns come by TMA into the other slot, two
+// pieces in turn.  M is evaluated in the log2 domain with per-column tables tf[s] = cs_f[s] log2e - log2 Delta[s] (tb
+// likewise): M = CB * 2^(f2[l] - tf[s]) below the diagonal, CB * 2^(b2[l] - tb[s]) above it, twice that on it.
 //
-// Shapes: headdim, dstate multiples of 64, chunk 128 or 256, everything resident must fit (checked on the host).
+// Shapes: headdim 64 or 128, dstate a multiple of 64 up to 256, chunk 128 or 256.
 #pragma once
 #include "tc_kernels.cuh"
 #include "tc_tma.cuh"
@@ -17,84 +20,118 @@ namespace bissd {
 namespace tc {
 
 struct ScanShared {
-    uint64_t bar_cs, bar_x, bar_st, bar_mid, free_bar[2], done_bar;   // bar_mid: every round of the state products but the last
+    uint64_t full[2], read[2], x_full[2], st_done, free_bar[2], done_bar;   // full / read: a slot has landed / its MMAs are done
     uint32_t tmem_base;
     int fail;
 };
+__host__ __device__ constexpr int scan_slot_bytes(int P) { return 16384 + 2 * P * 128; }   // [128 x 64] of C, [P x 64] of either state
+inline size_t scan_tma_smem(int P, int Q) { return 1024 + 2 * (size_t)scan_slot_bytes(P) + 4 * (size_t)Q * 4; }
+inline bool scan_tma_ok(int P, int N, int Q) { return (P == 64 || P == 128) && N % 64 == 0 && N <= 256 && (Q == 128 || Q == 256); }
 
-// The operands of the two state products (C or B rows and both state tiles) take dstate/64 slabs each.  Where all of
-// them do not fit beside x (headdim 128 with dstate 256), they come in `rounds` = 2 halves of dstate, the second
-// loaded into the same buffers once the MMAs of the first have read them.
-inline size_t scan_tma_smem(int P, int N, int Q, int rounds = 1) {
-    const size_t nsr = (size_t)(N / 64) / rounds;
-    return 1024 + nsr * 16384 + 2 * nsr * P * 128 + (size_t)(P / 64) * Q * 128 + 4 * Q * 4;
-}
-inline int scan_tma_rounds(int P, int N, int Q) {                // 0: shape not supported
-    if (P % 64 || N % 64 || (Q != 128 && Q != 256) || P > 128 || N > 256) return 0;
-    for (int rounds = 1; rounds <= 2; ++rounds) {
-        if ((N / 64) % rounds) continue;
-        const size_t nsr = (size_t)(N / 64) / rounds;
-        if (nsr * 16384 + 2 * nsr * P * 128 < 32768) continue;       // room for the two M stages
-        if (scan_tma_smem(P, N, Q, rounds) <= 200 * 1024) return rounds;
+// The loads and products of one tile up to both state products, for chunk_scan_tma and dx_tma; one thread.
+struct ScanFeed {
+    ScanShared &sh;
+    const Dims &d;
+    uint8_t *base_sm;
+    const CUtensorMap *mA, *mSf, *mSb, *mX;                     // rows (C or B), both states, x or g in boxes of 64 rows
+    int b, c, h, grp, l0;
+    __device__ __forceinline__ void init_barriers() {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&sh.full[i], 1);
+            mbar_init(&sh.read[i], 1);
+            mbar_init(&sh.x_full[i], 1);
+            mbar_init(&sh.free_bar[i], 1);
+        }
+        mbar_init(&sh.st_done, 1);
+        mbar_init(&sh.done_bar, 1);
+        sh.fail = 0;
+        fence_mbar_init();
     }
-    return 0;
-}
-inline bool scan_tma_ok(int P, int N, int Q) { return scan_tma_rounds(P, N, Q) > 0; }
+    __device__ __forceinline__ uint8_t *slot(int k) { return base_sm + (k & 1) * scan_slot_bytes(d.P); }
+    __device__ __forceinline__ uint8_t *stages() { return slot(d.N / 64 - 1); }   // two M stages, over the last slab
+    __device__ __forceinline__ uint8_t *x_piece(int i) { return slot(d.N / 64) + (i & 1) * d.P * 128; }
+    __device__ __forceinline__ void load_slab(int k) {
+        const int P = d.P, n0 = k * 64, row = ((b * d.nc + c) * d.H + h) * P;
+        uint8_t *dst = slot(k);
+        mbar_expect_tx(&sh.full[k & 1], (uint32_t)scan_slot_bytes(P));
+        tma_load4(dst, mA, n0, grp, c * d.Q + l0, b, &sh.full[k & 1]);
+        tma_load2(dst + 16384, mSf, n0, row, &sh.full[k & 1]);
+        tma_load2(dst + 16384 + P * 128, mSb, n0, row, &sh.full[k & 1]);
+    }
+    __device__ __forceinline__ void load_x(int i) {             // rows 64 i ... of the chunk
+        mbar_expect_tx(&sh.x_full[i & 1], (uint32_t)(d.P * 128));
+        for (int j = 0; j < d.P / 64; ++j) tma_load4(x_piece(i) + j * 8192, mX, j * 64, h, c * d.Q + i * 64, b, &sh.x_full[i & 1]);
+    }
+    __device__ __forceinline__ void start() {
+        load_slab(0);
+        if (d.N > 64) load_slab(1);
+        else { load_x(0); load_x(1); }
+    }
+    template <class T> __device__ __forceinline__ bool products(uint32_t tmem) {
+        const int P = d.P, ns = d.N / 64;
+        const uint32_t idesc = instr_desc(AbFmt<T>::v, false, false, P);
+        for (int k = 0; k < ns; ++k) {
+            if (!mbar_wait(&sh.full[k & 1], (k >> 1) & 1)) return false;
+            tc_fence_after();
+            const uint32_t sa = smem_u32(slot(k));
+            for (int dir = 0; dir < 2; ++dir)
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    umma(tmem + dir * P, smem_desc(sa + kk * 32, 16, 1024), smem_desc(sa + 16384 + dir * P * 128 + kk * 32, 16, 1024),
+                         idesc, (k > 0 || kk > 0) ? 1u : 0u);
+            umma_commit(k + 1 < ns ? &sh.read[k & 1] : &sh.st_done);
+            if (k >= 1) {                                       // slab k - 1 has been read: its slot takes slab k + 1, or x
+                if (!mbar_wait(&sh.read[(k - 1) & 1], ((k - 1) >> 1) & 1)) return false;
+                if (k + 1 < ns) load_slab(k + 1);
+                else { load_x(0); load_x(1); }
+            }
+        }
+        return true;
+    }
+    // M stage `it` is in place: its product with the x rows of the same columns, on top of the accumulator
+    template <class T> __device__ __forceinline__ bool stage_product(uint32_t tmem, int it) {
+        if (it >= 2) load_x(it);                                // the stage's buffers, x included, were free before it was built
+        if (!mbar_wait(&sh.x_full[it & 1], (it >> 1) & 1)) return false;
+        tc_fence_after();
+        const uint32_t idesc = instr_desc(AbFmt<T>::v, false, true, d.P);
+        const uint32_t sa = smem_u32(stages() + (it & 1) * kAStageBytes), sx = smem_u32(x_piece(it));
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+            umma(tmem, smem_desc(sa + kk * 32, 16, 1024), smem_desc(sx + kk * 16 * 128, 8192, 1024), idesc, 1u);
+        umma_commit(&sh.free_bar[it & 1]);
+        return true;
+    }
+};
 
 template <class T>
 __global__ void __launch_bounds__(kThreads, 2)
 chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmSf,
                const __grid_constant__ CUtensorMap tmSb, const __grid_constant__ CUtensorMap tmX, View x, View z,
                const float *D, const float *dt_out, const float *cs_f, const float *cs_b, const float *CB, MutView out,
-               MutView out_x, int rounds, int *status) {
+               MutView out_x, int *status) {
+    pdl_begin();
     extern __shared__ uint8_t dyn[];
     __shared__ ScanShared sh;
-    const int P = d.P, N = d.N, Q = d.Q;
-    const int nsr = N / 64 / rounds, npb = P / 64;            // slabs of 64 dstate columns resident at a time
+    const int P = d.P, Q = d.Q;
     uint8_t *base_sm = smem_align1024(dyn);
-    uint8_t *smC = base_sm;                                   // nsr slabs [128 x 64]
-    uint8_t *smSf = smC + nsr * 16384;                        // nsr slabs [P x 64]
-    uint8_t *smSb = smSf + nsr * P * 128;
-    uint8_t *smX = smSb + nsr * P * 128;                      // npb blocks [Q x 64]
-    float *f2 = reinterpret_cast<float *>(smX + npb * Q * 128), *b2 = f2 + Q, *tf = b2 + Q, *tb = tf + Q;
+    float *f2 = reinterpret_cast<float *>(base_sm + 2 * scan_slot_bytes(P)), *b2 = f2 + Q, *tf = b2 + Q, *tb = tf + Q;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int h = blockIdx.x % d.H, c = (blockIdx.x / d.H) % d.nc, b = blockIdx.x / (d.H * d.nc);
     const int g = h / d.R;
     const int lim = min(Q, d.L - c * Q);
     const int l0 = blockIdx.y * kTileM;
     const long long base = ((long long)(b * d.H + h) * d.nc + c) * Q;
-    const uint32_t ncols = tmem_cols(3 * P);
+    const uint32_t ncols = 2 * P;
+    ScanFeed feed{sh, d, base_sm, &tmC, &tmSf, &tmSb, &tmX, b, c, h, g, l0};
     if (warp == 0) tmem_alloc(&sh.tmem_base, ncols);
-    if (tid == 32) {
-        mbar_init(&sh.bar_cs, 1);
-        mbar_init(&sh.bar_x, 1);
-        mbar_init(&sh.bar_st, 1);
-        mbar_init(&sh.bar_mid, 1);
-        mbar_init(&sh.free_bar[0], 1);
-        mbar_init(&sh.free_bar[1], 1);
-        mbar_init(&sh.done_bar, 1);
-        sh.fail = 0;
-        fence_mbar_init();
+    if (tid == 32) {                                            // barriers and first loads by the same thread, before the sync
+        feed.init_barriers();
+        feed.start();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
-    const int tile = (b * d.nc + c) * d.H + h;
-    auto load_round = [&](int rd) {                             // thread 0: one dstate share of C and both states
-        mbar_expect_tx(&sh.bar_cs, (uint32_t)(nsr * 16384 + 2 * nsr * P * 128));
-        for (int j = 0; j < nsr; ++j) {
-            const int n0 = (rd * nsr + j) * 64;
-            tma_load4(smC + j * 16384, &tmC, n0, g, c * Q + l0, b, &sh.bar_cs);
-            tma_load2(smSf + j * P * 128, &tmSf, n0, tile * P, &sh.bar_cs);
-            tma_load2(smSb + j * P * 128, &tmSb, n0, tile * P, &sh.bar_cs);
-        }
-    };
-    if (tid == 0) {
-        load_round(0);
-        mbar_expect_tx(&sh.bar_x, (uint32_t)(npb * Q * 128));
-        for (int j = 0; j < npb; ++j) tma_load4(smX + j * Q * 128, &tmX, j * 64, h, c * Q, b, &sh.bar_x);
-    }
     const float *cbt = CB + ((long long)(b * d.nc + c) * d.G + g) * Q * Q;
     // the decay tables are built while the TMA loads are in flight
     for (int i = tid; i < Q; i += kThreads) {
@@ -150,37 +187,33 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
     load_raw(0);
     fetch(0);
     if (kStageK < Q) load_raw(kStageK);
-    bool ok = true;
-    if (tid == 0) {                                             // the two state products, straight from the TMA tiles
-        const uint32_t idesc = instr_desc(AbFmt<T>::v, false, false, P);
-        for (int rd = 0; rd < rounds; ++rd) {                   // bar_cs completes once per round, bar_st with the last one only
-            if (rd > 0) {                                       // the MMAs of the round before have read the tiles
-                if (!mbar_wait(&sh.bar_mid, (rd - 1) & 1)) {
-                    sh.fail = 1;
-                    break;
-                }
-                load_round(rd);
-            }
-            if (!mbar_wait(&sh.bar_cs, rd & 1)) {
-                sh.fail = 1;
-                break;
-            }
-            tc_fence_after();
-            for (int dir = 0; dir < 2; ++dir)
-                for (int j = 0; j < nsr; ++j)
+    const int l = l0 + (warp & 3) * 32 + lane;                  // this thread's row, in the sums and in the epilogue
+    const float ef = l < lim ? __expf(cs_f[base + l]) : 0.f, eb = l < lim ? __expf(cs_b[base + l]) : 0.f;
+    const uint32_t tl = tmem_lane_base(tmem);
+    if (tid == 0 && !feed.products<T>(tmem)) sh.fail = 1;
+    bool ok = mbar_wait(&sh.st_done, 0);
+    if (ok) {                                                   // the weighted sum of both products replaces the first
+        tc_fence_after();
+        for (int c0 = (warp >> 2) * 32; c0 < P; c0 += 64)
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        umma(tmem + dir * P, smem_desc(smem_u32(smC + j * 16384) + kk * 32, 16, 1024),
-                             smem_desc(smem_u32((dir ? smSb : smSf) + j * P * 128) + kk * 32, 16, 1024), idesc,
-                             (rd > 0 || j > 0 || kk > 0) ? 1u : 0u);
-            umma_commit(rd + 1 < rounds ? &sh.bar_mid : &sh.bar_st);
-        }
+            for (int q = 0; q < 32; q += 8) {
+                uint32_t vf[8], vb[8];
+                float y[8];
+                tmem_ld8_nowait(tl + c0 + q, vf);
+                tmem_ld8_nowait(tl + P + c0 + q, vb);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; ++j) y[j] = fmaf(eb, __uint_as_float(vb[j]), ef * __uint_as_float(vf[j]));
+                tmem_st8(tl + c0 + q, y);
+            }
+        tmem_st_wait();
+        tc_fence_before();
     }
     uint32_t it = 0;
     for (int s0 = 0; s0 < Q; s0 += kStageK, ++it) {
         const int st = it & 1;
-        uint8_t *stage = base_sm + st * kAStageBytes;           // reuses the C / state tiles
-        ok = (it < 2) ? mbar_wait(&sh.bar_st, 0) : mbar_wait(&sh.free_bar[st], ((it >> 1) - 1) & 1);
+        uint8_t *stage = feed.stages() + st * kAStageBytes;
+        if (it >= 2) ok = mbar_wait(&sh.free_bar[st], ((it >> 1) - 1) & 1);
         if (ok) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -195,33 +228,17 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
         ok = __syncthreads_and(ok) && !sh.fail;
         if (!ok) break;
         if (tid == 0) {
-            bool xok = (it > 0) || mbar_wait(&sh.bar_x, 0);
-            if (xok) {
-                tc_fence_after();
-                const uint32_t idesc = instr_desc(AbFmt<T>::v, false, true, P);
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                    umma(tmem + 2 * P, smem_desc(smem_u32(stage) + kk * 32, 16, 1024),
-                         smem_desc(smem_u32(smX) + (s0 + kk * 16) * 128, (uint32_t)Q * 128, 1024), idesc,
-                         (s0 > 0 || kk > 0) ? 1u : 0u);
-                umma_commit(&sh.free_bar[st]);
-            } else {
-                sh.fail = 1;
-            }
+            tc_fence_after();
+            if (!feed.stage_product<T>(tmem, it)) sh.fail = 1;
         }
     }
     // epilogue operands of the first strip are requested before waiting for the last MMAs
-    const int el = l0 + (warp & 3) * 32 + lane, ec0 = (warp >> 2) * 32;
+    const int ec0 = (warp >> 2) * 32;
     uint4 xr[4], zr[4];
-    float ecf = 0.f, ecb = 0.f;
-    if (ok && el < lim) {
-        ecf = cs_f[base + el];
-        ecb = cs_b[base + el];
-    }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        xr[q] = (ok && el < lim && d.has_D && ec0 < P) ? ld8v<T>(x, b, c * Q + el, h, ec0 + q * 8) : zero8();
-        zr[q] = (ok && el < lim && d.has_z && ec0 < P) ? ld8v<T>(z, b, c * Q + el, h, ec0 + q * 8) : zero8();
+        xr[q] = (ok && l < lim && d.has_D && ec0 < P) ? ld8v<T>(x, b, c * Q + l, h, ec0 + q * 8) : zero8();
+        zr[q] = (ok && l < lim && d.has_z && ec0 < P) ? ld8v<T>(z, b, c * Q + l, h, ec0 + q * 8) : zero8();
     }
     if (ok) {
         if (tid == 0) umma_commit(&sh.done_bar);
@@ -231,9 +248,6 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
     }
     if (!ok && tid == 0) atomicExch(status, kErrMmaTimeout);
     if (ok) {
-        const int l = l0 + (warp & 3) * 32 + lane;
-        const float ef = (l < lim) ? __expf(ecf) : 0.f, eb = (l < lim) ? __expf(ecb) : 0.f;
-        const uint32_t tl = tmem_lane_base(tmem);
         for (int c0 = (warp >> 2) * 32; c0 < P; c0 += 64) {
             // all global operands of this strip are requested before anything is consumed: one round trip, not eight
             if (c0 != ec0) {
@@ -243,14 +257,8 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
                     zr[q] = (l < lim && d.has_z) ? ld8v<T>(z, b, c * Q + l, h, c0 + q * 8) : zero8();
                 }
             }
-            float y[32], v[32];
-            tmem_ld32(tl + 2 * P + c0, y);
-            tmem_ld32(tl + c0, v);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) y[j] = fmaf(ef, v[j], y[j]);
-            tmem_ld32(tl + P + c0, v);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) y[j] = fmaf(eb, v[j], y[j]);
+            float y[32];
+            tmem_ld32(tl + c0, y);
             if (l < lim) {
 #pragma unroll
                 for (int j = 0; j < 32; j += 8) {
