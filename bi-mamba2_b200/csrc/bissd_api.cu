@@ -605,7 +605,7 @@ do {                                                                            
                         d, mC, mSf, mSb, mG128, ks, a.cs_f, a.cs_b, F(w.pf), F(w.pb), status));
                 } else {
                     BISSD_ALLOW(tc::prev_terms_tma<T>, smem_p);
-                    BISSD_LAUNCH("tc_prev_terms_tma", tc::prev_terms_tma<T><<<dim3(bch, nlt_tc), tc::kThreads, smem_p, s>>>(
+                    BISSD_LAUNCH("tc_prev_terms_tma", launch_pdl(tc::prev_terms_tma<T>, dim3(bch, nlt_tc), tc::kThreads, smem_p, s,
                         d, mC, mSf, mSb, gv, a.cs_f, a.cs_b, F(w.pf), F(w.pb), status));
                 }
                 BISSD_ALLOW(tc::dbc_accum_tma<T>, smem_a);
@@ -617,7 +617,7 @@ do {                                                                            
                         part_heads = d.G * dbc_slots(d, w.dbc_ks);
                     }
                 } else
-                BISSD_LAUNCH("tc_dbc_accum_tma", tc::dbc_accum_tma<T><<<dim3(d.b * d.nc * d.G * w.nsplit, nlt_tc, 2), tc::kThreads, smem_a, s>>>(
+                BISSD_LAUNCH("tc_dbc_accum_tma", launch_pdl(tc::dbc_accum_tma<T>, dim3(d.b * d.nc * d.G * w.nsplit, nlt_tc, 2), tc::kDbcTmaThreads, smem_a, s,
                     d, mEf, mEb, mSf, mSb, mX128, mG128, a.dt_out, a.cs_f, a.cs_b, F(w.dB_part), F(w.dC_part), status));
                 dbc_done = true;
                 nsplit = 1;                                      // nf/nb/pf/pb now hold complete row sums

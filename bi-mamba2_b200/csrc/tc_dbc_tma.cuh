@@ -14,9 +14,11 @@
 namespace bissd {
 namespace tc {
 
+constexpr int kDbcTmaThreads = kThreads + 64;
 struct DbcShared {
-    uint64_t full[3], free_bar[3], done_bar;
+    uint64_t full[3], scaled[3], free_bar[3], wbar, done_bar;
     uint32_t tmem_base;
+    int fail;
 };
 
 inline size_t dbc_tma_smem(int P, int nt) {
@@ -25,15 +27,17 @@ inline size_t dbc_tma_smem(int P, int nt) {
 
 // grid (b*nc*G*nsplit, Q/128, 2); blockIdx.z: 0 = dB (left = x, right operand = E16), 1 = dC (left = g, right = states).
 // part layout [b, nc*Q, G, N] fp32.  tmL: x or g, box [64 x 128 rows].
-// Both operands of every (head, direction) stage arrive by TMA into a three-deep ring; the threads only scale the
-// 128 rows of the left tile in place (packed multiply for bf16) before thread 0 issues the stage's MMAs.  The row
-// factors of head h+1 are loaded while head h is being worked on.
+// Both operands of every (head, direction) stage arrive by TMA into a three-deep ring, requested by lane 0 of warp 9; warps
+// 0-7 scale the 128 rows of the left tile in place, lane 0 of warp 8 issues the stage's MMAs.  (One thread doing loads, MMAs
+// and its share of the scaling, a CTA barrier per stage, the kernel took 113 us at b8 L1024 H16 P128 G2 N256
+// chunk 128.)  The row factors of head h+1 are loaded while head h is being worked on.  Bounded waits, ids 81-85 in the status word.
 template <class T>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kDbcTmaThreads, 1)
 dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_constant__ CUtensorMap tmEb,
               const __grid_constant__ CUtensorMap tmSf, const __grid_constant__ CUtensorMap tmSb,
               const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG, const float *dt_out,
               const float *cs_f, const float *cs_b, float *dB_part, float *dC_part, int *status) {
+    pdl_begin();
     extern __shared__ uint8_t dyn[];
     __shared__ DbcShared sh;
     const int P = d.P, N = d.N, Q = d.Q, R = d.R;
@@ -51,7 +55,8 @@ dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
     const int l0 = blockIdx.y * kTileM, n0 = split * 128;
     const int total = 2 * R;
     const uint32_t ncols = tmem_cols(nt);
-    auto load_stage = [&](int it) {                             // thread 0: both operands of stage it = (head, dir)
+    volatile int *fail = &sh.fail;
+    auto load_stage = [&](int it) {                             // both operands of stage it = (head, dir)
         const int hr = it >> 1, dir = it & 1, slot = it % 3;
         const int h = grp * R + hr;
         const int tile = (b * d.nc + c) * d.H + h;
@@ -62,16 +67,17 @@ dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
         for (int j = 0; j < nnb; ++j) tma_load2(sb + j * P * 128, m, n0 + j * 64, tile * P, &sh.full[slot]);
     };
     if (warp == 0) tmem_alloc(&sh.tmem_base, ncols);
-    if (tid == 0) {                                             // barriers and the first loads by the same thread
+    if (tid == kThreads + 32) {                                 // the loading thread: barriers and the first loads
         for (int i = 0; i < 3; ++i) {
             mbar_init(&sh.full[i], 1);
+            mbar_init(&sh.scaled[i], 8);
             mbar_init(&sh.free_bar[i], 1);
         }
+        mbar_init(&sh.wbar, 8);
         mbar_init(&sh.done_bar, 1);
+        sh.fail = 0;
         fence_mbar_init();
-        load_stage(0);
-        if (total > 1) load_stage(1);
-        if (total > 2) load_stage(2);
+        for (int it = 0; it < 3 && it < total; ++it) load_stage(it);
     }
     // one (dir, row) per thread: the inputs of the row factor of head hr, then the factor itself
     const int sdir = tid >> 7, srow = tid & 127, sl = l0 + srow;
@@ -92,83 +98,96 @@ dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
         if (sl < lim) v = which ? __expf(pcs) : pdt * __expf(pT - pcs);
         sc[((hr & 1) * 2 + sdir) * 128 + srow] = v;
     };
-    fetch_scale(0);
-    write_scale(0);
-    if (R > 1) fetch_scale(1);
+    if (warp < 8) {
+        fetch_scale(0);
+        write_scale(0);
+        if (R > 1) fetch_scale(1);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
-    bool ok = true;
-#pragma unroll 1
-    for (int it = 0; it < total; ++it) {
-        const int slot = it % 3, hr = it >> 1, dir = it & 1;
-        uint8_t *sa = base_sm + slot * slot_bytes;
-        ok = mbar_wait(&sh.full[slot], (it / 3) & 1);
-        if (ok) {                                               // scale row r of the left tile by its factor, in place
-            const float *sf_ = sc + ((hr & 1) * 2 + dir) * 128;
-            for (int q = tid; q < npb * 1024; q += kThreads) {
-                uint4 *ptr = reinterpret_cast<uint4 *>(sa) + q;
-                *ptr = scale8_packed<T>(*ptr, sf_[(q >> 3) & 127]);
+    if (warp == 8) {
+        if (lane == 0) {
+            const uint32_t idesc = instr_desc(AbFmt<T>::v, false, true, nt);
+            int slot = 0, phase = 0;
+            for (int it = 0; it < total; ++it) {
+                if (!ws_wait(&sh.scaled[slot], phase, fail, 82)) break;
+                tc_fence_after();
+                const uint32_t sa = smem_u32(base_sm + slot * slot_bytes), sb = sa + a_bytes;
+                for (int j = 0; j < npb; ++j)
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        umma(tmem, smem_desc(sa + j * 16384 + kk * 32, 16, 1024), smem_desc(sb + (j * 64 + kk * 16) * 128, (uint32_t)P * 128, 1024),
+                             idesc, (it > 0 || j > 0 || kk > 0) ? 1u : 0u);
+                umma_commit(it + 1 < total ? &sh.free_bar[slot] : &sh.done_bar);
+                if (++slot == 3) { slot = 0; phase ^= 1; }
             }
+        }
+    } else if (warp == 9) {
+        if (lane == 0) {
+            int slot = 0, phase = 0;
+            for (int it = 3; it < total; ++it) {
+                if (!ws_wait(&sh.free_bar[slot], phase, fail, 81)) break;
+                load_stage(it);
+                if (++slot == 3) { slot = 0; phase ^= 1; }
+            }
+        }
+    } else {
+        bool ok = true;
+        int slot = 0, phase = 0;
+#pragma unroll 1
+        for (int it = 0; it < total && ok; ++it) {
+            const int hr = it >> 1, dir = it & 1;
+            ok = ws_wait_warp(&sh.full[slot], phase, fail, 83);
+            if (!ok) break;
+            uint4 *sa = reinterpret_cast<uint4 *>(base_sm + slot * slot_bytes);   // the left tile's rows times their factors, in place
+            const float *sf_ = sc + ((hr & 1) * 2 + dir) * 128;
+#pragma unroll 4
+            for (int q = tid; q < npb * 1024; q += kThreads) sa[q] = scale8_packed<T>(sa[q], sf_[(q >> 3) & 127]);
             fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.scaled[slot]);
             if (dir == 1 && hr + 1 < R) {                       // next head's factors; then the loads for the one after
                 write_scale(hr + 1);
                 if (hr + 2 < R) fetch_scale(hr + 2);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sh.wbar);
+                ok = ws_wait_warp(&sh.wbar, hr & 1, fail, 84);  // every warp is done with head hr and has written the next factors
             }
+            if (++slot == 3) { slot = 0; phase ^= 1; }
         }
-        ok = __syncthreads_and(ok);
-        if (!ok) break;
-        if (tid == 0) {
+        if (ok) ok = ws_wait_warp(&sh.done_bar, 0, fail, 85);
+        if (ok) {
             tc_fence_after();
-            const uint32_t idesc = instr_desc(AbFmt<T>::v, false, true, nt);
-            const uint8_t *sb = sa + a_bytes;
-            for (int j = 0; j < npb; ++j)
+            const int l = l0 + (warp & 3) * 32 + lane;
+            float *part = (which ? dC_part : dB_part) + (((long long)b * d.nc * Q + c * Q + l) * d.G + grp) * N + n0;
+            for (int c0 = (warp >> 2) * 32; c0 < nt; c0 += 64) {
+                float v[32];
+                tmem_ld32(tmem_lane_base(tmem) + c0, v);
+                if (l < lim) {
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                    umma(tmem, smem_desc(smem_u32(sa + j * 16384) + kk * 32, 16, 1024),
-                         smem_desc(smem_u32(sb) + (j * 64 + kk * 16) * 128, (uint32_t)P * 128, 1024), idesc,
-                         (it > 0 || j > 0 || kk > 0) ? 1u : 0u);
-            umma_commit(&sh.free_bar[slot]);
-            if (it >= 1 && it + 2 < total) {                    // refill the slot stage it-1 used, once its MMAs are done
-                ok = mbar_wait(&sh.free_bar[(it + 2) % 3], ((it - 1) / 3) & 1);
-                if (ok) load_stage(it + 2);
-            }
-        }
-    }
-    // a failure seen only by thread 0 in the last iteration is caught here
-    if (ok) {
-        if (tid == 0) umma_commit(&sh.done_bar);
-        ok = mbar_wait(&sh.done_bar, 0);
-    }
-    ok = __syncthreads_and(ok);
-    tc_fence_after();
-    if (!ok && tid == 0) atomicExch(status, kErrMmaTimeout);
-    if (ok) {
-        const int l = l0 + (warp & 3) * 32 + lane;
-        float *part = (which ? dC_part : dB_part) + (((long long)b * d.nc * Q + c * Q + l) * d.G + grp) * N + n0;
-        for (int c0 = (warp >> 2) * 32; c0 < nt; c0 += 64) {
-            float v[32];
-            tmem_ld32(tmem_lane_base(tmem) + c0, v);
-            if (l < lim) {
-#pragma unroll
-                for (int j = 0; j < 32; j += 4)
-                    *reinterpret_cast<float4 *>(part + c0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                    for (int j = 0; j < 32; j += 4)
+                        *reinterpret_cast<float4 *>(part + c0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                }
             }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, ncols);
+    if (sh.fail && tid == 0) atomicExch(status, kErrWsWait + sh.fail);
+    if (warp == 0) {
+        __syncwarp();
+        tmem_dealloc(tmem, ncols);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------------------
 // The same sums with one CTA per (batch, chunk, group, 128 state columns) that walks the heads of its group: the CTA
 // owns all Q rows (one 128-column accumulator per 128-row block), so the state tiles E_f / E_b (or S_f / S_b) of a head
-// are fetched once instead of once per row block, and the x / g tile once.  Roles as in state_gemm_grp: warps 0-7
-// turn the left tile as it landed into its two row-scaled copies (one buffer: the copies of head i + 1 are written
-// once the MMAs of head i are done), lane 0 of warp 8 issues every TMA load and every MMA; two stages of (left
-// tile + 2 right tiles).  The heads accumulate in tensor memory, two parts of them (head_parts) side by side; a pair of
+// are fetched once instead of once per row block, and the x / g tile once.  Warps 0-7 turn the left tile as it landed into
+// its two row-scaled copies - the backward one in place, the forward one beside the ring - lane 0 of warp 8 issues the
+// MMAs, lane 0 of warp 9 the loads; two stages of (left tile + 2 right tiles).  The heads accumulate in tensor memory, two parts of them (head_parts) side by side; a pair of
 // parts is read out together.  With few blocks the parts are dealt to ks of them (dbc_ksplit).  Bounded waits, ids 51-58
 // in the status word.
 // grid (b*nc*G*ks*nsplit, 1, 2); blockIdx.z: 0 = dB, 1 = dC.  part layout [b, nc*Q, G, slots, N] fp32: a slot per pair of
@@ -180,7 +199,7 @@ dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
 // partial results (268 MB at b2 L8192 G8 N128) and a launch; taken where the heads are one part (head_parts), so that
 // the order of additions does not depend on the batch.
 struct DbcGrpShared {
-    uint64_t full[2], scaled, done[2], wbar, last_in, last_done;
+    uint64_t full[2], scaled[2], done[2], wbar, last_in, last_done;
     uint32_t tmem_base;
     int fail;
 };
@@ -188,7 +207,7 @@ inline bool dbc_grp_ok(int P, int N, int Q) { return P == 64 && (N == 64 || N % 
 inline size_t dbc_grp_smem(int Q, int nt) {
     return 1024 + 2 * ((size_t)Q * 128 + 2 * (size_t)(nt / 64) * 64 * 128) + 2 * (size_t)Q * 128 + 2 * 2 * (size_t)Q * 4;
 }
-constexpr int kDbcGrpThreads = kThreads + 32;
+constexpr int kDbcGrpThreads = kThreads + 64;
 struct LastMaps {                                               // operands and results of the product with dCB
     CUtensorMap Dm, Dk, B, C;
     MutView dB, dC;
@@ -208,7 +227,7 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
     const int nsplit = (N + 127) / 128, nt = min(N, 128), nnb = nt / 64, nrb = Q / 128;
     const int left_bytes = Q * 128, right_bytes = 2 * nnb * P * 128, stage_bytes = left_bytes + right_bytes;
     uint8_t *base_sm = smem_align1024(dyn);                     // per stage: left [Q rows x 128 B], right [dir][nnb][P x 128 B]
-    uint8_t *smScaled = base_sm + 2 * stage_bytes;              // [dir][Q rows x 128 B]
+    uint8_t *smScaled = base_sm + 2 * stage_bytes;              // [2 stages][Q rows x 128 B]: the forward copy; the backward one replaces the left tile
     float *sc = reinterpret_cast<float *>(smScaled + 2 * left_bytes);   // [2 bufs][2 dirs][Q]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int split = blockIdx.x % nsplit, part_id = blockIdx.x / nsplit % ks, bx = blockIdx.x / nsplit / ks;
@@ -234,10 +253,10 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
         }
     };
     if (warp == 0) tmem_alloc(&sh.tmem_base, ncols);
-    if (tid == kThreads) {                                      // the controller: barriers and the first loads
+    if (tid == kThreads + 32) {                                 // the loading thread: barriers and the first loads
         mbar_init(&sh.wbar, 8);
-        mbar_init(&sh.scaled, 8);
         for (int i = 0; i < 2; ++i) {
+            mbar_init(&sh.scaled[i], 8);
             mbar_init(&sh.full[i], 1);
             mbar_init(&sh.done[i], 1);
         }
@@ -292,19 +311,15 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
                     ++p;
                     start = i;
                 }
-                if (i >= 1 && i + 1 < R) {                      // stage (i + 1) & 1 is free once the MMAs of head i - 1 are done
-                    ok = ws_wait(&sh.done[(i - 1) & 1], ((i - 1) >> 1) & 1, fail, 51);
-                    if (ok) load_head(i + 1);
-                }
-                ok = ok && ws_wait(&sh.scaled, i & 1, fail, 52);
+                ok = ws_wait(&sh.scaled[i & 1], (i >> 1) & 1, fail, 52);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t sl = smem_u32(smScaled), sr = smem_u32(base_sm + (i & 1) * stage_bytes) + left_bytes;
+                const uint32_t sb = smem_u32(base_sm + (i & 1) * stage_bytes), sf = smem_u32(smScaled + (i & 1) * left_bytes), sr = sb + left_bytes;
                 for (int rb = 0; rb < nrb; ++rb)
                     for (int dir = 0; dir < 2; ++dir)
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk)
-                            umma(tmem + (p & 1) * acc_cols + rb * nt, smem_desc(sl + (dir * nrb + rb) * 16384 + kk * 32, 16, 1024),
+                            umma(tmem + (p & 1) * acc_cols + rb * nt, smem_desc((dir ? sb : sf) + rb * 16384 + kk * 32, 16, 1024),
                                  smem_desc(sr + dir * nnb * P * 128 + kk * 16 * 128, (uint32_t)P * 128, 1024), idesc,
                                  (i > start || dir > 0 || kk > 0) ? 1u : 0u);
                 umma_commit(&sh.done[i & 1]);
@@ -338,6 +353,9 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
                 }
             }
         }
+    } else if (warp == 9) {                                     // the ring's loads: stage i & 1 is free once the MMAs of head i - 2 are done
+        if (lane == 0)
+            for (int i = 2; i < R && ws_wait(&sh.done[i & 1], ((i >> 1) - 1) & 1, fail, 51); ++i) load_head(i);
     } else {
         // the sum of local parts 2 pair and 2 pair + 1 (`two`) as this block's next partial result
         auto write_out = [&](int pair, bool two) {
@@ -370,19 +388,21 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
         for (int i = 0; i < R && ok; ++i) {
             uint8_t *sl = base_sm + (i & 1) * stage_bytes;
             ok = ws_wait_warp(&sh.full[i & 1], (i >> 1) & 1, fail, 53);
-            // the scaled copies of head i - 1 have been read by its MMAs
-            if (ok && i >= 1) ok = ws_wait_warp(&sh.done[(i - 1) & 1], ((i - 1) >> 1) & 1, fail, 56);
             if (!ok) break;
-            if (nparts > 2 && i == part_end(2 * pair + 1)) write_out(pair++, true);   // both accumulators are complete: out, before the next part starts
+            if (nparts > 2 && i == part_end(2 * pair + 1)) {    // both accumulators are complete: out, before the next part starts
+                ok = ws_wait_warp(&sh.done[(i - 1) & 1], ((i - 1) >> 1) & 1, fail, 56);
+                if (!ok) break;
+                write_out(pair++, true);
+            }
             const float *wf = sc + ((i & 1) * 2) * Q, *wb = wf + Q;
             for (int q = tid; q < Q * 8; q += kThreads) {
                 const uint4 raw = reinterpret_cast<const uint4 *>(sl)[q];
-                reinterpret_cast<uint4 *>(smScaled)[q] = scale8_packed<T>(raw, wf[q >> 3]);
-                reinterpret_cast<uint4 *>(smScaled + left_bytes)[q] = scale8_packed<T>(raw, wb[q >> 3]);
+                reinterpret_cast<uint4 *>(smScaled + (i & 1) * left_bytes)[q] = scale8_packed<T>(raw, wf[q >> 3]);
+                reinterpret_cast<uint4 *>(sl)[q] = scale8_packed<T>(raw, wb[q >> 3]);
             }
             fence_async_smem();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sh.scaled);
+            if (lane == 0) mbar_arrive(&sh.scaled[i & 1]);
             if (i + 1 < R) {
                 write_scale(i + 1);
                 if (i + 2 < R) fetch_scale(i + 2);
@@ -435,6 +455,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 prev_terms_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmSf,
                const __grid_constant__ CUtensorMap tmSb, View g, const float *cs_f, const float *cs_b, float *pf, float *pb,
                int *status) {
+    pdl_begin();
     extern __shared__ uint8_t dyn[];
     __shared__ uint64_t bar_in, bar_done;
     __shared__ uint32_t tmem_slot;
@@ -548,7 +569,7 @@ inline bool prev_grp_ok(int P, int N, int Q, int R) { return P == 64 && (N == 64
 inline size_t prev_grp_smem(int N, int Q) {
     return 1024 + (size_t)(Q / 128) * (N / 64) * 16384 + 2 * 2 * (size_t)(N / 64) * 8192 + 2 * (size_t)(Q / 128) * 16384;
 }
-constexpr int kPrevGrpThreads = kThreads + 32;
+constexpr int kPrevGrpThreads = kThreads + 64;
 
 template <class T>
 __global__ void __launch_bounds__(kPrevGrpThreads, 1)
@@ -587,7 +608,7 @@ prev_terms_grp(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
     };
     const uint32_t ncols = 2 * nrb * 128;                       // two accumulator sets of nrb x 128 columns
     if (warp == 0) tmem_alloc(&sh.tmem_base, ncols);
-    if (tid == kThreads) {                                      // the controller: barriers and the first loads
+    if (tid == kThreads + 32) {                                 // the loading thread: barriers and the first loads
         mbar_init(&sh.bar_c, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&sh.full_s[i], 1);
@@ -630,14 +651,16 @@ prev_terms_grp(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
                             umma(tmem + ((i & 1) * nrb + rb) * 128, smem_desc(smem_u32(smC + (rb * nsl + j) * 16384) + kk * 32, 16, 1024),
                                  smem_desc(ss + j * 16384 + kk * 32, 16, 1024), idesc, (j > 0 || kk > 0) ? 1u : 0u);
                 umma_commit(&sh.done[i & 1]);
-                if (i >= 1 && i + 1 < nh) {                     // the rings of head i - 1 are refilled as they drain
-                    ok = ws_wait(&sh.done[(i - 1) & 1], ((i - 1) >> 1) & 1, fail, 64);
-                    if (ok) load_s(i + 1);
-                    ok = ok && ws_wait(&sh.gfree[(i - 1) & 1], ((i - 1) >> 1) & 1, fail, 65);
-                    if (ok) load_g(i + 1);
-                }
             }
         }
+    } else if (warp == 9) {                                     // the rings of head i - 2 are refilled as they drain
+        if (lane == 0)
+            for (int i = 2; i < nh; ++i) {
+                if (!ws_wait(&sh.done[i & 1], ((i >> 1) - 1) & 1, fail, 64)) break;
+                load_s(i);
+                if (!ws_wait(&sh.gfree[i & 1], ((i >> 1) - 1) & 1, fail, 65)) break;
+                load_g(i);
+            }
     } else {
         const int quad = warp & 3, dir = warp >> 2;             // rows quad * 32 + lane of every row block, one direction
         const float *cs = dir ? cs_b : cs_f;
