@@ -279,7 +279,12 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
                 const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, false);
                 BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
                 BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
-                    d, mCc, mBc, mCBo, mCBo, true, false, nullptr, status));
+                    d, mCc, mBc, mCBo, mCBo, true, false, nullptr, nullptr, nullptr, status));
+            } else if (!ws_path && !no_tma() && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc)) {
+                const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, false, true);
+                BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
+                BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
+                    d, mCc, mBc, mCc, mCc, false, false, nullptr, CB, nullptr, status));
             } else
             BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_cb, s>>>(
                 d, Cm, Bm, ws_path ? nullptr : CB, nullptr, ws_path ? CB16 : nullptr, nullptr, nullptr, status));
@@ -475,7 +480,12 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
             const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, true);
             BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
             BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
-                d, mCc, mBc, mCBo, mCBto, fused_cb, true, fused_cb ? nullptr : F(w.cbs), status));
+                d, mCc, mBc, mCBo, mCBto, fused_cb, true, fused_cb ? nullptr : F(w.cbs), nullptr, nullptr, status));
+        } else if (!ws_path && sums_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc)) {
+            const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, true, true);
+            BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
+            BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
+                d, mCc, mBc, mCc, mCc, false, false, F(w.cbs), F(w.cb), F(w.cbt), status));
         } else
         BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
             d, Cm, Bm, (sums_path && ws_path) ? nullptr : F(w.cb), ws_path ? nullptr : F(w.cbt), nullptr,

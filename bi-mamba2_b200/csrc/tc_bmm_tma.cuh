@@ -4,7 +4,8 @@
 // each optional: the bf16 tile (tmO), its transpose (tmOt), CBs (fp32 in strips of 16 columns, [Q/16][Q rows][16]).
 // The 16-bit tiles leave by TMA from shared memory, over C and B, which are dead by then: as per-lane row pieces, 32
 // different lines per store instruction, they were most of this kernel's time (b2 L8192 G8: 51 us a launch; bound by
-// the 67 or 134 MB it writes).  Rows past the end of the sequence read as zeros.
+// the 67 or 134 MB it writes).  CB and its transpose in fp32, which the headdim 128 kernels read, are likewise turned in shared
+// memory into whole rows per warp.  Rows past the end of the sequence read as zeros.
 // grid (b*nc*G, Q/128, Q/128).
 #pragma once
 #include "tc_scan_tma.cuh"
@@ -13,8 +14,9 @@ namespace bissd {
 namespace tc {
 
 inline bool bmm_cb_tma_ok(int N, int Q) { return N % 64 == 0 && N <= 256 && (Q == 128 || Q == 256); }
-inline size_t bmm_cb_tma_smem(int N, bool transposed) {         // C and B, then the tile and its transpose
-    const size_t in = 2 * (size_t)(N / 64) * 16384, out = transposed ? 65536 : 32768;
+constexpr int kCbRow = 132;                                      // floats a row of the fp32 tile takes in shared memory: no bank conflicts
+inline size_t bmm_cb_tma_smem(int N, bool transposed, bool fp32 = false) {   // C and B, then the tile and its transpose, or an fp32 tile
+    const size_t in = 2 * (size_t)(N / 64) * 16384, out = fp32 ? 128 * kCbRow * 4 : (transposed ? 65536 : 32768);
     return 1024 + (in > out ? in : out);
 }
 
@@ -22,7 +24,7 @@ template <class T>
 __global__ void __launch_bounds__(kThreads)
 bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmB,
            const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmOt, bool plain, bool transposed, float *CBs,
-           int *status) {
+           float *CB32, float *CBt32, int *status) {
     pdl_begin();
     extern __shared__ uint8_t dyn[];
     __shared__ uint64_t bar_in, bar_done;
@@ -32,7 +34,8 @@ bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constan
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = blockIdx.x % d.G, c = (blockIdx.x / d.G) % d.nc, b = blockIdx.x / (d.G * d.nc);
     const int l0 = blockIdx.y * kTileM, s0 = blockIdx.z * 128;
-    const uint32_t ncols = transposed ? 256 : 128;
+    const bool two = transposed || CBt32;                       // the transpose is wanted
+    const uint32_t ncols = two ? 256 : 128;
     if (warp == 0) tmem_alloc(&tmem_slot, ncols);
     if (tid == 32) {                                            // barriers and loads by the same thread, before the sync
         mbar_init(&bar_in, 1);
@@ -54,7 +57,7 @@ bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constan
         if (ok) {
             tc_fence_after();
             const uint32_t idesc = instr_desc(AbFmt<T>::v, false, false, 128);
-            for (int t = 0; t < (transposed ? 2 : 1); ++t)
+            for (int t = 0; t < (two ? 2 : 1); ++t)
                 for (int j = 0; j < nsl; ++j)
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk) {
@@ -81,6 +84,23 @@ bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constan
                 *reinterpret_cast<uint4 *>(slab + r * 128 + ((((hc + j) >> 3) ^ (r & 7)) << 4)) = pack8<__nv_bfloat16>(o);
             }
         };
+        auto rows_out = [&](int t, float *out) {                // accumulator t, to out[rows of Q floats]
+            float *buf = reinterpret_cast<float *>(smC);
+#pragma unroll
+            for (int hc = 0; hc < 64; hc += 32) {
+                float v[32];
+                tmem_ld32(tl + t * 128 + hc, v);
+#pragma unroll
+                for (int j = 0; j < 32; j += 4)
+                    *reinterpret_cast<float4 *>(buf + r * kCbRow + c0 + hc + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            }
+            __syncthreads();
+            for (int i = warp; i < 128; i += kThreads / 32)
+                *reinterpret_cast<float4 *>(out + (long long)i * Q + lane * 4) = *reinterpret_cast<const float4 *>(buf + i * kCbRow + lane * 4);
+            __syncthreads();
+        };
+        if (CB32) rows_out(0, CB32 + tile + (long long)l0 * Q + s0);
+        if (CBt32) rows_out(1, CBt32 + tile + (long long)s0 * Q + l0);
         uint8_t *so = smC, *st = smC + 32768;                   // [2 slabs of 128 x 64]
         if (plain || CBs) {
 #pragma unroll
@@ -107,7 +127,7 @@ bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constan
         }
         fence_async_smem();
         __syncthreads();
-        if (tid == 0) {
+        if (tid == 0 && (plain || transposed)) {
             const int row = ((b * d.nc + c) * d.G + g) * Q;
             for (int k = 0; k < 2; ++k) {
                 if (plain) tma_store2(&tmO, so + k * 16384, s0 + k * 64, row + l0);

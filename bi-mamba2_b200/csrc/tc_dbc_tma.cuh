@@ -43,16 +43,16 @@ dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
     const int P = d.P, N = d.N, Q = d.Q, R = d.R;
     const int npb = P / 64;
     const int nsplit = (N + 127) / 128;
-    const int nt = min(N, 128), nnb = nt / 64;
+    const int split = blockIdx.x % nsplit, bx = blockIdx.x / nsplit, n0 = split * 128;
+    const int nt = min(N - n0, 128), nnb = nt / 64;             // dstate 192: the second split has 64 columns
     const int a_bytes = npb * 16384, b_bytes = nnb * P * 128, slot_bytes = a_bytes + b_bytes;
     uint8_t *base_sm = smem_align1024(dyn);
     float *sc = reinterpret_cast<float *>(base_sm + 3 * slot_bytes);               // [2 bufs][2 dirs][128 rows]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int split = blockIdx.x % nsplit, bx = blockIdx.x / nsplit;
     const int grp = bx % d.G, c = (bx / d.G) % d.nc, b = bx / (d.G * d.nc);
     const int which = blockIdx.z;
     const int lim = min(Q, d.L - c * Q);
-    const int l0 = blockIdx.y * kTileM, n0 = split * 128;
+    const int l0 = blockIdx.y * kTileM;
     const int total = 2 * R;
     const uint32_t ncols = tmem_cols(nt);
     volatile int *fail = &sh.fail;
