@@ -221,7 +221,7 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
     if (a.phases & BISSD_PHASE_LOCAL) {
         int rc = note_cuda(cudaMemsetAsync(ws, 0, kWsHeader, s), "cudaMemsetAsync");
         if (rc != BISSD_OK) return rc;
-        BISSD_LAUNCH("cumsum_fwd", launch_pdl(d.Q <= 128 ? tc::cumsum_fwd<4> : tc::cumsum_fwd<8>, tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s,
+        BISSD_LAUNCH("cumsum_fwd", launch_pdl(tc::cumsum_share(d) == 1 ? (d.Q <= 128 ? tc::cumsum_fwd<4, 1> : tc::cumsum_fwd<8, 1>) : (d.Q <= 128 ? tc::cumsum_fwd<1, 4> : tc::cumsum_fwd<2, 4>), tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s,
             d, a.dt.ptr, a.p.dt_dtype, a.dt.stride_batch, a.dt.stride_seq, a.dt.stride_head, a.A, a.dt_bias, a.dt_out,
             a.cs_f, a.cs_b, all_aligned16(a.dt_out, a.cs_f, a.cs_b)));
         if (!walk.use) {
@@ -779,7 +779,7 @@ do {                                                                            
     if (use_u4) { cs.u4 = F(w.u4); cs.u4_tiles = u4_tiles; }
     else { cs.da_f = F(w.da_f); cs.da_b = F(w.da_b); }
     cs.dTpart = F(w.dTpart); cs.nblk = walk.use ? tc::walk_slots(d) : pass_slots(d); cs.nsplit = nsplit; cs.ddt = gr.ddt; cs.dApart = F(w.dApart); cs.dbiaspart = F(w.dbiaspart);
-    BISSD_LAUNCH("cumsum_bwd", launch_pdl(d.Q <= 128 ? tc::cumsum_bwd<4> : tc::cumsum_bwd<8>, tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s,
+    BISSD_LAUNCH("cumsum_bwd", launch_pdl(tc::cumsum_share(d) == 1 ? (d.Q <= 128 ? tc::cumsum_bwd<4, 1> : tc::cumsum_bwd<8, 1>) : (d.Q <= 128 ? tc::cumsum_bwd<1, 4> : tc::cumsum_bwd<2, 4>), tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s,
         d, cs, all_aligned16(a.dt_out, a.dt_out, a.dt_out)));
     BISSD_LAUNCH("final_reduce", launch_pdl(simt::final_reduce<1024>, d.H, 1024, 0, s, 
         d, F(w.dApart), F(w.dbiaspart), d.has_D ? F(w.dDpart) : nullptr, dd_slots ? dd_slots : nlt, dd_compact ? 1 : 0, a.dA, d.has_bias ? a.ddt_bias : nullptr,

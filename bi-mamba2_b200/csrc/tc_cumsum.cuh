@@ -1,7 +1,9 @@
 // Discretisation + both cumulative sums of the tensor-core family, and their backward (formulas at simt::chunk_cumsum and
-// simt::cumsum_bwd_role).  A warp has one (batch, chunk, head), a lane E consecutive positions: every operand is requested
-// at once in 16-byte pieces, the scans are register sums and five shuffles, and nothing waits for a barrier.  The block's
-// eight warps have eight neighbouring heads, whose dt and ddt values share 32-byte sectors.  One block per (batch, chunk,
+// simt::cumsum_bwd_role).  A lane has E consecutive positions, W warps one (batch, chunk, head): every operand is requested at
+// once in wide pieces, the scans are register sums and five shuffles.  Where a row of the batch brings many chunks W is 1 and
+// nothing waits for a barrier; where it does not, the length of a lane's work is the length of the kernel, and four warps share a
+// chunk (W = 1 cost the smallest forward call 1.6 of 20 us).  The block's heads are neighbours, whose dt and ddt values share
+// 32-byte sectors.  One block per (batch, chunk,
 // head) left these kernels waiting for launches and barriers: at b16 L4096 H32 chunk 256 / 128 backward 88 / 151 us,
 // forward 23 / 33 us.
 #pragma once
@@ -11,12 +13,13 @@ namespace bissd {
 namespace tc {
 
 constexpr int kCumsumWarps = 8;
-inline int cumsum_blocks(const Dims &d) { return d.b * d.nc * ceil_div(d.H, kCumsumWarps); }
+inline int cumsum_share(const Dims &d) { return d.nc * d.H < 256 ? 4 : 1; }   // W: by one row of the batch, so that a row's bits do not depend on the others
+inline int cumsum_blocks(const Dims &d) { return d.b * d.nc * ceil_div(d.H, kCumsumWarps / cumsum_share(d)); }
 
 template <int E> __device__ __forceinline__ void load_e(const float *p, bool wide, float (&v)[E]) {
-    if (wide) {
+    if (E % 4 == 0 && wide) {
 #pragma unroll
-        for (int j = 0; j < E; j += 4) {
+        for (int j = 0; j + 3 < E; j += 4) {
             const float4 t = *reinterpret_cast<const float4 *>(p + j);
             v[j] = t.x; v[j + 1] = t.y; v[j + 2] = t.z; v[j + 3] = t.w;
         }
@@ -26,9 +29,9 @@ template <int E> __device__ __forceinline__ void load_e(const float *p, bool wid
     }
 }
 template <int E> __device__ __forceinline__ void store_e(float *p, bool wide, const float (&v)[E]) {
-    if (wide) {
+    if (E % 4 == 0 && wide) {
 #pragma unroll
-        for (int j = 0; j < E; j += 4) *reinterpret_cast<float4 *>(p + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        for (int j = 0; j + 3 < E; j += 4) *reinterpret_cast<float4 *>(p + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
     } else {
 #pragma unroll
         for (int j = 0; j < E; ++j) p[j] = v[j];
@@ -87,15 +90,37 @@ template <int E> __device__ __forceinline__ void scan_down(float (&v)[E], int la
     for (int j = 0; j < E; ++j) v[j] += lane < 31 ? after : 0.f;
 }
 
-// grid cumsum_blocks; E = 4 for chunks up to 128, else 8; chunk_size a multiple of E.  wide: dt_out, cs_f and cs_b are 16-byte aligned
-template <int E>
+// W warps a chunk: add the totals of the warps before (ascending scans) or after (descending ones); K scans at once, the first UP
+// of them ascending.  last / first positions hold a warp's totals.  One barrier; every warp of the block takes part.
+template <int E, int W, int K, int UP> __device__ __forceinline__ void across_warps(float (*const (&v)[K])[E], int lane) {
+    if (W == 1) return;
+    __shared__ float tot[K][kCumsumWarps];
+    const int warp = threadIdx.x >> 5, part = warp % W, first = warp - part;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (lane == (k < UP ? 31 : 0)) tot[k][warp] = (*v[k])[k < UP ? E - 1 : 0];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        float s = 0.f;
+        for (int w = 0; w < W; ++w) s += (k < UP ? w < part : w > part) ? tot[k][first + w] : 0.f;
+#pragma unroll
+        for (int j = 0; j < E; ++j) (*v[k])[j] += s;
+    }
+}
+
+// grid cumsum_blocks; 32 E W >= chunk_size: E W = 4 for chunks up to 128, else 8; chunk_size a multiple of E.  wide: dt_out, cs_f and cs_b are 16-byte aligned
+template <int E, int W>
 __global__ void __launch_bounds__(32 * kCumsumWarps)
 cumsum_fwd(Dims d, const void *dt, int dt_dtype, long long dsb, long long dsl, long long dsh, const float *A, const float *dt_bias,
            float *dt_out, float *cs_f, float *cs_b, int wide) {
     pdl_begin();
-    const int lane = threadIdx.x & 31, l0 = lane * E, nhb = (d.H + kCumsumWarps - 1) / kCumsumWarps;
-    const int h = blockIdx.x % nhb * kCumsumWarps + (threadIdx.x >> 5), c = blockIdx.x / nhb % d.nc, b = blockIdx.x / nhb / d.nc;
-    if (h >= d.H) return;
+    constexpr int kHeads = kCumsumWarps / W;                    // per block
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l0 = (warp % W * 32 + lane) * E, nhb = (d.H + kHeads - 1) / kHeads;
+    const int hw = blockIdx.x % nhb * kHeads + warp / W, c = blockIdx.x / nhb % d.nc, b = blockIdx.x / nhb / d.nc;
+    if (W == 1 && hw >= d.H) return;
+    const bool on = l0 < d.Q && hw < d.H;                       // W > 1: warps beyond the heads redo the last one and store nothing
+    const int h = min(hw, d.H - 1);
     const long long base = ((long long)(b * d.H + h) * d.nc + c) * d.Q + l0;
     const int lim = min(d.Q, d.L - c * d.Q);
     const float Ah = A[h], bias = d.has_bias ? dt_bias[h] : 0.f;
@@ -110,7 +135,8 @@ cumsum_fwd(Dims d, const void *dt, int dt_dtype, long long dsb, long long dsl, l
     }
     scan_up(f, lane);
     scan_down(r, lane);
-    if (l0 < d.Q) {
+    across_warps<E, W, 2, 1>({&f, &r}, lane);
+    if (on) {
         store_e(dt_out + base, wide, v);
         store_e(cs_f + base, wide, f);
         store_e(cs_b + base, wide, r);
@@ -118,13 +144,16 @@ cumsum_fwd(Dims d, const void *dt, int dt_dtype, long long dsb, long long dsl, l
 }
 
 // a.u4 (with a.u4_tiles) or a.da_f / a.da_b as in simt::cumsum_bwd_role.  wide: dt_out is 16-byte aligned
-template <int E>
+template <int E, int W>
 __global__ void __launch_bounds__(32 * kCumsumWarps)
 cumsum_bwd(Dims d, simt::CumsumBwd a, int wide) {
     pdl_begin();
-    const int lane = threadIdx.x & 31, l0 = lane * E, nhb = (d.H + kCumsumWarps - 1) / kCumsumWarps;
-    const int h = blockIdx.x % nhb * kCumsumWarps + (threadIdx.x >> 5), c = blockIdx.x / nhb % d.nc, b = blockIdx.x / nhb / d.nc;
-    if (h >= d.H) return;
+    constexpr int kHeads = kCumsumWarps / W;                    // per block
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l0 = (warp % W * 32 + lane) * E, nhb = (d.H + kHeads - 1) / kHeads;
+    const int hw = blockIdx.x % nhb * kHeads + warp / W, c = blockIdx.x / nhb % d.nc, b = blockIdx.x / nhb / d.nc;
+    if (W == 1 && hw >= d.H) return;
+    const bool on = l0 < d.Q && hw < d.H;                       // W > 1: warps beyond the heads redo the last one and store nothing
+    const int h = min(hw, d.H - 1);
     const int lim = min(d.Q, d.L - c * d.Q);
     const long long tix = (long long)(b * d.H + h) * d.nc + c, base = tix * d.Q + l0;
     const long long copies = (long long)d.b * d.H * d.nc * d.Q;        // nf / nb / pf / pb hold nsplit partial copies, u4 its tiles
@@ -195,6 +224,7 @@ cumsum_bwd(Dims d, simt::CumsumBwd a, int wide) {
     scan_up(v2, lane);
     scan_down(w1, lane);
     scan_down(w2, lane);
+    across_warps<E, W, 4, 2>({&v1, &v2, &w1, &w2}, lane);
     float sumA = 0.f, sumB = 0.f, g[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) {
@@ -206,10 +236,23 @@ cumsum_bwd(Dims d, simt::CumsumBwd a, int wide) {
         sumA += l0 + j < lim ? ddA * dlo[j] : 0.f;
         sumB += l0 + j < lim ? g[j] : 0.f;
     }
-    store_strided(a.ddt.ptr, a.dt_dtype, b * a.ddt.sb + (long long)(c * d.Q + l0) * a.ddt.sl + h * a.ddt.sh, a.ddt.sl, lim - l0, g);
+    store_strided(a.ddt.ptr, a.dt_dtype, b * a.ddt.sb + (long long)(c * d.Q + l0) * a.ddt.sl + h * a.ddt.sh, a.ddt.sl, on ? lim - l0 : 0, g);
     sumA = simt::warp_sum(sumA);
     sumB = simt::warp_sum(sumB);
-    if (lane == 0) {
+    if (W > 1) {
+        __shared__ float red[2][kCumsumWarps];
+        if (lane == 0) {
+            red[0][warp] = sumA;
+            red[1][warp] = sumB;
+        }
+        __syncthreads();
+        sumA = sumB = 0.f;
+        for (int w = 0; w < W; ++w) {
+            sumA += red[0][warp - warp % W + w];
+            sumB += red[1][warp - warp % W + w];
+        }
+    }
+    if (lane == 0 && warp % W == 0 && hw < d.H) {
         a.dApart[(long long)(b * d.nc + c) * d.H + h] = sumA;
         a.dbiaspart[(long long)(b * d.nc + c) * d.H + h] = sumB;
     }
