@@ -221,7 +221,7 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
     if (a.phases & BISSD_PHASE_LOCAL) {
         int rc = note_cuda(cudaMemsetAsync(ws, 0, kWsHeader, s), "cudaMemsetAsync");
         if (rc != BISSD_OK) return rc;
-        BISSD_LAUNCH("cumsum_fwd", launch_pdl(tc::cumsum_share(d) == 1 ? (d.Q <= 128 ? tc::cumsum_fwd<4, 1> : tc::cumsum_fwd<8, 1>) : (d.Q <= 128 ? tc::cumsum_fwd<1, 4> : tc::cumsum_fwd<2, 4>), tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s,
+        BISSD_LAUNCH("cumsum_fwd", launch_pdl(d.Q <= 128 ? tc::cumsum_fwd<1> : tc::cumsum_fwd<2>, tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s,
             d, a.dt.ptr, a.p.dt_dtype, a.dt.stride_batch, a.dt.stride_seq, a.dt.stride_head, a.A, a.dt_bias, a.dt_out,
             a.cs_f, a.cs_b, all_aligned16(a.dt_out, a.cs_f, a.cs_b)));
         if (!walk.use) {
@@ -277,13 +277,13 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
             CUtensorMap mCc, mBc, mCBo;
             if (ws_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc) && make_tile_map(d, CB16, &mCBo)) {
                 const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, false);
-                BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
-                BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
+                BISSD_ALLOW((tc::bmm_cb_tma<T, false>), smem_ct);
+                BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T, false>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
                     d, mCc, mBc, mCBo, mCBo, true, false, nullptr, nullptr, nullptr, status));
             } else if (!ws_path && !no_tma() && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc)) {
                 const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, false, true);
-                BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
-                BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
+                BISSD_ALLOW((tc::bmm_cb_tma<T, true>), smem_ct);
+                BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T, true>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
                     d, mCc, mBc, mCc, mCc, false, false, nullptr, CB, nullptr, status));
             } else
             BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_cb, s>>>(
@@ -478,13 +478,13 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
             // reads the fp32 strips
             fused_cb = !no_fused() && tc::intra_tile_ok(d.P, d.Q);
             const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, true);
-            BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
-            BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
+            BISSD_ALLOW((tc::bmm_cb_tma<T, false>), smem_ct);
+            BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T, false>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
                 d, mCc, mBc, mCBo, mCBto, fused_cb, true, fused_cb ? nullptr : F(w.cbs), nullptr, nullptr, status));
         } else if (!ws_path && sums_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc)) {
             const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, true, true);
-            BISSD_ALLOW(tc::bmm_cb_tma<T>, smem_ct);
-            BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
+            BISSD_ALLOW((tc::bmm_cb_tma<T, true>), smem_ct);
+            BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T, true>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
                 d, mCc, mBc, mCc, mCc, false, false, F(w.cbs), F(w.cb), F(w.cbt), status));
         } else
         BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
@@ -779,7 +779,7 @@ do {                                                                            
     if (use_u4) { cs.u4 = F(w.u4); cs.u4_tiles = u4_tiles; }
     else { cs.da_f = F(w.da_f); cs.da_b = F(w.da_b); }
     cs.dTpart = F(w.dTpart); cs.nblk = walk.use ? tc::walk_slots(d) : pass_slots(d); cs.nsplit = nsplit; cs.ddt = gr.ddt; cs.dApart = F(w.dApart); cs.dbiaspart = F(w.dbiaspart);
-    BISSD_LAUNCH("cumsum_bwd", launch_pdl(tc::cumsum_share(d) == 1 ? (d.Q <= 128 ? tc::cumsum_bwd<4, 1> : tc::cumsum_bwd<8, 1>) : (d.Q <= 128 ? tc::cumsum_bwd<1, 4> : tc::cumsum_bwd<2, 4>), tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s,
+    BISSD_LAUNCH("cumsum_bwd", launch_pdl(d.Q <= 128 ? tc::cumsum_bwd<1> : tc::cumsum_bwd<2>, tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s,
         d, cs, all_aligned16(a.dt_out, a.dt_out, a.dt_out)));
     BISSD_LAUNCH("final_reduce", launch_pdl(simt::final_reduce<1024>, d.H, 1024, 0, s, 
         d, F(w.dApart), F(w.dbiaspart), d.has_D ? F(w.dDpart) : nullptr, dd_slots ? dd_slots : nlt, dd_compact ? 1 : 0, a.dA, d.has_bias ? a.ddt_bias : nullptr,

@@ -20,7 +20,8 @@ inline size_t bmm_cb_tma_smem(int N, bool transposed, bool fp32 = false) {   // 
     return 1024 + (in > out ? in : out);
 }
 
-template <class T>
+// FP32: CB32 / CBt32 / CBs are written, not the 16-bit tiles
+template <class T, bool FP32>
 __global__ void __launch_bounds__(kThreads)
 bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmB,
            const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmOt, bool plain, bool transposed, float *CBs,
@@ -34,7 +35,7 @@ bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constan
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = blockIdx.x % d.G, c = (blockIdx.x / d.G) % d.nc, b = blockIdx.x / (d.G * d.nc);
     const int l0 = blockIdx.y * kTileM, s0 = blockIdx.z * 128;
-    const bool two = transposed || CBt32;                       // the transpose is wanted
+    const bool two = FP32 ? CBt32 != nullptr : transposed;                       // the transpose is wanted
     const uint32_t ncols = two ? 256 : 128;
     if (warp == 0) tmem_alloc(&tmem_slot, ncols);
     if (tid == 32) {                                            // barriers and loads by the same thread, before the sync
@@ -99,8 +100,8 @@ bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constan
                 *reinterpret_cast<float4 *>(out + (long long)i * Q + lane * 4) = *reinterpret_cast<const float4 *>(buf + i * kCbRow + lane * 4);
             __syncthreads();
         };
-        if (CB32) rows_out(0, CB32 + tile + (long long)l0 * Q + s0);
-        if (CBt32) rows_out(1, CBt32 + tile + (long long)s0 * Q + l0);
+        if (FP32 && CB32) rows_out(0, CB32 + tile + (long long)l0 * Q + s0);
+        if (FP32 && CBt32) rows_out(1, CBt32 + tile + (long long)s0 * Q + l0);
         uint8_t *so = smC, *st = smC + 32768;                   // [2 slabs of 128 x 64]
         if (plain || CBs) {
 #pragma unroll

@@ -1,41 +1,32 @@
 // Discretisation + both cumulative sums of the tensor-core family, and their backward (formulas at simt::chunk_cumsum and
-// simt::cumsum_bwd_role).  A lane has E consecutive positions, W warps one (batch, chunk, head): every operand is requested at
-// once in wide pieces, the scans are register sums and five shuffles.  Where a row of the batch brings many chunks W is 1 and
-// nothing waits for a barrier; where it does not, the length of a lane's work is the length of the kernel, and four warps share a
-// chunk (W = 1 cost the smallest forward call 1.6 of 20 us).  The block's heads are neighbours, whose dt and ddt values share
-// 32-byte sectors.  One block per (batch, chunk,
-// head) left these kernels waiting for launches and barriers: at b16 L4096 H32 chunk 256 / 128 backward 88 / 151 us,
-// forward 23 / 33 us.
+// simt::cumsum_bwd_role).  Four warps share one (batch, chunk, head), a lane has E consecutive positions: every operand is
+// requested at once in wide pieces, the scans are register sums, five shuffles and one barrier.  The block's two heads are
+// neighbours, whose dt and ddt values share 32-byte sectors.  us, forward and backward, with a block of one position a
+// thread, a warp per chunk, and this: b16 L4096 H32 23 + 88, 15 + 60, 15.6 + 51; b2 L8192 H32 7 + 24, -, 5.3 + 14;
+// b8 L2048 H24 6 + 18, 5.5 + 16, 4.4 + 11.
 #pragma once
 #include "simt_kernels.cuh"
 
 namespace bissd {
 namespace tc {
 
-constexpr int kCumsumWarps = 8;
-inline int cumsum_share(const Dims &d) { return d.nc * d.H < 256 ? 4 : 1; }   // W: by one row of the batch, so that a row's bits do not depend on the others
-inline int cumsum_blocks(const Dims &d) { return d.b * d.nc * ceil_div(d.H, kCumsumWarps / cumsum_share(d)); }
+constexpr int kCumsumWarps = 8, kCumsumShare = 4;              // per block, per chunk
+inline int cumsum_blocks(const Dims &d) { return d.b * d.nc * ceil_div(d.H, kCumsumWarps / kCumsumShare); }
 
 template <int E> __device__ __forceinline__ void load_e(const float *p, bool wide, float (&v)[E]) {
-    if (E % 4 == 0 && wide) {
-#pragma unroll
-        for (int j = 0; j + 3 < E; j += 4) {
-            const float4 t = *reinterpret_cast<const float4 *>(p + j);
-            v[j] = t.x; v[j + 1] = t.y; v[j + 2] = t.z; v[j + 3] = t.w;
-        }
+    if (E == 2 && wide) {
+        const float2 t = *reinterpret_cast<const float2 *>(p);
+        v[0] = t.x; v[E - 1] = t.y;
     } else {
 #pragma unroll
         for (int j = 0; j < E; ++j) v[j] = p[j];
     }
 }
 template <int E> __device__ __forceinline__ void store_e(float *p, bool wide, const float (&v)[E]) {
-    if (E % 4 == 0 && wide) {
-#pragma unroll
-        for (int j = 0; j + 3 < E; j += 4) *reinterpret_cast<float4 *>(p + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-    } else {
+    if (E == 2 && wide) *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[E - 1]);
+    else
 #pragma unroll
         for (int j = 0; j < E; ++j) p[j] = v[j];
-    }
 }
 // dt and ddt, strided and of a type known at run time only: the choice of type stands outside the loop, so that the E loads
 // are in flight together (decided element by element, each waited for the one before).  Zero beyond n.
@@ -90,10 +81,10 @@ template <int E> __device__ __forceinline__ void scan_down(float (&v)[E], int la
     for (int j = 0; j < E; ++j) v[j] += lane < 31 ? after : 0.f;
 }
 
-// W warps a chunk: add the totals of the warps before (ascending scans) or after (descending ones); K scans at once, the first UP
+// Add the totals of the warps before (ascending scans) or after (descending ones); K scans at once, the first UP
 // of them ascending.  last / first positions hold a warp's totals.  One barrier; every warp of the block takes part.
-template <int E, int W, int K, int UP> __device__ __forceinline__ void across_warps(float (*const (&v)[K])[E], int lane) {
-    if (W == 1) return;
+template <int E, int K, int UP> __device__ __forceinline__ void across_warps(float (*const (&v)[K])[E], int lane) {
+    constexpr int W = kCumsumShare;
     __shared__ float tot[K][kCumsumWarps];
     const int warp = threadIdx.x >> 5, part = warp % W, first = warp - part;
 #pragma unroll
@@ -109,17 +100,16 @@ template <int E, int W, int K, int UP> __device__ __forceinline__ void across_wa
     }
 }
 
-// grid cumsum_blocks; 32 E W >= chunk_size: E W = 4 for chunks up to 128, else 8; chunk_size a multiple of E.  wide: dt_out, cs_f and cs_b are 16-byte aligned
-template <int E, int W>
+// grid cumsum_blocks; E = 1 for chunks up to 128, else 2; chunk_size a multiple of E.  wide: dt_out, cs_f and cs_b are 16-byte aligned
+template <int E>
 __global__ void __launch_bounds__(32 * kCumsumWarps)
 cumsum_fwd(Dims d, const void *dt, int dt_dtype, long long dsb, long long dsl, long long dsh, const float *A, const float *dt_bias,
            float *dt_out, float *cs_f, float *cs_b, int wide) {
     pdl_begin();
-    constexpr int kHeads = kCumsumWarps / W;                    // per block
+    constexpr int W = kCumsumShare, kHeads = kCumsumWarps / W;                    // per block
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l0 = (warp % W * 32 + lane) * E, nhb = (d.H + kHeads - 1) / kHeads;
     const int hw = blockIdx.x % nhb * kHeads + warp / W, c = blockIdx.x / nhb % d.nc, b = blockIdx.x / nhb / d.nc;
-    if (W == 1 && hw >= d.H) return;
-    const bool on = l0 < d.Q && hw < d.H;                       // W > 1: warps beyond the heads redo the last one and store nothing
+    const bool on = l0 < d.Q && hw < d.H;                       // warps beyond the heads redo the last one and store nothing
     const int h = min(hw, d.H - 1);
     const long long base = ((long long)(b * d.H + h) * d.nc + c) * d.Q + l0;
     const int lim = min(d.Q, d.L - c * d.Q);
@@ -135,7 +125,7 @@ cumsum_fwd(Dims d, const void *dt, int dt_dtype, long long dsb, long long dsl, l
     }
     scan_up(f, lane);
     scan_down(r, lane);
-    across_warps<E, W, 2, 1>({&f, &r}, lane);
+    across_warps<E, 2, 1>({&f, &r}, lane);
     if (on) {
         store_e(dt_out + base, wide, v);
         store_e(cs_f + base, wide, f);
@@ -144,15 +134,14 @@ cumsum_fwd(Dims d, const void *dt, int dt_dtype, long long dsb, long long dsl, l
 }
 
 // a.u4 (with a.u4_tiles) or a.da_f / a.da_b as in simt::cumsum_bwd_role.  wide: dt_out is 16-byte aligned
-template <int E, int W>
+template <int E>
 __global__ void __launch_bounds__(32 * kCumsumWarps)
 cumsum_bwd(Dims d, simt::CumsumBwd a, int wide) {
     pdl_begin();
-    constexpr int kHeads = kCumsumWarps / W;                    // per block
+    constexpr int W = kCumsumShare, kHeads = kCumsumWarps / W;                    // per block
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l0 = (warp % W * 32 + lane) * E, nhb = (d.H + kHeads - 1) / kHeads;
     const int hw = blockIdx.x % nhb * kHeads + warp / W, c = blockIdx.x / nhb % d.nc, b = blockIdx.x / nhb / d.nc;
-    if (W == 1 && hw >= d.H) return;
-    const bool on = l0 < d.Q && hw < d.H;                       // W > 1: warps beyond the heads redo the last one and store nothing
+    const bool on = l0 < d.Q && hw < d.H;                       // warps beyond the heads redo the last one and store nothing
     const int h = min(hw, d.H - 1);
     const int lim = min(d.Q, d.L - c * d.Q);
     const long long tix = (long long)(b * d.H + h) * d.nc + c, base = tix * d.Q + l0;
@@ -224,7 +213,7 @@ cumsum_bwd(Dims d, simt::CumsumBwd a, int wide) {
     scan_up(v2, lane);
     scan_down(w1, lane);
     scan_down(w2, lane);
-    across_warps<E, W, 4, 2>({&v1, &v2, &w1, &w2}, lane);
+    across_warps<E, 4, 2>({&v1, &v2, &w1, &w2}, lane);
     float sumA = 0.f, sumB = 0.f, g[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) {
@@ -239,18 +228,16 @@ cumsum_bwd(Dims d, simt::CumsumBwd a, int wide) {
     store_strided(a.ddt.ptr, a.dt_dtype, b * a.ddt.sb + (long long)(c * d.Q + l0) * a.ddt.sl + h * a.ddt.sh, a.ddt.sl, on ? lim - l0 : 0, g);
     sumA = simt::warp_sum(sumA);
     sumB = simt::warp_sum(sumB);
-    if (W > 1) {
-        __shared__ float red[2][kCumsumWarps];
-        if (lane == 0) {
-            red[0][warp] = sumA;
-            red[1][warp] = sumB;
-        }
-        __syncthreads();
-        sumA = sumB = 0.f;
-        for (int w = 0; w < W; ++w) {
-            sumA += red[0][warp - warp % W + w];
-            sumB += red[1][warp - warp % W + w];
-        }
+    __shared__ float red[2][kCumsumWarps];
+    if (lane == 0) {
+        red[0][warp] = sumA;
+        red[1][warp] = sumB;
+    }
+    __syncthreads();
+    sumA = sumB = 0.f;
+    for (int w = 0; w < W; ++w) {
+        sumA += red[0][warp - warp % W + w];
+        sumB += red[1][warp - warp % W + w];
     }
     if (lane == 0 && warp % W == 0 && hw < d.H) {
         a.dApart[(long long)(b * d.nc + c) * d.H + h] = sumA;
