@@ -128,6 +128,8 @@ def kernel_model(name, cfg, batch=None):
         # transpose - the mean of the two launches
         "bmm_cb": (tg * 2 * Q * Q * N, 2 * BC + CB16 + CB16 // 2),
         "chunk_scan": (state_f + intra_f, X * (2 + 2 * zf) + BC + CB16 + 2 * ST16 + 3 * HQ),
+        "state_walk": (state_f, X + BC + 3 * HQ + 2 * ST16),         # chunk states and their recurrence
+        "dstate_walk": (state_f, X + BC + 2 * HQ + 4 * ST16),
         "gate_bwd": (0, 5 * X),
         "dstates": (state_f, X + BC + 2 * HQ + 2 * ST32),
         "state_passing_bwd": (0, 2 * ST32 + 4 * ST16),
