@@ -218,12 +218,34 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
     const int bch = d.b * d.nc * d.H;
     const int ntP = tc::round_up(d.P, 16), ntQ = tc::round_up(d.Q, 16);
     const Walk walk = plan_walk(d, a.p.x_dtype, a.phases, a.B, x, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
+    const tc::CumsumFwd cs{a.dt.ptr, a.p.dt_dtype, a.dt.stride_batch, a.dt.stride_seq, a.dt.stride_head, a.A, a.dt_bias, a.dt_out, a.cs_f, a.cs_b,
+                           all_aligned16(a.dt_out, a.cs_f, a.cs_b)};
+    // C.B^T by TMA: a bf16 copy for the persistent scan, fp32 for the others; in one launch with the cumulative sums where
+    // all blocks are resident at once (b1 L384 H8: 20.5 us a forward call with two launches and a memset for the status word)
+    const bool ws_path = !no_tma() && !no_ws() && tc::scan_ws_ok(d.P, d.N, d.Q);
+    __nv_bfloat16 *CB16 = reinterpret_cast<__nv_bfloat16 *>(ws + w.cb16);
+    CUtensorMap mCc, mBc, mCBo;
+    const bool cb_tma = !no_tma() && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc) && (!ws_path || make_tile_map(d, CB16, &mCBo));
+    if (!ws_path) mCBo = mCc;                                    // not used
+    const size_t cb_smem = tc::bmm_cb_tma_smem(d.N, false, !ws_path);
+    const tc::CbArgs cb_args{ws_path, 0, nullptr, ws_path ? nullptr : CB, nullptr};
+    const long long first_blocks = (long long)d.b * d.nc * d.G * (d.Q / 128) * (d.Q / 128) + tc::cumsum_blocks(d);
+    const bool cb_with_cumsum = cb_tma && (a.phases & BISSD_PHASE_LOCAL) && (a.phases & BISSD_PHASE_FINISH) &&
+                                first_blocks <= (long long)sm_count() * std::min<size_t>(4, 227 * 1024 / (cb_smem + 2048));
     if (a.phases & BISSD_PHASE_LOCAL) {
-        int rc = note_cuda(cudaMemsetAsync(ws, 0, kWsHeader, s), "cudaMemsetAsync");
-        if (rc != BISSD_OK) return rc;
-        BISSD_LAUNCH("cumsum_fwd", launch_pdl(d.Q <= 128 ? tc::cumsum_fwd<1> : tc::cumsum_fwd<2>, tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s,
-            d, a.dt.ptr, a.p.dt_dtype, a.dt.stride_batch, a.dt.stride_seq, a.dt.stride_head, a.A, a.dt_bias, a.dt_out,
-            a.cs_f, a.cs_b, all_aligned16(a.dt_out, a.cs_f, a.cs_b)));
+        if (cb_with_cumsum) {
+            auto launch = [&](auto kernel) -> int {
+                const int tiles = d.b * d.nc * d.G * (d.Q / 128) * (d.Q / 128);
+                BISSD_ALLOW(kernel, cb_smem);
+                BISSD_LAUNCH("cumsum_cb", launch_pdl(kernel, tiles + tc::cumsum_blocks(d), tc::kThreads, cb_smem, s, d, mCc, mBc, mCBo, cb_args, cs, tiles, status));
+                return BISSD_OK;
+            };
+            const int rc = ws_path ? (d.Q == 128 ? launch(tc::cumsum_cb<T, false, 1>) : launch(tc::cumsum_cb<T, false, 2>))
+                                   : (d.Q == 128 ? launch(tc::cumsum_cb<T, true, 1>) : launch(tc::cumsum_cb<T, true, 2>));
+            if (rc != BISSD_OK) return rc;
+        } else {
+            BISSD_LAUNCH("cumsum_fwd", launch_pdl(d.Q <= 128 ? tc::cumsum_fwd<1> : tc::cumsum_fwd<2>, tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s, d, cs, status));
+        }
         if (!walk.use) {
             const size_t smem = tc::smem_bytes(ntP, 2 * d.Q);
             bool st_done = false;
@@ -272,19 +294,16 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
         {
             const size_t smem_cb = tc::smem_bytes(ntQ, 0), smem_sc = tc::smem_bytes(ntP, 3 * d.Q);
             BISSD_ALLOW(tc::bmm_cb<T>, smem_cb);
-            const bool ws_path = !no_tma() && !no_ws() && tc::scan_ws_ok(d.P, d.N, d.Q);
-            __nv_bfloat16 *CB16 = reinterpret_cast<__nv_bfloat16 *>(ws + w.cb16);
-            CUtensorMap mCc, mBc, mCBo;
-            if (ws_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc) && make_tile_map(d, CB16, &mCBo)) {
-                const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, false);
-                BISSD_ALLOW((tc::bmm_cb_tma<T, false>), smem_ct);
-                BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T, false>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
-                    d, mCc, mBc, mCBo, mCBo, true, false, nullptr, nullptr, nullptr, status));
-            } else if (!ws_path && !no_tma() && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc)) {
-                const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, false, true);
-                BISSD_ALLOW((tc::bmm_cb_tma<T, true>), smem_ct);
-                BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T, true>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
-                    d, mCc, mBc, mCc, mCc, false, false, nullptr, CB, nullptr, status));
+            if (cb_with_cumsum) {
+            } else if (cb_tma) {
+                auto launch = [&](auto kernel) -> int {
+                    BISSD_ALLOW(kernel, cb_smem);
+                    BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(kernel, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, cb_smem, s,
+                        d, mCc, mBc, mCBo, mCBo, cb_args, status));
+                    return BISSD_OK;
+                };
+                const int rc = ws_path ? launch(tc::bmm_cb_tma<T, false>) : launch(tc::bmm_cb_tma<T, true>);
+                if (rc != BISSD_OK) return rc;
             } else
             BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_cb, s>>>(
                 d, Cm, Bm, ws_path ? nullptr : CB, nullptr, ws_path ? CB16 : nullptr, nullptr, nullptr, status));
@@ -391,12 +410,13 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
     }
     const Walk walk = plan_walk(d, a.p.x_dtype, a.phases, a.C, gv, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
     if (a.phases & BISSD_PHASE_LOCAL) {
-        int rc = note_cuda(cudaMemsetAsync(ws, 0, kWsHeader, s), "cudaMemsetAsync");
-        if (rc != BISSD_OK) return rc;
-        if (d.has_z) {
+        if (!d.has_z) {                                          // the gate kernel clears the status word
+            const int rc = note_cuda(cudaMemsetAsync(ws, 0, kWsHeader, s), "cudaMemsetAsync");
+            if (rc != BISSD_OK) return rc;
+        } else {
             const long long chunks = (long long)d.b * d.L * d.H * (d.P / 8);
             BISSD_LAUNCH("gate_bwd", launch_pdl(tc::gate_bwd<T>, (unsigned)((chunks + 255) / 256), 256, 0, s, 
-                d, dout, z, out_x, ws + w.g, a.dz));
+                d, dout, z, out_x, ws + w.g, a.dz, status));
         }
         if (!walk.use) {
             const size_t smem = tc::smem_bytes(ntP, 2 * d.Q);
@@ -480,12 +500,12 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
             const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, true);
             BISSD_ALLOW((tc::bmm_cb_tma<T, false>), smem_ct);
             BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T, false>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
-                d, mCc, mBc, mCBo, mCBto, fused_cb, true, fused_cb ? nullptr : F(w.cbs), nullptr, nullptr, status));
+                d, mCc, mBc, mCBo, mCBto, tc::CbArgs{fused_cb, 1, fused_cb ? nullptr : F(w.cbs), nullptr, nullptr}, status));
         } else if (!ws_path && sums_path && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc)) {
             const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, true, true);
             BISSD_ALLOW((tc::bmm_cb_tma<T, true>), smem_ct);
             BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T, true>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
-                d, mCc, mBc, mCc, mCc, false, false, F(w.cbs), F(w.cb), F(w.cbt), status));
+                d, mCc, mBc, mCc, mCc, tc::CbArgs{0, 0, F(w.cbs), F(w.cb), F(w.cbt)}, status));
         } else
         BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
             d, Cm, Bm, (sums_path && ws_path) ? nullptr : F(w.cb), ws_path ? nullptr : F(w.cbt), nullptr,

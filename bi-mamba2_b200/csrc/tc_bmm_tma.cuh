@@ -8,6 +8,7 @@
 // memory into whole rows per warp.  Rows past the end of the sequence read as zeros.
 // grid (b*nc*G, Q/128, Q/128).
 #pragma once
+#include "tc_cumsum.cuh"
 #include "tc_scan_tma.cuh"
 
 namespace bissd {
@@ -20,21 +21,24 @@ inline size_t bmm_cb_tma_smem(int N, bool transposed, bool fp32 = false) {   // 
     return 1024 + (in > out ? in : out);
 }
 
-// FP32: CB32 / CBt32 / CBs are written, not the 16-bit tiles
+struct CbArgs {
+    int plain, transposed;                                      // which 16-bit tiles
+    float *CBs, *CB32, *CBt32;
+};
+// One tile; bx: (batch, chunk, group), row and column tile.  FP32: CB32 / CBt32 / CBs are written, not the 16-bit tiles
 template <class T, bool FP32>
-__global__ void __launch_bounds__(kThreads)
-bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmB,
-           const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmOt, bool plain, bool transposed, float *CBs,
-           float *CB32, float *CBt32, int *status) {
-    pdl_begin();
+__device__ __forceinline__ void bmm_cb_role(const Dims &d, const CUtensorMap &tmC, const CUtensorMap &tmB, const CUtensorMap &tmO,
+                                            const CUtensorMap &tmOt, const CbArgs &a, int bx, int by, int bz, int *status) {
+    const bool plain = a.plain, transposed = a.transposed;
+    float *CBs = a.CBs, *CB32 = a.CB32, *CBt32 = a.CBt32;
     extern __shared__ uint8_t dyn[];
     __shared__ uint64_t bar_in, bar_done;
     __shared__ uint32_t tmem_slot;
     const int Q = d.Q, nsl = d.N / 64;
     uint8_t *smC = smem_align1024(dyn), *smB = smC + nsl * 16384;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = blockIdx.x % d.G, c = (blockIdx.x / d.G) % d.nc, b = blockIdx.x / (d.G * d.nc);
-    const int l0 = blockIdx.y * kTileM, s0 = blockIdx.z * 128;
+    const int g = bx % d.G, c = (bx / d.G) % d.nc, b = bx / (d.G * d.nc);
+    const int l0 = by * kTileM, s0 = bz * 128;
     const bool two = FP32 ? CBt32 != nullptr : transposed;                       // the transpose is wanted
     const uint32_t ncols = two ? 256 : 128;
     if (warp == 0) tmem_alloc(&tmem_slot, ncols);
@@ -140,6 +144,28 @@ bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constan
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, ncols);
+}
+
+template <class T, bool FP32>
+__global__ void __launch_bounds__(kThreads)
+bmm_cb_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmB,
+           const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmOt, CbArgs a, int *status) {
+    pdl_begin();
+    bmm_cb_role<T, FP32>(d, tmC, tmB, tmO, tmOt, a, blockIdx.x, blockIdx.y, blockIdx.z, status);
+}
+
+// The cumulative sums and C.B^T of a forward pass in one launch: neither needs the other, and where all blocks are
+// resident at once (the caller's rule) the pass is as long as its chain of launches.  The first `tiles` blocks have a C.B^T
+// tile each.  The status word is cleared here; a wait that runs out reports long after.
+template <class T, bool FP32, int E>
+__global__ void __launch_bounds__(kThreads)
+cumsum_cb(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmB,
+          const __grid_constant__ CUtensorMap tmO, CbArgs a, CumsumFwd cs, int tiles, int *status) {
+    pdl_begin();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+    const int nt = d.Q / 128, bcg = tiles / (nt * nt), i = blockIdx.x;
+    if (i < tiles) bmm_cb_role<T, FP32>(d, tmC, tmB, tmO, tmO, a, i % bcg, i / bcg % nt, i / bcg / nt, status);
+    else cumsum_fwd_role<E>(d, cs, i - tiles);
 }
 
 }  // namespace tc

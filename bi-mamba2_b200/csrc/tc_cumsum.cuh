@@ -100,22 +100,27 @@ template <int E, int K, int UP> __device__ __forceinline__ void across_warps(flo
     }
 }
 
-// grid cumsum_blocks; E = 1 for chunks up to 128, else 2; chunk_size a multiple of E.  wide: dt_out, cs_f and cs_b are 16-byte aligned
-template <int E>
-__global__ void __launch_bounds__(32 * kCumsumWarps)
-cumsum_fwd(Dims d, const void *dt, int dt_dtype, long long dsb, long long dsl, long long dsh, const float *A, const float *dt_bias,
-           float *dt_out, float *cs_f, float *cs_b, int wide) {
-    pdl_begin();
+// The forward sums as a role of a launch (block of cumsum_blocks).  E = 1 for chunks up to 128, else 2; chunk_size a multiple
+// of E.  wide: dt_out, cs_f and cs_b are 16-byte aligned
+struct CumsumFwd {
+    const void *dt;
+    int dt_dtype;
+    long long dsb, dsl, dsh;
+    const float *A, *dt_bias;
+    float *dt_out, *cs_f, *cs_b;
+    int wide;
+};
+template <int E> __device__ __forceinline__ void cumsum_fwd_role(const Dims &d, const CumsumFwd &a, int block) {
     constexpr int W = kCumsumShare, kHeads = kCumsumWarps / W;                    // per block
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l0 = (warp % W * 32 + lane) * E, nhb = (d.H + kHeads - 1) / kHeads;
-    const int hw = blockIdx.x % nhb * kHeads + warp / W, c = blockIdx.x / nhb % d.nc, b = blockIdx.x / nhb / d.nc;
+    const int hw = block % nhb * kHeads + warp / W, c = block / nhb % d.nc, b = block / nhb / d.nc;
     const bool on = l0 < d.Q && hw < d.H;                       // warps beyond the heads redo the last one and store nothing
     const int h = min(hw, d.H - 1);
     const long long base = ((long long)(b * d.H + h) * d.nc + c) * d.Q + l0;
     const int lim = min(d.Q, d.L - c * d.Q);
-    const float Ah = A[h], bias = d.has_bias ? dt_bias[h] : 0.f;
+    const float Ah = a.A[h], bias = d.has_bias ? a.dt_bias[h] : 0.f;
     float v[E], f[E], r[E];
-    load_strided(dt, dt_dtype, b * dsb + (long long)(c * d.Q + l0) * dsl + h * dsh, dsl, lim - l0, v);
+    load_strided(a.dt, a.dt_dtype, b * a.dsb + (long long)(c * d.Q + l0) * a.dsl + h * a.dsh, a.dsl, lim - l0, v);
 #pragma unroll
     for (int j = 0; j < E; ++j) {
         float t = v[j] + bias;
@@ -127,10 +132,17 @@ cumsum_fwd(Dims d, const void *dt, int dt_dtype, long long dsb, long long dsl, l
     scan_down(r, lane);
     across_warps<E, 2, 1>({&f, &r}, lane);
     if (on) {
-        store_e(dt_out + base, wide, v);
-        store_e(cs_f + base, wide, f);
-        store_e(cs_b + base, wide, r);
+        store_e(a.dt_out + base, a.wide, v);
+        store_e(a.cs_f + base, a.wide, f);
+        store_e(a.cs_b + base, a.wide, r);
     }
+}
+// grid cumsum_blocks; the first kernel of a pass: it also clears the status word
+template <int E>
+__global__ void __launch_bounds__(32 * kCumsumWarps) cumsum_fwd(Dims d, CumsumFwd a, int *status) {
+    pdl_begin();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+    cumsum_fwd_role<E>(d, a, blockIdx.x);
 }
 
 // a.u4 (with a.u4_tiles) or a.da_f / a.da_b as in simt::cumsum_bwd_role.  wide: dt_out is 16-byte aligned

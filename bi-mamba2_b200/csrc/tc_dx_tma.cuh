@@ -15,8 +15,9 @@ namespace tc {
 // g = dout * z * sigmoid(z), dz = dout * out_x * sigmoid(z) * (1 + z (1 - sigmoid(z))); 8 elements per thread.
 // Takes over _chunk_scan_bwd_dz_kernel (src/ssd/bi/ssd_chunk_scan.py:357-440) except its dD partials.
 template <class T>
-__global__ void __launch_bounds__(256) gate_bwd(Dims d, View dout, View z, View out_x, void *g_out, void *dz) {
+__global__ void __launch_bounds__(256) gate_bwd(Dims d, View dout, View z, View out_x, void *g_out, void *dz, int *status) {
     pdl_begin();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;        // the first kernel of its pass
     const long long pc = d.P / 8;
     const long long total = (long long)d.b * d.L * d.H * pc;
     const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
