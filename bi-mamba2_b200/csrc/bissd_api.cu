@@ -183,10 +183,10 @@ static bool walk_pays(const Dims &d) {
     const double apart = 8.0 + 2.5e-6 * 2.0 * d.b * d.nc * d.H * d.P * d.N;
     return walk < apart;
 }
-static Walk plan_walk(const Dims &d, int dtype, int phases, const bissd_tensor &row, const View &col, const float *dt_out,
+static Walk plan_walk(const Dims &d, int dtype, const bissd_tensor &row, const View &col, const float *dt_out,
                       const float *cs_f, const float *cs_b, const void *states_f, const void *states_b) {
     Walk w;
-    if (no_tma() || no_ws() || (phases & 3) != 3 || !tc::walk_ok(d.P, d.N, d.Q) || !walk_pays(d)) return w;
+    if (no_tma() || no_ws() || !tc::walk_ok(d.P, d.N, d.Q) || !walk_pays(d)) return w;
     if (!all_aligned16(dt_out, cs_f, cs_b)) return w;
     const unsigned rows = tc::walk_rows(d.P / 64);
     const unsigned long long srows = (unsigned long long)d.b * d.nc * d.H * d.P;
@@ -217,7 +217,8 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
     const View x = view_of(a.x), Bm = view_of(a.B), Cm = view_of(a.C), z = view_of(a.z);
     const int bch = d.b * d.nc * d.H;
     const int ntP = tc::round_up(d.P, 16), ntQ = tc::round_up(d.Q, 16);
-    const Walk walk = plan_walk(d, a.p.x_dtype, a.phases, a.B, x, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
+    // (a FINISH phase with entering states walks again, from the inputs: the decision is the same in both phases)
+    const Walk walk = plan_walk(d, a.p.x_dtype, a.B, x, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
     const tc::CumsumFwd cs{a.dt.ptr, a.p.dt_dtype, a.dt.stride_batch, a.dt.stride_seq, a.dt.stride_head, a.A, a.dt_bias, a.dt_out, a.cs_f, a.cs_b,
                            all_aligned16(a.dt_out, a.cs_f, a.cs_b)};
     // C.B^T by TMA: a bf16 copy for the persistent scan, fp32 for the others; in one launch with the cumulative sums where
@@ -282,11 +283,12 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
     }
     // the recurrence runs in both phases: from zero (or init_*) in LOCAL, again with init_* in FINISH
     const bool need_pass = (a.phases & BISSD_PHASE_LOCAL) || (a.init_f || a.init_b);
-    if (walk.use) {
-        const tc::WalkArgs wa{a.dt_out, a.cs_f, a.cs_b, a.init_f, a.init_b, a.final_f, a.final_b, a.states_f, a.states_b, nullptr};
+    if (!need_pass) {
+    } else if (walk.use) {
+        const tc::WalkArgs wa{a.dt_out, a.cs_f, a.cs_b, a.init_f, a.init_b, a.final_f, a.final_b, a.states_f, a.states_b, nullptr, 0};
         const int rc = launch_walk<T, 0>(d, walk, wa, status, s);
         if (rc != BISSD_OK) return rc;
-    } else if (need_pass) {
+    } else {
         BISSD_LAUNCH("state_passing_fwd", launch_pdl(pass_ahead(d) ? simt::state_passing_fwd4<T, 8> : simt::state_passing_fwd4<T, 1>, pass_grid(d), pass_threads(d), 0, s,
             d, loc, a.cs_f, a.cs_b, a.init_f, a.init_b, a.states_f, a.states_b, a.final_f, a.final_b));
     }
@@ -408,12 +410,14 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
         dg.has_z = 0;
         gv = View{ws + w.g, (long long)d.L * d.H * d.P, (long long)d.H * d.P, (long long)d.P};
     }
-    const Walk walk = plan_walk(d, a.p.x_dtype, a.phases, a.C, gv, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
+    Walk walk;                                                   // whole passes only: a split one keeps its local gradients
+    if (a.phases == BISSD_PHASE_ALL) walk = plan_walk(d, a.p.x_dtype, a.C, gv, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
     if (a.phases & BISSD_PHASE_LOCAL) {
-        if (!d.has_z) {                                          // the gate kernel clears the status word
+        if (!d.has_z && !walk.use) {                             // else the gate kernel or the walk, whichever is first, clears the status word
             const int rc = note_cuda(cudaMemsetAsync(ws, 0, kWsHeader, s), "cudaMemsetAsync");
             if (rc != BISSD_OK) return rc;
-        } else {
+        }
+        if (d.has_z) {
             const long long chunks = (long long)d.b * d.L * d.H * (d.P / 8);
             BISSD_LAUNCH("gate_bwd", launch_pdl(tc::gate_bwd<T>, (unsigned)((chunks + 255) / 256), 256, 0, s, 
                 d, dout, z, out_x, ws + w.g, a.dz, status));
@@ -455,7 +459,7 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
     const bool need_pass = (a.phases & BISSD_PHASE_LOCAL) || (a.dfinal_f || a.dfinal_b);
     if (walk.use) {
         const tc::WalkArgs wa{a.dt_out, a.cs_f, a.cs_b, a.dfinal_f, a.dfinal_b, a.dinit_f, a.dinit_b, E16,
-                              static_cast<char *>(E16) + (size_t)d.b * d.nc * d.H * d.P * d.N * 2, F(w.dTpart)};
+                              static_cast<char *>(E16) + (size_t)d.b * d.nc * d.H * d.P * d.N * 2, F(w.dTpart), !d.has_z};
         const int rc = launch_walk<T, 1>(d, walk, wa, status, s);
         if (rc != BISSD_OK) return rc;
     } else if (need_pass) {

@@ -44,6 +44,7 @@ struct WalkArgs {
     float *end_f, *end_b;                                       // final_* or dinit_*: the same, or null
     void *out_f, *out_b;                                        // states_* or E16 per direction: (b, nc, H, P, N) 16-bit
     float *dTpart;                                              // MODE 1
+    int first;                                                  // first kernel of its pass: clears the status word (a wait that runs out reports long after)
 };
 
 // grid 2 b H tiles; tmRow: B or C, box [64 n x a stage's positions]; tmCol: x or g, the same; tmS*: states, box [64 n x P
@@ -53,6 +54,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1)
 state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_constant__ CUtensorMap tmCol,
            const __grid_constant__ CUtensorMap tmSf, const __grid_constant__ CUtensorMap tmSb, WalkArgs a, int *status) {
     pdl_begin();
+    if (a.first && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
     extern __shared__ uint8_t dyn[];
     __shared__ WalkShared sh;
     constexpr int P = 64 * PB, SR = walk_rows(PB), NS = walk_ring(PB, MODE);
