@@ -627,7 +627,7 @@ do {                                                                            
                 tc::make_map2(&mEb, a.p.x_dtype, e16 + rows * d.N * 2, d.N, rows, 64, d.P) &&
                 tc::make_map2(&mSf, a.p.x_dtype, a.states_f, d.N, rows, 64, d.P) &&
                 tc::make_map2(&mSb, a.p.x_dtype, a.states_b, d.N, rows, 64, d.P)) {
-                const size_t smem_p = tc::prev_tma_smem(d.P, d.N), smem_a = tc::dbc_tma_smem(d.P, std::min(d.N, 128));
+                const size_t smem_p = tc::prev_tma_smem(d.P), smem_a = tc::dbc_tma_smem(d.P, std::min(d.N, 128));
                 if (!map_bshd(&mX128, a.p.x_dtype, a.x.ptr, a.x.stride_batch, a.x.stride_seq, a.x.stride_head, d.P, d.H, d.L, d.b, 128) ||
                     !map_bshd(&mG128, a.p.x_dtype, gv.ptr, gv.sb, gv.sl, gv.sh, d.P, d.H, d.L, d.b, 128))
                     return BISSD_ERR_ALIGN;

@@ -447,8 +447,9 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
 // ---------------------------------------------------------------------------------------------------------
 // "prev" decay terms:  pf[l] = e^{cs_f[l]} sum_p g[l,p] (C[l,:].S_f[p,:]),  pb[l] likewise with S_b / cs_b  - the row sums
 // the reference takes inside _chunk_scan_bwd_dc_kernel (src/ssd/bi/ssd_chunk_scan.py:598-623).  C and both entering
-// states arrive by TMA; nothing is staged by threads.   grid (b*nc*H, Q/128).
-inline size_t prev_tma_smem(int P, int N) { return 1024 + (size_t)(N / 64) * 16384 + 2 * (size_t)(N / 64) * P * 128; }
+// states arrive by TMA, 64 dstate columns at a time (ScanFeed), so that two CTAs share an SM (everything resident, one CTA
+// an SM: 55 us at b8 L1024 H16 P128 N256); nothing is staged by threads.   grid (b*nc*H, Q/128).
+inline size_t prev_tma_smem(int P) { return 1024 + 2 * (size_t)scan_slot_bytes(P); }
 
 template <class T>
 __global__ void __launch_bounds__(kThreads, 2)
@@ -457,32 +458,20 @@ prev_terms_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
                int *status) {
     pdl_begin();
     extern __shared__ uint8_t dyn[];
-    __shared__ uint64_t bar_in, bar_done;
-    __shared__ uint32_t tmem_slot;
+    __shared__ ScanShared sh;
     __shared__ float rowred[2][kTileM];
-    const int P = d.P, N = d.N, Q = d.Q;
-    const int nsl = N / 64;
-    uint8_t *smC = smem_align1024(dyn);
-    uint8_t *smSf = smC + nsl * 16384, *smSb = smSf + nsl * P * 128;
+    const int P = d.P, Q = d.Q;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int h = blockIdx.x % d.H, c = (blockIdx.x / d.H) % d.nc, b = blockIdx.x / (d.H * d.nc);
-    const int grp = h / d.R;
     const int lim = min(Q, d.L - c * Q);
     const int l0 = blockIdx.y * kTileM;
     const long long base = ((long long)(b * d.H + h) * d.nc + c) * Q;
-    const uint32_t ncols = tmem_cols(2 * P);
-    if (warp == 0) tmem_alloc(&tmem_slot, ncols);
-    if (tid == 0) {                                             // barriers and loads by the same thread, before the sync
-        mbar_init(&bar_in, 1);
-        mbar_init(&bar_done, 1);
-        fence_mbar_init();
-        const int tile = (b * d.nc + c) * d.H + h;
-        mbar_expect_tx(&bar_in, (uint32_t)(nsl * 16384 + 2 * nsl * P * 128));
-        for (int j = 0; j < nsl; ++j) {
-            tma_load4(smC + j * 16384, &tmC, j * 64, grp, c * Q + l0, b, &bar_in);
-            tma_load2(smSf + j * P * 128, &tmSf, j * 64, tile * P, &bar_in);
-            tma_load2(smSb + j * P * 128, &tmSb, j * 64, tile * P, &bar_in);
-        }
+    const uint32_t ncols = 2 * P;
+    ScanFeed feed{sh, d, smem_align1024(dyn), &tmC, &tmSf, &tmSb, nullptr, b, c, h, h / d.R, l0};
+    if (warp == 0) tmem_alloc(&sh.tmem_base, ncols);
+    if (tid == 32) {                                            // barriers and first loads by the same thread, before the sync
+        feed.init_barriers();
+        feed.start();
     }
     // this thread's g row piece and row factors are requested while the tiles are in flight
     const int quad = warp & 3, half = warp >> 2;
@@ -498,25 +487,10 @@ prev_terms_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
-    bool ok = true;
-    if (tid == 0) {
-        ok = mbar_wait(&bar_in, 0);
-        if (ok) {
-            tc_fence_after();
-            const uint32_t idesc = instr_desc(AbFmt<T>::v, false, false, P);
-            for (int dir = 0; dir < 2; ++dir)
-                for (int j = 0; j < nsl; ++j)
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        umma(tmem + dir * P, smem_desc(smem_u32(smC + j * 16384) + kk * 32, 16, 1024),
-                             smem_desc(smem_u32((dir ? smSb : smSf) + j * P * 128) + kk * 32, 16, 1024), idesc,
-                             (j > 0 || kk > 0) ? 1u : 0u);
-            umma_commit(&bar_done);
-        }
-    }
-    if (ok) ok = mbar_wait(&bar_done, 0);
-    ok = __syncthreads_and(ok);
+    const uint32_t tmem = sh.tmem_base;
+    if (tid == 0 && !feed.products<T>(tmem)) sh.fail = 1;
+    bool ok = mbar_wait(&sh.st_done, 0);
+    ok = __syncthreads_and(ok) && !sh.fail;
     tc_fence_after();
     if (!ok && tid == 0) atomicExch(status, kErrMmaTimeout);
     float sf_ = 0.f, sb_ = 0.f;

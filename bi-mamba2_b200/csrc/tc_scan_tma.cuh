@@ -28,7 +28,7 @@ __host__ __device__ constexpr int scan_slot_bytes(int P) { return 16384 + 2 * P 
 inline size_t scan_tma_smem(int P, int Q) { return 1024 + 2 * (size_t)scan_slot_bytes(P) + 4 * (size_t)Q * 4; }
 inline bool scan_tma_ok(int P, int N, int Q) { return (P == 64 || P == 128) && N % 64 == 0 && N <= 256 && (Q == 128 || Q == 256); }
 
-// The loads and products of one tile up to both state products, for chunk_scan_tma and dx_tma; one thread.
+// The loads and products of one tile, for chunk_scan_tma, dx_tma and prev_terms_tma (which needs no x: mX null); one thread.
 struct ScanFeed {
     ScanShared &sh;
     const Dims &d;
@@ -59,6 +59,7 @@ struct ScanFeed {
         tma_load2(dst + 16384 + P * 128, mSb, n0, row, &sh.full[k & 1]);
     }
     __device__ __forceinline__ void load_x(int i) {             // rows 64 i ... of the chunk
+        if (!mX) return;
         mbar_expect_tx(&sh.x_full[i & 1], (uint32_t)(d.P * 128));
         for (int j = 0; j < d.P / 64; ++j) tma_load4(x_piece(i) + j * 8192, mX, j * 64, h, c * d.Q + i * 64, b, &sh.x_full[i & 1]);
     }
