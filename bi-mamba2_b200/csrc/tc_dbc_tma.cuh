@@ -30,7 +30,7 @@ inline size_t dbc_tma_smem(int P, int nt) {
 // Both operands of every (head, direction) stage arrive by TMA into a three-deep ring, requested by lane 0 of warp 9; warps
 // 0-7 scale the 128 rows of the left tile in place, lane 0 of warp 8 issues the stage's MMAs.  (One thread doing loads, MMAs
 // and its share of the scaling, a CTA barrier per stage, the kernel took 113 us at b8 L1024 H16 P128 G2 N256
-// chunk 128.)  The row factors of head h+1 are loaded while head h is being worked on.  Bounded waits, ids 81-85 in the status word.
+// chunk 128, 87 now.)  The row factors of head h+1 are loaded while head h is being worked on.  Bounded waits, ids 81-85 in the status word.
 template <class T>
 __global__ void __launch_bounds__(kDbcTmaThreads, 1)
 dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_constant__ CUtensorMap tmEb,
@@ -448,7 +448,7 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
 // "prev" decay terms:  pf[l] = e^{cs_f[l]} sum_p g[l,p] (C[l,:].S_f[p,:]),  pb[l] likewise with S_b / cs_b  - the row sums
 // the reference takes inside _chunk_scan_bwd_dc_kernel (src/ssd/bi/ssd_chunk_scan.py:598-623).  C and both entering
 // states arrive by TMA, 64 dstate columns at a time (ScanFeed), so that two CTAs share an SM (everything resident, one CTA
-// an SM: 55 us at b8 L1024 H16 P128 N256); nothing is staged by threads.   grid (b*nc*H, Q/128).
+// an SM: 55 us at b8 L1024 H16 P128 N256, 43 now); nothing is staged by threads.   grid (b*nc*H, Q/128).
 inline size_t prev_tma_smem(int P) { return 1024 + 2 * (size_t)scan_slot_bytes(P); }
 
 template <class T>

@@ -2,7 +2,7 @@
 //
 // Per CTA: one (batch, chunk, head) and 128 rows l; two CTAs an SM - one tile is a chain of loads, products and sums, and the
 // other CTA's work fills the waits (headdim 128, dstate 256, b8 L1024 H16 chunk 128: one CTA an SM, everything resident,
-// took 129 us).  For that the products C.S_f^T and C.S_b^T take 64 dstate columns at a time: a slot holds a slab of C and
+// took 129 us; 111 now).  For that the products C.S_f^T and C.S_b^T take 64 dstate columns at a time: a slot holds a slab of C and
 // of both entering states, the next slab lands in the second slot meanwhile.  Both products have a TMEM accumulator; when
 // they are complete their sum, weighted by e^{cs_f[l]} and e^{cs_b[l]}, replaces the first of them, and the masked-decay
 // product is accumulated on top: 2 P columns of tensor memory instead of 3 P, which would round up to all of it.
