@@ -11,6 +11,7 @@
 #include "common.cuh"
 #include "host.cuh"
 #include "layouts.cuh"
+#include "side_stream.h"
 #include "simt_kernels.cuh"
 #include "tc_intra.cuh"
 #include "tc_intra_sums.cuh"
@@ -40,57 +41,12 @@ std::atomic<unsigned long long> g_launches{0};
 // the caller's stream after the dx kernel and shares the GPU with the fused dCB / decay-gradient kernel; dbc_accum_grp goes
 // with it where it writes partial results, or follows that kernel where it finishes dB and dC itself, then beside
 // cumsum_bwd and final_reduce.  Each of these leaves a seventh of the SMs idle when it runs alone.  Stream order as the
-// caller sees it is unchanged, also under stream capture (the side stream joins the capture through the events).  A call
-// leases one (stream, events) set of its device for its duration; sets are created on first need - in practice by the
-// first call on a device, so not inside a later capture.  BISSD_NO_SIDE=1 keeps everything on the caller's stream.
-struct Side {
-    cudaStream_t st = nullptr;
-    cudaEvent_t fork = nullptr, fork2 = nullptr, join = nullptr;
-    int dev = -1;
-    bool busy = false;
-};
-static std::mutex g_side_mu;
-static std::vector<Side *> g_side;
-static Side *side_acquire(cudaStream_t s) {
+// caller sees it is unchanged, also under stream capture (the side stream joins the capture through the events) and when a
+// launch fails (side_stream.h).  BISSD_NO_SIDE=1 keeps everything on the caller's stream.
+static bool side_allowed() {
     static const bool off = [] { const char *e = getenv("BISSD_NO_SIDE"); return e && e[0] == '1'; }();
-    if (off || g_trace_on.load(std::memory_order_relaxed)) return nullptr;   // traced runs time every kernel alone, in line
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-    std::lock_guard<std::mutex> lk(g_side_mu);
-    for (Side *sd : g_side)
-        if (sd->dev == dev && !sd->busy) {
-            sd->busy = true;
-            return sd;
-        }
-    // nothing free: make a set - but not while the caller's stream is being captured (creation belongs outside a capture)
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    cudaStream_t st = nullptr;
-    cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
-    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&e0, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&e1, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&e2, cudaEventDisableTiming) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;                                           // no side stream: the launch stays in line
-    }
-    Side *sd = new Side;
-    sd->st = st; sd->fork = e0; sd->join = e1; sd->fork2 = e2; sd->dev = dev; sd->busy = true;
-    g_side.push_back(sd);
-    return sd;
+    return !off && !g_trace_on.load(std::memory_order_relaxed);  // traced runs time every kernel alone, in line
 }
-struct SideLease {                                                // gives the set back when the call returns
-    Side *sd = nullptr;
-    ~SideLease() {
-        if (sd) {
-            std::lock_guard<std::mutex> lk(g_side_mu);
-            sd->busy = false;
-        }
-    }
-};
 
 // C and B as (dstate, group, seqlen, batch) tensors read in boxes of 64 state columns x 128 rows
 template <class Args> static bool make_cb_maps(const Args &a, const Dims &d, CUtensorMap *mC, CUtensorMap *mB) {
@@ -480,8 +436,7 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
     bool have_fp32_cb = true;                                    // fp32 CB (and its transpose) are in the workspace
     bool use_u4 = false;                                         // decay gradients arrive as u_f / u_b (tc::intra_sums)
     bool fused_cb = false;                                       // the bf16 C.B^T tile for tc::intra_dcb_tile has been written
-    SideLease lease;
-    cudaStream_t s_side = s;                                     // where prev_terms_grp and dbc_accum_grp are launched
+    SideStream side(s);                                          // where prev_terms_grp and dbc_accum_grp are launched
     int u4_tiles = 2;                                            // (u_f, u_b) vector pairs per chunk in u4
     int dd_slots = 0;                                            // dD partial rows per (b,c,h) when not nlt
     bool dd_compact = false;                                     // per-head D from the persistent dx kernel: dd_slots scalars, no channel axis
@@ -565,13 +520,7 @@ do {                                                                            
                 else BISSD_DX_WS(1, 2);
 #undef BISSD_DX_WS
                 dx_done = true;
-                if (fused_cb && (lease.sd = side_acquire(s)) != nullptr) {      // the two group-walking kernels branch off here
-                    if (cudaEventRecord(lease.sd->fork, s) == cudaSuccess && cudaStreamWaitEvent(lease.sd->st, lease.sd->fork, 0) == cudaSuccess) {
-                        s_side = lease.sd->st;
-                    } else {
-                        cudaGetLastError();
-                    }
-                }
+                if (fused_cb && side_allowed() && side.fork() != cudaSuccess) cudaGetLastError();   // the group-walking kernels branch off here, or stay in line
                 dd_slots = nlt_tc * 4;
                 if (d.has_D && !d.D_hdim) {
                     dd_slots = nlt_tc * 8;                       // one scalar per epilogue warp and tile
@@ -635,7 +584,7 @@ do {                                                                            
                     const size_t smem_g = tc::prev_grp_smem(d.N, d.Q);
                     const int ks = tc::state_grp_ksplit(d.b * d.nc * d.G, d.R, sm_count());
                     BISSD_ALLOW(tc::prev_terms_grp<T>, smem_g);
-                    BISSD_LAUNCH_ON(s_side, "tc_prev_terms_grp", launch_pdl(tc::prev_terms_grp<T>, dim3(d.b * d.nc * d.G * ks), tc::kPrevGrpThreads, smem_g, s_side, 
+                    BISSD_LAUNCH_ON(side.stream(), "tc_prev_terms_grp", launch_pdl(tc::prev_terms_grp<T>, dim3(d.b * d.nc * d.G * ks), tc::kPrevGrpThreads, smem_g, side.stream(),
                         d, mC, mSf, mSb, mG128, ks, a.cs_f, a.cs_b, F(w.pf), F(w.pb), status));
                 } else {
                     BISSD_ALLOW(tc::prev_terms_tma<T>, smem_p);
@@ -646,7 +595,7 @@ do {                                                                            
                 if (!no_ws() && tc::dbc_grp_ok(d.P, d.N, d.Q)) {
                     dbc_last = fused_cb && head_parts(d) == 1 && tc::bmm_bwd_tma_ok(d.N, d.Q);   // launched after the dCB kernel, below
                     if (!dbc_last) {
-                        const int rc = launch_dbc(tc::dbc_accum_grp<T, false>, tc::LastMaps{}, s_side);
+                        const int rc = launch_dbc(tc::dbc_accum_grp<T, false>, tc::LastMaps{}, side.stream());
                         if (rc != BISSD_OK) return rc;
                         part_heads = d.G * dbc_slots(d, w.dbc_ks);
                     }
@@ -766,24 +715,17 @@ do {                                                                            
                 dg, none, none, x, z, gv, a.dt_out, a.cs_f, a.cs_b, F(w.cb), F(w.da_f), F(w.da_b), status));
         }
     }
-    auto join = [&]() -> int {                                   // the side stream's kernels rejoin before their results are read
-        if (s_side == s) return BISSD_OK;
-        int rcj = note_cuda(cudaEventRecord(lease.sd->join, s_side), "cudaEventRecord");
-        if (rcj == BISSD_OK) rcj = note_cuda(cudaStreamWaitEvent(s, lease.sd->join, 0), "cudaStreamWaitEvent");
-        return rcj;
-    };
-    {
-        const int rcj = join();
-        if (rcj != BISSD_OK) return rcj;
-    }
+    // the side stream's kernels rejoin before their results are read
+    const bool beside = side.stream() != s;
+    int rcj = note_cuda(side.join(), "join of the second stream");
+    if (rcj != BISSD_OK) return rcj;
     if (dbc_last) {
         if (!bmm_tma) return BISSD_ERR_ALIGN;                    // its operands are the ones the dCB kernel's branch has mapped
-        if (s_side != s) {
-            int rcj = note_cuda(cudaEventRecord(lease.sd->fork2, s), "cudaEventRecord");
-            if (rcj == BISSD_OK) rcj = note_cuda(cudaStreamWaitEvent(s_side, lease.sd->fork2, 0), "cudaStreamWaitEvent");
+        if (beside) {
+            rcj = note_cuda(side.fork(), "fork of the second stream");
             if (rcj != BISSD_OK) return rcj;
         }
-        const int rcl = launch_dbc(tc::dbc_accum_grp<T, true>, tc::LastMaps{mDm, mDk, mBb, mCb, gr.dB, gr.dC}, s_side);
+        const int rcl = launch_dbc(tc::dbc_accum_grp<T, true>, tc::LastMaps{mDm, mDk, mBb, mCb, gr.dB, gr.dC}, side.stream());
         if (rcl != BISSD_OK) return rcl;
     } else if (bmm_tma) {
         const size_t smem_b = tc::bmm_bwd_tma_smem(d.Q);
@@ -808,7 +750,7 @@ do {                                                                            
     BISSD_LAUNCH("final_reduce", launch_pdl(simt::final_reduce<1024>, d.H, 1024, 0, s, 
         d, F(w.dApart), F(w.dbiaspart), d.has_D ? F(w.dDpart) : nullptr, dd_slots ? dd_slots : nlt, dd_compact ? 1 : 0, a.dA, d.has_bias ? a.ddt_bias : nullptr,
         d.has_D ? a.dD : nullptr));
-    return dbc_last ? join() : BISSD_OK;
+    return note_cuda(side.join(), "join of the second stream");
 }
 
 }  // namespace bissd
