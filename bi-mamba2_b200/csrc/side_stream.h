@@ -16,6 +16,16 @@ struct SideSet {
 inline std::mutex g_side_mu;
 inline std::vector<SideSet *> g_side;
 
+// May what `main` launches go to `side` now?  A stream that was forked into a capture belongs to it until the capture ends, long
+// after its lease: only calls of the same capture may use it, anything else would break the capture.
+inline bool side_usable(cudaStream_t side, cudaStream_t main) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone, st_main = st;
+    unsigned long long id = 0, id_main = 0;
+    if (cudaStreamGetCaptureInfo(side, &st, &id) != cudaSuccess) return false;
+    if (st == cudaStreamCaptureStatusNone) return true;
+    return st == cudaStreamCaptureStatusActive && cudaStreamGetCaptureInfo(main, &st_main, &id_main) == cudaSuccess && st_main == st && id_main == id;
+}
+
 // A free set of the current device, or null: the launch then stays in line.  Sets are created on first need - in practice
 // by the first call on a device - but not while the caller's stream is being captured (creation belongs outside a capture).
 inline SideSet *side_acquire(cudaStream_t s) {
@@ -23,7 +33,7 @@ inline SideSet *side_acquire(cudaStream_t s) {
     if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
     std::lock_guard<std::mutex> lk(g_side_mu);
     for (SideSet *set : g_side)
-        if (set->dev == dev && !set->busy) {
+        if (set->dev == dev && !set->busy && side_usable(set->st, s)) {
             set->busy = true;
             return set;
         }

@@ -1,14 +1,14 @@
 // Drives csrc/side_stream.h against a CUDA runtime of a few fake functions that write down what is called.  Prints "ok".
 #include <cstdio>
 #include <cstdlib>
-#include <set>
+#include <map>
 #include <string>
 
 #include "../bi-mamba2_b200/csrc/side_stream.h"
 
 static std::string calls;                                        // one letter per call: R record, W wait, S synchronize, C create
 static std::string refuse;                                       // letters whose next call fails
-static std::set<cudaStream_t> capturing;
+static std::map<cudaStream_t, unsigned long long> capture;      // streams in a capture, and which
 static long made = 100;
 static cudaError_t note(char c) {
     const size_t at = refuse.find(c);
@@ -30,9 +30,15 @@ cudaError_t cudaStreamDestroy(cudaStream_t) { return note('c'); }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return note('e'); }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return note('R'); }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return note('W'); }
+cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, cudaStreamCaptureStatus *st, unsigned long long *id, cudaGraph_t *,
+                                     const cudaGraphNode_t **, size_t *) {
+    *st = capture.count(s) ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    *id = capture.count(s) ? capture[s] : 0;
+    return cudaSuccess;
+}
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return note('S'); }
 cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus *st) {
-    *st = capturing.count(s) ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    *st = capture.count(s) ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
     return cudaSuccess;
 }
 }
@@ -89,6 +95,16 @@ int main() {
         take();
     }
     expect(take().empty(), "and has nothing to join");
+    {                                                            // `first` was forked into capture 7 of s, which goes on after the call
+        capture[s] = capture[first] = 7;
+        SideStream beside(other);
+        expect(beside.fork() == cudaSuccess && beside.stream() != first, "a stream in another's capture is left alone");
+        SideStream same(s);
+        expect(same.fork() == cudaSuccess && same.stream() == first, "the capture's own calls use it");
+        capture[other] = 8;
+        SideStream later(other);
+        expect(later.fork() == cudaSuccess && later.stream() == other, "no set is made inside a capture");
+    }
     std::printf("ok\n");
     return 0;
 }
