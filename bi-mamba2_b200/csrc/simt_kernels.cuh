@@ -432,10 +432,10 @@ __global__ void __launch_bounds__(TB) state_passing_fwd4(Dims d, const float *lo
             const int c = dir ? d.nc - 1 - i0 - u : i0 + u;
             const float ed = expf(dec[u]);
             st4<T>(states, off0 + c * cstride, run.x, run.y, run.z, run.w);
-            run.x = ed * run.x + v[u].x;
-            run.y = ed * run.y + v[u].y;
-            run.z = ed * run.z + v[u].z;
-            run.w = ed * run.w + v[u].w;
+            run.x = fmaf(ed, run.x, v[u].x);
+            run.y = fmaf(ed, run.y, v[u].y);
+            run.z = fmaf(ed, run.z, v[u].z);
+            run.w = fmaf(ed, run.w, v[u].w);
         }
     }
     if (fin) *reinterpret_cast<float4 *>(fin + (long long)(b * d.H + h) * PN + e) = run;
@@ -484,16 +484,16 @@ __global__ void __launch_bounds__(TB) state_passing_bwd4(Dims d, const float *gl
             const int c = dir ? i0 + u : d.nc - 1 - i0 - u;
             const long long off = off0 + c * cstride;
             const float ed = expf(dec[u]);
-            part[u] = ed * (sv[u].x * run.x + sv[u].y * run.y + sv[u].z * run.z + sv[u].w * run.w);
+            part[u] = ed * fmaf(sv[u].x, run.x, fmaf(sv[u].y, run.y, fmaf(sv[u].z, run.z, sv[u].w * run.w)));   // one order, whatever U
             if (i0 + u < d.nc) {
                 if (on) {
                     if (E) *reinterpret_cast<float4 *>(E + dir * per_dir + off) = run;
                     if (E16) st4<T>(E16, dir * per_dir + off, run.x, run.y, run.z, run.w);
                 }
-                run.x = ed * run.x + gv[u].x;
-                run.y = ed * run.y + gv[u].y;
-                run.z = ed * run.z + gv[u].z;
-                run.w = ed * run.w + gv[u].w;
+                run.x = fmaf(ed, run.x, gv[u].x);
+                run.y = fmaf(ed, run.y, gv[u].y);
+                run.z = fmaf(ed, run.z, gv[u].z);
+                run.w = fmaf(ed, run.w, gv[u].w);
             }
         }
 #pragma unroll

@@ -1,0 +1,41 @@
+"""A row's results do not depend on how many rows there are: sizes where the batch changes the kernels, or how they share work."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def rows(dtype, b, L, H, P, G, N, Q, z, few=1):
+    """out, dx, ddt, dB, dC (and dz) of `few` rows run alone and of the same rows among b, with the kernels of each run."""
+    from ssd import _cabi
+    from ssd.bi.ssd_combined import bimamba_chunk_scan_combined
+    g = torch.Generator(device="cuda").manual_seed(L + H + P)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, B, C, dout, gate = (t.to(dtype) for t in (mk(b, L, H, P), mk(b, L, G, N), mk(b, L, G, N), mk(b, L, H, P), mk(b, L, H, P)))
+    per_row, shared = [x, mk(b, L, H) - 4.0, B, C] + ([gate] if z else []), [-torch.exp(torch.rand(H, generator=g, device="cuda") * 2.7), mk(H)]
+    results = []
+    for n in (few, b):
+        leaves = [t[:n].clone().requires_grad_(True) for t in per_row]
+        _cabi.trace_enable(True)
+        out = bimamba_chunk_scan_combined(leaves[0], leaves[1], shared[0], leaves[2], leaves[3], Q, D=shared[1], z=leaves[4] if z else None,
+                                          dt_softplus=True)
+        got = [out, *torch.autograd.grad(out, leaves, dout[:n])]
+        torch.cuda.synchronize()
+        ran = set(_cabi.trace_read())
+        _cabi.trace_enable(False)
+        results.append((dict(zip(("out", "dx", "ddt", "dB", "dC", "dz"), (t[:few] for t in got))), ran))
+    return results
+
+
+def check(*case, **kw):
+    (alone, _), (among, _) = results = rows(*case, **kw)
+    for k in alone:
+        assert torch.equal(alone[k], among[k]), k
+    return [ran for _, ran in results]
+
+
+@pytest.mark.parametrize("case", [(torch.float16, 11, 916, 1, 128, 1, 128, 128, True), (torch.float32, 5, 175, 32, 32, 4, 16, 64, False),
+                                  (torch.bfloat16, 8, 600, 12, 32, 1, 32, 64, True)])
+def test_recurrence_with_chunks_in_flight(case):
+    """Few threads keep eight chunks' loads in flight, many one: the same sums."""
+    check(*case)
