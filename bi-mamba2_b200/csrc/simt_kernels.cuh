@@ -396,6 +396,18 @@ template <class T> __device__ __forceinline__ float4 ld4(const void *p, long lon
     return make_float4(to_f<T>(v[0]), to_f<T>(v[1]), to_f<T>(v[2]), to_f<T>(v[3]));
 }
 
+// The states a pass starts from and ends in are the caller's fp32 arrays, of any alignment; once per thread.
+__device__ __forceinline__ float4 load_state4(const float *p) {
+    return reinterpret_cast<uintptr_t>(p) % 16 == 0 ? *reinterpret_cast<const float4 *>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+__device__ __forceinline__ void store_state4(float *p, float4 v) {
+    if (reinterpret_cast<uintptr_t>(p) % 16 == 0) {
+        *reinterpret_cast<float4 *>(p) = v;
+    } else {
+        p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w;
+    }
+}
+
 // grid (b*H, ceil(P*N/4/blockDim), 2)
 template <class T, int U>
 __global__ void __launch_bounds__(TB) state_passing_fwd4(Dims d, const float *loc, const float *cs_f, const float *cs_b,
@@ -412,7 +424,7 @@ __global__ void __launch_bounds__(TB) state_passing_fwd4(Dims d, const float *lo
     const float *init = dir ? init_b : init_f;
     void *states = dir ? states_b : states_f;
     float *fin = dir ? final_b : final_f;
-    float4 run = init ? *reinterpret_cast<const float4 *>(init + (long long)(b * d.H + h) * PN + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 run = init ? load_state4(init + (long long)(b * d.H + h) * PN + e) : make_float4(0.f, 0.f, 0.f, 0.f);
     const long long cstride = (long long)d.H * PN;
     const long long off0 = ((long long)b * d.nc * d.H + h) * PN + e;
     const long long cb0 = (long long)(b * d.H + h) * d.nc * d.Q;
@@ -438,7 +450,7 @@ __global__ void __launch_bounds__(TB) state_passing_fwd4(Dims d, const float *lo
             run.w = fmaf(ed, run.w, v[u].w);
         }
     }
-    if (fin) *reinterpret_cast<float4 *>(fin + (long long)(b * d.H + h) * PN + e) = run;
+    if (fin) store_state4(fin + (long long)(b * d.H + h) * PN + e, run);
 }
 
 // grid (b*H, ceil(P*N/4/blockDim), 2), blockDim a multiple of 32; dTpart has one slot per warp of a (dir, b, h): gridDim.y *
@@ -462,7 +474,7 @@ __global__ void __launch_bounds__(TB) state_passing_bwd4(Dims d, const float *gl
     const float *dfin = dir ? dfinal_b : dfinal_f;
     float *dinit = dir ? dinit_b : dinit_f;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 run = (on && dfin) ? *reinterpret_cast<const float4 *>(dfin + (long long)(b * d.H + h) * PN + e) : zero;
+    float4 run = (on && dfin) ? load_state4(dfin + (long long)(b * d.H + h) * PN + e) : zero;
     const long long cstride = (long long)d.H * PN;
     const long long off0 = ((long long)b * d.nc * d.H + h) * PN + e;
     const float *total = (dir ? cs_b : cs_f + d.Q - 1) + (long long)(b * d.H + h) * d.nc * d.Q;      // T of chunk 0
@@ -504,7 +516,7 @@ __global__ void __launch_bounds__(TB) state_passing_bwd4(Dims d, const float *gl
         for (int u = 0; u < U; ++u)
             if ((threadIdx.x & 31) == 0 && i0 + u < d.nc) slots[(long long)(dir ? i0 + u : d.nc - 1 - i0 - u) * nslots] = part[u];
     }
-    if (on && dinit) *reinterpret_cast<float4 *>(dinit + (long long)(b * d.H + h) * PN + e) = run;
+    if (on && dinit) store_state4(dinit + (long long)(b * d.H + h) * PN + e, run);
 }
 
 // ---------------------------------------------------------------------------------------------------------
