@@ -87,8 +87,13 @@ static bool aligned16(const bissd_tensor &t) {
     return (reinterpret_cast<uintptr_t>(t.ptr) % 16 == 0) && t.stride_batch % 8 == 0 && t.stride_seq % 8 == 0 &&
            t.stride_head % 8 == 0;
 }
-static bool all_aligned16(const float *a, const float *b, const float *c) {
+static bool all_aligned16(const void *a, const void *b, const void *c) {
     return (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) % 16 == 0;
+}
+// states_f and states_b: 16-byte pieces, or four elements where the CUDA-core kernels take four at a time
+static bool states_aligned(const bissd_problem &p, bool tcp, const void *f, const void *b) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(f) | reinterpret_cast<uintptr_t>(b);
+    return at % (tcp || p.x_dtype == BISSD_F32 ? 16 : 8) == 0 || (!tcp && (long long)p.headdim * p.dstate % 4 != 0);
 }
 static bool force_simt() {
     static const bool v = [] { const char *e = getenv("BISSD_FORCE_SIMT"); return e && e[0] == '1'; }();
@@ -903,12 +908,13 @@ int bissd_forward(const bissd_fwd_args *a, void *workspace, size_t workspace_byt
     if (a->p.has_dt_bias && !a->dt_bias) return BISSD_ERR_NULL;
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) || workspace_bytes < fwd_layout(d).total)
         return BISSD_ERR_WORKSPACE;
+    const bool tcp = !force_simt() && tc_shape_ok(a->p) && aligned16(a->x) && aligned16(a->B) && aligned16(a->C) &&
+                     aligned16(a->z) && aligned16(a->out) && aligned16(a->out_x);
+    if (!states_aligned(a->p, tcp, a->states_f, a->states_b)) return BISSD_ERR_ALIGN;
     rc = check_device();
     if (rc != BISSD_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char *ws = static_cast<char *>(workspace);
-    const bool tcp = !force_simt() && tc_shape_ok(a->p) && aligned16(a->x) && aligned16(a->B) && aligned16(a->C) &&
-                     aligned16(a->z) && aligned16(a->out) && aligned16(a->out_x);
     if (!tcp) return simt_forward(*a, d, ws, s);
     return a->p.x_dtype == BISSD_BF16 ? forward_impl<__nv_bfloat16>(*a, d, ws, s) : forward_impl<__half>(*a, d, ws, s);
 }
@@ -1016,19 +1022,20 @@ int bissd_backward_into(const bissd_bwd_args *a, const bissd_grad_strides *gs, v
                      aligned16(a->z) && aligned16(a->dout) && aligned16(a->out_x);
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) || workspace_bytes < bwd_layout(d, tcp).total)
         return BISSD_ERR_WORKSPACE;
-    rc = check_device();
-    if (rc != BISSD_OK) return rc;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    char *ws = static_cast<char *>(workspace);
     const long long L = d.L, hp = (long long)d.H * d.P, gn = (long long)d.G * d.N;
     GradViews gr{MutView{a->dx, L * hp, hp, d.P}, MutView{a->dB, L * gn, gn, d.N}, MutView{a->dC, L * gn, gn, d.N},
                  MutView{a->ddt, L * d.H, d.H, 1}};
     if (gs) {
         auto set = [](MutView &v, const int64_t *st) { v.sb = st[0]; v.sl = st[1]; v.sh = st[2]; };
         set(gr.dx, gs->dx); set(gr.dB, gs->dB); set(gr.dC, gs->dC); set(gr.ddt, gs->ddt);
-        auto al = [](const MutView &v) { return reinterpret_cast<uintptr_t>(v.ptr) % 16 == 0 && v.sb % 8 == 0 && v.sl % 8 == 0 && v.sh % 8 == 0; };
-        if (tcp && !(al(gr.dx) && al(gr.dB) && al(gr.dC))) return BISSD_ERR_ALIGN;   // 16-byte stores
     }
+    auto al = [](const MutView &v) { return reinterpret_cast<uintptr_t>(v.ptr) % 16 == 0 && v.sb % 8 == 0 && v.sl % 8 == 0 && v.sh % 8 == 0; };
+    if (tcp && !(al(gr.dx) && al(gr.dB) && al(gr.dC) && all_aligned16(a->dz, a->dz, a->dz))) return BISSD_ERR_ALIGN;   // 16-byte stores
+    if (!states_aligned(a->p, tcp, a->states_f, a->states_b)) return BISSD_ERR_ALIGN;
+    rc = check_device();
+    if (rc != BISSD_OK) return rc;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    char *ws = static_cast<char *>(workspace);
     if (!tcp) return simt_backward(*a, gr, d, ws, s);
     return a->p.x_dtype == BISSD_BF16 ? backward_impl<__nv_bfloat16>(*a, gr, d, ws, s) : backward_impl<__half>(*a, gr, d, ws, s);
 }

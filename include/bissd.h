@@ -94,7 +94,8 @@ typedef struct bissd_fwd_args {
     /* saved for the backward pass, contiguous: */
     float *dt_out, *cs_f, *cs_b;          /* (batch, nheads, nchunks, chunk_size) fp32 */
     void *states_f, *states_b;            /* (batch, nchunks, nheads, headdim, dstate), x_dtype: state entering
-                                             each chunk from the left (f) / from the right (b) */
+                                             each chunk from the left (f) / from the right (b); 16-byte
+                                             aligned, else BISSD_ERR_ALIGN */
     float *final_f, *final_b;             /* (batch, nheads, headdim, dstate) fp32; may be NULL */
     const float *init_f, *init_b;         /* optional (batch, nheads, headdim, dstate) fp32 incoming states:
                                              init_f precedes token 0, init_b follows the last token */
@@ -113,7 +114,8 @@ typedef struct bissd_bwd_args {
     const float *A, *D, *dt_bias;
     const float *dt_out, *cs_f, *cs_b;    /* as written by the forward */
     const void *states_f, *states_b;      /* as written by the forward */
-    /* gradients, all contiguous in the layout of the tensor they belong to: */
+    /* gradients, all contiguous in the layout of the tensor they belong to (16-bit dx, dz, dB and dC of the
+     * tensor-core kernels 16-byte aligned, else BISSD_ERR_ALIGN): */
     void *dx, *dz;                        /* x_dtype; dz NULL unless p.has_z */
     void *dB, *dC;                        /* x_dtype */
     void *ddt;                            /* dt_dtype, (batch, seqlen, nheads) */

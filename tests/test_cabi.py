@@ -119,6 +119,41 @@ def test_forward_rejects_bad_arguments_before_any_launch(lib):
     assert b"NULL" in lib.bissd_strerror(-1)
 
 
+@pytest.mark.parametrize("x_dtype,headdim,dstate,off,refused", [
+    (1, 64, 128, 8, True), (0, 16, 20, 4, True), (0, 15, 17, 4, False), (2, 20, 6, 4, True), (2, 20, 6, 8, False)])
+def test_unaligned_states_and_gradients_are_refused_before_any_launch(lib, x_dtype, headdim, dstate, off, refused):
+    """The kernels move states and 16-bit gradients in pieces of several elements: addresses that would fault come back
+    as an error.  (What is accepted goes on to the device check, which fails here without a GPU.)"""
+    import torch
+    if torch.cuda.is_available():
+        pytest.skip("made-up addresses")
+    p = _problem(x_dtype=x_dtype, headdim=headdim, dstate=dstate, has_D=0, has_z=1)
+    t = lambda: _cabi.Tensor(4096, 128 * 4 * headdim * 8, 4 * headdim * 8, headdim * 8)
+    f, b = _cabi.FwdArgs(), _cabi.BwdArgs()
+    for a, names in ((f, ("x", "B", "C", "z", "out", "out_x")), (b, ("x", "B", "C", "z", "dout", "out_x"))):
+        a.p, a.phases, a.dt = p, 3, _cabi.Tensor(4096, 512, 4, 1)
+        for n in names:
+            setattr(a, n, t())
+        for n in ("A", "dt_out", "cs_f", "cs_b", "states_f", "states_b"):
+            setattr(a, n, 4096)
+    for n in ("dx", "dz", "dB", "dC", "ddt", "dA"):
+        setattr(b, n, 4096)
+    size = 1 << 40
+    fwd, bwd = (lambda: lib.bissd_forward(ctypes.byref(f), 4096, size, None)), (lambda: lib.bissd_backward(ctypes.byref(b), 4096, size, None))
+    ALIGN = -4
+    assert fwd() != ALIGN and bwd() != ALIGN
+    for field in ("states_f", "states_b"):
+        for a, call in ((f, fwd), (b, bwd)):
+            setattr(a, field, 4096 + off)
+            assert (call() == ALIGN) == refused, field
+            setattr(a, field, 4096)
+    if lib.bissd_kernel_path(ctypes.byref(p)) == b"tcgen05":
+        for field in ("dx", "dz", "dB", "dC"):
+            setattr(b, field, 4096 + off)
+            assert bwd() == ALIGN, field
+            setattr(b, field, 4096)
+
+
 def test_operator_refuses_cpu_tensors(lib):
     import torch
     from ssd.bi.ssd_combined import bimamba_chunk_scan_combined
