@@ -224,7 +224,7 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
                     } else {
                         const size_t smem_t = tc::state_tma_smem(d.P, d.Q);
                         BISSD_ALLOW((tc::state_gemm_tma<T, 0>), smem_t);
-                        BISSD_LAUNCH("tc_chunk_state_tma", tc::state_gemm_tma<T, 0><<<dim3(bch, 2, d.N / 128), tc::kThreads, smem_t, s>>>(
+                        BISSD_LAUNCH("tc_chunk_state_tma", tc::state_gemm_tma<T, 0><<<dim3(bch, 2, ceil_div(d.N, 128)), tc::kThreads, smem_t, s>>>(
                             d, mRow, mCol, a.dt_out, a.cs_f, a.cs_b, loc, status));
                     }
                     st_done = true;
@@ -399,7 +399,7 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
                     } else {
                         const size_t smem_t = tc::state_tma_smem(d.P, d.Q);
                         BISSD_ALLOW((tc::state_gemm_tma<T, 1>), smem_t);
-                        BISSD_LAUNCH("tc_dstates_tma", tc::state_gemm_tma<T, 1><<<dim3(bch, 2, d.N / 128), tc::kThreads, smem_t, s>>>(
+                        BISSD_LAUNCH("tc_dstates_tma", tc::state_gemm_tma<T, 1><<<dim3(bch, 2, ceil_div(d.N, 128)), tc::kThreads, smem_t, s>>>(
                             d, mRow, mCol, a.dt_out, a.cs_f, a.cs_b, F(w.gloc), status));
                     }
                     st_done = true;

@@ -5,7 +5,10 @@
 // Per CTA: one (batch, chunk, head), one direction, 128 state columns n.  Both operand tiles arrive by TMA with the
 // sequence index as their row (= K) index, i.e. as MN-major operands; the per-row factor is applied IN PLACE to the
 // smaller one (the [Q x headdim] x / g tile) by the threads, and one thread then issues the Q/16 MMAs.
-// Needs dstate % 128 == 0, headdim % 64 == 0, chunk in {128, 256}.
+// Needs dstate 64, 128 or 256, headdim 64 or 128, chunk in {128, 256}.  dstate 64 runs as half a 128-row tile: the TMA box of the
+// second 64 state columns lies outside the tensor and reads as zeros, the epilogue skips those rows.  These are the sizes
+// of the walk (tc_walk_tma.cuh), and every number is rounded where the walk rounds it: which of the two runs depends on
+// the batch, a row's results do not.
 #pragma once
 #include "tc_scan_tma.cuh"
 
@@ -27,11 +30,11 @@ template <> __device__ __forceinline__ uint4 scale8_packed<__nv_bfloat16>(uint4 
 }
 
 inline bool state_tma_ok(int P, int N, int Q) {
-    return P % 64 == 0 && P <= 128 && N % 128 == 0 && N <= 256 && (Q == 128 || Q == 256);
+    return (P == 64 || P == 128) && (N == 64 || (N % 128 == 0 && N <= 256)) && (Q == 128 || Q == 256);
 }
 inline size_t state_tma_smem(int P, int Q) { return 1024 + 2 * (size_t)Q * 128 + (size_t)(P / 64) * Q * 128 + Q * 4; }
 
-// grid (b*nc*H, 2, N/128)
+// grid (b*nc*H, 2, ceil(N/128))
 template <class T, int MODE>
 __global__ void __launch_bounds__(kThreads, 2)
 state_gemm_tma(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_constant__ CUtensorMap tmCol,
@@ -110,8 +113,9 @@ state_gemm_tma(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_c
         for (int c0 = (warp >> 2) * 32; c0 < P; c0 += 64) {
             float v[32];
             tmem_ld32(tmem_lane_base(tmem) + c0, v);
+            if (n < N)
 #pragma unroll
-            for (int j = 0; j < 32; ++j) o[(long long)(c0 + j) * N] = v[j];
+                for (int j = 0; j < 32; ++j) o[(long long)(c0 + j) * N] = v[j];
         }
     }
     tc_fence_before();
@@ -132,8 +136,6 @@ struct StateGrpShared {
     uint32_t tmem_base;
     int fail;
 };
-// dstate 64 runs as half a 128-row tile: the TMA box of the second 64 state columns lies outside the tensor and reads
-// as zeros, the epilogue skips those rows.
 inline bool state_grp_ok(int P, int N, int Q, int R) {
     return P == 64 && (N == 64 || (N % 128 == 0 && N <= 256)) && (Q == 128 || Q == 256) && R >= 2;
 }

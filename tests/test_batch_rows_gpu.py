@@ -39,3 +39,11 @@ def check(*case, **kw):
 def test_recurrence_with_chunks_in_flight(case):
     """Few threads keep eight chunks' loads in flight, many one: the same sums."""
     check(*case)
+
+
+@pytest.mark.parametrize("case", [(torch.bfloat16, 16, 1000, 4, 128, 2, 64, 128, True), (torch.float16, 16, 1024, 4, 128, 2, 64, 128, False),
+                                  (torch.bfloat16, 16, 2000, 4, 64, 4, 64, 256, False), (torch.bfloat16, 7, 517, 16, 128, 2, 64, 256, False)])
+def test_walk_and_two_kernels_dstate_64(case):
+    """Few rows: chunk states and the recurrence as two kernels; many: the walk.  The states round alike."""
+    few, many = check(*case)
+    assert "tc_chunk_state_tma" in few and "tc_state_walk" in many, (few, many)
