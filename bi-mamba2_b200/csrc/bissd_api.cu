@@ -424,8 +424,19 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
         const int rc = launch_walk<T, 1>(d, walk, wa, status, s);
         if (rc != BISSD_OK) return rc;
     } else if (need_pass) {
-        BISSD_LAUNCH("state_passing_bwd", launch_pdl(pass_ahead(d) ? simt::state_passing_bwd4<T, 8> : simt::state_passing_bwd4<T, 1>, pass_grid(d), pass_threads(d), 0, s,
-            d, F(w.gloc), a.states_f, a.states_b, a.cs_f, a.cs_b, a.dfinal_f, a.dfinal_b, nullptr, E16, F(w.dTpart), a.dinit_f, a.dinit_b));
+        auto launch = [&](auto wn) -> int {
+            constexpr int WN = decltype(wn)::value;
+            const auto kernel = pass_ahead(d) ? simt::state_passing_bwd4<T, 8, WN> : simt::state_passing_bwd4<T, 1, WN>;
+            BISSD_LAUNCH("state_passing_bwd", launch_pdl(kernel, pass_grid(d), pass_threads(d), 0, s,
+                d, F(w.gloc), a.states_f, a.states_b, a.cs_f, a.cs_b, a.dfinal_f, a.dfinal_b, nullptr, E16, F(w.dTpart), a.dinit_f, a.dinit_b));
+            return BISSD_OK;
+        };
+        int rc;
+        if (!tc::walk_ok(d.P, d.N, d.Q)) rc = launch(std::integral_constant<int, 0>());
+        else if (d.N == 64) rc = launch(std::integral_constant<int, 64>());
+        else if (d.N == 128) rc = launch(std::integral_constant<int, 128>());
+        else rc = launch(std::integral_constant<int, 256>());
+        if (rc != BISSD_OK) return rc;
     }
     if (!(a.phases & BISSD_PHASE_FINISH)) return BISSD_OK;
     int nlt = w.nlt, nsplit = 1, part_heads = d.H;
@@ -749,7 +760,7 @@ do {                                                                            
     cs.nf = F(w.nf); cs.nb = F(w.nb); cs.pf = F(w.pf); cs.pb = F(w.pb);
     if (use_u4) { cs.u4 = F(w.u4); cs.u4_tiles = u4_tiles; }
     else { cs.da_f = F(w.da_f); cs.da_b = F(w.da_b); }
-    cs.dTpart = F(w.dTpart); cs.nblk = walk.use ? tc::walk_slots(d) : pass_slots(d); cs.nsplit = nsplit; cs.ddt = gr.ddt; cs.dApart = F(w.dApart); cs.dbiaspart = F(w.dbiaspart);
+    cs.dTpart = F(w.dTpart); cs.nblk = w.nslots; cs.nsplit = nsplit; cs.ddt = gr.ddt; cs.dApart = F(w.dApart); cs.dbiaspart = F(w.dbiaspart);
     BISSD_LAUNCH("cumsum_bwd", launch_pdl(d.Q <= 128 ? tc::cumsum_bwd<1> : tc::cumsum_bwd<2>, tc::cumsum_blocks(d), 32 * tc::kCumsumWarps, 0, s,
         d, cs, all_aligned16(a.dt_out, a.dt_out, a.dt_out)));
     BISSD_LAUNCH("final_reduce", launch_pdl(simt::final_reduce<1024>, d.H, 1024, 0, s, 

@@ -96,7 +96,7 @@ template <class T> static int backward_t(const bissd_bwd_args &a, const GradView
     if (rc != BISSD_OK) return rc;
     if (local || a.dfinal_f || a.dfinal_b) {
         if (pass_by4(d)) {
-            BISSD_LAUNCH("state_passing_bwd", launch_pdl(pass_ahead(d) ? simt::state_passing_bwd4<T, 8> : simt::state_passing_bwd4<T, 1>, pass_grid(d), pass_threads(d), 0, s,
+            BISSD_LAUNCH("state_passing_bwd", launch_pdl(pass_ahead(d) ? simt::state_passing_bwd4<T, 8, 0> : simt::state_passing_bwd4<T, 1, 0>, pass_grid(d), pass_threads(d), 0, s,
                 d, F(w.gloc), a.states_f, a.states_b, a.cs_f, a.cs_b, a.dfinal_f, a.dfinal_b, F(w.E), nullptr, F(w.dTpart), a.dinit_f, a.dinit_b));
         } else {
             BISSD_LAUNCH("state_passing_bwd", simt::state_passing_bwd<T><<<dim3(d.b * d.H, ceil_div(d.P * d.N, simt::TB), 2), simt::TB, 0, s>>>(

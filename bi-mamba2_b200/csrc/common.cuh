@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "../../include/bissd.h"
 
 namespace bissd {
@@ -79,6 +81,24 @@ __device__ __forceinline__ void st_any(void *p, int dtype, long long i, float v)
 __device__ __forceinline__ float softplus_ref(float v) { return v <= 20.f ? log1pf(expf(v)) : v; }
 __device__ __forceinline__ float sigmoidf_(float v) { return 1.f / (1.f + expf(-v)); }
 
+// Sums over the warp of V values a lane, value(integral_constant<G>) the lane's G-th: lane l gets that of value l V / 32.  Each is
+// added up in the order of one shuffle per distance 16, 8 ... 1, but the values are dealt to the lanes on the way: V + 4 -
+// log2 V shuffles instead of 5 V, and no more than log2 V + 1 values held.
+template <int V, int S, int G, class F> __device__ __forceinline__ float dealt_sums(F &value, int lane) {
+    if constexpr (S == V) {
+        return value(std::integral_constant<int, G>());
+    } else {
+        const float a = dealt_sums<V, 2 * S, G>(value, lane), b = dealt_sums<V, 2 * S, G + S>(value, lane);
+        constexpr int o = 32 * S / V;
+        return ((lane & o) ? b : a) + __shfl_xor_sync(0xffffffffu, (lane & o) ? a : b, o);
+    }
+}
+template <int V, class F> __device__ __forceinline__ float warp_sums(F &value, int lane) {
+    float v = dealt_sums<V, 1, 0>(value, lane);
+#pragma unroll
+    for (int o = 16 / V; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
 
 // Programmatic dependent launch: a kernel launched with the stream-serialisation attribute may be scheduled while
 // the kernel before it in the stream is still draining.  Every such kernel opens with pdl_begin(): it lets its own

@@ -29,7 +29,7 @@ inline bool pass_ahead(const Dims &d) {
     const dim3 g = pass_grid(d);
     return (long long)g.x * g.y * g.z * pass_threads(d) < 256LL * sm_count();
 }
-inline int pass_slots(const Dims &d) {                           // partial dT per (direction, batch, head, chunk)
+inline int pass_slots(const Dims &d) {                           // partial dT per (direction, batch, head, chunk), the walk's included
     return pass_grid(d).y * (pass_by4(d) ? pass_threads(d) / 32 : 1);
 }
 
@@ -81,7 +81,6 @@ inline BwdWs bwd_layout(const Dims &d, bool tc) {
     const size_t st = (size_t)d.b * d.nc * d.H * d.P * d.N;
     const size_t hq = (size_t)d.b * d.H * d.nc * d.Q, qq = (size_t)d.b * d.nc * d.G * d.Q * d.Q;
     w.nslots = pass_slots(d);
-    if (tc) w.nslots = std::max(w.nslots, 8 * ceil_div(d.N, 128));   // tc::state_walk: one per warp
     w.nlt = ceil_div(d.Q, simt::TILE);
     w.nsplit = tc ? ceil_div(d.N, 128) : 1;
     w.hsplit = tc ? 1 : simt_hsplit(d);

@@ -396,6 +396,15 @@ template <class T> __device__ __forceinline__ float4 ld4(const void *p, long lon
     return make_float4(to_f<T>(v[0]), to_f<T>(v[1]), to_f<T>(v[2]), to_f<T>(v[3]));
 }
 
+template <class T> __device__ __forceinline__ void st2(void *p, long long i, float a, float b) {   // 16-bit T
+    T v[2] = {from_f<T>(a), from_f<T>(b)};
+    *reinterpret_cast<uint32_t *>(static_cast<T *>(p) + i) = *reinterpret_cast<uint32_t *>(v);
+}
+template <class T> __device__ __forceinline__ float2 ld2(const void *p, long long i) {
+    const uint32_t u = *reinterpret_cast<const uint32_t *>(static_cast<const T *>(p) + i);
+    const T *v = reinterpret_cast<const T *>(&u);
+    return make_float2(to_f<T>(v[0]), to_f<T>(v[1]));
+}
 // The states a pass starts from and ends in are the caller's fp32 arrays, of any alignment; once per thread.
 __device__ __forceinline__ float4 load_state4(const float *p) {
     return reinterpret_cast<uintptr_t>(p) % 16 == 0 ? *reinterpret_cast<const float4 *>(p) : make_float4(p[0], p[1], p[2], p[3]);
@@ -455,26 +464,40 @@ __global__ void __launch_bounds__(TB) state_passing_fwd4(Dims d, const float *lo
 
 // grid (b*H, ceil(P*N/4/blockDim), 2), blockDim a multiple of 32; dTpart has one slot per warp of a (dir, b, h): gridDim.y *
 // blockDim / 32 - one per warp instead of one per block keeps barriers out of the loop (b8 H24 nc8 P64 N128 bf16: 43 -> 39
-// us).  U: chunks whose loads are in flight together, see pass_ahead().
-template <class T, int U>
+// us).  U: chunks whose loads are in flight together, see pass_ahead(); with few threads the instructions of a group of
+// chunks are most of the time, so its U sums share their shuffles (b1 L8192 H8 P64 N128 chunk 256: 16.7 -> 14 us).
+// WN (dstate, at the sizes of tc::state_walk, 16-bit states; else 0): a thread has the elements, and a slot the sum, that tc::state_walk gives a
+// lane and a slot - four columns of 32 n, a lane two adjacent n of two columns - and everything is added up in its order.
+// Which of the two runs depends on the batch; dT, and through it ddt and dA, does not.  (dstate is a constant so that the
+// distance to a thread's second column is part of the instructions.)
+template <class T, int U, int WN>
 __global__ void __launch_bounds__(TB) state_passing_bwd4(Dims d, const float *gloc, const void *states_f,
                                                          const void *states_b, const float *cs_f, const float *cs_b,
                                                          const float *dfinal_f, const float *dfinal_b, float *E,
                                                          void *E16, float *dTpart, float *dinit_f, float *dinit_b) {
     pdl_begin();
     const int h = blockIdx.x % d.H, b = blockIdx.x / d.H;
-    const int dir = blockIdx.z;
+    const int dir = blockIdx.z, lane = threadIdx.x & 31;
     const int PN = d.P * d.N;
     const int nslots = gridDim.y * (blockDim.x >> 5), slot = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int e = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
-    const bool on = e < PN;
+    int e = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    constexpr int gap = WN ? 2 * WN : 2;                         // from the first two elements to the others
+    if (WN) {
+        constexpr bool half = WN == 64;                          // both halves of the 128-row tile are the same 64 n
+        const int cols = half ? d.P / 4 : d.P / 2, V = cols / 4, ew = slot / V % 8, quad = ew & 3;
+        const int col = (half ? (quad >> 1) * 2 + (ew >> 2) : ew >> 2) * cols + slot % V * 4 + (lane & 1);
+        e = col * WN + slot / (8 * V) * 128 + (half ? quad & 1 : quad) * 32 + (lane & ~1);
+    }
+    const bool on = WN || e < PN;
     const long long per_dir = (long long)d.b * d.nc * d.H * PN;
     const float *gp = gloc + dir * per_dir;
     const void *states = dir ? states_b : states_f;
     const float *dfin = dir ? dfinal_b : dfinal_f;
     float *dinit = dir ? dinit_b : dinit_f;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 run = (on && dfin) ? load_state4(dfin + (long long)(b * d.H + h) * PN + e) : zero;
+    const long long bh0 = (long long)(b * d.H + h) * PN + e;
+    float4 run = zero;
+    if (on && dfin) run = WN ? make_float4(dfin[bh0], dfin[bh0 + 1], dfin[bh0 + gap], dfin[bh0 + gap + 1]) : load_state4(dfin + bh0);
     const long long cstride = (long long)d.H * PN;
     const long long off0 = ((long long)b * d.nc * d.H + h) * PN + e;
     const float *total = (dir ? cs_b : cs_f + d.Q - 1) + (long long)(b * d.H + h) * d.nc * d.Q;      // T of chunk 0
@@ -484,6 +507,16 @@ __global__ void __launch_bounds__(TB) state_passing_bwd4(Dims d, const float *gl
         float dec[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
+            if (WN) {                                            // past the last chunk: its values again, not used
+                const int k = min(i0 + u, d.nc - 1), c = dir ? k : d.nc - 1 - k;
+                const long long off = off0 + c * cstride;
+                const float2 lo = __ldg(reinterpret_cast<const float2 *>(gp + off)), hi = __ldg(reinterpret_cast<const float2 *>(gp + off + gap));
+                const float2 s0 = ld2<T>(states, off), s1 = ld2<T>(states, off + gap);
+                gv[u] = make_float4(lo.x, lo.y, hi.x, hi.y);
+                sv[u] = make_float4(s0.x, s0.y, s1.x, s1.y);
+                dec[u] = total[(long long)c * d.Q];
+                continue;
+            }
             const int c = dir ? i0 + u : d.nc - 1 - i0 - u;
             const bool have = on && i0 + u < d.nc;
             gv[u] = have ? __ldg(reinterpret_cast<const float4 *>(gp + off0 + c * cstride)) : zero;
@@ -495,28 +528,42 @@ __global__ void __launch_bounds__(TB) state_passing_bwd4(Dims d, const float *gl
         for (int u = 0; u < U; ++u) {
             const int c = dir ? i0 + u : d.nc - 1 - i0 - u;
             const long long off = off0 + c * cstride;
-            const float ed = expf(dec[u]);
-            part[u] = ed * fmaf(sv[u].x, run.x, fmaf(sv[u].y, run.y, fmaf(sv[u].z, run.z, sv[u].w * run.w)));   // one order, whatever U
+            dec[u] = expf(dec[u]);
+            // the order is written out: the same whatever U
+            if (WN) part[u] = fmaf(sv[u].z, run.z, fmaf(sv[u].w, run.w, fmaf(sv[u].x, run.x, fmaf(sv[u].y, run.y, 0.f))));
+            else part[u] = fmaf(sv[u].x, run.x, fmaf(sv[u].y, run.y, fmaf(sv[u].z, run.z, sv[u].w * run.w)));
             if (i0 + u < d.nc) {
                 if (on) {
-                    if (E) *reinterpret_cast<float4 *>(E + dir * per_dir + off) = run;
-                    if (E16) st4<T>(E16, dir * per_dir + off, run.x, run.y, run.z, run.w);
+                    if (WN) {
+                        st2<T>(E16, dir * per_dir + off, run.x, run.y);
+                        st2<T>(E16, dir * per_dir + off + gap, run.z, run.w);
+                    } else {
+                        if (E) *reinterpret_cast<float4 *>(E + dir * per_dir + off) = run;
+                        if (E16) st4<T>(E16, dir * per_dir + off, run.x, run.y, run.z, run.w);
+                    }
                 }
-                run.x = fmaf(ed, run.x, gv[u].x);
-                run.y = fmaf(ed, run.y, gv[u].y);
-                run.z = fmaf(ed, run.z, gv[u].z);
-                run.w = fmaf(ed, run.w, gv[u].w);
+                run.x = fmaf(dec[u], run.x, gv[u].x);
+                run.y = fmaf(dec[u], run.y, gv[u].y);
+                run.z = fmaf(dec[u], run.z, gv[u].z);
+                run.w = fmaf(dec[u], run.w, gv[u].w);
             }
         }
+        // lane 32 u / U writes chunk u's sum, times its decay
+        auto value = [&](auto k) -> float { return part[decltype(k)::value]; };
+        const float sum = warp_sums<U>(value, lane);
+        float ed = dec[0];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int u = 0; u < U; ++u) part[u] += __shfl_xor_sync(0xffffffffu, part[u], o);
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if ((threadIdx.x & 31) == 0 && i0 + u < d.nc) slots[(long long)(dir ? i0 + u : d.nc - 1 - i0 - u) * nslots] = part[u];
+        for (int u = 1; u < U; ++u) ed = lane == 32 / U * u ? dec[u] : ed;
+        const int i = i0 + lane * U / 32;
+        if (lane % (32 / U) == 0 && i < d.nc) slots[(long long)(dir ? i : d.nc - 1 - i) * nslots] = ed * sum;
     }
-    if (on && dinit) store_state4(dinit + (long long)(b * d.H + h) * PN + e, run);
+    if (on && dinit) {
+        if (WN) {
+            dinit[bh0] = run.x; dinit[bh0 + 1] = run.y; dinit[bh0 + gap] = run.z; dinit[bh0 + gap + 1] = run.w;
+        } else {
+            store_state4(dinit + bh0, run);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------------------------------------

@@ -163,9 +163,19 @@ cumsum_bwd(Dims d, simt::CumsumBwd a, int wide) {
 #pragma unroll
     for (int j = 0; j < E; ++j) v1[j] = v2[j] = w1[j] = w2[j] = ex[j] = dto[j] = dlo[j] = pre[j] = 0.f;
     float ts = 0.f, te = 0.f;                                          // dT_b, dT_f
-    for (int k = lane; k < a.nblk; k += 32) {
-        te += a.dTpart[tix * a.nblk + k];
-        ts += a.dTpart[((long long)d.b * d.H * d.nc + tix) * a.nblk + k];
+    for (int k0 = lane; k0 < a.nblk; k0 += 256) {                      // 16 loads in flight: dstate 256 of headdim 128 brings 256 partial values
+        float pe[8], ps[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = k0 + 32 * j;
+            pe[j] = k < a.nblk ? a.dTpart[tix * a.nblk + k] : 0.f;
+            ps[j] = k < a.nblk ? a.dTpart[((long long)d.b * d.H * d.nc + tix) * a.nblk + k] : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            te += pe[j];
+            ts += ps[j];
+        }
     }
     if (l0 < d.Q) {
         load_strided(a.dt, a.dt_dtype, b * a.dsb + (long long)(c * d.Q + l0) * a.dsl + h * a.dsh, a.dsl, lim - l0, pre);

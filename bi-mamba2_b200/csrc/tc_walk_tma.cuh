@@ -32,7 +32,6 @@ inline size_t walk_smem(int P, int mode) {
     return 1024 + (size_t)walk_ring(P / 64, mode) * walk_stage_bytes(P / 64) + (mode ? 2 * (size_t)P * 256 : 0);
 }
 inline int walk_tiles(const Dims &d) { return d.N == 64 ? 1 : d.N / 128; }
-inline int walk_slots(const Dims &d) { return 8 * walk_tiles(d); }  // partial dT per (direction, batch, head, chunk): one per warp
 
 struct WalkShared {
     uint64_t full[6], scaled[6], empty[6], acc[2], acc_free[2], s_full[2], s_free[2];
@@ -203,28 +202,30 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
             }
             // Neighbouring lanes swap one of two columns, so that each has two adjacent n of one column: half as many
             // stores (and reads of the entering states), of twice the width.
-            float part = 0.f;
             T *o = out + c * cstride;
             const uint8_t *sp = smS + (i & 1) * P * 256 + (n >> 6) * P * 128 + (n & 6) * 2;
-#pragma unroll
-            for (int j = 0; j < NC; j += 2) {
+            auto put = [&](int j, float part) -> float {        // columns j and j + 1; part + their share of <S, run>
                 const float got = __shfl_xor_sync(0xffffffffu, odd ? run[j] : run[j + 1], 1);
                 const float lo = odd ? got : run[j], hi = odd ? run[j + 1] : got;   // column j + odd, at n & ~1 and n | 1
                 *reinterpret_cast<uint32_t *>(o + (long long)j * N) = pack2<T>(lo, hi);
-                if (MODE == 1) {
-                    const int p = col0 + j + odd;
-                    float s0, s1;
-                    unpack2<T>(*reinterpret_cast<const uint32_t *>(sp + p * 128 + ((((n & 63) >> 3) ^ (p & 7)) << 4)), s0, s1);
-                    part = fmaf(s0, lo, fmaf(s1, hi, part));
-                }
-            }
-            if (MODE == 1) {
+                if (MODE == 0) return 0.f;
+                const int p = col0 + j + odd;
+                float s0, s1;
+                unpack2<T>(*reinterpret_cast<const uint32_t *>(sp + p * 128 + ((((n & 63) >> 3) ^ (p & 7)) << 4)), s0, s1);
+                return fmaf(s0, lo, fmaf(s1, hi, part));
+            };
+            if constexpr (MODE == 0) {
 #pragma unroll
-                for (int o2 = 16; o2 > 0; o2 >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o2);
-                if (lane == 0) {
-                    mbar_arrive(&sh.s_free[i & 1]);
+                for (int j = 0; j < NC; j += 2) put(j, 0.f);
+            } else {
+                // A partial dT per four columns and 32 n: a warp's worth of simt::state_passing_bwd4, in its order
+                constexpr int V = NC / 4;
+                auto four = [&](auto k) -> float { return put(4 * decltype(k)::value + 2, put(4 * decltype(k)::value, 0.f)); };
+                const float part = warp_sums<V>(four, lane);
+                if (lane == 0) mbar_arrive(&sh.s_free[i & 1]);
+                if (lane % (32 / V) == 0) {
                     const long long hc = ((long long)dir * d.b * d.H + (long long)b * d.H + h) * nc + c;
-                    a.dTpart[hc * (8 * tiles) + tile * 8 + ew] = e * part;
+                    a.dTpart[(hc * tiles + tile) * (8 * V) + ew * V + lane * V / 32] = e * part;
                 }
             }
             ok = ws_wait_warp(&sh.acc[i & 1], (i >> 1) & 1, fail, 78);

@@ -47,3 +47,34 @@ def test_walk_and_two_kernels_dstate_64(case):
     """Few rows: chunk states and the recurrence as two kernels; many: the walk.  The states round alike."""
     few, many = check(*case)
     assert "tc_chunk_state_tma" in few and "tc_state_walk" in many, (few, many)
+
+
+@pytest.mark.parametrize("case", [(torch.bfloat16, 4, 8192, 8, 64, 1, 128, 256, False), (torch.bfloat16, 64, 1000, 4, 64, 2, 64, 128, True),
+                                  (torch.float16, 14, 822, 4, 64, 4, 256, 128, True), (torch.bfloat16, 11, 842, 12, 128, 4, 128, 128, False),
+                                  (torch.float16, 16, 1000, 4, 128, 2, 256, 128, True), (torch.bfloat16, 20, 585, 6, 128, 2, 64, 128, True)])
+def test_walk_and_two_kernels(case):
+    """The sums over a chunk's states that enter ddt are added up in one order, whichever computes them."""
+    few, many = check(*case)
+    assert "state_passing_bwd" in few and "tc_dstate_walk" in many, (few, many)
+
+
+@pytest.mark.parametrize("P,N", [(64, 64), (64, 128), (64, 256), (128, 64), (128, 128), (128, 256)])
+def test_one_pass_and_two_phases(P, N):
+    """A whole backward pass walks; one in phases, as the sequence-sharded operator runs it, keeps its local gradients."""
+    from ssd.bi import sequence_parallel as sp
+    from ssd.bi.ssd_combined import bimamba_chunk_scan_combined
+    b, L, H, G, Q = 4, 700, 24, 2, 128
+    g = torch.Generator(device="cuda").manual_seed(P + N)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, B, C, dout = (t.bfloat16() for t in (mk(b, L, H, P), mk(b, L, G, N), mk(b, L, G, N), mk(b, L, H, P)))
+    leaves = [t.requires_grad_(True) for t in (x, mk(b, L, H) - 4.0, -torch.rand(H, generator=g, device="cuda") - 0.1, B, C)]
+    out = bimamba_chunk_scan_combined(*leaves, Q, dt_softplus=True)
+    want = [out, *torch.autograd.grad(out, leaves, dout)]
+    zero = torch.zeros(b, H, P, N, device="cuda")
+    for boundary in (None, zero):                            # nothing enters the shard
+        st = sp.local_forward(*(t.detach() for t in leaves), Q, dt_softplus=True)
+        got = [sp.finish_forward(st, boundary, boundary)]
+        sp.local_backward(st, dout)
+        got += sp.finish_backward(st, boundary, boundary)[:5]
+        for a, w, name in zip(got, want, ("out", "dx", "ddt", "dA", "dB", "dC")):
+            assert torch.equal(a, w), name
