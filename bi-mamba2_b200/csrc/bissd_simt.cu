@@ -111,7 +111,7 @@ template <class T> static int backward_t(const bissd_bwd_args &a, const GradView
     ba.dx = gr.dx; ba.dB = gr.dB; ba.dC = gr.dC; ba.dz = a.dz;
     ba.ddt_out = F(w.ddt_out); ba.dDpart = F(w.dDpart); ba.dB_part = F(w.dB_part); ba.dC_part = F(w.dC_part);
     ba.nf = F(w.nf); ba.nb = F(w.nb); ba.pf = F(w.pf); ba.pb = F(w.pb); ba.dCB = F(w.dCB); ba.u = F(w.u4);
-    ba.hsplit = w.hsplit;
+    ba.hsplit = w.hsplit; ba.parts = simt_parts(d);
     const int nt = w.nlt, bch = d.b * d.nc * d.H, bcg = d.b * d.nc * d.G;
     const int dcb = bcg * w.hsplit * nt * nt, dx = bch * nt, dbc = bch * nt * 2;
     const int twp = tile_width<T>(d.P), twn = tile_width<T>(d.N);

@@ -44,16 +44,27 @@ inline FwdWs fwd_layout(const Dims &d) {
     return w;
 }
 
-// Blocks the heads of a group are dealt to in the CUDA-core dCB product, each with a partial dCB of its own: one, unless
-// the problem has too few (batch, chunk, group, tile)s for two blocks an SM; a divisor of the heads per group.
-inline int simt_hsplit(const Dims &d) {
+// CUDA-core dCB product: are there blocks enough with one for all heads of a group?  Other blocks of the launch fill the SMs
+// beside them, so four for five SMs do (us a pass, two blocks an SM asked for and this: b4 L1000 H8 P32 N32 chunk 128,
+// 128 blocks, 167, 160; b2 L4000 H4 P64 N64, 256 blocks, 297, 290; b1 L8000 H8 chunk 64, 125 blocks, 267, 260).
+inline bool simt_dcb_fills(const Dims &d, int rows) {
     const int nt = ceil_div(d.Q, simt::TILE);
-    const long long blocks = (long long)d.b * d.nc * d.G * nt * nt;
-    int hs = 1;
-    for (int k = 2; k <= d.R && blocks * hs < 2LL * sm_count(); ++k)
-        if (d.R % k == 0) hs = k;
-    return hs;
+    return 5LL * rows * d.nc * d.G * nt * nt >= 4LL * sm_count();
 }
+// Parts the heads of a group are summed in: by one row of the batch, so that a row's results do not depend on how many rows
+// there are.  A divisor of the heads; enough for two blocks an SM where a row alone does not fill them.
+inline int simt_parts(const Dims &d) {
+    if (simt_dcb_fills(d, 1)) return 1;
+    const int nt = ceil_div(d.Q, simt::TILE);
+    const long long blocks = (long long)d.nc * d.G * nt * nt;
+    int parts = 1;
+    for (int k = 2; k <= d.R && blocks * parts < 2LL * sm_count(); ++k)
+        if (d.R % k == 0) parts = k;
+    return parts;
+}
+// Blocks that share the parts, each with a partial dCB of its own that the last product adds to the others: one a part, or
+// one for all of them where the rows fill the SMs.
+inline int simt_hsplit(const Dims &d) { return simt_dcb_fills(d, d.b) ? 1 : simt_parts(d); }
 
 // Blocks the heads of a group are dealt to in dbc_accum_grp (one block an SM, about 2 us a head), each writing a partial
 // dB / dC that the last product adds up again: more than one only where the blocks leave SMs idle.

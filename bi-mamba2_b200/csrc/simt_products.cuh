@@ -308,7 +308,7 @@ struct BwdArgs {
     MutView dx, dB, dC;
     void *dz;
     float *ddt_out, *dDpart, *dB_part, *dC_part, *nf, *nb, *pf, *pb, *dCB, *u;
-    int hsplit;                                                  // blocks the heads of a group are dealt to in dcb_intra
+    int hsplit, parts;                                           // blocks the heads of a group are dealt to in dcb_role, parts they are summed in
 };
 
 // dx, ddt_out, dz and per-block dD partials.
@@ -508,19 +508,29 @@ template <class T, int TW> __device__ __forceinline__ void dbc_role(Panels &sm, 
 //   u = (column sums - row sums) of W, which cumsum_bwd takes: u[t] for t < ceil(Q/64) holds the column sums over row
 //   tile t, the rest minus the row sums over column tile t - ceil(Q/64), forward and reverse in turn.
 // Takes over _chunk_scan_bwd_dcb_kernel (src/ssd/bi/ssd_chunk_scan.py:776-859) and the "stable" decay kernels
-// (:1361-1446, :1078-1157).  dCB: [b,c,g][hsplit][Q][Q], summed by bmm_bwd.  Blocks: b nc G hsplit ceil(Q/64)^2.
+// (:1361-1446, :1078-1157).  dCB: [b,c,g][hsplit][Q][Q], summed by bmm_bwd; a block with several
+// parts adds them up in the same order.  Blocks: b nc G hsplit ceil(Q/64)^2.
 template <class T> __device__ __forceinline__ void dcb_role(Panels &sm, const Dims &d, const BwdArgs &a, int vec, int block) {
     const int nt = ceil_div(d.Q, TILE), tile = block % (nt * nt), part = block / (nt * nt) % a.hsplit, bcg = block / (nt * nt) / a.hsplit;
     const int g = bcg % d.G, c = (bcg / d.G) % d.nc, b = bcg / (d.G * d.nc), lim = min(d.Q, d.L - c * d.Q);
     const int lt = tile / nt, st = tile % nt, l0 = lt * TILE, s0 = st * TILE, heads = d.R / a.hsplit, shP = shift_for(d.P);
+    const int per = d.R / a.parts;                               // heads a part
     const int lr = l0 + Acc<64>::row0(), sc = s0 + Acc<64>::col0(), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long stride = (long long)d.b * d.H * d.nc * d.Q;
-    float tot[4][4];
+    float tot[4][4], before[4][4];                               // the part's sums, and those of the block's parts before it
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) tot[i][j] = 0.f;
+        for (int j = 0; j < 4; ++j) tot[i][j] = before[i][j] = 0.f;
     for (int r = 0; r < heads; ++r) {
+        if (r > 0 && r % per == 0)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    before[i][j] += tot[i][j];
+                    tot[i][j] = 0.f;
+                }
         Where w(d, (b * d.nc + c) * d.H + g * d.R + part * heads + r);
         __syncthreads();                                         // the vectors' and sums' last readers are done
         const Vectors vec4 = load_vectors(sm, d, w, a.dt_out, a.cs_f, a.cs_b);
@@ -614,7 +624,8 @@ template <class T> __device__ __forceinline__ void dcb_role(Panels &sm, const Di
 #pragma unroll
     for (int i = 0; i < 4; ++i)
         if (lr + i < d.Q)
-            store4<float>(out + (long long)(lr + i) * d.Q + sc, d.Q - sc, vec & VEC_Q, make_float4(tot[i][0], tot[i][1], tot[i][2], tot[i][3]));
+            store4<float>(out + (long long)(lr + i) * d.Q + sc, d.Q - sc, vec & VEC_Q,
+                          make_float4(before[i][0] + tot[i][0], before[i][1] + tot[i][1], before[i][2] + tot[i][2], before[i][3] + tot[i][3]));
 }
 
 // dB[s,n] = sum_l dCB[l,s] C[l,n] + sum_{h in g} dB_part[s,h,n];  dC[l,n] = sum_s dCB[l,s] B[s,n] + sum_h dC_part.

@@ -58,6 +58,14 @@ def test_walk_and_two_kernels(case):
     assert "state_passing_bwd" in few and "tc_dstate_walk" in many, (few, many)
 
 
+@pytest.mark.parametrize("case,few", [((torch.float32, 8, 1000, 8, 32, 1, 32, 128, True), 1), ((torch.float32, 6, 700, 8, 64, 2, 64, 128, False), 1),
+                                      ((torch.float32, 30, 294, 12, 16, 1, 16, 64, True), 5), ((torch.float32, 9, 242, 48, 64, 4, 64, 64, True), 1),
+                                      ((torch.float32, 9, 222, 9, 16, 1, 17, 66, False), 2), ((torch.bfloat16, 40, 200, 6, 20, 1, 12, 40, False), 1)])
+def test_cuda_core_heads_in_parts(case, few):
+    """Heads of a group dealt to several blocks, or all to one: dCB is summed in the same parts."""
+    check(*case, few=few)
+
+
 @pytest.mark.parametrize("P,N", [(64, 64), (64, 128), (64, 256), (128, 64), (128, 128), (128, 256)])
 def test_one_pass_and_two_phases(P, N):
     """A whole backward pass walks; one in phases, as the sequence-sharded operator runs it, keeps its local gradients."""
