@@ -144,11 +144,24 @@ static bool walk_pays(const Dims &d) {
     const double apart = 8.0 + 2.5e-6 * 2.0 * d.b * d.nc * d.H * d.P * d.N;
     return walk < apart;
 }
+static bool walk_wanted(const Dims &d) { return !no_tma() && !no_ws() && tc::walk_ok(d.P, d.N, d.Q) && walk_pays(d); }
+
+// What the sizes alone say of the tensor-core family's kernels, and so which arrays of the workspace a pass does without.
+// Operands that no tensor map describes are found out later: such a pass takes other kernels, and needs them all.
+static bool ws_wanted(const Dims &d) { return !no_tma() && !no_ws() && tc::scan_ws_ok(d.P, d.N, d.Q); }
+static bool fused_wanted(const Dims &d) {                        // tc::intra_dcb_tile, on the bf16 C.B^T tile only
+    return ws_wanted(d) && !no_sums() && !no_fused() && tc::scan_tma_ok(d.P, d.N, d.Q) && tc::bmm_cb_tma_ok(d.N, d.Q) && tc::intra_tile_ok(d.P, d.Q);
+}
+static bool last_wanted(const Dims &d) {                         // dbc_accum_grp finishes dB and dC
+    return fused_wanted(d) && head_parts(d) == 1 && tc::bmm_bwd_tma_ok(d.N, d.Q) && tc::dbc_grp_ok(d.P, d.N, d.Q);
+}
+static FwdWs least_fwd(const Dims &d) { return fwd_layout(d, FwdNeed{!walk_wanted(d), !ws_wanted(d), ws_wanted(d)}); }
+static BwdWs least_bwd(const Dims &d) { return bwd_layout(d, true, BwdNeed{!walk_wanted(d), !last_wanted(d), !fused_wanted(d)}); }
+
 static Walk plan_walk(const Dims &d, int dtype, const bissd_tensor &row, const View &col, const float *dt_out,
                       const float *cs_f, const float *cs_b, const void *states_f, const void *states_b) {
     Walk w;
-    if (no_tma() || no_ws() || !tc::walk_ok(d.P, d.N, d.Q) || !walk_pays(d)) return w;
-    if (!all_aligned16(dt_out, cs_f, cs_b)) return w;
+    if (!walk_wanted(d) || !all_aligned16(dt_out, cs_f, cs_b)) return w;
     const unsigned rows = tc::walk_rows(d.P / 64);
     const unsigned long long srows = (unsigned long long)d.b * d.nc * d.H * d.P;
     w.use = map_bshd(&w.mRow, dtype, row.ptr, row.stride_batch, row.stride_seq, row.stride_head, d.N, d.G, d.L, d.b, rows) &&
@@ -170,8 +183,9 @@ static int launch_walk(const Dims &d, const Walk &w, const tc::WalkArgs &args, i
 }
 
 template <class T>
-static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaStream_t s) {
-    const FwdWs w = fwd_layout(d);
+static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, size_t ws_bytes, cudaStream_t s) {
+    const bool lean = ws_bytes < fwd_layout(d).total;            // no room for what least_fwd leaves out
+    const FwdWs w = lean ? least_fwd(d) : fwd_layout(d);
     int *status = reinterpret_cast<int *>(ws);
     float *loc = reinterpret_cast<float *>(ws + w.loc);
     float *CB = reinterpret_cast<float *>(ws + w.cb);
@@ -180,11 +194,12 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, cudaSt
     const int ntP = tc::round_up(d.P, 16), ntQ = tc::round_up(d.Q, 16);
     // (a FINISH phase with entering states walks again, from the inputs: the decision is the same in both phases)
     const Walk walk = plan_walk(d, a.p.x_dtype, a.B, x, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
+    if (lean && walk_wanted(d) && !walk.use) return BISSD_ERR_WORKSPACE;
     const tc::CumsumFwd cs{a.dt.ptr, a.p.dt_dtype, a.dt.stride_batch, a.dt.stride_seq, a.dt.stride_head, a.A, a.dt_bias, a.dt_out, a.cs_f, a.cs_b,
                            all_aligned16(a.dt_out, a.cs_f, a.cs_b)};
     // C.B^T by TMA: a bf16 copy for the persistent scan, fp32 for the others; in one launch with the cumulative sums where
     // all blocks are resident at once (b1 L384 H8: 20.5 us a forward call with two launches and a memset for the status word)
-    const bool ws_path = !no_tma() && !no_ws() && tc::scan_ws_ok(d.P, d.N, d.Q);
+    const bool ws_path = ws_wanted(d);
     __nv_bfloat16 *CB16 = reinterpret_cast<__nv_bfloat16 *>(ws + w.cb16);
     CUtensorMap mCc, mBc, mCBo;
     const bool cb_tma = !no_tma() && tc::bmm_cb_tma_ok(d.N, d.Q) && make_cb_maps(a, d, &mCc, &mBc) && (!ws_path || make_tile_map(d, CB16, &mCBo));
@@ -314,6 +329,7 @@ do {                                                                            
 #undef BISSD_SCAN_WS
                     tma_done = true;
                 } else {                                     // maps refused: produce the fp32 tile after all
+                    if (lean) return BISSD_ERR_WORKSPACE;
                     BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, ceil_div(d.Q, tc::kTileM)), tc::kThreads, smem_cb, s>>>(
                         d, Cm, Bm, CB, nullptr, nullptr, nullptr, nullptr, status));
                 }
@@ -353,8 +369,9 @@ do {                                                                            
 }
 
 template <class T>
-static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dims &d, char *ws, cudaStream_t s) {
-    const BwdWs w = bwd_layout(d, true);
+static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dims &d, char *ws, size_t ws_bytes, cudaStream_t s) {
+    const bool lean = ws_bytes < bwd_layout(d, true).total;      // no room for what least_bwd leaves out
+    const BwdWs w = lean ? least_bwd(d) : bwd_layout(d, true);
     int *status = reinterpret_cast<int *>(ws);
     auto F = [&](size_t off) { return reinterpret_cast<float *>(ws + off); };
     const View x = view_of(a.x), Bm = view_of(a.B), Cm = view_of(a.C), z = view_of(a.z), dout = view_of(a.dout),
@@ -373,6 +390,7 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
     }
     Walk walk;                                                   // whole passes only: a split one keeps its local gradients
     if (a.phases == BISSD_PHASE_ALL) walk = plan_walk(d, a.p.x_dtype, a.C, gv, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
+    if (lean && walk_wanted(d) && !walk.use) return BISSD_ERR_WORKSPACE;
     if (a.phases & BISSD_PHASE_LOCAL) {
         if (!d.has_z && !walk.use) {                             // else the gate kernel or the walk, whichever is first, clears the status word
             const int rc = note_cuda(cudaMemsetAsync(ws, 0, kWsHeader, s), "cudaMemsetAsync");
@@ -462,7 +480,7 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
         part_heads = d.G;
         const size_t smem_cb = tc::smem_bytes(ntQ, 0), smem_dx = tc::smem_bytes(ntP, 3 * d.Q), smem_n = tc::smem_bytes(ntN, 0);
         BISSD_ALLOW(tc::bmm_cb<T>, smem_cb);
-        const bool ws_path = !no_tma() && !no_ws() && tc::scan_ws_ok(d.P, d.N, d.Q);
+        const bool ws_path = ws_wanted(d);
         const bool sums_path = !no_tma() && !no_sums() && tc::scan_tma_ok(d.P, d.N, d.Q);
         __nv_bfloat16 *CBt16 = reinterpret_cast<__nv_bfloat16 *>(ws + w.cbt16);
         __nv_bfloat16 *CB16b = reinterpret_cast<__nv_bfloat16 *>(ws + w.cb16);
@@ -471,7 +489,7 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
             make_tile_map(d, CBt16, &mCBto)) {
             // the fused dCB / decay-gradient kernel reads the bf16 tile by TMA; the separate intra_sums kernel
             // reads the fp32 strips
-            fused_cb = !no_fused() && tc::intra_tile_ok(d.P, d.Q);
+            fused_cb = fused_wanted(d);
             const size_t smem_ct = tc::bmm_cb_tma_smem(d.N, true);
             BISSD_ALLOW((tc::bmm_cb_tma<T, false>), smem_ct);
             BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T, false>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
@@ -481,13 +499,16 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
             BISSD_ALLOW((tc::bmm_cb_tma<T, true>), smem_ct);
             BISSD_LAUNCH("tc_bmm_cb_tma", launch_pdl(tc::bmm_cb_tma<T, true>, dim3(d.b * d.nc * d.G, d.Q / 128, d.Q / 128), tc::kThreads, smem_ct, s,
                 d, mCc, mBc, mCc, mCc, tc::CbArgs{0, 0, F(w.cbs), F(w.cb), F(w.cbt)}, status));
-        } else
-        BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
-            d, Cm, Bm, (sums_path && ws_path) ? nullptr : F(w.cb), ws_path ? nullptr : F(w.cbt), nullptr,
-            ws_path ? CBt16 : nullptr, sums_path ? F(w.cbs) : nullptr, status));   // only the copies that will be read
+        } else {
+            if (lean && fused_wanted(d)) return BISSD_ERR_WORKSPACE;
+            BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
+                d, Cm, Bm, (sums_path && ws_path) ? nullptr : F(w.cb), ws_path ? nullptr : F(w.cbt), nullptr,
+                ws_path ? CBt16 : nullptr, sums_path ? F(w.cbs) : nullptr, status));   // only the copies that will be read
+        }
         have_fp32_cb = !ws_path;                             // ws path: only the copies its kernels read were written
         auto ensure_fp32_cb = [&]() -> int {                 // for the kernels that read them, should a planned path fall through
             if (have_fp32_cb) return BISSD_OK;
+            if (lean && fused_wanted(d)) return BISSD_ERR_WORKSPACE;
             BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
                 d, Cm, Bm, F(w.cb), F(w.cbt), nullptr, nullptr, nullptr, status));
             have_fp32_cb = true;
@@ -609,7 +630,7 @@ do {                                                                            
                 }
                 BISSD_ALLOW(tc::dbc_accum_tma<T>, smem_a);
                 if (!no_ws() && tc::dbc_grp_ok(d.P, d.N, d.Q)) {
-                    dbc_last = fused_cb && head_parts(d) == 1 && tc::bmm_bwd_tma_ok(d.N, d.Q);   // launched after the dCB kernel, below
+                    dbc_last = fused_cb && last_wanted(d);       // launched after the dCB kernel, below
                     if (!dbc_last) {
                         const int rc = launch_dbc(tc::dbc_accum_grp<T, false>, tc::LastMaps{}, side.stream());
                         if (rc != BISSD_OK) return rc;
@@ -622,6 +643,7 @@ do {                                                                            
                 nsplit = 1;                                      // nf/nb/pf/pb now hold complete row sums
             }
         }
+        if (lean && last_wanted(d) && !dbc_last) return BISSD_ERR_WORKSPACE;
         if (!dbc_done) {
             BISSD_ALLOW(tc::dbc_states<T>, smem_n);
             BISSD_LAUNCH("tc_dbc_states", tc::dbc_states<T><<<dim3(d.b * d.nc * d.G * w.nsplit, nlt_tc, 2), tc::kThreads, smem_n, s>>>(
@@ -709,6 +731,7 @@ do {                                                                            
             }
         }
         if (!intra_done && !have_fp32_cb) {                  // the prefix-sweep kernels read the fp32 matrix
+            if (lean && fused_wanted(d)) return BISSD_ERR_WORKSPACE;
             const size_t smem_cb = tc::smem_bytes(ntQ, 0);
             BISSD_LAUNCH("tc_bmm_cb", tc::bmm_cb<T><<<dim3(d.b * d.nc * d.G, nlt_tc), tc::kThreads, smem_cb, s>>>(
                 d, Cm, Bm, F(w.cb), F(w.cbt), nullptr, nullptr, nullptr, status));
@@ -802,6 +825,17 @@ int bissd_workspace_bytes(const bissd_problem *p, size_t *fwd_bytes, size_t *bwd
     if (rc != BISSD_OK) return rc;
     if (fwd_bytes) *fwd_bytes = fwd_layout(d).total;
     if (bwd_bytes) *bwd_bytes = bwd_layout(d, !force_simt() && tc_shape_ok(*p)).total;
+    return BISSD_OK;
+}
+
+int bissd_workspace_bytes_least(const bissd_problem *p, size_t *fwd_bytes, size_t *bwd_bytes) {
+    if (!p) return BISSD_ERR_NULL;
+    Dims d;
+    int rc = make_dims(*p, &d);
+    if (rc != BISSD_OK) return rc;
+    const bool tcp = !force_simt() && tc_shape_ok(*p);
+    if (fwd_bytes) *fwd_bytes = (tcp ? least_fwd(d) : fwd_layout(d)).total;
+    if (bwd_bytes) *bwd_bytes = (tcp ? least_bwd(d) : bwd_layout(d, false)).total;
     return BISSD_OK;
 }
 
@@ -917,17 +951,17 @@ int bissd_forward(const bissd_fwd_args *a, void *workspace, size_t workspace_byt
     if (a->p.has_z && (!a->z.ptr || ((a->phases & BISSD_PHASE_FINISH) && !a->out_x.ptr))) return BISSD_ERR_NULL;
     if (a->p.has_D && !a->D) return BISSD_ERR_NULL;
     if (a->p.has_dt_bias && !a->dt_bias) return BISSD_ERR_NULL;
-    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) || workspace_bytes < fwd_layout(d).total)
-        return BISSD_ERR_WORKSPACE;
     const bool tcp = !force_simt() && tc_shape_ok(a->p) && aligned16(a->x) && aligned16(a->B) && aligned16(a->C) &&
                      aligned16(a->z) && aligned16(a->out) && aligned16(a->out_x);
+    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) || workspace_bytes < (tcp ? least_fwd(d) : fwd_layout(d)).total)
+        return BISSD_ERR_WORKSPACE;
     if (!states_aligned(a->p, tcp, a->states_f, a->states_b)) return BISSD_ERR_ALIGN;
     rc = check_device();
     if (rc != BISSD_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char *ws = static_cast<char *>(workspace);
     if (!tcp) return simt_forward(*a, d, ws, s);
-    return a->p.x_dtype == BISSD_BF16 ? forward_impl<__nv_bfloat16>(*a, d, ws, s) : forward_impl<__half>(*a, d, ws, s);
+    return a->p.x_dtype == BISSD_BF16 ? forward_impl<__nv_bfloat16>(*a, d, ws, workspace_bytes, s) : forward_impl<__half>(*a, d, ws, workspace_bytes, s);
 }
 
 // ---- forward pass on library-owned scratch -------------------------------------------------------------------
@@ -1031,8 +1065,8 @@ int bissd_backward_into(const bissd_bwd_args *a, const bissd_grad_strides *gs, v
     // larger workspace that bissd_workspace_bytes reports for the same sizes with fp32 inputs
     const bool tcp = !force_simt() && tc_shape_ok(a->p) && aligned16(a->x) && aligned16(a->B) && aligned16(a->C) &&
                      aligned16(a->z) && aligned16(a->dout) && aligned16(a->out_x);
-    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) || workspace_bytes < bwd_layout(d, tcp).total)
-        return BISSD_ERR_WORKSPACE;
+    const size_t need = (tcp && a->phases == BISSD_PHASE_ALL ? least_bwd(d) : bwd_layout(d, tcp)).total;   // a split pass keeps its local gradients
+    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) || workspace_bytes < need) return BISSD_ERR_WORKSPACE;
     const long long L = d.L, hp = (long long)d.H * d.P, gn = (long long)d.G * d.N;
     GradViews gr{MutView{a->dx, L * hp, hp, d.P}, MutView{a->dB, L * gn, gn, d.N}, MutView{a->dC, L * gn, gn, d.N},
                  MutView{a->ddt, L * d.H, d.H, 1}};
@@ -1048,7 +1082,7 @@ int bissd_backward_into(const bissd_bwd_args *a, const bissd_grad_strides *gs, v
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char *ws = static_cast<char *>(workspace);
     if (!tcp) return simt_backward(*a, gr, d, ws, s);
-    return a->p.x_dtype == BISSD_BF16 ? backward_impl<__nv_bfloat16>(*a, gr, d, ws, s) : backward_impl<__half>(*a, gr, d, ws, s);
+    return a->p.x_dtype == BISSD_BF16 ? backward_impl<__nv_bfloat16>(*a, gr, d, ws, workspace_bytes, s) : backward_impl<__half>(*a, gr, d, ws, workspace_bytes, s);
 }
 
 }  // extern "C"

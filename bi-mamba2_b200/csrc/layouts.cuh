@@ -33,13 +33,19 @@ inline int pass_slots(const Dims &d) {                           // partial dT p
     return pass_grid(d).y * (pass_by4(d) ? pass_threads(d) / 32 : 1);
 }
 
-inline FwdWs fwd_layout(const Dims &d) {
+// Arrays that only some kernels need.  bissd_workspace_bytes reports room for all of them; a pass whose kernels are known to
+// do without also runs in less (bissd_workspace_bytes_least).  They lie at the end: the others are where they are either way.
+struct FwdNeed {
+    bool loc = true, cb = true, cb16 = true;                     // local states; C.B^T in fp32; rounded to bf16 (TMA-fed scan)
+};
+inline FwdWs fwd_layout(const Dims &d, FwdNeed need = FwdNeed()) {
     FwdWs w;
     size_t o = kWsHeader;
-    const size_t st = (size_t)d.b * d.nc * d.H * d.P * d.N;
-    w.loc = o; o = align256(o + 2 * st * 4);
-    w.cb = o; o = align256(o + (size_t)d.b * d.nc * d.G * d.Q * d.Q * 4);
-    w.cb16 = o; o = align256(o + (size_t)d.b * d.nc * d.G * d.Q * d.Q * 2);      // C.B^T rounded to bf16 (TMA-fed scan)
+    auto take = [&](size_t bytes) { size_t at = o; o = align256(o + bytes); return at; };
+    const size_t qq = (size_t)d.b * d.nc * d.G * d.Q * d.Q;
+    w.cb16 = take(need.cb16 ? qq * 2 : 0);
+    w.cb = take(need.cb ? qq * 4 : 0);
+    w.loc = take(need.loc ? 2 * (size_t)d.b * d.nc * d.H * d.P * d.N * 4 : 0);
     w.total = o;
     return w;
 }
@@ -86,7 +92,10 @@ inline int dbc_ksplit(const Dims &d) {
 // tc: sized for the tensor-core family (16-bit inputs that meet its alignment rules): the passed state gradients are
 // kept in the input dtype only, and the "states" parts of dB / dC arrive summed over the heads of a group.  The
 // CUDA-core family needs the fp32 copy and one partial per head.
-inline BwdWs bwd_layout(const Dims &d, bool tc) {
+struct BwdNeed {
+    bool gloc = true, parts = true, cb32 = true;                 // local state gradients; partial dB / dC; C.B^T in fp32 and its copies
+};
+inline BwdWs bwd_layout(const Dims &d, bool tc, BwdNeed need = BwdNeed()) {
     BwdWs w;
     size_t o = kWsHeader;
     const size_t st = (size_t)d.b * d.nc * d.H * d.P * d.N;
@@ -98,13 +107,9 @@ inline BwdWs bwd_layout(const Dims &d, bool tc) {
     w.dbc_ks = tc ? dbc_ksplit(d) : 1;
     const int slots = dbc_slots(d, w.dbc_ks);
     auto take = [&](size_t bytes) { size_t at = o; o = align256(o + bytes); return at; };
-    w.cb = take(qq * 4);
-    w.gloc = take(2 * st * 4);
     w.E = take(tc ? 0 : 2 * st * 4);                                 // fp32 passed state gradients (CUDA-core family)
     w.E16 = take(tc ? 2 * st * 2 : 0);                               // passed state gradients in the input dtype
     w.g = take(tc ? (size_t)d.b * d.L * d.H * d.P * 2 : 0);          // gated output gradient dout * silu(z)
-    w.cbt = take(tc ? qq * 4 : 0);                                   // CB transposed
-    w.cbs = take(tc ? qq * 4 : 0);                                   // CB in strips of 16 columns (tc::intra_sums)
     w.cbt16 = take(tc ? qq * 2 : 0);                                 // CB transposed, rounded to bf16 (TMA-fed dx)
     w.cb16 = take(tc ? qq * 2 : 0);                                  // CB rounded to bf16 (tc::intra_dcb_tile)
     w.dTpart = take((size_t)2 * d.b * d.H * d.nc * w.nslots * 4);
@@ -113,12 +118,17 @@ inline BwdWs bwd_layout(const Dims &d, bool tc) {
     w.pf = take(hq * 4 * w.nsplit); w.pb = take(hq * 4 * w.nsplit);
     w.da_f = take(tc ? hq * 4 : 0); w.da_b = take(tc ? hq * 4 : 0);
     w.u4 = take((tc ? 8 : 4 * w.nlt) * hq * 4);                      // u_f / u_b per tile (tc::intra_sums: 2 row tiles; tc::intra_dcb_tile: 4; simt: 2 nlt)
-    w.dB_part = take((size_t)d.b * d.nc * d.Q * (tc ? d.G * slots : d.H) * d.N * 4);
-    w.dC_part = take((size_t)d.b * d.nc * d.Q * (tc ? d.G * slots : d.H) * d.N * 4);
     w.dCB = take(qq * 4 * w.hsplit);
     w.dDpart = take((size_t)d.b * d.nc * d.H * std::max(w.nlt, 8) * d.P * 4);   // up to 8 partial rows per (b,c,h)
     w.dApart = take((size_t)d.b * d.nc * d.H * 4);
     w.dbiaspart = take((size_t)d.b * d.nc * d.H * 4);
+    w.cb = take(need.cb32 ? qq * 4 : 0);
+    w.cbt = take(tc && need.cb32 ? qq * 4 : 0);                      // CB transposed
+    w.cbs = take(tc && need.cb32 ? qq * 4 : 0);                      // CB in strips of 16 columns (tc::intra_sums)
+    const size_t part = need.parts ? (size_t)d.b * d.nc * d.Q * (tc ? d.G * slots : d.H) * d.N * 4 : 0;
+    w.dB_part = take(part);
+    w.dC_part = take(part);
+    w.gloc = take(need.gloc ? 2 * st * 4 : 0);
     w.total = o;
     return w;
 }

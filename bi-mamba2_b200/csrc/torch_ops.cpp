@@ -122,6 +122,22 @@ bissd_problem problem_of(const Tensor &x, const Tensor &dt, const Tensor &B, con
     return p;
 }
 
+// `call` with the least scratch its sizes need (and `extra` bytes behind it), and once more with all there may be if that
+// turns out to be too little.
+template <class F>
+void with_workspace(const bissd_problem &p, bool forward, size_t extra, bool check_status, void *stream, F call) {
+    int rc = BISSD_ERR_WORKSPACE;
+    for (const auto size_of : {bissd_workspace_bytes_least, bissd_workspace_bytes}) {
+        size_t bytes = 0;
+        check(size_of(&p, forward ? &bytes : nullptr, forward ? nullptr : &bytes));
+        const c10::DataPtr ws = c10::cuda::CUDACachingAllocator::get()->allocate(bytes + extra);
+        rc = call(static_cast<char *>(ws.get()), bytes);
+        if (rc == BISSD_OK) check_device_status(check_status, ws.get(), stream);
+        if (rc != BISSD_ERR_WORKSPACE) break;
+    }
+    check(rc);
+}
+
 struct ScanOut {
     Tensor out, out_x, saved, fin_f, fin_b;                      // fin_*: only when asked for
 };
@@ -134,8 +150,6 @@ ScanOut scan_forward(const Tensor &x_, const Tensor &dt, const Tensor &A, const 
     const Tensor x = inner_contig(x_), B = inner_contig(B_), C = inner_contig(C_), z = inner_contig(z_);
     const Tensor A32 = f32c(A), D32 = f32c(D), bias32 = f32c(dt_bias), if32 = f32c(init_f), ib32 = f32c(init_b);
     const bissd_problem p = problem_of(x, dt, B, D, z, dt_bias, cfg);
-    size_t ws_bytes = 0;
-    check(bissd_workspace_bytes(&p, &ws_bytes, nullptr));
     const auto stream = c10::cuda::getCurrentCUDAStream(x.device().index());
     ScanOut r;
     if (phases & BISSD_PHASE_FINISH) {
@@ -143,16 +157,7 @@ ScanOut scan_forward(const Tensor &x_, const Tensor &dt, const Tensor &A, const 
         if (z.defined()) r.out_x = at::empty(x.sizes(), x.options());
     }
     const Saved at_(p, x.element_size());
-    const size_t own = keep ? 0 : align256(at_.total);
-    c10::DataPtr ws = c10::cuda::CUDACachingAllocator::get()->allocate(ws_bytes + own);
-    char *ws_ptr = static_cast<char *>(ws.get());
-    char *sv;
-    if (keep) {
-        r.saved = at::empty({(int64_t)at_.total}, x.options().dtype(at::kByte));
-        sv = static_cast<char *>(r.saved.mutable_data_ptr());
-    } else {
-        sv = ws_ptr + align256(ws_bytes);
-    }
+    if (keep) r.saved = at::empty({(int64_t)at_.total}, x.options().dtype(at::kByte));
     if (finals) {
         const Tensor fin = at::empty({2, x.size(0), x.size(2), x.size(3), B.size(3)}, x.options().dtype(at::kFloat));
         r.fin_f = fin.select(0, 0);
@@ -164,14 +169,17 @@ ScanOut scan_forward(const Tensor &x_, const Tensor &dt, const Tensor &A, const 
     a.A = static_cast<const float *>(ptr(A32)); a.D = static_cast<const float *>(ptr(D32));
     a.dt_bias = static_cast<const float *>(ptr(bias32));
     a.out = tensor4(r.out); a.out_x = tensor4(r.out_x);
-    a.dt_out = reinterpret_cast<float *>(sv + at_.dt_out); a.cs_f = reinterpret_cast<float *>(sv + at_.cs_f);
-    a.cs_b = reinterpret_cast<float *>(sv + at_.cs_b);
-    a.states_f = sv + at_.states_f; a.states_b = sv + at_.states_b;
     a.final_f = static_cast<float *>(ptr(r.fin_f)); a.final_b = static_cast<float *>(ptr(r.fin_b));
     a.init_f = static_cast<const float *>(ptr(if32)); a.init_b = static_cast<const float *>(ptr(ib32));
     a.phases = phases;
-    check(bissd_forward(&a, ws_ptr, ws_bytes, stream.stream()));
-    check_device_status(cfg.check_status, ws_ptr, stream.stream());
+    const size_t own = keep ? 0 : align256(at_.total);
+    with_workspace(p, true, own, cfg.check_status, stream.stream(), [&](char *ws, size_t bytes) {
+        char *sv = keep ? static_cast<char *>(r.saved.mutable_data_ptr()) : ws + align256(bytes);
+        a.dt_out = reinterpret_cast<float *>(sv + at_.dt_out); a.cs_f = reinterpret_cast<float *>(sv + at_.cs_f);
+        a.cs_b = reinterpret_cast<float *>(sv + at_.cs_b);
+        a.states_f = sv + at_.states_f; a.states_b = sv + at_.states_b;
+        return bissd_forward(&a, ws, bytes, stream.stream());
+    });
     return r;
 }
 
@@ -188,8 +196,6 @@ void scan_backward(ScanGrads &g, const Tensor &dout_, const Tensor &x_, const Te
     const Tensor x = inner_contig(x_), B = inner_contig(B_), C = inner_contig(C_), z = inner_contig(z_), dout = inner_contig(dout_);
     const Tensor A32 = f32c(A), D32 = f32c(D), bias32 = f32c(dt_bias), ff32 = f32c(dfin_f), fb32 = f32c(dfin_b);
     const bissd_problem p = problem_of(x, dt, B, D, z, dt_bias, cfg);
-    size_t ws_bytes = 0;
-    check(bissd_workspace_bytes(&p, nullptr, &ws_bytes));
     const auto stream = c10::cuda::getCurrentCUDAStream(x.device().index());
     if (!g.dx.defined()) g.dx = at::empty(x.sizes(), x.options());
     if (z.defined()) g.dz = at::empty(x.sizes(), x.options());
@@ -207,7 +213,6 @@ void scan_backward(ScanGrads &g, const Tensor &dout_, const Tensor &x_, const Te
     }
     const Saved at_(p, x.element_size());
     char *sv = static_cast<char *>(ptr(saved));
-    c10::DataPtr ws = c10::cuda::CUDACachingAllocator::get()->allocate(ws_bytes);
     auto F = [](const Tensor &t) { return static_cast<float *>(ptr(t)); };
     bissd_bwd_args a{};
     a.p = p;
@@ -224,8 +229,8 @@ void scan_backward(ScanGrads &g, const Tensor &dout_, const Tensor &x_, const Te
     bissd_grad_strides gs;
     auto strides = [](int64_t *to, const Tensor &t) { for (int i = 0; i < 3; ++i) to[i] = t.stride(i); };
     strides(gs.dx, g.dx); strides(gs.dB, g.dB); strides(gs.dC, g.dC); strides(gs.ddt, g.ddt);
-    check(bissd_backward_into(&a, &gs, ws.get(), ws_bytes, stream.stream()));
-    check_device_status(cfg.check_status, ws.get(), stream.stream());
+    with_workspace(p, false, 0, cfg.check_status, stream.stream(),
+                   [&](char *ws, size_t bytes) { return bissd_backward_into(&a, &gs, ws, bytes, stream.stream()); });
 }
 
 Tensor to_dtype_of(const Tensor &g, const Tensor &like) {

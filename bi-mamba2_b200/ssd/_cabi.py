@@ -65,14 +65,14 @@ class ConvArgs(C.Structure):
                 ("dout", C.c_void_p), ("dx", C.c_void_p), ("dweight", C.c_void_p), ("dbias", C.c_void_p)]
 
 
-EXPORTS = ("bissd_abi_version", "bissd_strerror", "bissd_last_cuda_error", "bissd_workspace_bytes", "bissd_forward",
+EXPORTS = ("bissd_abi_version", "bissd_strerror", "bissd_last_cuda_error", "bissd_workspace_bytes", "bissd_workspace_bytes_least", "bissd_forward",
            "bissd_backward", "bissd_kernel_path", "bissd_launch_count", "bissd_trace_enable", "bissd_trace_read", "bissd_selftest_gemm", "bissd_read_status",
            "bissd_forward_static_scratch", "bissd_chain_boundaries", "bissd_rmsnorm_gated_workspace_bytes", "bissd_rmsnorm_gated_forward",
            "bissd_rmsnorm_gated_backward", "bissd_dwconv_silu_workspace_bytes", "bissd_dwconv_silu_forward",
            "bissd_dwconv_silu_backward", "bissd_backward_into", "bissd_layer_params_in", "bissd_layer_params_out")
 
 STATIC_SCRATCH_BYTES = 16 << 20      # BISSD_STATIC_SCRATCH_BYTES
-ERR_TOO_LARGE = -9
+ERR_WORKSPACE, ERR_TOO_LARGE = -5, -9
 
 _lib = None
 
@@ -96,6 +96,8 @@ def load():
     lib.bissd_last_cuda_error.restype = C.c_char_p
     lib.bissd_workspace_bytes.restype = C.c_int
     lib.bissd_workspace_bytes.argtypes = [C.POINTER(Problem), C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]
+    lib.bissd_workspace_bytes_least.restype = C.c_int
+    lib.bissd_workspace_bytes_least.argtypes = [C.POINTER(Problem), C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]
     lib.bissd_forward.restype = C.c_int
     lib.bissd_forward.argtypes = [C.POINTER(FwdArgs), C.c_void_p, C.c_size_t, C.c_void_p]
     lib.bissd_backward.restype = C.c_int

@@ -57,19 +57,35 @@ def _problem(x, dt, B, chunk_size, D, z, dt_bias, dt_softplus, dt_min, dt_max):
                          float(dt_min), float(dt_max))
 
 
-_ws_bytes = {}                                    # problem fields -> (forward bytes, backward bytes)
+_ws_bytes = {}                                    # problem fields, least -> (forward bytes, backward bytes)
 
 
-def _workspace(problem, device, which):
-    key = tuple(getattr(problem, name) for name, _ in problem._fields_)
+def _workspace(problem, device, which, least=False):
+    key = (least, *(getattr(problem, name) for name, _ in problem._fields_))
     sizes = _ws_bytes.get(key)
     if sizes is None:
         import ctypes
         f, b = ctypes.c_size_t(0), ctypes.c_size_t(0)
-        _cabi.check(_cabi.load().bissd_workspace_bytes(ctypes.byref(problem), ctypes.byref(f), ctypes.byref(b)))
+        lib = _cabi.load()
+        size_of = lib.bissd_workspace_bytes_least if least else lib.bissd_workspace_bytes
+        _cabi.check(size_of(ctypes.byref(problem), ctypes.byref(f), ctypes.byref(b)))
         sizes = _ws_bytes[key] = (f.value, b.value)
     nbytes = sizes[0] if which == "fwd" else sizes[1]
     return torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device), nbytes
+
+
+def _with_workspace(problem, device, which, call):
+    """call(workspace address, bytes, stream) with the least scratch the sizes need, and once more with all there may be
+    if that turns out to be too little."""
+    with torch.cuda.device(device):
+        stream = torch.cuda.current_stream(device).cuda_stream
+        for least in (True, False):
+            ws, nbytes = _workspace(problem, device, which, least)
+            rc = call(ws.data_ptr(), nbytes, stream)
+            if rc != _cabi.ERR_WORKSPACE:
+                break
+        _cabi.check(rc)
+        _check_status(ws, stream)
 
 
 def _require_cuda(*tensors):
@@ -147,16 +163,12 @@ def _scan_fwd_core(x, dt, A, B, C, chunk_size, D, z, dt_bias, init_f, init_b, dt
     dt_out, cs_f, cs_b = _family(3, (batch, nheads, nchunks, chunk_size), fused, dtype=torch.float32, device=dev)
     states_f, states_b = _family(2, (batch, nchunks, nheads, headdim, dstate), fused, dtype=x.dtype, device=dev)
     final_f, final_b = _family(2, (batch, nheads, headdim, dstate), fused, dtype=torch.float32, device=dev)
-    ws, nbytes = _workspace(p, dev, "fwd")
     args = _cabi.FwdArgs(p, _tensor4(x), _tensor4(B), _tensor4(C), _tensor4(z),
                          _cabi.Tensor(dt.data_ptr(), dt.stride(0), dt.stride(1), dt.stride(2)),
                          _ptr(A32), _ptr(D32), _ptr(bias32), _tensor4(out), _tensor4(out_x if z is not None else None),
                          _ptr(dt_out), _ptr(cs_f), _ptr(cs_b), _ptr(states_f), _ptr(states_b), _ptr(final_f),
                          _ptr(final_b), _ptr(init_f), _ptr(init_b), phases)
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        _cabi.check(lib.bissd_forward(ctypes.byref(args), ws.data_ptr(), nbytes, stream))
-        _check_status(ws, stream)
+    _with_workspace(p, dev, "fwd", lambda ws, nbytes, stream: lib.bissd_forward(ctypes.byref(args), ws, nbytes, stream))
     return out, out_x, dt_out, cs_f, cs_b, states_f, states_b, final_f, final_b
 
 
@@ -220,7 +232,6 @@ def _scan_bwd_core(dout, x, dt, A, B, C, chunk_size, D, z, dt_bias, out_x, dt_ou
         dinit_f, dinit_b = _family(2, (batch, nheads, headdim, dstate), fused, **f32)
     else:
         dinit_f, dinit_b = empty(), empty()
-    ws, nbytes = _workspace(p, dev, "bwd")
     opt = lambda t, present: _ptr(t) if present else None
     args = _cabi.BwdArgs(p, _tensor4(x), _tensor4(B), _tensor4(C), _tensor4(z), _tensor4(dout),
                          _tensor4(out_x if z is not None else None),
@@ -229,10 +240,7 @@ def _scan_bwd_core(dout, x, dt, A, B, C, chunk_size, D, z, dt_bias, out_x, dt_ou
                          _ptr(states_b), _ptr(dx), opt(dz, z is not None), _ptr(dB), _ptr(dC), _ptr(ddt), _ptr(dA),
                          opt(dD, D is not None), opt(ddt_bias, dt_bias is not None), _ptr(dfinal_f), _ptr(dfinal_b),
                          opt(dinit_f, want_dinit), opt(dinit_b, want_dinit), _cabi.PHASE_ALL)
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        _cabi.check(lib.bissd_backward(ctypes.byref(args), ws.data_ptr(), nbytes, stream))
-        _check_status(ws, stream)
+    _with_workspace(p, dev, "bwd", lambda ws, nbytes, stream: lib.bissd_backward(ctypes.byref(args), ws, nbytes, stream))
     return dx, ddt, dA, dB, dC, dD, dz, ddt_bias, dinit_f, dinit_b
 
 

@@ -40,7 +40,7 @@ typedef enum bissd_status {
     BISSD_ERR_SHAPE = -2,         /* inconsistent or unsupported sizes */
     BISSD_ERR_DTYPE = -3,         /* unsupported dtype combination */
     BISSD_ERR_ALIGN = -4,         /* pointer or stride not aligned as required */
-    BISSD_ERR_WORKSPACE = -5,     /* workspace smaller than bissd_workspace_bytes() reports */
+    BISSD_ERR_WORKSPACE = -5,     /* workspace smaller than the call needs, see bissd_workspace_bytes() */
     BISSD_ERR_LAUNCH = -6,        /* a CUDA launch or API call failed (see bissd_last_cuda_error) */
     BISSD_ERR_ARCH = -7,          /* the current device is not compute capability 10.x */
     BISSD_ERR_PHASE = -8,         /* invalid phase mask */
@@ -142,6 +142,13 @@ const char *bissd_last_cuda_error(void);
  * function reports for the same sizes with x_dtype = BISSD_F32; with less, bissd_backward returns
  * BISSD_ERR_WORKSPACE. */
 int bissd_workspace_bytes(const bissd_problem *p, size_t *fwd_bytes, size_t *bwd_bytes);
+
+/* The least scratch that bissd_forward, and bissd_backward with all phases in one call, run `p` in: without the arrays
+ * of kernels that these sizes do not normally take.  They do take them for a few operands (strides that no TMA
+ * descriptor holds, dt_out or cs_* not 16-byte aligned); such a call returns BISSD_ERR_WORKSPACE, possibly with outputs
+ * half written, and succeeds when made again with bissd_workspace_bytes().  A backward pass in two phases needs that
+ * size too.  Both phases of a forward pass must be given the same size. */
+int bissd_workspace_bytes_least(const bissd_problem *p, size_t *fwd_bytes, size_t *bwd_bytes);
 
 /* Forward pass.  workspace must be 256-byte aligned. */
 int bissd_forward(const bissd_fwd_args *args, void *workspace, size_t workspace_bytes, void *stream);

@@ -108,6 +108,34 @@ def test_backward_workspace_is_sized_by_kernel_family(lib):
     assert lib.bissd_backward(ctypes.byref(a), 4096, tc.value, None) == -5     # BISSD_ERR_WORKSPACE
 
 
+def test_least_workspace(lib):
+    """Without the arrays of kernels that the sizes do not take: in whole passes only, and never more than all of it."""
+    def sizes(p):
+        out = []
+        for f in (lib.bissd_workspace_bytes, lib.bissd_workspace_bytes_least):
+            fwd, bwd = ctypes.c_size_t(0), ctypes.c_size_t(0)
+            assert f(ctypes.byref(p), ctypes.byref(fwd), ctypes.byref(bwd)) == 0
+            out += [fwd.value, bwd.value]
+        return out
+    cfg2 = dict(batch=8, seqlen=2048, nheads=24, headdim=64, ngroups=1, dstate=128, chunk_size=256, x_dtype=1)
+    fwd, bwd, fwd_least, bwd_least = sizes(_problem(**cfg2))
+    assert fwd_least < fwd / 10 and bwd_least < bwd / 2       # no local states, no fp32 C.B^T, no partial dB and dC
+    for kw in (dict(), dict(x_dtype=1, headdim=20, dstate=12), dict(x_dtype=0, **{k: v for k, v in cfg2.items() if k != "x_dtype"})):
+        all_ = sizes(_problem(**kw))
+        assert all_[:2] == all_[2:] or lib.bissd_kernel_path(ctypes.byref(_problem(**kw))) == b"tcgen05"
+    assert lib.bissd_workspace_bytes_least(None, None, None) == -1
+    a = _cabi.BwdArgs()
+    a.p = _problem(has_D=0, **cfg2)
+    t = lambda: _cabi.Tensor(4096, 2048 * 24 * 64, 24 * 64, 64)
+    a.x, a.B, a.C, a.dout, a.dt = t(), t(), t(), t(), _cabi.Tensor(4096, 2048 * 24, 24, 1)
+    for f in ("A", "dt_out", "cs_f", "cs_b", "states_f", "states_b", "dx", "dB", "dC", "ddt", "dA"):
+        setattr(a, f, 4096)
+    a.phases = 1
+    assert lib.bissd_backward(ctypes.byref(a), 4096, bwd - 256, None) == -5      # a split pass keeps its local gradients
+    a.phases = 3
+    assert lib.bissd_backward(ctypes.byref(a), 4096, bwd_least - 256, None) == -5
+
+
 def test_forward_rejects_bad_arguments_before_any_launch(lib):
     args = _cabi.FwdArgs()
     args.p = _problem()
