@@ -1017,10 +1017,8 @@ int bissd_forward_static_scratch(const bissd_fwd_args *a, void *stream) {
     void *scratch = nullptr;
     rc = static_scratch_on_current_device(&scratch);
     if (rc != BISSD_OK) return rc;
-    // The array still holds whatever the previous call left.  Only the status word at its start is read before it
-    // is written, so that is what gets cleared; every other region is fully rewritten by the kernels that use it.
-    rc = note_cuda(cudaMemsetAsync(scratch, 0, kWsHeader, static_cast<cudaStream_t>(stream)), "cudaMemsetAsync");
-    if (rc != BISSD_OK) return rc;
+    // The array still holds whatever the previous call left.  Only the status word at its start is read before it is written:
+    // the first kernel of the pass clears it.
     return bissd_forward(a, scratch, kStaticScratchBytes, stream);
 }
 

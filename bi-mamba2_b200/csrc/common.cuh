@@ -58,12 +58,6 @@ template <class T> __device__ __forceinline__ float ld(const void *p, long long 
 template <class T> __device__ __forceinline__ void st(void *p, long long i, float v) {
     static_cast<T *>(p)[i] = from_f<T>(v);
 }
-template <class T> __device__ __forceinline__ float ldv(const View &t, int b, int l, int h, int i) {
-    return ld<T>(t.ptr, b * t.sb + l * t.sl + h * t.sh + i);
-}
-template <class T> __device__ __forceinline__ void stv(const MutView &t, int b, int l, int h, int i, float v) {
-    st<T>(t.ptr, b * t.sb + l * t.sl + h * t.sh + i, v);
-}
 
 // Load / store with a run-time dtype (used only for dt / ddt, which are tiny).
 __device__ __forceinline__ float ld_any(const void *p, int dtype, long long i) {

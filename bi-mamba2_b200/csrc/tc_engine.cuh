@@ -18,7 +18,6 @@ namespace tc {
 constexpr int kThreads = 256;
 constexpr int kStageK = 64;
 constexpr int kTileM = 128;
-constexpr uint32_t kSpinLimit = 1u << 22;      // mbarrier polls before a wait gives up and reports an error
 constexpr int kAStageBytes = kTileM * kStageK * 2;
 
 // error codes written to the status word

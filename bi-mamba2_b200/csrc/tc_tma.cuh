@@ -60,9 +60,6 @@ inline bool make_map2(CUtensorMap *m, int dtype, const void *ptr, unsigned long 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *m) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
-}
 // x = innermost coordinate (elements; x * 2 bytes must be a multiple of 16)
 __device__ __forceinline__ void tma_load4(void *dst, const CUtensorMap *m, int x, int y, int z, int w, uint64_t *bar) {
     asm volatile(
