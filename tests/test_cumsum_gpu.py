@@ -1,4 +1,5 @@
-"""A warp per (batch, chunk, head) of the cumulative sums: lane, chunk and head remainders, clamps and dt types, against the oracle."""
+"""Four warps per (batch, chunk, head) of the cumulative sums: lane, warp, chunk and head remainders, clamps and dt types, against
+the oracle."""
 import pytest
 import torch
 from oracle.bissd_oracle import max_rel_err, reference_with_grads
