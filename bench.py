@@ -120,8 +120,10 @@ def kernel_model(name, cfg, batch=None):
     zf = 1 if cfg["z"] else 0
     DTB = (2 if cfg["dt"] == "positive_bf16" else 4) * b * L * H
     state_f, intra_f = t * 4 * Q * P * N, t * 2 * Q * Q * P
+    finishes = P == 64 and nc * G * ((Q + 127) // 128) ** 2 >= 32
     model = {
         "cumsum_fwd": (0, DTB + 3 * HQ),
+        "cumsum_cb": (tg * 2 * Q * Q * N, DTB + 3 * HQ + 2 * BC + CB16),   # cumulative sums and C.B^T in one launch
         "chunk_state": (state_f, X + BC + 3 * HQ + 2 * ST32),
         "state_passing_fwd": (0, 2 * ST32 + 2 * ST16),
         # launched twice per step under one name: the forward writes one 16-bit copy, the backward that copy and its
@@ -135,7 +137,9 @@ def kernel_model(name, cfg, batch=None):
         "state_passing_bwd": (0, 2 * ST32 + 4 * ST16),
         "dx": (state_f + intra_f, 3 * X + BC + CB16 + 2 * ST16 + 6 * HQ),
         "prev_terms": (state_f, X + BC + 2 * ST16 + 4 * HQ),
-        "dbc_accum": (2 * state_f, 2 * X + 4 * ST16 + 3 * HQ + 4 * BC),
+        # where a row of the batch brings 32 tiles it also forms the product with dCB and writes dB and dC, else fp32 parts
+        "dbc_accum": (2 * state_f + tg * 4 * Q * Q * N, 2 * X + 4 * ST16 + 3 * HQ + CB16 + 4 * BC) if finishes else
+                     (2 * state_f, 2 * X + 4 * ST16 + 3 * HQ + 4 * BC),
         "dcb": (intra_f, 2 * X + 3 * HQ + CB16),
         "intra_sums": (intra_f, 2 * X + 3 * HQ + CB32 + 4 * HQ),
         # dCB and the intra-chunk decay gradients from one g.x^T product per head: reads g, x, the bf16 C.B^T tile and
@@ -167,9 +171,13 @@ def _source_hash(*files):
 # kernel's source file(s) at capture time; when the source has changed since, `traffic` prints as null instead of a
 # stale figure.  {kernel: (bytes per launch at batch 2, source files, hash)}
 NCU_TRAFFIC_B2 = {
-    "tc_intra_dcb_tile": (28.53e6, ("tc_intra_grp.cuh",), "4be93440f93a1481"),
-    "tc_dx_ws": (42.33e6, ("tc_scan_ws.cuh",), "b0a507b61400027a"),
-    "tc_chunk_scan_ws": (43.41e6, ("tc_scan_ws.cuh",), "b0a507b61400027a"),
+    "tc_intra_dcb_tile": (28.53e6, ("tc_intra_grp.cuh",), "41e3ef286fa48f36"),
+    "tc_dx_ws": (42.42e6, ("tc_scan_ws.cuh",), "b0a507b61400027a"),
+    "tc_chunk_scan_ws": (43.23e6, ("tc_scan_ws.cuh",), "b0a507b61400027a"),
+    "tc_state_walk": (14.86e6, ("tc_walk_tma.cuh",), "95d10f31667c0eed"),
+    "tc_dstate_walk": (27.06e6, ("tc_walk_tma.cuh",), "95d10f31667c0eed"),
+    "tc_dbc_accum_grp": (55.89e6, ("tc_dbc_tma.cuh",), "421cb86a24d9bcde"),
+    "tc_prev_terms_grp": (27.05e6, ("tc_dbc_tma.cuh",), "421cb86a24d9bcde"),
 }
 
 
