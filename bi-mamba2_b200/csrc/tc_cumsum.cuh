@@ -1,9 +1,10 @@
 // Discretisation + both cumulative sums of the tensor-core family, and their backward (formulas at simt::chunk_cumsum and
 // simt::cumsum_bwd_role).  Four warps share one (batch, chunk, head), a lane has E consecutive positions: every operand is
 // requested at once in wide pieces, the scans are register sums, five shuffles and one barrier.  The block's two heads are
-// neighbours, whose dt and ddt values share 32-byte sectors.  us, forward and backward, with a block of one position a
-// thread, a warp per chunk, and this: b16 L4096 H32 23 + 88, 15 + 60, 15.6 + 51; b2 L8192 H32 7 + 24, -, 5.3 + 14;
-// b8 L2048 H24 6 + 18, 5.5 + 16, 4.4 + 11.
+// neighbours, whose dt and ddt values share 32-byte sectors.  Device time by the profiler, us, forward and backward: b16
+// L4096 H32 16.5 + 44; b2 L8192 H32 6.5 + 15.2; b8 L2048 H24 5.5 + 12.5 (event brackets around each launch add 3 - 5).  With a
+// block of one position a thread: 23 + 88, 7 + 24, 6 + 18 by CUDA events; a warp per chunk 15 + 60 and 5.5 + 16
+// for the first and the last.
 #pragma once
 #include "simt_kernels.cuh"
 
