@@ -673,10 +673,15 @@ do {                                                                            
                 tc::make_map4(&mBb, a.p.x_dtype, a.B.ptr, dBC4, sB4, bx4) && tc::make_map4(&mCb, a.p.x_dtype, a.C.ptr, dBC4, sC4b, bx4) &&
                 tc::make_map2(&mDm, a.p.x_dtype, F(w.dCB), d.Q, dcb_rows, 64, d.Q) &&
                 tc::make_map2(&mDk, a.p.x_dtype, F(w.dCB), d.Q, dcb_rows, 64, 128)) {
-                const size_t smem_f = tc::intra_tile_smem(d.Q);
-                const auto intra = head_parts(d) > 1 ? tc::intra_dcb_tile<T, true> : tc::intra_dcb_tile<T, false>;
+                const size_t smem_f = tc::intra_tile_smem();
+                const auto intra = tc::intra_dcb_tile<T>;
+                const int ks = head_parts(d);                    // one block of a cluster for each part of the heads
                 BISSD_ALLOW(intra, smem_f);
-                const int ks = tc::intra_ksplit(d, sm_count());
+                static const bool split_fits = [&] {             // its warps deal out the registers of the launch: with fewer they would wait for more
+                    cudaFuncAttributes at;
+                    return cudaFuncGetAttributes(&at, intra) == cudaSuccess && at.numRegs >= tc::kIntraLaunchRegs;
+                }();
+                if (!split_fits) return note_cuda(cudaErrorLaunchOutOfResources, "tc_intra_dcb_tile");
                 BISSD_LAUNCH("tc_intra_dcb_tile", launch_cluster(intra, dim3(d.b * d.nc * d.G * ks, nlt_tc, nlt_tc), tc::kIntraTileThreads, smem_f, s, ks,
                     dg, mG, mX128, mCB, a.dt_out, a.cs_f, a.cs_b, F(w.u4), (long long)d.b * d.H * d.nc * d.Q,
                     static_cast<void *>(F(w.dCB)), ks, status));

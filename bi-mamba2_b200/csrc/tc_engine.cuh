@@ -201,6 +201,14 @@ template <class T> struct AbFmt;
 template <> struct AbFmt<__nv_bfloat16> { static constexpr int v = 1; };
 template <> struct AbFmt<__half> { static constexpr int v = 0; };
 
+// One lane of a converged warp, always the same.  The compiler knows that a single thread runs what follows and builds the
+// MMAs' descriptors in uniform registers: 3 instructions an MMA, 8 behind `lane == 0`.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 // D[tmem] (+)= A[smem] * B[smem]; one thread issues.
 __device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
