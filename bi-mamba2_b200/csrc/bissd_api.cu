@@ -677,11 +677,8 @@ do {                                                                            
                 const auto intra = tc::intra_dcb_tile<T>;
                 const int ks = head_parts(d);                    // one block of a cluster for each part of the heads
                 BISSD_ALLOW(intra, smem_f);
-                static const bool split_fits = [&] {             // its warps deal out the registers of the launch: with fewer they would wait for more
-                    cudaFuncAttributes at;
-                    return cudaFuncGetAttributes(&at, intra) == cudaSuccess && at.numRegs >= tc::kIntraLaunchRegs;
-                }();
-                if (!split_fits) return note_cuda(cudaErrorLaunchOutOfResources, "tc_intra_dcb_tile");
+                const int rc_regs = check_registers(intra, tc::kIntraLaunchRegs);
+                if (rc_regs != BISSD_OK) return rc_regs;
                 BISSD_LAUNCH("tc_intra_dcb_tile", launch_cluster(intra, dim3(d.b * d.nc * d.G * ks, nlt_tc, nlt_tc), tc::kIntraTileThreads, smem_f, s, ks,
                     dg, mG, mX128, mCB, a.dt_out, a.cs_f, a.cs_b, F(w.u4), (long long)d.b * d.H * d.nc * d.Q,
                     static_cast<void *>(F(w.dCB)), ks, status));

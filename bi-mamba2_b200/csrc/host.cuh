@@ -134,6 +134,22 @@ inline int sm_count() {
     return n[dev];
 }
 
+// Kernels that deal their registers anew (setmaxnreg) wait for ever if they were launched with fewer than the sum of the shares:
+// has the compiler given `kernel` that many a thread?
+template <class K> inline int check_registers(K kernel, int regs) {
+    static std::mutex mu;
+    static std::map<const void *, int> known;
+    std::lock_guard<std::mutex> lk(mu);
+    int &n = known[reinterpret_cast<const void *>(kernel)];
+    if (n == 0) {
+        cudaFuncAttributes at;
+        const int rc = note_cuda(cudaFuncGetAttributes(&at, kernel), "cudaFuncGetAttributes");
+        if (rc != BISSD_OK) return rc;
+        n = at.numRegs;
+    }
+    return n >= regs ? BISSD_OK : note_cuda(cudaErrorLaunchOutOfResources, "registers of a kernel that deals them anew");
+}
+
 #define BISSD_ALLOW(kernel, bytes)                  \
     do {                                             \
         int rc_ = allow_smem(kernel, bytes);         \

@@ -57,7 +57,7 @@ __device__ __forceinline__ void bmm_cb_role(const Dims &d, const CUtensorMap &tm
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     bool ok = true;
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
         ok = mbar_wait(&bar_in, 0);
         if (ok) {
             tc_fence_after();

@@ -302,7 +302,7 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
     if (warp == 8) {
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             const uint32_t idesc = instr_desc(AbFmt<T>::v, false, true, nt);
             int p = 0, start = 0;                               // local part of head i and its first head
@@ -354,7 +354,7 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
             }
         }
     } else if (warp == 9) {                                     // the ring's loads: stage i & 1 is free once the MMAs of head i - 2 are done
-        if (lane == 0)
+        if (elect_one())
             for (int i = 2; i < R && ws_wait(&sh.done[i & 1], ((i >> 1) - 1) & 1, fail, 51); ++i) load_head(i);
     } else {
         // the sum of local parts 2 pair and 2 pair + 1 (`two`) as this block's next partial result
@@ -488,7 +488,7 @@ prev_terms_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
-    if (tid == 0 && !feed.products<T>(tmem)) sh.fail = 1;
+    if (warp == 0 && elect_one() && !feed.products<T>(tmem)) sh.fail = 1;
     bool ok = mbar_wait(&sh.st_done, 0);
     ok = __syncthreads_and(ok) && !sh.fail;
     tc_fence_after();
@@ -609,7 +609,7 @@ prev_terms_grp(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
     if (warp == 8) {
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = ws_wait(&sh.bar_c, 0, fail, 61);
             const uint32_t idesc = instr_desc(AbFmt<T>::v, false, false, 2 * P);
             for (int i = 0; i < nh && ok; ++i) {
@@ -628,7 +628,7 @@ prev_terms_grp(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
             }
         }
     } else if (warp == 9) {                                     // the rings of head i - 2 are refilled as they drain
-        if (lane == 0)
+        if (elect_one())
             for (int i = 2; i < nh; ++i) {
                 if (!ws_wait(&sh.done[i & 1], ((i >> 1) - 1) & 1, fail, 64)) break;
                 load_s(i);

@@ -103,7 +103,7 @@ dcb_tma(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_constant__
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
     bool ok = true;
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
         for (int hr = 0; hr < 3 && hr < R; ++hr) load_head(hr);
         ok = issue_head(0, tmem);
     }
@@ -113,7 +113,7 @@ dcb_tma(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_constant__
     const uint32_t tl = tmem_lane_base(tmem);
 #pragma unroll 1
     for (int hr = 0; hr < R; ++hr) {
-        if (tid == 0 && ok && hr + 1 < R) ok = issue_head(hr + 1, tmem);
+        if (warp == 0 && elect_one() && ok && hr + 1 < R) ok = issue_head(hr + 1, tmem);
         if (hr + 1 < R) {
             write_tab(hr + 1);
             if (hr + 2 < R) fetch_tab(hr + 2);
@@ -227,7 +227,7 @@ bmm_bwd_tma(Dims d, const __grid_constant__ CUtensorMap tmDm, const __grid_const
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     bool ok = true;
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
         ok = mbar_wait(&bar_in, 0);
         if (ok) {
             tc_fence_after();

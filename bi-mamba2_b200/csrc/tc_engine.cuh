@@ -206,7 +206,8 @@ template <> struct AbFmt<__nv_bfloat16> { static constexpr int v = 1; };
 template <> struct AbFmt<__half> { static constexpr int v = 0; };
 
 // One lane of a converged warp, always the same.  The compiler knows that a single thread runs what follows and builds the
-// MMAs' descriptors in uniform registers: 3 instructions an MMA, 8 behind `lane == 0`.
+// MMAs' descriptors in uniform registers: 3 instructions an MMA, 8 behind `lane == 0` (one lane's work is a chain: eight MMAs of the
+// walk took 600 cycles to issue, half of a stage).
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
@@ -394,7 +395,7 @@ __device__ __forceinline__ bool umma_gemm(Pipe &p, uint32_t d_tmem, int n_tile, 
             if (tid == 0) atomicExch(p.status, kErrMmaTimeout);
             return false;
         }
-        if (tid == 0) {
+        if (tid < 32 && elect_one()) {
             tc_fence_after();
             const uint32_t a0 = smem_u32(p.a_stage[st]), b0 = smem_u32(p.b_stage[st]);
 #pragma unroll
@@ -438,7 +439,7 @@ __device__ __forceinline__ bool mbar_wait_cta(uint64_t *bar, uint32_t parity, bo
 
 // Wait until every MMA issued so far has completed, so the accumulators can be read with tmem_ld32.
 __device__ __forceinline__ bool umma_drain(Pipe &p) {
-    if (threadIdx.x == 0) umma_commit(&p.sh->done_bar);
+    if (threadIdx.x < 32 && elect_one()) umma_commit(&p.sh->done_bar);   // the thread that issued them
     bool ok = mbar_wait(&p.sh->done_bar, p.done_uses & 1);
     ++p.done_uses;
     ok = __syncthreads_and(ok);

@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, 2) intra_decay_grad(Dims d, const __
     if (TMA) {
         // g (128 rows) and x (Q rows) tiles by TMA into the engine's stage buffers, one 64-wide headdim slab per buffer
         const int npb = d.P / 64;
-        if (threadIdx.x == 0) {
+        if (threadIdx.x < 32 && elect_one()) {
             mbar_expect_tx(&sh.free_bar[0], (uint32_t)(npb * (16384 + Q * 128)));
             for (int j = 0; j < npb; ++j) {
                 tma_load4(p.a_stage[j], &tmG, j * 64, h, c * Q + l0, b, &sh.free_bar[0]);
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kThreads, 2) intra_decay_grad(Dims d, const __
     }
     tmem_reads_done();
     if (ok) {
-        if (threadIdx.x == 0) {
+        if (threadIdx.x < 32 && elect_one()) {
             tc_fence_after();
             umma_issue_stage<false, true>(p.tmem, nt, 1, p.a_stage[0], p.b_stage[0], 0u);
             umma_issue_stage<false, true>(p.tmem, nt, 1, p.a_stage[0], p.b_stage[1], 1u);

@@ -73,7 +73,7 @@ intra_sums(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_constan
             colF[i] = ex2_approx(cs_f[base + (i | 15)] * 1.4426950408889634f - (cf - lg));
             colB[i] = ex2_approx(cs_b[base + (i & ~15)] * 1.4426950408889634f - (cb_ - lg));
         }
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             ok = mbar_wait(&sh.free_bar[0], 0);
             if (ok) {
                 tc_fence_after();
@@ -199,7 +199,7 @@ intra_sums(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_constan
     }
     tmem_reads_done();
     if (ok) {
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             tc_fence_after();
             umma_issue_stage<false, true>(p.tmem, nt, 1, p.a_stage[0], p.b_stage[0], 0u);
             umma_issue_stage<false, true>(p.tmem, nt, 1, p.a_stage[1], p.b_stage[1], 1u);

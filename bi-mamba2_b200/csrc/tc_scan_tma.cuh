@@ -191,7 +191,7 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
     const int l = l0 + (warp & 3) * 32 + lane;                  // this thread's row, in the sums and in the epilogue
     const float ef = l < lim ? __expf(cs_f[base + l]) : 0.f, eb = l < lim ? __expf(cs_b[base + l]) : 0.f;
     const uint32_t tl = tmem_lane_base(tmem);
-    if (tid == 0 && !feed.products<T>(tmem)) sh.fail = 1;
+    if (warp == 0 && elect_one() && !feed.products<T>(tmem)) sh.fail = 1;
     bool ok = mbar_wait(&sh.st_done, 0);
     if (ok) {                                                   // the weighted sum of both products replaces the first
         tc_fence_after();
@@ -228,7 +228,7 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
         }
         ok = __syncthreads_and(ok) && !sh.fail;
         if (!ok) break;
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             tc_fence_after();
             if (!feed.stage_product<T>(tmem, it)) sh.fail = 1;
         }
@@ -242,7 +242,7 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
         zr[q] = (ok && l < lim && d.has_z && ec0 < P) ? ld8v<T>(z, b, c * Q + l, h, ec0 + q * 8) : zero8();
     }
     if (ok) {
-        if (tid == 0) umma_commit(&sh.done_bar);
+        if (warp == 0 && elect_one()) umma_commit(&sh.done_bar);
         ok = mbar_wait(&sh.done_bar, 0);
         ok = __syncthreads_and(ok) && !sh.fail;
         tc_fence_after();

@@ -510,7 +510,7 @@ ws_kernel(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant
 
     if (warp == 0) {
         // --------------------------------------------------------------------------------------------- MMA issue
-        if (lane == 0) {
+        if (elect_one()) {
             const uint64_t dC = smem_desc(smem_u32(smC), 16, 1024), dS = smem_desc(smem_u32(smS), 16, 1024);
             const uint64_t dM = smem_desc(smem_u32(smM), 16, 1024), dX = smem_desc(smem_u32(smX), (uint32_t)Q * 128, 1024);
             constexpr uint32_t idesc_st = instr_desc(AbFmt<T>::v, false, false, 2 * P);
@@ -567,7 +567,7 @@ ws_kernel(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------------------------------------- TMA loads
-        if (lane == 0) {
+        if (elect_one()) {
             WsIter it;
             it.init(d, nrt, t0);
             bool ok = true;

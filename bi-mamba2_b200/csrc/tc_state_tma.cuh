@@ -91,7 +91,7 @@ state_gemm_tma(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_c
         fence_async_smem();
     }
     ok = __syncthreads_and(ok);
-    if (ok && tid == 0) {
+    if (ok && warp == 0 && elect_one()) {
         ok = mbar_wait(&bar_a, 0);
         if (ok) {
             tc_fence_after();
@@ -229,7 +229,7 @@ state_gemm_grp(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_c
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
     if (warp == 16) {
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             for (int i = 0; i < nh && ok; ++i) {
                 uint8_t *sx = smX + (i & 1) * stage_bytes;

@@ -8,7 +8,7 @@
 // headdim 128, dstate 256 313, 164.
 //
 // Warps 0-3 scale the x / g rows in place; warps 4-11 keep the running state (TMEM lane = n, P / 2 columns each) and move it
-// from chunk to chunk; lane 0 of warp 13 fills the ring, lane 0 of warp 12 issues the MMAs (one thread doing both, a
+// from chunk to chunk; one lane of warp 13 fills the ring, one of warp 12 issues the MMAs (one thread doing both, a
 // stage took 0.75 us whatever was loaded, scaled or multiplied).  Stages are 128 positions (64 at P = 128): [128 x 128 n] of
 // B / C and [128 x P] of x / g, both MN-major as they land, with the rows' cumulative sums and Delta beside them (read from
 // global memory by the scaling warps, their latency was the length of a stage).  Accumulators and, in MODE 1, the entering
@@ -122,8 +122,11 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
+    // At headdim 128 the walk is bound elsewhere, and slower with elect_one (forward, b8 L1024 H16 N256: 69.6, 72.2 us; headdim 64,
+    // b8 L2048 H24 N128: 48.7, 45.2).
+    auto one_lane = [&] { return PB == 1 ? elect_one() : lane == 0; };
     if (warp == 12) {
-        if (lane == 0) {
+        if (one_lane()) {
             const uint32_t idesc = instr_desc(AbFmt<T>::v, true, true, P);
             bool ok = true;
             Pos m;
@@ -147,7 +150,7 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
             }
         }
     } else if (warp == 13) {                                    // the ring's loads
-        if (lane == 0) {
+        if (one_lane()) {
             Pos p;
             for (int s = 0; s < total; ++s, advance(p)) {
                 if (s >= NS && !ws_wait(&sh.empty[p.slot], p.phase ^ 1, fail, 71)) break;
