@@ -30,8 +30,8 @@ static int norm_check(const bissd_norm_args *a, norm::NormDims *d, bool backward
 }
 // hidden / 8 threads a row, rows side by side up to about 256 threads
 static dim3 norm_block(int hidden) { return dim3(hidden / norm::kCh, std::max(1, 256 * norm::kCh / hidden)); }
-// Persistent blocks: about 768 threads an SM forward and 512 backward (what their registers allow), fewer when the rows
-// run out first.  The backward's count is also its number of partial weight-gradient rows.
+// Persistent blocks: about 1024 threads an SM forward and 512 backward (what their registers allow), fewer when the rows
+// run out first (forward, 65536 rows of 2048 with strided z: 768 threads 201 us, 1024 191; one or four rows a thread and step 202).  The backward's count is also its number of partial weight-gradient rows.
 static int norm_blocks(long long rows, int hidden, int rows_per_thread, int threads_per_sm) {
     const dim3 b = norm_block(hidden);
     const long long want = (rows + b.y * rows_per_thread - 1) / (b.y * rows_per_thread);
@@ -42,7 +42,7 @@ static int norm_bwd_blocks(long long rows, int hidden) { return norm_blocks(rows
 template <class T, class W>
 static int norm_forward_impl(const bissd_norm_args *a, const norm::NormDims &d, cudaStream_t s) {
     const dim3 block = norm_block(d.hidden);
-    const int grid = norm_blocks(d.rows, d.hidden, norm::kFwdRows, 768);
+    const int grid = norm_blocks(d.rows, d.hidden, norm::kFwdRows, 1024);
     const size_t smem = 2 * block.y * norm::kFwdRows * 16 * sizeof(float);
     const auto kernel = !a->z ? norm::rmsnorm_gated_fwd<T, W, 0>
                               : (a->norm_before_gate ? norm::rmsnorm_gated_fwd<T, W, 1> : norm::rmsnorm_gated_fwd<T, W, 2>);

@@ -7,8 +7,8 @@
 // two kernels' time.  us, forward + backward, two kernels and walk: b8 L2048 H24 133, 95; b2 L8192 H32 195, 109; b8 L1024 H16
 // headdim 128, dstate 256 313, 164.
 //
-// Warps 0-3 scale the x / g rows in place; warps 4-11 keep the running state (TMEM lane = n, P / 2 columns each) and move it
-// from chunk to chunk; one lane of warp 13 fills the ring, one of warp 12 issues the MMAs (one thread doing both, a
+// Warps 0-3 scale the x / g rows in place; warps 4-11 (4-19) keep the running state (TMEM lane = n, P / 2 or P / 4 columns each) and
+// move it from chunk to chunk; one lane of the last warp fills the ring, one of the warp before it issues the MMAs (one thread doing both, a
 // stage took 0.75 us whatever was loaded, scaled or multiplied).  Stages are 128 positions (64 at P = 128): [128 x 128 n] of
 // B / C and [128 x P] of x / g, both MN-major as they land, with the rows' cumulative sums and Delta beside them (read from
 // global memory by the scaling warps, their latency was the length of a stage).  Accumulators and, in MODE 1, the entering
@@ -21,7 +21,12 @@
 namespace bissd {
 namespace tc {
 
-constexpr int kWalkScale = 128, kWalkThreads = kWalkScale + kThreads + 64;   // 14 warps, 128 registers each
+// Threads that keep the running state.  Sixteen warps in the backward walk at headdim 128, where eight are what it waits for
+// (dot products with the entering states; us, b8 L1024 H16 N256: 103, 87); elsewhere eight are as good or better (forward 69.6, 70.9;
+// headdim 64, b8 L2048 H24 N128: forward 45.2, 45.5, backward 53.6, 55.4).
+constexpr int kWalkScale = 128;
+__host__ __device__ constexpr int walk_state_threads(int pb, int mode) { return pb == 2 && mode == 1 ? 512 : 256; }
+__host__ __device__ constexpr int walk_threads(int pb, int mode) { return kWalkScale + walk_state_threads(pb, mode) + 64; }   // 14 or 22 warps
 __host__ __device__ constexpr int walk_rows(int pb) { return pb == 1 ? 128 : 64; }   // positions per stage
 __host__ __device__ constexpr int walk_ring(int pb, int mode) { return pb == 1 ? (mode ? 3 : 4) : (mode ? 4 : 6); }
 __host__ __device__ constexpr int walk_stage_bytes(int pb) { return walk_rows(pb) * (256 + pb * 128) + 2048; }
@@ -50,7 +55,7 @@ struct WalkArgs {
 // grid 2 b H tiles; tmRow: B or C, box [64 n x a stage's positions]; tmCol: x or g, the same; tmS*: states, box [64 n x P
 // rows].  PB = P / 64; HALF: dstate 64.  cs_* and dt_out are 16-byte aligned.
 template <class T, int MODE, int PB, bool HALF>
-__global__ void __launch_bounds__(kWalkThreads, 1)
+__global__ void __launch_bounds__(walk_threads(PB, MODE), 1)
 state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_constant__ CUtensorMap tmCol,
            const __grid_constant__ CUtensorMap tmSf, const __grid_constant__ CUtensorMap tmSb, WalkArgs a, int *status) {
     pdl_begin();
@@ -59,7 +64,8 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
     __shared__ WalkShared sh;
     constexpr int P = 64 * PB, SR = walk_rows(PB), NS = walk_ring(PB, MODE);
     constexpr int kA = 2 * SR * 128, kX = PB * SR * 128, kStage = walk_stage_bytes(PB);   // + the rows' cs, Delta and the chunk's T
-    constexpr int NC = HALF ? P / 4 : P / 2;                    // columns a thread keeps
+    constexpr int kState = walk_state_threads(PB, MODE), CS = kState / 128;   // CS warps share a row quarter's columns
+    constexpr int NC = (HALF ? P / 2 : P) / CS;                 // columns a thread keeps
     const int N = d.N, Q = d.Q, nc = d.nc, spc = Q / SR;        // stages per chunk
     uint8_t *base_sm = smem_align1024(dyn), *smS = base_sm + NS * kStage;   // smS: [2 buffers][2][P rows x 128 B]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -101,7 +107,7 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
             tma_load2(smS + (i & 1) * P * 256 + j * P * 128, dir ? &tmSb : &tmSf, n0 + j * 64, row, &sh.s_full[i & 1]);
     };
     if (warp == 0) tmem_alloc(&sh.tmem_base, 2 * P);
-    if (tid == kWalkScale + kThreads + 32) {
+    if (tid == kWalkScale + kState + 32) {
         for (int i = 0; i < NS; ++i) {
             mbar_init(&sh.full[i], 1);
             mbar_init(&sh.scaled[i], kWalkScale / 32);
@@ -109,9 +115,9 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&sh.acc[i], 1);
-            mbar_init(&sh.acc_free[i], 8);
+            mbar_init(&sh.acc_free[i], kState / 32);
             mbar_init(&sh.s_full[i], 1);
-            mbar_init(&sh.s_free[i], 8);
+            mbar_init(&sh.s_free[i], kState / 32);
         }
         sh.fail = 0;
         fence_mbar_init();
@@ -125,7 +131,7 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
     // At headdim 128 the walk is bound elsewhere, and slower with elect_one (forward, b8 L1024 H16 N256: 69.6, 72.2 us; headdim 64,
     // b8 L2048 H24 N128: 48.7, 45.2).
     auto one_lane = [&] { return PB == 1 ? elect_one() : lane == 0; };
-    if (warp == 12) {
+    if (warp == (kWalkScale + kState) / 32) {
         if (one_lane()) {
             const uint32_t idesc = instr_desc(AbFmt<T>::v, true, true, P);
             bool ok = true;
@@ -149,7 +155,7 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
                 if (m.part == spc - 1) umma_commit(&sh.acc[i & 1]);
             }
         }
-    } else if (warp == 13) {                                    // the ring's loads
+    } else if (warp > (kWalkScale + kState) / 32) {                                    // the ring's loads
         if (one_lane()) {
             Pos p;
             for (int s = 0; s < total; ++s, advance(p)) {
@@ -181,9 +187,9 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
             if (lane == 0) mbar_arrive(&sh.scaled[p.slot]);
         }
     } else {
-        const int ew = warp - 4, quad = ew & 3, odd = lane & 1;
+        const int quad = warp & 3, colq = (warp - 4) >> 2, odd = lane & 1;
         const int n = HALF ? (quad & 1) * 32 + lane : quad * 32 + lane;       // within the 128-column tile
-        const int col0 = HALF ? ((quad >> 1) * 2 + (ew >> 2)) * NC : (ew >> 2) * NC;
+        const int col0 = HALF ? ((quad >> 1) * CS + colq) * NC : colq * NC;
         const long long hp = ((long long)b * d.H + h) * P * N, cstride = (long long)d.H * P * N;
         const long long off0 = (long long)b * nc * cstride + (long long)h * P * N;
         const float *start = dir ? a.start_b : a.start_f;
@@ -228,18 +234,21 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
                 if (lane == 0) mbar_arrive(&sh.s_free[i & 1]);
                 if (lane % (32 / V) == 0) {
                     const long long hc = ((long long)dir * d.b * d.H + (long long)b * d.H + h) * nc + c;
-                    a.dTpart[(hc * tiles + tile) * (8 * V) + ew * V + lane * V / 32] = e * part;
+                    a.dTpart[(hc * tiles + tile) * (4 * CS * V) + ((quad + 4 * (colq / (CS / 2))) * (CS / 2) + colq % (CS / 2)) * V + lane * V / 32] = e * part;
                 }
             }
             ok = ws_wait_warp(&sh.acc[i & 1], (i >> 1) & 1, fail, 78);
             if (!ok) break;
             tc_fence_after();
+            constexpr int LD = CS == 4 ? NC : 16;                // columns read at once: what the registers allow
 #pragma unroll
-            for (int q = 0; q < NC; q += 16) {
-                float v[16];
-                tmem_ld16(tmem_lane_base(tmem) + (i & 1) * P + col0 + q, v);
+            for (int q = 0; q < NC; q += LD) {
+                uint32_t v[LD];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) run[q + j] = fmaf(e, run[q + j], v[j]);
+                for (int k = 0; k < LD; k += 8) tmem_ld8_nowait(tmem_lane_base(tmem) + (i & 1) * P + col0 + q + k, *reinterpret_cast<uint32_t(*)[8]>(&v[k]));
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < LD; ++j) run[q + j] = fmaf(e, run[q + j], __uint_as_float(v[j]));
             }
             tc_fence_before();
             __syncwarp();
