@@ -171,13 +171,13 @@ def _source_hash(*files):
 # kernel's source file(s) at capture time; when the source has changed since, `traffic` prints as null instead of a
 # stale figure.  {kernel: (bytes per launch at batch 2, source files, hash)}
 NCU_TRAFFIC_B2 = {
-    "tc_intra_dcb_tile": (28.53e6, ("tc_intra_grp.cuh",), "41e3ef286fa48f36"),
-    "tc_dx_ws": (42.42e6, ("tc_scan_ws.cuh",), "b0a507b61400027a"),
-    "tc_chunk_scan_ws": (43.23e6, ("tc_scan_ws.cuh",), "b0a507b61400027a"),
-    "tc_state_walk": (14.86e6, ("tc_walk_tma.cuh",), "95d10f31667c0eed"),
-    "tc_dstate_walk": (27.06e6, ("tc_walk_tma.cuh",), "95d10f31667c0eed"),
-    "tc_dbc_accum_grp": (55.89e6, ("tc_dbc_tma.cuh",), "421cb86a24d9bcde"),
-    "tc_prev_terms_grp": (27.05e6, ("tc_dbc_tma.cuh",), "421cb86a24d9bcde"),
+    "tc_intra_dcb_tile": (28.51e6, ("tc_intra_grp.cuh",), "94b1d27c4df4692a"),
+    "tc_dx_ws": (42.24e6, ("tc_scan_ws.cuh",), "73d12e220dc08075"),
+    "tc_chunk_scan_ws": (42.89e6, ("tc_scan_ws.cuh",), "73d12e220dc08075"),
+    "tc_state_walk": (14.85e6, ("tc_walk_tma.cuh",), "99fef3862fb25eaa"),
+    "tc_dstate_walk": (27.05e6, ("tc_walk_tma.cuh",), "99fef3862fb25eaa"),
+    "tc_dbc_accum_grp": (55.94e6, ("tc_dbc_tma.cuh",), "344d370efeb1baa0"),
+    "tc_prev_terms_grp": (27.04e6, ("tc_dbc_tma.cuh",), "344d370efeb1baa0"),
 }
 
 

@@ -31,8 +31,8 @@ struct MutView {
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Parts the heads of a group are summed in by the kernels that walk them (dCB, dB, dC): heads R i / S ... R (i + 1) / S of part
-// i, the parts' sums then added in a fixed order.  Blocks may share the parts or one block take them all - the numbers
-// are the same, and the rule looks at one row of the batch only, so a row's results do not depend on how many rows there
+// i, the parts' sums then added in a fixed order.  dB and dC: blocks may share the parts or one block take them all, dCB: a
+// block of a cluster each - the numbers are the same, and the rule looks at one row of the batch only, so a row's results do not depend on how many rows there
 // are.  One part where a row alone brings 32 tiles (b >= 5 such rows fill the chip; summing in parts costs one block 5 %)
 // or the heads are few.
 __host__ __device__ inline int head_parts(const Dims &d) {

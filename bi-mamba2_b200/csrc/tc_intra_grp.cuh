@@ -31,8 +31,9 @@
 // heads' loads, products, weighting and sums in one chain (256 threads, a triangular ones matrix for the column
 // sums) and this form: b8 L2048 H24 136, 84; b2 L8192 H32 G8 194, 142; b16 L4096 H32 dstate 64 732, 441.
 // Tried: V in a buffer of its own (106: the weighting warps wait for the sums), the MMAs behind `lane == 0` instead of
-// elect_one (1250 cycles for sixteen of them, now 730), strips of 16 columns a load (spills), the warp's number made uniform
-// by a shuffle (90), and, before this form, a 128 x Q tile per CTA with sixteen warps (183).
+// elect_one (1250 cycles for sixteen of them, now 730), strips of 16 columns a load (spills), the next columns of G2 read ahead
+// (88: more registers than there are), 96 and 48 registers (91), the warp's number made uniform by a shuffle (90), and, before
+// this form, a 128 x Q tile per CTA with sixteen warps (183).
 //
 // Shapes: headdim 64, chunk 128 or 256, 16-bit inputs.
 #pragma once

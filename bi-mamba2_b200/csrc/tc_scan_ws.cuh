@@ -9,7 +9,7 @@
 // share the C rows [128 x N] and the 16-bit C.B^T rows [128 x Q]; both stay resident in shared memory while the heads
 // of the group stream through:
 //
-//   warp 0 (one lane)   issues every tcgen05.mma
+//   warp 0 (one lane)   issues every tcgen05.mma (elect_one: lane 0 by name, dx took 115 us instead of 110)
 //   warp 1 (one lane)   issues every TMA load
 //   warps 2-9           epilogue: TMEM -> registers -> out_x / out in 32-byte pieces (row factors, gate);
 //                       warps w and w+4 share 32 rows and take 32 columns each
@@ -33,6 +33,12 @@
 //
 // Every blocking point is an mbarrier wait with an attempt limit; a wait that runs out raises a CTA-wide flag that
 // every other wait polls, the status word is set and all roles leave their loops.
+//
+// What bounds it: a stage that is built while the epilogue of the tile before runs takes twice the time it takes alone (2000
+// and 1000 cycles at dstate 128, chunk 256); the two share the load / store path, and a row per lane is 32 lines an access.
+// Tried on this form (scan / dx, us, b8 L2048 H24: 101 / 110): the diagonal's squares split into blocks of 32 so that half as
+// many elements pay an ex2 (102 / 110), with sixteen builder warps (110 / 115), with the next half's operands and tables
+// fetched ahead by warps of their own (110 - 115 / 118 - 126), the epilogues in fp32x2 arithmetic (103 / 113).
 //
 // Shapes: headdim 64, dstate 64 or 128, chunk 128 or 256, 16-bit inputs.
 #pragma once
