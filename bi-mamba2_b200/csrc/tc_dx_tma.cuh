@@ -236,7 +236,7 @@ dx_tma(Dims d, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
                         gx[i] = gv[i] * xv[i];
                     }
                     if (l < lim)
-                        *reinterpret_cast<uint4 *>(static_cast<T *>(dx.ptr) + b * dx.sb + (long long)(c * Q + l) * dx.sl + h * dx.sh + p0) = pack8<T>(o);
+                        stg8_once(static_cast<T *>(dx.ptr) + b * dx.sb + (long long)(c * Q + l) * dx.sl + h * dx.sh + p0, pack8<T>(o));
                     if (d.has_D) {                              // column sums of g*x over this warp's 32 rows
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {

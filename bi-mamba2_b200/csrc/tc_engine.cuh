@@ -269,6 +269,11 @@ __device__ __forceinline__ void ldg8f(const float *p, float (&v)[8]) {
     const float4 b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
+// Eight elements to global memory, leaving no line in the L1 cache: where a lane stores pieces of a row of its own, a warp's 32
+// lines push out what loads could still use (chunk_scan_tma at b8 L1024 H16 P128 N256: 107.6, 104.4 us; the walk gains nothing).
+__device__ __forceinline__ void stg8_once(void *p, uint4 v) {
+    asm volatile("st.global.L1::no_allocate.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 __device__ __forceinline__ uint4 zero8() { return make_uint4(0u, 0u, 0u, 0u); }
 
 // ---- the pipeline --------------------------------------------------------------------------------------------------

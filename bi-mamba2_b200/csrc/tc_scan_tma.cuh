@@ -276,13 +276,13 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
                     const long long oo = b * out.sb + (long long)(c * Q + l) * out.sl + h * out.sh + p0;
                     if (d.has_z) {
                         const long long ox = b * out_x.sb + (long long)(c * Q + l) * out_x.sl + h * out_x.sh + p0;
-                        *reinterpret_cast<uint4 *>(static_cast<T *>(out_x.ptr) + ox) = pack8<T>(o);
+                        stg8_once(static_cast<T *>(out_x.ptr) + ox, pack8<T>(o));
                         float zz[8];
                         unpack8<T>(zr[j >> 3], zz);
 #pragma unroll
                         for (int i = 0; i < 8; ++i) o[i] *= __fdividef(zz[i], 1.f + __expf(-zz[i]));
                     }
-                    *reinterpret_cast<uint4 *>(static_cast<T *>(out.ptr) + oo) = pack8<T>(o);
+                    stg8_once(static_cast<T *>(out.ptr) + oo, pack8<T>(o));
                 }
             }
         }

@@ -5,7 +5,7 @@
 // (see simt::chunk_state / simt::dstates and simt::state_passing_fwd / _bwd for the reference line numbers).  As two kernels
 // the local states made a round trip through memory in fp32 - 16 bytes for every 4 that are kept - and that was most of the
 // two kernels' time.  us, forward + backward, two kernels and walk: b8 L2048 H24 133, 91; b2 L8192 H32 195, 109; b8 L1024 H16
-// headdim 128, dstate 256 313, 148.
+// headdim 128, dstate 256 313, 157 (the last with the 2 - 5 us a launch of event brackets).
 //
 // Warps 0-3 scale the x / g rows in place; warps 4-11 (4-19) keep the running state (TMEM lane = n, P / 2 or P / 4 columns each) and
 // move it from chunk to chunk; one lane of the last warp fills the ring, one of the warp before it issues the MMAs (one thread doing both, a
