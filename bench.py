@@ -172,10 +172,10 @@ def _source_hash(*files):
 # stale figure.  {kernel: (bytes per launch at batch 2, source files, hash)}
 NCU_TRAFFIC_B2 = {
     "tc_intra_dcb_tile": (28.51e6, ("tc_intra_grp.cuh",), "94b1d27c4df4692a"),
-    "tc_dx_ws": (42.24e6, ("tc_scan_ws.cuh",), "73d12e220dc08075"),
-    "tc_chunk_scan_ws": (42.89e6, ("tc_scan_ws.cuh",), "73d12e220dc08075"),
-    "tc_state_walk": (14.85e6, ("tc_walk_tma.cuh",), "99fef3862fb25eaa"),
-    "tc_dstate_walk": (27.05e6, ("tc_walk_tma.cuh",), "99fef3862fb25eaa"),
+    "tc_dx_ws": (42.15e6, ("tc_scan_ws.cuh",), "2df4cd23913b872f"),
+    "tc_chunk_scan_ws": (42.73e6, ("tc_scan_ws.cuh",), "2df4cd23913b872f"),
+    "tc_state_walk": (14.85e6, ("tc_walk_tma.cuh",), "a7200e6550b4e35a"),
+    "tc_dstate_walk": (27.05e6, ("tc_walk_tma.cuh",), "a7200e6550b4e35a"),
     "tc_dbc_accum_grp": (55.94e6, ("tc_dbc_tma.cuh",), "344d370efeb1baa0"),
     "tc_prev_terms_grp": (27.04e6, ("tc_dbc_tma.cuh",), "344d370efeb1baa0"),
 }
