@@ -171,7 +171,7 @@ def _source_hash(*files):
 # kernel's source file(s) at capture time; when the source has changed since, `traffic` prints as null instead of a
 # stale figure.  {kernel: (bytes per launch at batch 2, source files, hash)}
 NCU_TRAFFIC_B2 = {
-    "tc_intra_dcb_tile": (28.51e6, ("tc_intra_grp.cuh",), "94b1d27c4df4692a"),
+    "tc_intra_dcb_tile": (28.51e6, ("tc_intra_grp.cuh",), "c00b372537a40c24"),
     "tc_dx_ws": (42.15e6, ("tc_scan_ws.cuh",), "2df4cd23913b872f"),
     "tc_chunk_scan_ws": (42.73e6, ("tc_scan_ws.cuh",), "2df4cd23913b872f"),
     "tc_state_walk": (14.85e6, ("tc_walk_tma.cuh",), "a7200e6550b4e35a"),

@@ -35,6 +35,8 @@
 // (88: more registers than there are), 96 and 48 registers (91), the warp's number made uniform by a shuffle (90), and, before
 // this form, a 128 x Q tile per CTA with sixteen warps (183).
 //
+// Every blocking point is a bounded mbarrier wait, ids 91-97 in the status word.
+//
 // Shapes: headdim 64, chunk 128 or 256, 16-bit inputs.
 #pragma once
 #include "tc_scan_tma.cuh"
@@ -115,13 +117,13 @@ __device__ __forceinline__ bool intra_weight(IntraGrpShared &sh, uint32_t tabs, 
     const int quad = warp & 3, chalf = warp >> 2, r = quad * 32 + lane;
     const uint32_t own = cb + r * 128 + ((chalf << 5) ^ ((r & 7) << 4));   // the row's first columns of C.B^T
     const int mixed = diag ? quad : -1, edge = diag ? quad : below ? 4 : 0;   // the strip the diagonal crosses; those left of it
-    if (!ws_wait_warp(&sh.cb_full, 0, fail, 61)) return false;
+    if (!ws_wait_warp(&sh.cb_full, 0, fail, 91)) return false;
     if (diag && chalf == ((r >> 4) & 1))                          // V has no diagonal: the one thread that reads C.B^T[r, r] clears it
         asm volatile("st.shared.u16 [%0], %1;" ::"r"(cb + (r >> 6) * 16384 + r * 128 + ((((r & 63) >> 3) ^ (r & 7)) << 4) + (r & 7) * 2), "h"((short)0) : "memory");
 #pragma unroll 1
     for (int h = 0; h < nh; ++h) {
         const uint32_t t = tabs + (h & 1) * (uint32_t)sizeof(IntraTab);
-        if (!ws_wait_warp(&sh.ready[h & 1], (h >> 1) & 1, fail, 62)) return false;
+        if (!ws_wait_warp(&sh.ready[h & 1], (h >> 1) & 1, fail, 92)) return false;
         tc_fence_after();
         const float fl = lds4(t + offsetof(IntraTab, row_f) + r * 4), bl = lds4(t + offsetof(IntraTab, row_b) + r * 4);
         const uint32_t g2h = g2 + (h & 1) * 128 + chalf * 16;
@@ -333,7 +335,7 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
             tma_load4(to + 16384, &tmX, 0, h0 + h, c * Q + s0, b, bar);
         };
         auto issue_g2 = [&](int h) {                              // G2 of head h, by warp 9
-            if (!ws_wait_warp(&sh.in_full[h & 1], (h >> 1) & 1, fail, 65)) return false;
+            if (!ws_wait_warp(&sh.in_full[h & 1], (h >> 1) & 1, fail, 93)) return false;
             tc_fence_after();
             if (elect_one()) {
                 constexpr uint32_t idesc = instr_desc(AbFmt<T>::v, false, false, 128);
@@ -370,7 +372,7 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
 #pragma unroll 1
         for (int h = 0; h < nh && ok; ++h) {
             if (h + 2 < nh) fetch_tab();
-            ok = ws_wait_warp(&sh.v_full[h & 1], (h >> 1) & 1, fail, 68);       // V complete, G2 and the tables read
+            ok = ws_wait_warp(&sh.v_full[h & 1], (h >> 1) & 1, fail, 94);       // V complete, G2 and the tables read
             if (!ok) break;
             if (role == 0) {                                      // columns 0-7: column sums, 8-15: row sums, by block of 16
                 tc_fence_after();
@@ -407,11 +409,11 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.v_read);
-            ok = ws_wait_warp(&sh.sums_full[h & 1], (h >> 1) & 1, fail, 69);
+            ok = ws_wait_warp(&sh.sums_full[h & 1], (h >> 1) & 1, fail, 95);
             if (!ok) break;
             tc_fence_after();
             if (role == 1 && h + 2 < nh) {                        // V of this head has been read: room for head h + 2
-                ok = ws_wait_warp(&sh.v_read, h & 1, fail, 64);
+                ok = ws_wait_warp(&sh.v_read, h & 1, fail, 96);
                 if (!ok) break;
                 if (elect_one()) {
                     fence_async_smem();                           // the warps' reads precede the next TMA write
@@ -457,7 +459,7 @@ intra_dcb_tile(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_con
             }
             out += step;
             if (role == 1) {                                      // head h + 2's product takes the place of head h's sums
-                ok = ws_wait_warp(&sh.read_done, h & 1, fail, 70);
+                ok = ws_wait_warp(&sh.read_done, h & 1, fail, 97);
                 tc_fence_after();
                 if (ok && h + 2 < nh) ok = issue_g2(h + 2);
             }
