@@ -173,7 +173,7 @@ template <class T, int MODE>
 static int launch_walk(const Dims &d, const Walk &w, const tc::WalkArgs &args, int *status, cudaStream_t s) {
     auto launch = [&](auto kernel) -> int {
         const size_t smem = tc::walk_smem(d.P, MODE);
-        const int threads = tc::walk_threads(d.P / 64, MODE);
+        const int threads = tc::walk_threads(d.P / 64, MODE, d.N == 64);
         BISSD_ALLOW(kernel, smem);
         BISSD_LAUNCH(MODE ? "tc_dstate_walk" : "tc_state_walk", launch_pdl(kernel, dim3(2 * d.b * d.H * tc::walk_tiles(d)), threads, smem, s,
             d, w.mRow, w.mCol, w.mSf, w.mSb, args, status));

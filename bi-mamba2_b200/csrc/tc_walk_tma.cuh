@@ -21,12 +21,14 @@
 namespace bissd {
 namespace tc {
 
-// Threads that keep the running state.  Sixteen warps in the backward walk at headdim 128, where eight are what it waits for
-// (dot products with the entering states; us, b8 L1024 H16 N256: 103, 87); elsewhere eight are as good or better (forward 69.6, 70.9;
-// headdim 64, b8 L2048 H24 N128: forward 45.2, 45.5, backward 53.6, 55.4).
+// Threads that keep the running state.  Sixteen warps in the backward walk at headdim 128 with dstate 128 and 256, where eight are
+// what it waits for (dot products with the entering states); elsewhere eight are as good or better.  us, eight and sixteen warps,
+// backward, headdim 128: dstate 256 b8 L1024 H16 102.9, 85.1, b2 L4096 H24 chunk 256 109, 93.6; dstate 128 b8 L1024 H16 55.8, 45.5,
+// b1 L2048 H8 51.6, 38.8; dstate 64 (half the columns a thread) b8 L1024 H16 35.3, 37.4, b2 L8192 H32 101.5, 103.5.  Forward, b8 L1024
+// H16 dstate 256: 69.6, 70.9.  Headdim 64, b8 L2048 H24 dstate 128: forward 45.2, 45.5, backward 53.6, 55.4.
 constexpr int kWalkScale = 128;
-__host__ __device__ constexpr int walk_state_threads(int pb, int mode) { return pb == 2 && mode == 1 ? 512 : 256; }
-__host__ __device__ constexpr int walk_threads(int pb, int mode) { return kWalkScale + walk_state_threads(pb, mode) + 64; }   // 14 or 22 warps
+__host__ __device__ constexpr int walk_state_threads(int pb, int mode, bool half) { return pb == 2 && mode == 1 && !half ? 512 : 256; }
+__host__ __device__ constexpr int walk_threads(int pb, int mode, bool half) { return kWalkScale + walk_state_threads(pb, mode, half) + 64; }   // 14 or 22 warps
 __host__ __device__ constexpr int walk_rows(int pb) { return pb == 1 ? 128 : 64; }   // positions per stage
 __host__ __device__ constexpr int walk_ring(int pb, int mode) { return pb == 1 ? (mode ? 3 : 4) : (mode ? 4 : 6); }
 __host__ __device__ constexpr int walk_stage_bytes(int pb) { return walk_rows(pb) * (256 + pb * 128) + 2048; }
@@ -55,7 +57,7 @@ struct WalkArgs {
 // grid 2 b H tiles; tmRow: B or C, box [64 n x a stage's positions]; tmCol: x or g, the same; tmS*: states, box [64 n x P
 // rows].  PB = P / 64; HALF: dstate 64.  cs_* and dt_out are 16-byte aligned.
 template <class T, int MODE, int PB, bool HALF>
-__global__ void __launch_bounds__(walk_threads(PB, MODE), 1)
+__global__ void __launch_bounds__(walk_threads(PB, MODE, HALF), 1)
 state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_constant__ CUtensorMap tmCol,
            const __grid_constant__ CUtensorMap tmSf, const __grid_constant__ CUtensorMap tmSb, WalkArgs a, int *status) {
     pdl_begin();
@@ -64,7 +66,7 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
     __shared__ WalkShared sh;
     constexpr int P = 64 * PB, SR = walk_rows(PB), NS = walk_ring(PB, MODE);
     constexpr int kA = 2 * SR * 128, kX = PB * SR * 128, kStage = walk_stage_bytes(PB);   // + the rows' cs, Delta and the chunk's T
-    constexpr int kState = walk_state_threads(PB, MODE), CS = kState / 128;   // CS warps share a row quarter's columns
+    constexpr int kState = walk_state_threads(PB, MODE, HALF), CS = kState / 128;   // CS warps share a row quarter's columns
     constexpr int NC = (HALF ? P / 2 : P) / CS;                 // columns a thread keeps
     const int N = d.N, Q = d.Q, nc = d.nc, spc = Q / SR;        // stages per chunk
     uint8_t *base_sm = smem_align1024(dyn), *smS = base_sm + NS * kStage;   // smS: [2 buffers][2][P rows x 128 B]
