@@ -30,22 +30,28 @@ static int norm_check(const bissd_norm_args *a, norm::NormDims *d, bool backward
 }
 // hidden / 8 threads a row, rows side by side up to about 256 threads
 static dim3 norm_block(int hidden) { return dim3(hidden / norm::kCh, std::max(1, 256 * norm::kCh / hidden)); }
-// Persistent blocks: about 1024 threads an SM forward and 512 backward (what their registers allow), fewer when the rows
-// run out first (forward, 65536 rows of 2048 with strided z: 768 threads 201 us, 1024 191; one or four rows a thread and step 202).  The backward's count is also its number of partial weight-gradient rows.
-static int norm_blocks(long long rows, int hidden, int rows_per_thread, int threads_per_sm) {
-    const dim3 b = norm_block(hidden);
-    const long long want = (rows + b.y * rows_per_thread - 1) / (b.y * rows_per_thread);
-    return (int)std::min<long long>(want, (long long)sm_count() * std::max<int>(1, threads_per_sm / (b.x * b.y)));
+// Persistent blocks, fewer when the rows run out first; the backward's count is also its number of partial weight-gradient rows.
+static int norm_blocks(long long rows, int hidden, int rows_per_thread, int blocks_per_sm) {
+    const long long step = (long long)norm_block(hidden).y * rows_per_thread;
+    return (int)std::min<long long>((rows + step - 1) / step, (long long)sm_count() * std::max(1, blocks_per_sm));
 }
-static int norm_bwd_blocks(long long rows, int hidden) { return norm_blocks(rows, hidden, norm::kBwdRows, 512); }
+static int norm_bwd_blocks(long long rows, int hidden) {         // 512 threads an SM: what its registers allow
+    const dim3 b = norm_block(hidden);
+    return norm_blocks(rows, hidden, norm::kBwdRows, 512 / (b.x * b.y));
+}
 
 template <class T, class W>
 static int norm_forward_impl(const bissd_norm_args *a, const norm::NormDims &d, cudaStream_t s) {
     const dim3 block = norm_block(d.hidden);
-    const int grid = norm_blocks(d.rows, d.hidden, norm::kFwdRows, 1024);
     const size_t smem = 2 * block.y * norm::kFwdRows * 16 * sizeof(float);
     const auto kernel = !a->z ? norm::rmsnorm_gated_fwd<T, W, 0>
                               : (a->norm_before_gate ? norm::rmsnorm_gated_fwd<T, W, 1> : norm::rmsnorm_gated_fwd<T, W, 2>);
+    // As many blocks as are resident, up to 1024 threads an SM: one block more than fit walks its rows when the others are done.
+    // us, 768 threads an SM whatever fits, 1024 whatever fits, this: 16384 rows fp32 without z hidden 1536 34.2, 47.4, 34.0, 2048
+    // 44.4, 57.8, 44.6; fp32 with z 1536 53.4, 61.5, 52.8, 2048 76.3, 62.1, 62.2; 65536 rows bf16 with z 2048 174.8, 166.6, 166.7, 4096
+    // 424, 345, 345.  (Up to 1536 threads: as 1024.)
+    const int threads = block.x * block.y;
+    const int grid = norm_blocks(d.rows, d.hidden, norm::kFwdRows, std::min(resident_blocks(kernel, threads, smem), 1024 / threads));
     BISSD_LAUNCH("rmsnorm_gated_fwd", launch_pdl(kernel, grid, block, smem, s, d, a->x, a->z, a->weight, a->out, a->rstd));
     return BISSD_OK;
 }

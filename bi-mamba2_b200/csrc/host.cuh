@@ -6,6 +6,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -148,6 +149,16 @@ template <class K> inline int check_registers(K kernel, int regs) {
         n = at.numRegs;
     }
     return n >= regs ? BISSD_OK : note_cuda(cudaErrorLaunchOutOfResources, "registers of a kernel that deals them anew");
+}
+
+// Blocks of `kernel` an SM holds at once.  Asked once per form of a launch.
+template <class K> inline int resident_blocks(K kernel, int threads, size_t smem) {
+    static std::mutex mu;
+    static std::map<std::tuple<const void *, int, size_t>, int> known;
+    std::lock_guard<std::mutex> lk(mu);
+    int &n = known[{reinterpret_cast<const void *>(kernel), threads, smem}];
+    if (n == 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess) n = 0;
+    return std::max(n, 1);
 }
 
 #define BISSD_ALLOW(kernel, bytes)                  \
