@@ -106,16 +106,15 @@ state_gemm_tma(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_c
     ok = __syncthreads_and(ok);
     tc_fence_after();
     if (!ok && tid == 0) atomicExch(status, kErrMmaTimeout);
-    if (ok) {
-        const int n = n0 + (warp & 3) * 32 + lane;
-        const long long per_dir = (long long)d.b * d.nc * d.H * P * N;
+    const int n = n0 + (warp & 3) * 32 + lane;
+    if (ok && n < N) {                                          // whole warps (a condition inside, around the stores: 120 registers
+        const long long per_dir = (long long)d.b * d.nc * d.H * P * N;   // instead of 64, two CTAs an SM by registers)
         float *o = out + dir * per_dir + ((long long)(b * d.nc + c) * d.H + h) * P * N + n;
         for (int c0 = (warp >> 2) * 32; c0 < P; c0 += 64) {
             float v[32];
             tmem_ld32(tmem_lane_base(tmem) + c0, v);
-            if (n < N)
 #pragma unroll
-                for (int j = 0; j < 32; ++j) o[(long long)(c0 + j) * N] = v[j];
+            for (int j = 0; j < 32; ++j) o[(long long)(c0 + j) * N] = v[j];
         }
     }
     tc_fence_before();
