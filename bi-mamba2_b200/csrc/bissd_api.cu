@@ -135,13 +135,16 @@ struct Walk {
     CUtensorMap mRow, mCol, mSf, mSb;
 };
 // The walk takes a fixed time per chunk whatever else runs, one CTA an SM; the two kernels it replaces take the time of their
-// memory traffic.  Measured (us, forward and backward averaged): a chunk of the walk 1.0 / 1.4 at chunk 128 / 256 and headdim
-// 64, 2.1 / 2.9 at headdim 128; the two kernels 8 + 2.5 per million state elements, both directions.  So the walk wins unless
-// a long sequence of few heads leaves most SMs without one (b1 L8192 H8 chunk 256: 46 us against 16).
+// memory traffic - states in fp32 twice, x or g and their products - and a launch.  So the walk wins unless a long sequence of
+// few heads leaves most SMs without one.  Coefficients (us): fitted to 1000 drawn sizes, b 1 - 16, L 200 - 20000, H 2 - 64, both
+// headdims, every dstate and chunk, whole passes replayed from a graph with either form.  On 400 other sizes the form taken is
+// more than 5 % and 1.5 us behind the other at 9 forward (17 % at most) and 4 in training (7 %); by the coefficients of the
+// first walk at 42 (43 %) and 39 (31 %).  us a forward call, two kernels and walk: b1 L16747 H24 dstate 64 chunk 128 213, 153; b2
+// L15326 H16 223, 170; and the other way b1 L8192 H8 dstate 128 chunk 256 46, 69, b1 L17397 H2 headdim 128 dstate 256 85, 230.
 static bool walk_pays(const Dims &d) {
     const double ctas = 2.0 * d.b * d.H * tc::walk_tiles(d), waves = std::ceil(ctas / sm_count());
-    const double walk = 4.0 + waves * d.nc * (d.P / 64) * (0.6 + 0.8 * d.Q / 256);
-    const double apart = 8.0 + 2.5e-6 * 2.0 * d.b * d.nc * d.H * d.P * d.N;
+    const double walk = waves * d.nc * (0.06 + 0.41 * d.Q / 128 + (d.P == 128 ? 0.75 : 0.0));
+    const double rows = (double)d.b * d.H * d.P, apart = 1.8 + 2.25e-6 * rows * d.nc * d.N + 2e-6 * rows * d.L;
     return walk < apart;
 }
 static bool walk_wanted(const Dims &d) { return !no_tma() && !no_ws() && tc::walk_ok(d.P, d.N, d.Q) && walk_pays(d); }
