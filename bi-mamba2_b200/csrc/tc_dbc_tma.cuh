@@ -16,9 +16,9 @@ namespace tc {
 
 constexpr int kDbcTmaThreads = kThreads + 64;
 struct DbcShared {
-    uint64_t full[3], scaled[3], free_bar[3], wbar, done_bar;
+    uint64_t full[3], scaled[3], free_bar[3], wbar, done_bar, drain_bar;
     uint32_t tmem_base;
-    int fail;
+    int fail, loads;                                            // loads: stages requested
 };
 
 inline size_t dbc_tma_smem(int P, int nt) {
@@ -126,12 +126,13 @@ dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
         }
     } else if (warp == 9) {
         if (lane == 0) {
-            int slot = 0, phase = 0;
-            for (int it = 3; it < total; ++it) {
+            int slot = 0, phase = 0, it = min(3, total);
+            for (; it < total; ++it) {
                 if (!ws_wait(&sh.free_bar[slot], phase, fail, 81)) break;
                 load_stage(it);
                 if (++slot == 3) { slot = 0; phase ^= 1; }
             }
+            sh.loads = it;
         }
     } else {
         bool ok = true;
@@ -175,7 +176,12 @@ dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
     }
     tc_fence_before();
     __syncthreads();
-    if (sh.fail && tid == 0) atomicExch(status, kErrWsWait + sh.fail);
+    if (sh.fail) {                                              // leave nothing in flight
+        if (tid == 0) atomicExch(status, kErrWsWait + sh.fail);
+        if (tid == 256) drain_mmas(&sh.drain_bar);
+        if (tid == 0) drain_loads(sh.full, 3, sh.loads);
+        __syncthreads();
+    }
     if (warp == 0) {
         __syncwarp();
         tmem_dealloc(tmem, ncols);
@@ -199,9 +205,9 @@ dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
 // partial results (268 MB at b2 L8192 G8 N128) and a launch; taken where the heads are one part (head_parts), so that
 // the order of additions does not depend on the batch.
 struct DbcGrpShared {
-    uint64_t full[2], scaled[2], done[2], wbar, last_in, last_done;
+    uint64_t full[2], scaled[2], done[2], wbar, last_in, last_done, drain_bar;
     uint32_t tmem_base;
-    int fail;
+    int fail, loads, last_loads;                                // heads requested; are the operands of the product with dCB?
 };
 inline bool dbc_grp_ok(int P, int N, int Q) { return P == 64 && (N == 64 || N % 128 == 0) && (Q == 128 || Q == 256); }
 inline size_t dbc_grp_smem(int Q, int nt) {
@@ -262,7 +268,7 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
         }
         mbar_init(&sh.last_in, 1);
         mbar_init(&sh.last_done, 1);
-        sh.fail = 0;
+        sh.fail = sh.last_loads = 0;
         fence_mbar_init();
         load_head(0);
         if (R > 1) load_head(1);
@@ -327,6 +333,7 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
             if (LAST) {                                         // every buffer is free once the last head's MMAs are done
                 ok = ok && ws_wait(&sh.done[(R - 1) & 1], ((R - 1) >> 1) & 1, fail, 55);
                 if (ok) {
+                    sh.last_loads = 1;
                     const int row0 = ((b * d.nc + c) * d.G + grp) * Q, nsl = Q / 64;
                     uint8_t *smD = base_sm, *smY = base_sm + Q * Q * 2;
                     mbar_expect_tx(&sh.last_in, (uint32_t)(Q * Q * 2 + Q * nt * 2));
@@ -354,8 +361,11 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
             }
         }
     } else if (warp == 9) {                                     // the ring's loads: stage i & 1 is free once the MMAs of head i - 2 are done
-        if (elect_one())
-            for (int i = 2; i < R && ws_wait(&sh.done[i & 1], ((i >> 1) - 1) & 1, fail, 51); ++i) load_head(i);
+        if (elect_one()) {
+            int i = min(2, R);
+            for (; i < R && ws_wait(&sh.done[i & 1], ((i >> 1) - 1) & 1, fail, 51); ++i) load_head(i);
+            sh.loads = i;
+        }
     } else {
         // the sum of local parts 2 pair and 2 pair + 1 (`two`) as this block's next partial result
         auto write_out = [&](int pair, bool two) {
@@ -437,7 +447,15 @@ dbc_accum_grp(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
     }
     tc_fence_before();
     __syncthreads();
-    if (sh.fail && tid == 0) atomicExch(status, kErrWsWait + sh.fail);
+    if (sh.fail) {                                              // leave nothing in flight
+        if (tid == 0) atomicExch(status, kErrWsWait + sh.fail);
+        if (warp == 8 && elect_one()) drain_mmas(&sh.drain_bar);
+        if (tid == 0) {
+            drain_loads(sh.full, 2, sh.loads);
+            drain_loads(&sh.last_in, 1, sh.last_loads);
+        }
+        __syncthreads();
+    }
     if (warp == 0) {
         __syncwarp();
         tmem_dealloc(tmem, ncols);
@@ -518,6 +536,7 @@ prev_terms_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
         rowred[0][r] = sf_;
         rowred[1][r] = sb_;
     }
+    if (!ok && warp == 0 && elect_one()) feed.leave();
     tc_fence_before();
     __syncthreads();
     if (ok && half == 0 && l < Q) {
@@ -535,9 +554,9 @@ prev_terms_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
 // tensor memory and dot them with their g row while lane 0 of warp 8 issues the loads and MMAs of the next head.
 // Bounded waits, ids 61-66 in the status word.   grid (b*nc*G*ks).
 struct PrevGrpShared {
-    uint64_t bar_c, full_s[2], full_g[2], done[2], accfree[2], gfree[2];
+    uint64_t bar_c, full_s[2], full_g[2], done[2], accfree[2], gfree[2], drain_bar;
     uint32_t tmem_base;
-    int fail;
+    int fail, loads_s, loads_g;                                 // heads whose states, whose g have been requested
 };
 inline bool prev_grp_ok(int P, int N, int Q, int R) { return P == 64 && (N == 64 || N == 128) && (Q == 128 || Q == 256) && R >= 2; }
 inline size_t prev_grp_smem(int N, int Q) {
@@ -628,13 +647,17 @@ prev_terms_grp(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
             }
         }
     } else if (warp == 9) {                                     // the rings of head i - 2 are refilled as they drain
-        if (elect_one())
-            for (int i = 2; i < nh; ++i) {
-                if (!ws_wait(&sh.done[i & 1], ((i >> 1) - 1) & 1, fail, 64)) break;
-                load_s(i);
-                if (!ws_wait(&sh.gfree[i & 1], ((i >> 1) - 1) & 1, fail, 65)) break;
-                load_g(i);
+        if (elect_one()) {
+            int s = min(2, nh), g = s;
+            while (g < nh) {
+                if (!ws_wait(&sh.done[s & 1], ((s >> 1) - 1) & 1, fail, 64)) break;
+                load_s(s++);
+                if (!ws_wait(&sh.gfree[g & 1], ((g >> 1) - 1) & 1, fail, 65)) break;
+                load_g(g++);
             }
+            sh.loads_s = s;
+            sh.loads_g = g;
+        }
     } else {
         const int quad = warp & 3, dir = warp >> 2;             // rows quad * 32 + lane of every row block, one direction
         const float *cs = dir ? cs_b : cs_f;
@@ -702,7 +725,16 @@ prev_terms_grp(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
     }
     tc_fence_before();
     __syncthreads();
-    if (sh.fail && tid == 0) atomicExch(status, kErrWsWait + sh.fail);
+    if (sh.fail) {                                              // leave nothing in flight
+        if (tid == 0) atomicExch(status, kErrWsWait + sh.fail);
+        if (warp == 8 && elect_one()) drain_mmas(&sh.drain_bar);
+        if (tid == 0) {
+            drain_loads(&sh.bar_c, 1, 1);
+            drain_loads(sh.full_s, 2, sh.loads_s);
+            drain_loads(sh.full_g, 2, sh.loads_g);
+        }
+        __syncthreads();
+    }
     if (warp == 0) {
         __syncwarp();
         tmem_dealloc(tmem, ncols);

@@ -15,8 +15,9 @@ namespace bissd {
 namespace tc {
 
 struct DcbShared {
-    uint64_t full[3], mma_done[2];
+    uint64_t full[3], mma_done[2], drain_bar;
     uint32_t tmem_base;
+    int loads;                                                  // heads requested
 };
 
 inline size_t dcb_tma_smem(int P, int Q) { return 1024 + 3 * 2 * (size_t)(P / 64) * 16384 + 2 * 6 * (size_t)Q * 4; }
@@ -72,7 +73,7 @@ dcb_tma(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_constant__
             t[5 * Q + tid] = ex2_approx(pcbr * 1.4426950408889634f - (cb_ - lg));
         }
     };
-    auto load_head = [&](int hr) {                              // thread 0: both tiles of head hr into ring slot hr % 3
+    auto load_head = [&](int hr) {                              // one thread: both tiles of head hr into ring slot hr % 3
         const int h = g * R + hr, slot = hr % 3;
         uint8_t *sg = base_sm + slot * stage_bytes, *sx = sg + npb * 16384;
         mbar_expect_tx(&sh.full[slot], (uint32_t)stage_bytes);
@@ -80,8 +81,9 @@ dcb_tma(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_constant__
             tma_load4(sg + j * 16384, &tmG, j * 64, h, c * Q + l0, b, &sh.full[slot]);
             tma_load4(sx + j * 16384, &tmX, j * 64, h, c * Q + s0, b, &sh.full[slot]);
         }
+        sh.loads = hr + 1;
     };
-    auto issue_head = [&](int hr, uint32_t tmem) -> bool {      // thread 0: G2 of head hr into accumulator hr & 1
+    auto issue_head = [&](int hr, uint32_t tmem) -> bool {      // the same thread: G2 of head hr into accumulator hr & 1
         const int slot = hr % 3;
         if (!mbar_wait(&sh.full[slot], (hr / 3) & 1)) return false;
         tc_fence_after();
@@ -148,12 +150,16 @@ dcb_tma(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_constant__
                 }
             }
         }
-        if (tid == 0 && ok && hr + 3 < R) load_head(hr + 3);   // slot hr % 3 is free: the MMA that read it has completed
+        if (warp == 0 && elect_one() && ok && hr + 3 < R) load_head(hr + 3);   // slot hr % 3 is free: the MMA that read it has completed
         tc_fence_before();
         ok = __syncthreads_and(ok);
         if (!ok) break;
     }
     if (!ok && tid == 0) atomicExch(status, kErrMmaTimeout);
+    if (!ok && warp == 0 && elect_one()) {                      // leave nothing in flight
+        drain_mmas(&sh.drain_bar);
+        drain_loads(sh.full, 3, sh.loads);
+    }
     if (ok && l < Q && dCB16) {                                 // the rounded copy bmm_bwd_tma multiplies with; zero outside the sequence
         const int lim = min(Q, d.L - c * Q);
         T *out = static_cast<T *>(dCB16) + ((long long)(b * d.nc + c) * d.G + g) * Q * Q + (long long)l * Q + s0;

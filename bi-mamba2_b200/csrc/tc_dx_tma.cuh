@@ -187,7 +187,10 @@ dx_tma(Dims d, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
             if (s0 + 2 * kStageK < Q) load_raw(s0 + 2 * kStageK);
         }
         ok = __syncthreads_and(ok) && !sh.fail;
-        if (!ok) break;
+        if (!ok) {
+            if (tid == 0) feed.stopped(it);
+            break;
+        }
         if (tid == 0) {
             tc_fence_after();
             if (!feed.stage_product<T>(tmem, it)) sh.fail = 1;
@@ -255,6 +258,7 @@ dx_tma(Dims d, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
         rowred[1][r] = rsf;
         rowred[2][r] = rsb;
     }
+    if (!ok && tid == 0) feed.leave();
     tc_fence_before();
     __syncthreads();
     if (ok) {

@@ -11,6 +11,7 @@
 //   * accumulator: UMMA M = 128, cta_group::1 -> D row m lives in TMEM lane m, column n in TMEM column n.
 #pragma once
 #include "common.cuh"
+#include "drain.h"
 
 namespace bissd {
 namespace tc {
@@ -230,6 +231,19 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
                  : "memory");
 }
 
+// What a kernel that gives up has in flight would still write to memory that the next block gets as soon as this one ends.  So
+// before it frees its tensor memory and returns it waits, with the usual limit, for its MMAs - the thread that issued them does,
+// on a barrier that nothing else has used - and for its loads (`issued` of them, in turn over the ring `bars`).
+__device__ __forceinline__ void drain_mmas(uint64_t *unused) {
+    mbar_init(unused, 1);
+    fence_mbar_init();
+    umma_commit(unused);
+    mbar_wait(unused, 0);
+}
+__device__ __forceinline__ void drain_loads(uint64_t *bars, int depth, int issued) {
+    drain_ring(issued, depth, [&](int bar, int parity) { mbar_wait(&bars[bar], parity); });
+}
+
 // ---- packing ----------------------------------------------------------------------------------------------------------
 template <class T> __device__ __forceinline__ uint32_t pack2(float a, float b);
 template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
@@ -398,6 +412,10 @@ __device__ __forceinline__ bool umma_gemm(Pipe &p, uint32_t d_tmem, int n_tile, 
         ok = __syncthreads_and(ok);
         if (!ok) {
             if (tid == 0) atomicExch(p.status, kErrMmaTimeout);
+            if (tid < 32 && elect_one()) {                      // leave no MMA in flight
+                umma_commit(&p.sh->done_bar);
+                mbar_wait(&p.sh->done_bar, p.done_uses & 1);
+            }
             return false;
         }
         if (tid < 32 && elect_one()) {

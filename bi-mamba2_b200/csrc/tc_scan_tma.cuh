@@ -21,8 +21,9 @@ namespace tc {
 
 struct ScanShared {
     uint64_t full[2], read[2], x_full[2], st_done, free_bar[2], done_bar;   // full / read: a slot has landed / its MMAs are done
+    uint64_t drain_bar;
     uint32_t tmem_base;
-    int fail;
+    int fail, slabs, pieces;                                    // slabs and x pieces requested, once a wait has run out
 };
 __host__ __device__ constexpr int scan_slot_bytes(int P) { return 16384 + 2 * P * 128; }   // [128 x 64] of C, [P x 64] of either state
 inline size_t scan_tma_smem(int P, int Q) { return 1024 + 2 * (size_t)scan_slot_bytes(P) + 4 * (size_t)Q * 4; }
@@ -45,7 +46,16 @@ struct ScanFeed {
         mbar_init(&sh.st_done, 1);
         mbar_init(&sh.done_bar, 1);
         sh.fail = 0;
+        sh.slabs = d.N / 64;
+        sh.pieces = mX ? d.Q / 64 : 0;
         fence_mbar_init();
+    }
+    // A wait ran out (before stage it was built): nothing is left in flight.  The thread that issues the MMAs.
+    __device__ __forceinline__ void stopped(int it) { sh.pieces = min(sh.pieces, max(2, it)); }
+    __device__ __forceinline__ void leave() {
+        drain_mmas(&sh.drain_bar);
+        drain_loads(sh.full, 2, sh.slabs);
+        drain_loads(sh.x_full, 2, sh.pieces);
     }
     __device__ __forceinline__ uint8_t *slot(int k) { return base_sm + (k & 1) * scan_slot_bytes(d.P); }
     __device__ __forceinline__ uint8_t *stages() { return slot(d.N / 64 - 1); }   // two M stages, over the last slab
@@ -68,11 +78,16 @@ struct ScanFeed {
         if (d.N > 64) load_slab(1);
         else { load_x(0); load_x(1); }
     }
+    __device__ __forceinline__ bool gave_up(int k) {            // in products(), before it asked for anything beyond slab max(1, k)
+        sh.slabs = min(d.N / 64, max(2, k + 1));
+        sh.pieces = d.N > 64 ? 0 : min(sh.pieces, 2);
+        return false;
+    }
     template <class T> __device__ __forceinline__ bool products(uint32_t tmem) {
         const int P = d.P, ns = d.N / 64;
         const uint32_t idesc = instr_desc(AbFmt<T>::v, false, false, P);
         for (int k = 0; k < ns; ++k) {
-            if (!mbar_wait(&sh.full[k & 1], (k >> 1) & 1)) return false;
+            if (!mbar_wait(&sh.full[k & 1], (k >> 1) & 1)) return gave_up(k);
             tc_fence_after();
             const uint32_t sa = smem_u32(slot(k));
             for (int dir = 0; dir < 2; ++dir)
@@ -82,7 +97,7 @@ struct ScanFeed {
                          idesc, (k > 0 || kk > 0) ? 1u : 0u);
             umma_commit(k + 1 < ns ? &sh.read[k & 1] : &sh.st_done);
             if (k >= 1) {                                       // slab k - 1 has been read: its slot takes slab k + 1, or x
-                if (!mbar_wait(&sh.read[(k - 1) & 1], ((k - 1) >> 1) & 1)) return false;
+                if (!mbar_wait(&sh.read[(k - 1) & 1], ((k - 1) >> 1) & 1)) return gave_up(k);
                 if (k + 1 < ns) load_slab(k + 1);
                 else { load_x(0); load_x(1); }
             }
@@ -227,7 +242,10 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
             if (s0 + 2 * kStageK < Q) load_raw(s0 + 2 * kStageK);
         }
         ok = __syncthreads_and(ok) && !sh.fail;
-        if (!ok) break;
+        if (!ok) {
+            if (warp == 0 && elect_one()) feed.stopped(it);
+            break;
+        }
         if (warp == 0 && elect_one()) {
             tc_fence_after();
             if (!feed.stage_product<T>(tmem, it)) sh.fail = 1;
@@ -287,6 +305,7 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
             }
         }
     }
+    if (!ok && warp == 0 && elect_one()) feed.leave();
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, ncols);

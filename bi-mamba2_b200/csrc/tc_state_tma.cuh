@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 state_gemm_tma(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_constant__ CUtensorMap tmCol,
                const float *dt_out, const float *cs_f, const float *cs_b, float *out, int *status) {
     extern __shared__ uint8_t dyn[];
-    __shared__ uint64_t bar_a, bar_x, bar_done;
+    __shared__ uint64_t bar_a, bar_x, bar_done, bar_drain;
     __shared__ uint32_t tmem_slot;
     const int P = d.P, N = d.N, Q = d.Q;
     const int npb = P / 64;
@@ -106,6 +106,11 @@ state_gemm_tma(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_c
     ok = __syncthreads_and(ok);
     tc_fence_after();
     if (!ok && tid == 0) atomicExch(status, kErrMmaTimeout);
+    if (!ok && warp == 0 && elect_one()) {                      // leave nothing in flight
+        drain_mmas(&bar_drain);
+        drain_loads(&bar_x, 1, 1);
+        drain_loads(&bar_a, 1, 1);
+    }
     const int n = n0 + (warp & 3) * 32 + lane;
     if (ok && n < N) {                                          // whole warps (a condition inside, around the stores: 120 registers
         const long long per_dir = (long long)d.b * d.nc * d.H * P * N;   // instead of 64, two CTAs an SM by registers)
@@ -131,9 +136,9 @@ state_gemm_tma(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_c
 // factors are fetched one head ahead.
 // grid (b*nc*G*ks, N/128): ks CTAs share the heads of a group (R % ks == 0).
 struct StateGrpShared {
-    uint64_t bar_a, full[2], scaled[2], done[2], accfree[2], wbar;
+    uint64_t bar_a, full[2], scaled[2], done[2], accfree[2], wbar, drain_bar;
     uint32_t tmem_base;
-    int fail;
+    int fail, loads;                                            // loads: heads requested
 };
 inline bool state_grp_ok(int P, int N, int Q, int R) {
     return P == 64 && (N == 64 || (N % 128 == 0 && N <= 256)) && (Q == 128 || Q == 256) && R >= 2;
@@ -230,11 +235,12 @@ state_gemm_grp(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_c
     if (warp == 16) {
         if (elect_one()) {
             bool ok = true;
+            int loads = min(2, nh);
             for (int i = 0; i < nh && ok; ++i) {
                 uint8_t *sx = smX + (i & 1) * stage_bytes;
                 if (i >= 1 && i + 1 < nh) {                     // stage (i + 1) & 1 is free once the MMAs of head i - 1 are done
                     ok = ws_wait(&sh.done[(i - 1) & 1], ((i - 1) >> 1) & 1, fail, 44);
-                    if (ok) load_head(i + 1);
+                    if (ok) load_head(loads++);
                 }
                 ok = ok && ws_wait(&sh.scaled[i & 1], (i >> 1) & 1, fail, 41);
                 if (ok && i >= 2) ok = ws_wait(&sh.accfree[i & 1], ((i >> 1) - 1) & 1, fail, 42);
@@ -247,6 +253,7 @@ state_gemm_grp(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_c
                          smem_desc(smem_u32(sx) + kk * 2048, (uint32_t)Q * 128, 1024), idesc, kk > 0 ? 1u : 0u);
                 umma_commit(&sh.done[i & 1]);
             }
+            sh.loads = loads;
         }
     } else if (warp >= 8) {                                     // epilogue: accumulator i & 1 -> out[dir][p][n]
         const long long per_dir = (long long)d.b * d.nc * d.H * P * N;
@@ -303,7 +310,15 @@ state_gemm_grp(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_c
     }
     tc_fence_before();
     __syncthreads();
-    if (sh.fail && tid == 0) atomicExch(status, kErrWsWait + sh.fail);
+    if (sh.fail) {                                              // leave nothing in flight
+        if (tid == 0) atomicExch(status, kErrWsWait + sh.fail);
+        if (warp == 16 && elect_one()) drain_mmas(&sh.drain_bar);
+        if (tid == 0) {
+            drain_loads(&sh.bar_a, 1, 1);
+            drain_loads(sh.full, 2, sh.loads);
+        }
+        __syncthreads();
+    }
     if (warp == 0) {
         __syncwarp();
         tmem_dealloc(tmem, 256);

@@ -41,9 +41,9 @@ inline size_t walk_smem(int P, int mode) {
 inline int walk_tiles(const Dims &d) { return d.N == 64 ? 1 : d.N / 128; }
 
 struct WalkShared {
-    uint64_t full[6], scaled[6], empty[6], acc[2], acc_free[2], s_full[2], s_free[2];
+    uint64_t full[6], scaled[6], empty[6], acc[2], acc_free[2], s_full[2], s_free[2], drain_bar;
     uint32_t tmem_base;
-    int fail;
+    int fail, loads, s_loads;                                   // stages, and chunks whose entering states, requested
 };
 struct WalkArgs {
     const float *dt_out, *cs_f, *cs_b;
@@ -138,12 +138,13 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
             const uint32_t idesc = instr_desc(AbFmt<T>::v, true, true, P);
             bool ok = true;
             Pos m;
+            int states = min(2, nc);
             for (int s = 0; s < total; ++s, advance(m)) {
                 const int i = m.chunk;
                 if (m.part == 0 && i >= 2) {                    // the accumulator of chunk i - 2 (and its states) have been used
                     ok = ws_wait(&sh.acc_free[i & 1], ((i >> 1) - 1) & 1, fail, 73);
                     if (MODE == 1 && ok) ok = ws_wait(&sh.s_free[i & 1], ((i >> 1) - 1) & 1, fail, 74);
-                    if (MODE == 1 && ok) load_states(i);
+                    if (MODE == 1 && ok) load_states(states++);
                 }
                 ok = ok && ws_wait(&sh.scaled[m.slot], m.phase, fail, 72);
                 if (!ok) break;
@@ -156,14 +157,17 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
                 umma_commit(&sh.empty[m.slot]);
                 if (m.part == spc - 1) umma_commit(&sh.acc[i & 1]);
             }
+            sh.s_loads = states;
         }
-    } else if (warp > (kWalkScale + kState) / 32) {                                    // the ring's loads
+    } else if (warp > (kWalkScale + kState) / 32) {             // the ring's loads
         if (one_lane()) {
             Pos p;
-            for (int s = 0; s < total; ++s, advance(p)) {
+            int s = 0;
+            for (; s < total; ++s, advance(p)) {
                 if (s >= NS && !ws_wait(&sh.empty[p.slot], p.phase ^ 1, fail, 71)) break;
                 load_stage(p);
             }
+            sh.loads = s;
         }
     } else if (warp < 4) {
         // this thread scales 16-byte pieces of rows r0 + 16 k of a stage (in each of the PB blocks)
@@ -262,7 +266,15 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
     }
     tc_fence_before();
     __syncthreads();
-    if (sh.fail && tid == 0) atomicExch(status, kErrWsWait + sh.fail);
+    if (sh.fail) {                                              // leave nothing in flight
+        if (tid == 0) atomicExch(status, kErrWsWait + sh.fail);
+        if (warp == (kWalkScale + kState) / 32 && one_lane()) drain_mmas(&sh.drain_bar);
+        if (tid == 0) {
+            drain_loads(sh.full, NS, sh.loads);
+            if (MODE == 1) drain_loads(sh.s_full, 2, sh.s_loads);
+        }
+        __syncthreads();
+    }
     if (warp == 0) {
         __syncwarp();
         tmem_dealloc(tmem, 2 * P);
