@@ -31,10 +31,11 @@ struct MutView {
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Parts the heads of a group are summed in by the kernels that walk them (dCB, dB, dC): heads R i / S ... R (i + 1) / S of part
-// i, the parts' sums then added in a fixed order.  dB and dC: blocks may share the parts or one block take them all, dCB: a
-// block of a cluster each - the numbers are the same, and the rule looks at one row of the batch only, so a row's results do not depend on how many rows there
-// are.  One part where a row alone brings 32 tiles (b >= 5 such rows fill the chip; summing in parts costs one block 5 %)
-// or the heads are few.
+// i, the parts' sums then added in a fixed order.  dB and dC: blocks may share the parts or one block take them all.  dCB: a
+// block of a cluster for each.  The numbers are the same, and the rule looks at one row of the batch only, so a row's results do
+// not depend on how many rows there are.  One part where a row alone brings 32 tiles (b >= 5 such rows fill the chip; summing
+// in parts costs one block 5 %) or the heads are few.  dCB with many rows, us: the kernel before, where one block then took all
+// parts, and this one in clusters: b8 L1792 H24 143, 99; b16 L1792 276, 177; b64 L256 H24 145, 109; b16 L1500 H16 chunk 128 103, 70.
 __host__ __device__ inline int head_parts(const Dims &d) {
     const int nt = ceil_div(d.Q, 128);
     return d.nc * d.G * nt * nt >= 32 ? 1 : (d.R >= 16 ? 4 : (d.R >= 8 ? 2 : 1));

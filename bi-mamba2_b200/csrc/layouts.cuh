@@ -11,7 +11,8 @@ struct FwdWs {
     size_t loc, cb, cb16, total;
 };
 struct BwdWs {
-    size_t cb, cbt, cbt16, cb16, cbs, gloc, E, E16, g, dTpart, ddt_out, nf, nb, pf, pb, da_f, da_b, u4, dB_part, dC_part, dCB, dDpart, dApart, dbiaspart, total;
+    size_t cb, cbt, cbt16, cb16, cbs, gloc, E, E16, g, dTpart, ddt_out, nf, nb, pf, pb, da_f, da_b, u4, dB_part, dC_part, dCB, dDpart,
+        dApart, dbiaspart, total;
     int nslots, nlt, nsplit, hsplit, dbc_ks;
 };
 

@@ -30,7 +30,8 @@ inline size_t dbc_tma_smem(int P, int nt) {
 // Both operands of every (head, direction) stage arrive by TMA into a three-deep ring, requested by lane 0 of warp 9; warps
 // 0-7 scale the 128 rows of the left tile in place, lane 0 of warp 8 issues the stage's MMAs.  (One thread doing loads, MMAs
 // and its share of the scaling, a CTA barrier per stage, the kernel took 113 us at b8 L1024 H16 P128 G2 N256
-// chunk 128, 87 now.)  The row factors of head h+1 are loaded while head h is being worked on.  Bounded waits, ids 81-85 in the status word.
+// chunk 128, 90 now.)  Lane 0 rather than elect_one: 0.1 - 2 % faster at nine shapes (90.6, 91.5 there; b16 L700 H16 G16 158, 160).
+// The row factors of head h+1 are loaded while head h is being worked on.  Bounded waits, ids 81-85 in the status word.
 template <class T>
 __global__ void __launch_bounds__(kDbcTmaThreads, 1)
 dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_constant__ CUtensorMap tmEb,
@@ -192,9 +193,9 @@ dbc_accum_tma(Dims d, const __grid_constant__ CUtensorMap tmEf, const __grid_con
 // The same sums with one CTA per (batch, chunk, group, 128 state columns) that walks the heads of its group: the CTA
 // owns all Q rows (one 128-column accumulator per 128-row block), so the state tiles E_f / E_b (or S_f / S_b) of a head
 // are fetched once instead of once per row block, and the x / g tile once.  Warps 0-7 turn the left tile as it landed into
-// its two row-scaled copies - the backward one in place, the forward one beside the ring - lane 0 of warp 8 issues the
-// MMAs, lane 0 of warp 9 the loads; two stages of (left tile + 2 right tiles).  The heads accumulate in tensor memory, two parts of them (head_parts) side by side; a pair of
-// parts is read out together.  With few blocks the parts are dealt to ks of them (dbc_ksplit).  Bounded waits, ids 51-58
+// its two row-scaled copies - the backward one in place, the forward one beside the ring - one lane of warp 8 issues the
+// MMAs, one of warp 9 the loads; two stages of (left tile + 2 right tiles).  The heads accumulate in tensor memory, two parts of
+// them (head_parts) side by side; a pair of parts is read out together.  With few blocks the parts are dealt to ks of them (dbc_ksplit).  Bounded waits, ids 51-58
 // in the status word.
 // grid (b*nc*G*ks*nsplit, 1, 2); blockIdx.z: 0 = dB, 1 = dC.  part layout [b, nc*Q, G, slots, N] fp32: a slot per pair of
 // parts, or per part where every block has one.
@@ -551,7 +552,7 @@ prev_terms_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
 // The same row sums with one CTA per (batch, chunk, group[, head range]) that keeps the C tile of all Q rows resident
 // and walks its heads: per head both entering states (one [2P x dstate] K-major tile, so one N = 2P product per
 // 128-row block) and the g tile arrive by TMA into two-deep rings; warps 0-7 read the products out of double-buffered
-// tensor memory and dot them with their g row while lane 0 of warp 8 issues the loads and MMAs of the next head.
+// tensor memory and dot them with their g row while one lane of warp 8 issues the MMAs of the next head and one of warp 9 its loads.
 // Bounded waits, ids 61-66 in the status word.   grid (b*nc*G*ks).
 struct PrevGrpShared {
     uint64_t bar_c, full_s[2], full_g[2], done[2], accfree[2], gfree[2], drain_bar;

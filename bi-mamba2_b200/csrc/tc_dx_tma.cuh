@@ -137,7 +137,9 @@ dx_tma(Dims d, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
     }
     float rs = 0.f, rsf = 0.f, rsb = 0.f;
     const uint32_t tl = tmem_lane_base(tmem);
-    if (tid == 0 && !feed.products<T>(tmem)) sh.fail = 1;       // tid 0: with elect_one the kernel takes 116 us instead of 109 (b8 L1024 H16 P128 N256)
+    // tid 0, not elect_one, which is 1 - 7 % slower at nine shapes (us: b8 L1024 H16 dstate 256 105.5, 112, dstate 64 92.8, 98.8,
+    // b4 L2048 H16 dstate 128 chunk 256 112, 119, b2 L8192 H32 dstate 64 310, 328): the kernel is at its 128 registers
+    if (tid == 0 && !feed.products<T>(tmem)) sh.fail = 1;
     uint4 xr[4], gr[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) xr[q] = l < lim ? ld8v<T>(x, b, c * Q + l, h, half * 32 + q * 8) : zero8();

@@ -152,7 +152,7 @@ inline int state_grp_ksplit(int groups_total, int R, int sms) {      // CTAs per
 }
 constexpr int kStateGrpThreads = 2 * kThreads + 32;             // eight scaling warps, eight epilogue warps, one controller warp
 
-// Warps 0-7 scale the tiles of head i while warps 8-15 store the accumulator of head i - 1 and lane 0 of warp 16
+// Warps 0-7 scale the tiles of head i while warps 8-15 store the accumulator of head i - 1 and one lane of warp 16
 // issues every TMA load and every MMA, so that the three never wait behind one another.  Every blocking point is a
 // bounded mbarrier wait (ids 41-47 in the status word).
 template <class T, int MODE>

@@ -7,9 +7,9 @@
 // two kernels' time.  us, forward + backward, two kernels and walk: b8 L2048 H24 133, 91; b2 L8192 H32 195, 109; b8 L1024 H16
 // headdim 128, dstate 256 313, 157 (the last with the 2 - 5 us a launch of event brackets).
 //
-// Warps 0-3 scale the x / g rows in place; warps 4-11 (4-19) keep the running state (TMEM lane = n, P / 2 or P / 4 columns each) and
-// move it from chunk to chunk; one lane of the last warp fills the ring, one of the warp before it issues the MMAs (one thread doing both, a
-// stage took 0.75 us whatever was loaded, scaled or multiplied).  Stages are 128 positions (64 at P = 128): [128 x 128 n] of
+// Warps 0-3 scale the x / g rows in place; warps 4-11 (4-19) keep the running state (TMEM lane = n, P / 2 or P / 4 columns each)
+// and move it from chunk to chunk; one lane of the last warp fills the ring, one of the warp before it issues the MMAs (one
+// thread doing both, a stage took 0.75 us whatever was loaded, scaled or multiplied).  Stages are 128 positions (64 at P = 128): [128 x 128 n] of
 // B / C and [128 x P] of x / g, both MN-major as they land, with the rows' cumulative sums and Delta beside them (read from
 // global memory by the scaling warps, their latency was the length of a stage).  Accumulators and, in MODE 1, the entering
 // states that come by TMA are double-buffered.  dstate 64: the second 64 rows of the tile repeat the first, and each half of
@@ -130,8 +130,9 @@ state_walk(Dims d, const __grid_constant__ CUtensorMap tmRow, const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
-    // At headdim 128 the walk is bound elsewhere, and slower with elect_one (forward, b8 L1024 H16 N256: 69.6, 72.2 us; headdim 64,
-    // b8 L2048 H24 N128: 48.7, 45.2).
+    // At headdim 128 the walk is bound elsewhere, and no faster with elect_one but for dstate 64 (us, lane 0 and elect_one, forward:
+    // b8 L1024 H16 dstate 256 65.7, 68.0, dstate 128 35.4, 37.2, dstate 64 30.1, 29.2; b2 L8192 H32 dstate 64 88.7, 94.0; backward
+    // within 1.5 % but for b1 L2048 H8 38.7, 37.3).  Headdim 64, b8 L2048 H24 dstate 128: 48.7, 45.2.
     auto one_lane = [&] { return PB == 1 ? elect_one() : lane == 0; };
     if (warp == (kWalkScale + kState) / 32) {
         if (one_lane()) {

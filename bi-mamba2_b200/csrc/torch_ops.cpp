@@ -1,7 +1,7 @@
 // The operator's host path in native code: argument checks, output and scratch allocation, the library calls and the
 // autograd node of bimamba_chunk_scan_combined, for eager calls on CUDA tensors.
 //
-// What bounds a small problem is the host: a forward + backward pass enqueues 17 launches, and building the argument
+// What bounds a small problem is the host: a forward + backward pass enqueues 13 launches (8 in fp32), and building the argument
 // structures, allocating a dozen tensors and crossing into the library from Python took 200 us of the 300 us such a
 // pass cost.  Here the per-pass quantities live in one allocation, scratch comes straight from the caching allocator,
 // and nothing returns to the interpreter between the checks and the last launch.
