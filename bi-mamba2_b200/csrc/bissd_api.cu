@@ -136,16 +136,16 @@ struct Walk {
 };
 // The walk takes a fixed time per chunk whatever else runs, one CTA an SM; the two kernels it replaces take the time of their
 // memory traffic - states in fp32 twice, x or g and their products - and a launch.  So the walk wins unless a long sequence of
-// few heads leaves most SMs without one.  Coefficients (us): fitted to 1000 drawn sizes, b 1 - 16, L 200 - 20000, H 2 - 64, both
-// headdims, every dstate and chunk, whole passes replayed from a graph with either form.  On 400 other sizes the form taken is
-// more than 5 % and 1.5 us behind the other at 9 forward (17 % at most) and 4 in training (7 %); by the coefficients of the
-// first walk at 42 (43 %) and 39 (31 %).  us a forward call, two kernels and walk: b1 L16747 H24 dstate 64 chunk 128 213, 153; b2
-// L15326 H16 223, 170; and the other way b1 L8192 H8 dstate 128 chunk 256 46, 69, b1 L17397 H2 headdim 128 dstate 256 85, 230.
+// few heads leaves most SMs without one.  Coefficients (us) from 4600 drawn sizes in bf16 and fp16, b 1 - 16, L 200 - 20000, H
+// 2 - 64, both headdims, every dstate and chunk, whole passes replayed from a graph with either form: the form taken is more
+// than 10 % behind the other at 17 of them forward and 5 in training (22 % at most); by the coefficients of the first walk
+// at 242 (43 %) and 141 (38 %).  us a forward call, two kernels and walk: b1 L16747 H24 dstate 64 chunk 128 213, 153; b2 L15326 H16 223,
+// 170; and the other way b1 L8192 H8 dstate 128 chunk 256 46, 69, b1 L17397 H2 headdim 128 dstate 256 85, 230.
 static bool walk_pays(const Dims &d) {
-    const double ctas = 2.0 * d.b * d.H * tc::walk_tiles(d), waves = std::ceil(ctas / sm_count());
-    const double walk = waves * d.nc * (0.06 + 0.41 * d.Q / 128 + (d.P == 128 ? 0.75 : 0.0));
-    const double rows = (double)d.b * d.H * d.P, apart = 1.8 + 2.25e-6 * rows * d.nc * d.N + 2e-6 * rows * d.L;
-    return walk < apart;
+    const double ctas = 2.0 * d.b * d.H * tc::walk_tiles(d), waves = std::ceil(ctas / sm_count()), q = d.Q / 128;
+    const double chunk = d.P == 64 ? 0.08 + 0.41 * q : 1.0 + 0.32 * q;
+    const double rows = 1e-6 * d.b * d.H * d.P, apart = (d.P == 64 ? 1.75 : 1.45) + 2.7 * rows * d.nc * d.N + (d.P == 64 ? 1.75 : 1.5) * rows * d.L;
+    return waves * d.nc * chunk < apart;
 }
 static bool walk_wanted(const Dims &d) { return !no_tma() && !no_ws() && tc::walk_ok(d.P, d.N, d.Q) && walk_pays(d); }
 
