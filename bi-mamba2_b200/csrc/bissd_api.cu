@@ -141,13 +141,17 @@ struct Walk {
 // than 10 % behind the other at 17 of them forward and 5 in training (22 % at most); by the coefficients of the first walk
 // at 242 (43 %) and 141 (38 %).  us a forward call, two kernels and walk: b1 L16747 H24 dstate 64 chunk 128 213, 153; b2 L15326 H16 223,
 // 170; and the other way b1 L8192 H8 dstate 128 chunk 256 46, 69, b1 L17397 H2 headdim 128 dstate 256 85, 230.
-static bool walk_pays(const Dims &d) {
-    const double ctas = 2.0 * d.b * d.H * tc::walk_tiles(d), waves = std::ceil(ctas / sm_count()), q = d.Q / 128;
-    const double chunk = d.P == 64 ? 0.08 + 0.41 * q : 1.0 + 0.32 * q;
-    const double rows = 1e-6 * d.b * d.H * d.P, apart = (d.P == 64 ? 1.75 : 1.45) + 2.7 * rows * d.nc * d.N + (d.P == 64 ? 1.75 : 1.5) * rows * d.L;
-    return waves * d.nc * chunk < apart;
+// A forward pass in two phases (`twice`) would walk twice, where the two kernels repeat the recurrence only: coefficients of its own,
+// from 2000 sizes.  More than 10 % behind at 23 of them (22 % at most); with those of one pass at 258, by the first walk's at 147.
+static bool walk_pays(const Dims &d, bool twice) {
+    struct Cost { double chunk, per128, start, states, rows; };  // a wave's chunk; a chunk's 128 positions; then the two kernels'
+    static constexpr Cost cost[2][2] = {{{0.08, 0.41, 1.75, 2.7, 1.75}, {1.0, 0.32, 1.45, 2.7, 1.5}},      // headdim 64, 128
+                                        {{0.08, 0.41, 0.15, 1.8, 0.35}, {1.0, 0.32, 0.05, 1.7, 0.7}}};
+    const Cost &c = cost[twice][d.P / 64 - 1];
+    const double waves = std::ceil(2.0 * d.b * d.H * tc::walk_tiles(d) / sm_count()), rows = 1e-6 * d.b * d.H * d.P;
+    return waves * d.nc * (c.chunk + c.per128 * (d.Q / 128)) < c.start + c.states * rows * d.nc * d.N + c.rows * rows * d.L;
 }
-static bool walk_wanted(const Dims &d) { return !no_tma() && !no_ws() && tc::walk_ok(d.P, d.N, d.Q) && walk_pays(d); }
+static bool walk_wanted(const Dims &d, bool twice = false) { return !no_tma() && !no_ws() && tc::walk_ok(d.P, d.N, d.Q) && walk_pays(d, twice); }
 
 // What the sizes alone say of the tensor-core family's kernels, and so which arrays of the workspace a pass does without.
 // Operands that no tensor map describes are found out later: such a pass takes other kernels, and needs them all.
@@ -161,10 +165,10 @@ static bool last_wanted(const Dims &d) {                         // dbc_accum_gr
 static FwdWs least_fwd(const Dims &d) { return fwd_layout(d, FwdNeed{!walk_wanted(d), !ws_wanted(d), ws_wanted(d)}); }
 static BwdWs least_bwd(const Dims &d) { return bwd_layout(d, true, BwdNeed{!walk_wanted(d), !last_wanted(d), !fused_wanted(d)}); }
 
-static Walk plan_walk(const Dims &d, int dtype, const bissd_tensor &row, const View &col, const float *dt_out,
+static Walk plan_walk(const Dims &d, bool wanted, int dtype, const bissd_tensor &row, const View &col, const float *dt_out,
                       const float *cs_f, const float *cs_b, const void *states_f, const void *states_b) {
     Walk w;
-    if (!walk_wanted(d) || !all_aligned16(dt_out, cs_f, cs_b)) return w;
+    if (!wanted || !all_aligned16(dt_out, cs_f, cs_b)) return w;
     const unsigned rows = tc::walk_rows(d.P / 64);
     const unsigned long long srows = (unsigned long long)d.b * d.nc * d.H * d.P;
     w.use = map_bshd(&w.mRow, dtype, row.ptr, row.stride_batch, row.stride_seq, row.stride_head, d.N, d.G, d.L, d.b, rows) &&
@@ -196,9 +200,11 @@ static int forward_impl(const bissd_fwd_args &a, const Dims &d, char *ws, size_t
     const View x = view_of(a.x), Bm = view_of(a.B), Cm = view_of(a.C), z = view_of(a.z);
     const int bch = d.b * d.nc * d.H;
     const int ntP = tc::round_up(d.P, 16), ntQ = tc::round_up(d.Q, 16);
-    // (a FINISH phase with entering states walks again, from the inputs: the decision is the same in both phases)
-    const Walk walk = plan_walk(d, a.p.x_dtype, a.B, x, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
-    if (lean && walk_wanted(d) && !walk.use) return BISSD_ERR_WORKSPACE;
+    // A FINISH phase with entering states walks again, from the inputs: the decision is the same in both phases.  With the least
+    // scratch, which has no room for local states, LOCAL is all that is wanted.
+    const bool walks = walk_wanted(d, !lean && a.phases != BISSD_PHASE_ALL);
+    const Walk walk = plan_walk(d, walks, a.p.x_dtype, a.B, x, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
+    if (lean && walks && !walk.use) return BISSD_ERR_WORKSPACE;
     const tc::CumsumFwd cs{a.dt.ptr, a.p.dt_dtype, a.dt.stride_batch, a.dt.stride_seq, a.dt.stride_head, a.A, a.dt_bias, a.dt_out, a.cs_f, a.cs_b,
                            all_aligned16(a.dt_out, a.cs_f, a.cs_b)};
     // C.B^T by TMA: a bf16 copy for the persistent scan, fp32 for the others; in one launch with the cumulative sums where
@@ -393,7 +399,7 @@ static int backward_impl(const bissd_bwd_args &a, const GradViews &gr, const Dim
         gv = View{ws + w.g, (long long)d.L * d.H * d.P, (long long)d.H * d.P, (long long)d.P};
     }
     Walk walk;                                                   // whole passes only: a split one keeps its local gradients
-    if (a.phases == BISSD_PHASE_ALL) walk = plan_walk(d, a.p.x_dtype, a.C, gv, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
+    if (a.phases == BISSD_PHASE_ALL) walk = plan_walk(d, walk_wanted(d), a.p.x_dtype, a.C, gv, a.dt_out, a.cs_f, a.cs_b, a.states_f, a.states_b);
     if (lean && walk_wanted(d) && !walk.use) return BISSD_ERR_WORKSPACE;
     if (a.phases & BISSD_PHASE_LOCAL) {
         if (!d.has_z && !walk.use) {                             // else the gate kernel or the walk, whichever is first, clears the status word

@@ -21,3 +21,30 @@ def test_walk_or_two_kernels(b, L, H, P, N, Q, walks):
     assert lib.bissd_workspace_bytes(ctypes.byref(p), ctypes.byref(full), None) == 0
     local_states = 2 * b * -(-L // Q) * H * P * N * 4
     assert (full.value - least.value >= local_states) == walks
+
+
+@pytest.mark.gpu
+def test_a_pass_in_two_phases_does_not_walk_twice():
+    """Where one walk pays and two do not, the phases take the two kernels, which repeat the recurrence only: the same bits."""
+    import torch
+    from ssd.bi import sequence_parallel as sp
+    from ssd.bi.ssd_combined import bimamba_chunk_scan_combined
+    b, L, H, P, N, Q = 1, 2048, 16, 64, 128, 256
+    g = torch.Generator(device="cuda").manual_seed(1)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    ins = [mk(b, L, H, P).bfloat16(), mk(b, L, H) - 4.0, -torch.rand(H, generator=g, device="cuda") - 0.1, mk(b, L, 1, N).bfloat16(), mk(b, L, 1, N).bfloat16()]
+    start = [mk(b, H, P, N), mk(b, H, P, N)]
+    outs, ran = [], []
+    for phases in (False, True):
+        _cabi.trace_enable(True)
+        try:
+            if phases:
+                outs.append(sp.finish_forward(sp.local_forward(*ins, Q, dt_softplus=True), *start))
+            else:
+                outs.append(bimamba_chunk_scan_combined(*ins, Q, dt_softplus=True, initial_states_f=start[0], initial_states_b=start[1]))
+            torch.cuda.synchronize()
+            ran.append(_cabi.trace_read())
+        finally:
+            _cabi.trace_enable(False)
+    assert "tc_state_walk" in ran[0] and "tc_state_walk" not in ran[1], ran
+    assert torch.equal(*outs)
