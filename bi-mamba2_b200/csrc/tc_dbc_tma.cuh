@@ -507,7 +507,7 @@ prev_terms_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
-    if (warp == 0 && elect_one() && !feed.products<T>(tmem)) sh.fail = 1;
+    if (warp == 0 && elect_one()) feed.products<T>(tmem);
     bool ok = mbar_wait(&sh.st_done, 0);
     ok = __syncthreads_and(ok) && !sh.fail;
     tc_fence_after();
@@ -537,7 +537,6 @@ prev_terms_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
         rowred[0][r] = sf_;
         rowred[1][r] = sb_;
     }
-    if (!ok && warp == 0 && elect_one()) feed.leave();
     tc_fence_before();
     __syncthreads();
     if (ok && half == 0 && l < Q) {
@@ -545,7 +544,11 @@ prev_terms_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
         pf[base + l] = ef * (sf_ + (P > 32 ? rowred[0][r] : 0.f));
         pb[base + l] = eb * (sb_ + (P > 32 ? rowred[1][r] : 0.f));
     }
-    if (warp == 0) tmem_dealloc(tmem, ncols);
+    if (warp == 0) {
+        if (!ok && elect_one()) feed.leave();
+        __syncwarp();
+        tmem_dealloc(tmem, ncols);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------------------

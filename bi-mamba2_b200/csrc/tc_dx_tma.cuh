@@ -139,7 +139,7 @@ dx_tma(Dims d, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
     const uint32_t tl = tmem_lane_base(tmem);
     // tid 0, not elect_one, which is 1 - 7 % slower at nine shapes (us: b8 L1024 H16 dstate 256 105.5, 112, dstate 64 92.8, 98.8,
     // b4 L2048 H16 dstate 128 chunk 256 112, 119, b2 L8192 H32 dstate 64 310, 328): the kernel is at its 128 registers
-    if (tid == 0 && !feed.products<T>(tmem)) sh.fail = 1;
+    if (tid == 0) feed.products<T>(tmem);
     uint4 xr[4], gr[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) xr[q] = l < lim ? ld8v<T>(x, b, c * Q + l, h, half * 32 + q * 8) : zero8();
@@ -195,7 +195,7 @@ dx_tma(Dims d, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
         }
         if (tid == 0) {
             tc_fence_after();
-            if (!feed.stage_product<T>(tmem, it)) sh.fail = 1;
+            feed.stage_product<T>(tmem, it);
         }
     }
     // epilogue operands of the first strip are requested before waiting for the last MMAs
@@ -260,7 +260,6 @@ dx_tma(Dims d, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
         rowred[1][r] = rsf;
         rowred[2][r] = rsb;
     }
-    if (!ok && tid == 0) feed.leave();
     tc_fence_before();
     __syncthreads();
     if (ok) {
@@ -274,7 +273,11 @@ dx_tma(Dims d, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
             dDpart[(((long long)(b * d.nc + c) * d.H + h) * gridDim.y + blockIdx.y) * P + tid] =
                 colred[0][tid] + colred[1][tid] + colred[2][tid] + colred[3][tid];
     }
-    if (warp == 0) tmem_dealloc(tmem, ncols);
+    if (warp == 0) {
+        if (!ok && tid == 0) feed.leave();
+        __syncwarp();
+        tmem_dealloc(tmem, ncols);
+    }
 }
 
 }  // namespace tc

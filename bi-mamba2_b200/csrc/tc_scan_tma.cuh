@@ -23,7 +23,7 @@ struct ScanShared {
     uint64_t full[2], read[2], x_full[2], st_done, free_bar[2], done_bar;   // full / read: a slot has landed / its MMAs are done
     uint64_t drain_bar;
     uint32_t tmem_base;
-    int fail, slabs, pieces;                                    // slabs and x pieces requested, once a wait has run out
+    int fail;                                                   // where a wait ran out, as tile_asked reads it
 };
 __host__ __device__ constexpr int scan_slot_bytes(int P) { return 16384 + 2 * P * 128; }   // [128 x 64] of C, [P x 64] of either state
 inline size_t scan_tma_smem(int P, int Q) { return 1024 + 2 * (size_t)scan_slot_bytes(P) + 4 * (size_t)Q * 4; }
@@ -46,16 +46,19 @@ struct ScanFeed {
         mbar_init(&sh.st_done, 1);
         mbar_init(&sh.done_bar, 1);
         sh.fail = 0;
-        sh.slabs = d.N / 64;
-        sh.pieces = mX ? d.Q / 64 : 0;
         fence_mbar_init();
     }
-    // A wait ran out (before stage it was built): nothing is left in flight.  The thread that issues the MMAs.
-    __device__ __forceinline__ void stopped(int it) { sh.pieces = min(sh.pieces, max(2, it)); }
+    // Nothing is left in flight by a kernel that gives up: `stopped` notes the stage before which it did, unless a wait of this
+    // thread was first, `leave` waits.  Both by the thread that issues the MMAs.  What has been asked for follows from `fail`: kept
+    // in shared memory from the first load on, a training pass took 649 us, this way 647 (b8 L1024 H16 P128 N256).
+    __device__ __forceinline__ void stopped(int it) {
+        if (!sh.fail) sh.fail = kStages + it;
+    }
     __device__ __forceinline__ void leave() {
+        const Asked asked = tile_asked(sh.fail, d.N / 64, mX ? d.Q / 64 : 0);
         drain_mmas(&sh.drain_bar);
-        drain_loads(sh.full, 2, sh.slabs);
-        drain_loads(sh.x_full, 2, sh.pieces);
+        drain_loads(sh.full, 2, asked.slabs);
+        drain_loads(sh.x_full, 2, asked.pieces);
     }
     __device__ __forceinline__ uint8_t *slot(int k) { return base_sm + (k & 1) * scan_slot_bytes(d.P); }
     __device__ __forceinline__ uint8_t *stages() { return slot(d.N / 64 - 1); }   // two M stages, over the last slab
@@ -78,16 +81,11 @@ struct ScanFeed {
         if (d.N > 64) load_slab(1);
         else { load_x(0); load_x(1); }
     }
-    __device__ __forceinline__ bool gave_up(int k) {            // in products(), before it asked for anything beyond slab max(1, k)
-        sh.slabs = min(d.N / 64, max(2, k + 1));
-        sh.pieces = d.N > 64 ? 0 : min(sh.pieces, 2);
-        return false;
-    }
-    template <class T> __device__ __forceinline__ bool products(uint32_t tmem) {
+    template <class T> __device__ __forceinline__ void products(uint32_t tmem) {
         const int P = d.P, ns = d.N / 64;
         const uint32_t idesc = instr_desc(AbFmt<T>::v, false, false, P);
         for (int k = 0; k < ns; ++k) {
-            if (!mbar_wait(&sh.full[k & 1], (k >> 1) & 1)) return gave_up(k);
+            if (!mbar_wait(&sh.full[k & 1], (k >> 1) & 1)) { sh.fail = 1 + k; return; }
             tc_fence_after();
             const uint32_t sa = smem_u32(slot(k));
             for (int dir = 0; dir < 2; ++dir)
@@ -97,17 +95,16 @@ struct ScanFeed {
                          idesc, (k > 0 || kk > 0) ? 1u : 0u);
             umma_commit(k + 1 < ns ? &sh.read[k & 1] : &sh.st_done);
             if (k >= 1) {                                       // slab k - 1 has been read: its slot takes slab k + 1, or x
-                if (!mbar_wait(&sh.read[(k - 1) & 1], ((k - 1) >> 1) & 1)) return gave_up(k);
+                if (!mbar_wait(&sh.read[(k - 1) & 1], ((k - 1) >> 1) & 1)) { sh.fail = 1 + k; return; }
                 if (k + 1 < ns) load_slab(k + 1);
                 else { load_x(0); load_x(1); }
             }
         }
-        return true;
     }
     // M stage `it` is in place: its product with the x rows of the same columns, on top of the accumulator
-    template <class T> __device__ __forceinline__ bool stage_product(uint32_t tmem, int it) {
+    template <class T> __device__ __forceinline__ void stage_product(uint32_t tmem, int it) {
         if (it >= 2) load_x(it);                                // the stage's buffers, x included, were free before it was built
-        if (!mbar_wait(&sh.x_full[it & 1], (it >> 1) & 1)) return false;
+        if (!mbar_wait(&sh.x_full[it & 1], (it >> 1) & 1)) { sh.fail = kStages + it + 1; return; }
         tc_fence_after();
         const uint32_t idesc = instr_desc(AbFmt<T>::v, false, true, d.P);
         const uint32_t sa = smem_u32(stages() + (it & 1) * kAStageBytes), sx = smem_u32(x_piece(it));
@@ -115,7 +112,6 @@ struct ScanFeed {
         for (int kk = 0; kk < 4; ++kk)
             umma(tmem, smem_desc(sa + kk * 32, 16, 1024), smem_desc(sx + kk * 16 * 128, 8192, 1024), idesc, 1u);
         umma_commit(&sh.free_bar[it & 1]);
-        return true;
     }
 };
 
@@ -206,7 +202,7 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
     const int l = l0 + (warp & 3) * 32 + lane;                  // this thread's row, in the sums and in the epilogue
     const float ef = l < lim ? __expf(cs_f[base + l]) : 0.f, eb = l < lim ? __expf(cs_b[base + l]) : 0.f;
     const uint32_t tl = tmem_lane_base(tmem);
-    if (warp == 0 && elect_one() && !feed.products<T>(tmem)) sh.fail = 1;
+    if (warp == 0 && elect_one()) feed.products<T>(tmem);
     bool ok = mbar_wait(&sh.st_done, 0);
     if (ok) {                                                   // the weighted sum of both products replaces the first
         tc_fence_after();
@@ -248,7 +244,7 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
         }
         if (warp == 0 && elect_one()) {
             tc_fence_after();
-            if (!feed.stage_product<T>(tmem, it)) sh.fail = 1;
+            feed.stage_product<T>(tmem, it);
         }
     }
     // epilogue operands of the first strip are requested before waiting for the last MMAs
@@ -305,10 +301,13 @@ chunk_scan_tma(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_con
             }
         }
     }
-    if (!ok && warp == 0 && elect_one()) feed.leave();
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, ncols);
+    if (warp == 0) {
+        if (!ok && elect_one()) feed.leave();
+        __syncwarp();
+        tmem_dealloc(tmem, ncols);
+    }
 }
 
 }  // namespace tc
