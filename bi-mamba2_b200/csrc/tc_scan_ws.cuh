@@ -69,7 +69,7 @@ struct WsShared {
     uint64_t acc_full[2], acc_free[2];
     uint64_t r_full, r_free;     // the epilogue's row tile (z or x) has landed / every epilogue warp has taken its rows
     uint32_t tmem_base;
-    int fail;
+    int fail, groups, states, pieces;                            // fills of C and C.B^T, of the states, pieces of x: requested
 };
 
 inline size_t scan_ws_smem(int P, int N, int Q) {
@@ -568,10 +568,6 @@ ws_kernel(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant
                 it.next(d, nrt);
                 if (i + 1 < nt && it.grp != cur_grp) umma_commit(&sh.grp_done);   // C and C.B^T may be replaced
             }
-            if (!ok) {
-                umma_commit(&sh.fin_bar);                       // leave no MMA in flight
-                mbar_wait(&sh.fin_bar, 0);
-            }
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------------------------------------- TMA loads
@@ -580,7 +576,7 @@ ws_kernel(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant
             it.init(d, nrt, t0);
             bool ok = true;
             int cur_grp = -1;
-            int ngrp = 0, loads_st = 0, loads_x[4] = {0, 0, 0, 0};
+            int ngrp = 0, states = 0, pieces = 0;
             for (int j = 0; j < nt && ok; ++j) {
                 if (it.grp != cur_grp) {
                     if (ngrp > 0) ok = ws_wait(&sh.grp_done, (ngrp - 1) & 1, fail, 11);
@@ -604,24 +600,21 @@ ws_kernel(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant
                     tma_load2(smS + (2 * k) * P * 128, &tmSf, k * 64, tile * P, &sh.st_full);
                     tma_load2(smS + (2 * k + 1) * P * 128, &tmSb, k * 64, tile * P, &sh.st_full);
                 }
-                ++loads_st;
+                ++states;
 #pragma unroll
                 for (int s = 0; s < NS; ++s) {
                     if (j > 0) ok = ok && ws_wait(&sh.x_free[s], (j - 1) & 1, fail, 13);
                     if (ok) {
                         mbar_expect_tx(&sh.x_full[s], 8192u);
                         tma_load4(smX + s * 8192, &tmX, 0, it.h, it.c * Q + s * 64, it.b, &sh.x_full[s]);
-                        ++loads_x[s];
+                        ++pieces;
                     }
                 }
                 it.next(d, nrt);
             }
-            if (!ok) {                                          // leave no load in flight
-                if (loads_st) mbar_wait(&sh.st_full, (loads_st - 1) & 1);
-                for (int s = 0; s < NS; ++s)
-                    if (loads_x[s]) mbar_wait(&sh.x_full[s], (loads_x[s] - 1) & 1);
-                if (ngrp) mbar_wait(&sh.grp_full, (ngrp - 1) & 1);
-            }
+            sh.groups = ngrp;
+            sh.states = states;
+            sh.pieces = pieces;
         }
     } else if (warp < kWsFirstBuilder) {
         // ---------------------------------------------------------------------------------------------- epilogue
@@ -809,7 +802,18 @@ ws_kernel(Dims d, const __grid_constant__ CUtensorMap tmC, const __grid_constant
     }
     tc_fence_before();
     __syncthreads();
-    if (sh.fail && tid == 0) atomicExch(status, kErrWsWait + sh.fail);
+    if (sh.fail) {                                               // leave nothing in flight, whichever role it was that gave up
+        if (threadIdx.x == 0) atomicExch(status, kErrWsWait + sh.fail);
+        if (warp == 0 && elect_one()) {
+            umma_commit(&sh.fin_bar);
+            mbar_wait(&sh.fin_bar, 0);
+        }
+        if (warp == 1 && elect_one()) {
+            drain_loads(&sh.grp_full, 1, sh.groups);
+            drain_loads(&sh.st_full, 1, sh.states);
+            drain_loads(sh.x_full, NS, sh.pieces);
+        }
+    }
     if (warp == 0) {
         __syncwarp();
         tmem_dealloc(tmem, ncols);

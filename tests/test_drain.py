@@ -2,6 +2,8 @@
 import os
 import subprocess
 
+import pytest
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 
@@ -10,3 +12,14 @@ def test_drain_waits_for_what_is_in_flight(tmp_path):
     subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", os.path.join(HERE, "drain_check.cpp"), "-o", exe], check=True,
                    capture_output=True, text=True)
     assert subprocess.run([exe], capture_output=True, text=True, timeout=60).stdout == "ok\n"
+
+
+# tc_intra_grp.cuh has waits of its own for the two buffers that its loads take in turn
+@pytest.mark.parametrize("source", ["tc_dbc_tma", "tc_state_tma", "tc_walk_tma", "tc_scan_tma", "tc_dx_tma", "tc_scan_ws"])
+def test_every_kernel_with_loads_waits_for_them(source):
+    """A kernel's text, from one __global__ to the next (functions it shares stand before the first): a load is asked for, so one is waited
+    for on the way out.  What cannot be made to happen on a GPU without breaking the kernel."""
+    with open(os.path.join(HERE, "..", "bi-mamba2_b200", "csrc", source + ".cuh")) as f:
+        parts = f.read().split("__global__")
+    for part in parts:
+        assert ("tma_load" in part or "feed.start()" in part) <= ("drain_loads(" in part or "feed.leave()" in part), part[:200]
