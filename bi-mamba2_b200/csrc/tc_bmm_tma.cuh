@@ -32,7 +32,7 @@ __device__ __forceinline__ void bmm_cb_role(const Dims &d, const CUtensorMap &tm
     const bool plain = a.plain, transposed = a.transposed;
     float *CBs = a.CBs, *CB32 = a.CB32, *CBt32 = a.CBt32;
     extern __shared__ uint8_t dyn[];
-    __shared__ uint64_t bar_in, bar_done;
+    __shared__ uint64_t bar_in, bar_done, bar_drain;
     __shared__ uint32_t tmem_slot;
     const int Q = d.Q, nsl = d.N / 64;
     uint8_t *smC = smem_align1024(dyn), *smB = smC + nsl * 16384;
@@ -143,7 +143,14 @@ __device__ __forceinline__ void bmm_cb_role(const Dims &d, const CUtensorMap &tm
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, ncols);
+    if (warp == 0) {
+        if (!ok && elect_one()) {                               // leave nothing in flight
+            drain_mmas(&bar_drain);
+            drain_loads(&bar_in, 1, 1);
+        }
+        __syncwarp();
+        tmem_dealloc(tmem, ncols);
+    }
 }
 
 template <class T, bool FP32>

@@ -206,7 +206,7 @@ bmm_bwd_tma(Dims d, const __grid_constant__ CUtensorMap tmDm, const __grid_const
             const float *dC_part, int part_heads, MutView dB, MutView dC, int *status) {
     pdl_begin();
     extern __shared__ uint8_t dyn[];
-    __shared__ uint64_t bar_in, bar_done;
+    __shared__ uint64_t bar_in, bar_done, bar_drain;
     __shared__ uint32_t tmem_slot;
     const int N = d.N, Q = d.Q;
     uint8_t *smA = smem_align1024(dyn), *smB = smA + Q * 256;
@@ -293,7 +293,14 @@ bmm_bwd_tma(Dims d, const __grid_constant__ CUtensorMap tmDm, const __grid_const
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, 64);
+    if (warp == 0) {
+        if (!ok && elect_one()) {                               // leave nothing in flight
+            drain_mmas(&bar_drain);
+            drain_loads(&bar_in, 1, 1);
+        }
+        __syncwarp();
+        tmem_dealloc(tmem, 64);
+    }
 }
 
 }  // namespace tc

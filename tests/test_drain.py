@@ -15,7 +15,8 @@ def test_drain_waits_for_what_is_in_flight(tmp_path):
 
 
 # tc_intra_grp.cuh has waits of its own for the two buffers that its loads take in turn
-@pytest.mark.parametrize("source", ["tc_dbc_tma", "tc_state_tma", "tc_walk_tma", "tc_scan_tma", "tc_dx_tma", "tc_scan_ws"])
+@pytest.mark.parametrize("source", ["tc_dbc_tma", "tc_state_tma", "tc_walk_tma", "tc_scan_tma", "tc_dx_tma", "tc_scan_ws", "tc_bmm_tma",
+                                    "tc_dcb_tma"])
 def test_every_kernel_with_loads_waits_for_them(source):
     """A kernel's text, from one __global__ to the next (functions it shares stand before the first): a load is asked for, so one is waited
     for on the way out.  What cannot be made to happen on a GPU without breaking the kernel."""
