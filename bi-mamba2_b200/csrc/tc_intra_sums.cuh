@@ -83,6 +83,9 @@ intra_sums(Dims d, const __grid_constant__ CUtensorMap tmG, const __grid_constan
                     for (int kk = 0; kk < 4; ++kk)
                         umma(p.tmem, smem_desc(smem_u32(p.a_stage[j]) + kk * 32, 16, 1024),
                              smem_desc(smem_u32(p.b_stage[j]) + kk * 32, 16, 1024), idesc, (j > 0 || kk > 0) ? 1u : 0u);
+            } else {                                            // leave no load in flight
+                atomicExch(status, kErrMmaTimeout);
+                drain_loads(&sh.free_bar[0], 1, 1);
             }
         }
         ok = __syncthreads_and(ok);

@@ -16,7 +16,7 @@ def test_drain_waits_for_what_is_in_flight(tmp_path):
 
 # tc_intra_grp.cuh has waits of its own for the two buffers that its loads take in turn
 @pytest.mark.parametrize("source", ["tc_dbc_tma", "tc_state_tma", "tc_walk_tma", "tc_scan_tma", "tc_dx_tma", "tc_scan_ws", "tc_bmm_tma",
-                                    "tc_dcb_tma"])
+                                    "tc_dcb_tma", "tc_intra", "tc_intra_sums"])
 def test_every_kernel_with_loads_waits_for_them(source):
     """A kernel's text, from one __global__ to the next (functions it shares stand before the first): a load is asked for, so one is waited
     for on the way out.  What cannot be made to happen on a GPU without breaking the kernel."""
@@ -24,3 +24,11 @@ def test_every_kernel_with_loads_waits_for_them(source):
         parts = f.read().split("__global__")
     for part in parts:
         assert ("tma_load" in part or "feed.start()" in part) <= ("drain_loads(" in part or "feed.leave()" in part), part[:200]
+
+
+@pytest.mark.parametrize("source", ["tc_intra", "tc_intra_sums"])
+def test_a_load_that_does_not_arrive_is_reported(source):
+    """The intra-chunk kernels leave reporting to umma_drain, which a tile that never arrived does not reach."""
+    with open(os.path.join(HERE, "..", "bi-mamba2_b200", "csrc", source + ".cuh")) as f:
+        after = f.read().split("ok = mbar_wait(&sh.free_bar[0], 0);")[1]
+    assert "atomicExch(status, kErrMmaTimeout);" in after.split("__syncthreads_and")[0]
