@@ -18,12 +18,12 @@ def test_drain_waits_for_what_is_in_flight(tmp_path):
 @pytest.mark.parametrize("source", ["tc_dbc_tma", "tc_state_tma", "tc_walk_tma", "tc_scan_tma", "tc_dx_tma", "tc_scan_ws", "tc_bmm_tma",
                                     "tc_dcb_tma", "tc_intra", "tc_intra_sums"])
 def test_every_kernel_with_loads_waits_for_them(source):
-    """A kernel's text, from one __global__ to the next (functions it shares stand before the first): a load is asked for, so one is waited
-    for on the way out.  What cannot be made to happen on a GPU without breaking the kernel."""
+    """A kernel's text, from one __global__ to the next, and the functions before the first: a load is asked for, so one is waited for on
+    the way out.  It cannot be made to happen on a GPU without breaking the kernel."""
     with open(os.path.join(HERE, "..", "bi-mamba2_b200", "csrc", source + ".cuh")) as f:
-        parts = f.read().split("__global__")
-    for part in parts:
-        assert ("tma_load" in part or "feed.start()" in part) <= ("drain_loads(" in part or "feed.leave()" in part), part[:200]
+        before, *kernels = f.read().split("__global__")
+    for part in (before + k for k in kernels):
+        assert ("tma_load" in part or "feed.start()" in part) <= ("drain_loads(" in part or "feed.leave()" in part), part[len(before):][:200]
 
 
 @pytest.mark.parametrize("source", ["tc_intra", "tc_intra_sums"])
