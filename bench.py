@@ -172,14 +172,14 @@ def _source_hash(*files):
 # entry carries the hash of the kernel's source and of the waits, loads and MMAs it uses; when the code has changed since,
 # `traffic` prints as null instead of a stale figure.  {kernel: (bytes read, bytes written, its source, hash)}
 NCU_TRAFFIC = {
-    "tc_state_walk": (59.29e6, 13.23e6, "tc_walk_tma.cuh", "f303d92cf487a9fa"),
-    "tc_chunk_scan_ws": (197.53e6, 67.82e6, "tc_scan_ws.cuh", "346e9cdcb61f9fa3"),
-    "gate_bwd": (151.01e6, 59.49e6, "tc_dx_tma.cuh", "3f684ec7c336c486"),
-    "tc_dstate_walk": (108.18e6, 24.57e6, "tc_walk_tma.cuh", "f303d92cf487a9fa"),
-    "tc_dx_ws": (193.46e6, 33.37e6, "tc_scan_ws.cuh", "346e9cdcb61f9fa3"),
-    "tc_prev_terms_grp": (108.04e6, 0.32e6, "tc_dbc_tma.cuh", "0a9045a5206cb582"),
-    "tc_intra_dcb_tile": (113.89e6, 5.17e6, "tc_intra_grp.cuh", "c89cf173f62de2da"),
-    "tc_dbc_accum_grp": (222.87e6, 0.67e6, "tc_dbc_tma.cuh", "0a9045a5206cb582"),
+    "tc_state_walk": (59.29e6, 14.06e6, "tc_walk_tma.cuh", "f303d92cf487a9fa"),
+    "tc_chunk_scan_ws": (197.38e6, 67.65e6, "tc_scan_ws.cuh", "2fe47ae2492ed608"),
+    "gate_bwd": (151.01e6, 60.00e6, "tc_dx_tma.cuh", "3f684ec7c336c486"),
+    "tc_dstate_walk": (108.16e6, 24.01e6, "tc_walk_tma.cuh", "f303d92cf487a9fa"),
+    "tc_dx_ws": (193.30e6, 33.59e6, "tc_scan_ws.cuh", "2fe47ae2492ed608"),
+    "tc_prev_terms_grp": (108.04e6, 0.31e6, "tc_dbc_tma.cuh", "0a9045a5206cb582"),
+    "tc_intra_dcb_tile": (113.91e6, 4.94e6, "tc_intra_grp.cuh", "c89cf173f62de2da"),
+    "tc_dbc_accum_grp": (222.88e6, 0.34e6, "tc_dbc_tma.cuh", "0a9045a5206cb582"),
 }
 
 
